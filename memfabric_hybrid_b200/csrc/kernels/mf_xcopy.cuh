@@ -11,6 +11,8 @@
 #include <cuda_fp8.h>
 #include <stdint.h>
 
+#include "mf_shift.cuh"
+
 namespace mfk {
 
 struct CopyItem {
@@ -67,14 +69,7 @@ __device__ __forceinline__ void cta_copy(const uint8_t *__restrict__ src, uint8_
     const int tid = threadIdx.x;
     const int nt = blockDim.x;
     if (((reinterpret_cast<uint64_t>(src) ^ reinterpret_cast<uint64_t>(dst)) & 15) != 0) {
-        // Mutually misaligned: 4-byte words when possible, else bytes. Rare (KV segments are aligned).
-        if ((((reinterpret_cast<uint64_t>(src) | reinterpret_cast<uint64_t>(dst)) | len) & 3) == 0) {
-            const uint32_t *s = reinterpret_cast<const uint32_t *>(src);
-            uint32_t *d = reinterpret_cast<uint32_t *>(dst);
-            for (uint64_t i = tid; i < len / 4; i += nt) d[i] = s[i];
-        } else {
-            for (uint64_t i = tid; i < len; i += nt) dst[i] = src[i];
-        }
+        cta_copy_shifted<true>(src, dst, len);
         return;
     }
     uint64_t head = (16 - (reinterpret_cast<uint64_t>(src) & 15)) & 15;

@@ -202,3 +202,54 @@ def test_prepared_batch_launches_and_replays_in_a_cuda_graph():
     """mf_bm_batch_create / _launch: validated once, one launch per submission, capturable."""
     url = f"tcp://127.0.0.1:{free_port()}"
     assert run_ranks(_prepared_rank, 1, (url,), timeout=180) == [(True, True, True, True)]
+
+
+def _shifted_rank(rank, world, url):
+    import torch
+    import memfabric_hybrid as mf
+    from memfabric_hybrid import bm
+    torch.cuda.set_device(0)
+    assert mf.initialize() == 0
+    cfg = bm.BmConfig()
+    cfg.rank_id = 0
+    cfg.start_store = True
+    assert bm.initialize(url, 1, 0, cfg) == 0, mf.get_last_err_msg()
+    pool = 64 * MiB
+    h = bm.create2(id=4, local_dram_size=0, max_dram_size=0, local_hbm_size=pool, max_hbm_size=pool)
+    assert h.join() == 0, mf.get_last_err_msg()
+    base = h.peer_rank_ptr(0, bm.BmMemType.DEVICE)
+    # every pair of offsets inside a 16-byte granule; lengths around the granule, the warp's run (2 KiB), the CTA's step
+    # (32 KiB) and the work chunk
+    lens = [1, 15, 16, 17, 31, 32, 33, 47, 48, 63, 512, 2047, 2048, 2064, 2081, 4095, 32767, 32768 + 17, 70001]
+    segs, so, do = [], 0, 0
+    for s in range(16):
+        for d in range(16):
+            n = lens[(s * 16 + d) % len(lens)]
+            for ln in (n, lens[(s + d) % len(lens)]):
+                segs.append((so + s, do + d, ln))
+                so += (s + ln + 63) // 16 * 16
+                do += (d + ln + 63) // 16 * 16
+    g = torch.Generator("cuda").manual_seed(5)
+    src = torch.randint(0, 256, (so + 64,), dtype=torch.uint8, device="cuda", generator=g)
+    fill = torch.randint(0, 256, (do + 64,), dtype=torch.uint8, device="cuda", generator=g)
+    torch.cuda.synchronize()
+    assert h.copy_data(fill.data_ptr(), base, fill.numel(), bm.BmCopyType.L2G, 0) == 0, mf.get_last_err_msg()
+    assert h.copy_data_batch([src.data_ptr() + s for s, _, _ in segs], [base + d for _, d, _ in segs], [n for _, _, n in segs], len(segs),
+                             bm.BmCopyType.L2G, 0) == 0, mf.get_last_err_msg()
+    got = torch.empty_like(fill)
+    assert h.copy_data(base, got.data_ptr(), got.numel(), bm.BmCopyType.G2L, 0) == 0, mf.get_last_err_msg()
+    want = fill.clone()
+    for s, d, n in segs:
+        want[d:d + n] = src[s:s + n]
+    torch.cuda.synchronize()
+    ok = bool(torch.equal(got, want))   # the bytes between the pieces included
+    h.leave()
+    h.destroy()
+    bm.uninitialize(0)
+    mf.uninitialize()
+    return ok
+
+
+def test_pieces_at_every_pair_of_byte_offsets():
+    url = f"tcp://127.0.0.1:{free_port()}"
+    assert run_ranks(_shifted_rank, 1, (url,), timeout=180) == [True]
