@@ -47,8 +47,8 @@ class CopyParamsC(C.Structure):
 
 
 class BatchCopyParamsC(C.Structure):
-    _fields_ = [("sources", C.POINTER(vp)), ("destinations", C.POINTER(vp)), ("dataSizes", C.POINTER(u64)),
-                ("batchSize", u32), ("stream", vp)]
+    # the three lists as plain addresses: casting a numpy array to a typed ctypes pointer costs 2 us each
+    _fields_ = [("sources", vp), ("destinations", vp), ("dataSizes", vp), ("batchSize", u32), ("stream", vp)]
 
 
 class BatchCopyResultC(C.Structure):

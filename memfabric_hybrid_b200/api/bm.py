@@ -95,17 +95,17 @@ def _ptr_array(values: Sequence[int]):
     return (C.c_void_p * len(values))(*[int(v) for v in values])
 
 
-def _u64_view(values, n: int, ctype):
-    """``values`` as a C array of ``n`` 64-bit words plus the object that keeps it alive. A contiguous numpy array of
-    64-bit integers is passed as it is (no copy: the cost of a call on a large descriptor list is then the C call
+def _u64_view(values, n: int):
+    """Address of ``values`` as an array of ``n`` 64-bit words plus the object that keeps it alive. A contiguous numpy array
+    of 64-bit integers is passed as it is (no copy: the cost of a call on a large descriptor list is then the C call
     alone); any other sequence is converted once."""
     import numpy as np
     a = values if isinstance(values, np.ndarray) else np.asarray(values[:n], dtype=np.uint64)
-    if a.dtype not in (np.uint64, np.int64) or not a.flags["C_CONTIGUOUS"]:
+    if a.dtype not in (np.uint64, np.int64) or not a.flags.c_contiguous:
         a = np.ascontiguousarray(a, dtype=np.uint64)
     if a.shape[0] < n:
         raise ValueError(f"batch of {n} items but only {a.shape[0]} values")
-    return a.ctypes.data_as(C.POINTER(ctype)), a
+    return a.ctypes.data, a
 
 
 class _QuantParamsC(C.Structure):   # hybm_quant_copy_params
@@ -173,9 +173,9 @@ class BigMemory:
 
     def _batch(self, src_addrs, dst_addrs, sizes, count, stream):
         n = int(count)
-        srcs, k0 = _u64_view(src_addrs, n, C.c_void_p)
-        dsts, k1 = _u64_view(dst_addrs, n, C.c_void_p)
-        lens, k2 = _u64_view(sizes, n, C.c_uint64)
+        srcs, k0 = _u64_view(src_addrs, n)
+        dsts, k1 = _u64_view(dst_addrs, n)
+        lens, k2 = _u64_view(sizes, n)
         p = N.BatchCopyParamsC(srcs, dsts, lens, n, stream or None)
         return p, (k0, k1, k2)
 
