@@ -1,0 +1,318 @@
+// bf16 GEMM for few rows (decode steps, small batches): C[M,N] = A[M,K] . B[N,K]^T with K split over a thread-block cluster.
+//
+// What bounds it: reading B once from memory. The persistent kernel of mf_gemm.cu gives one SM a whole 128 x 256 tile over all
+// of K, so a layer with N = 7168 keeps 28 SMs busy and the other 120 idle. Measured with B from memory (us, the persistent kernel's
+// better tiling / this kernel): 32 x 7168 x 8192 SwiGLU 51.3 / 28.8, 32 x 8192 x 3584 24.7 / 16.6, 16 x 1024 x 8192 43.1 / 12.4. Here a tile is 128 x 128 and the S CTAs of a cluster
+// each take 1/S of K into their own tensor memory; the partial sums meet through distributed shared memory (every CTA adds up
+// and stores 1/S of the tile, in CTA order: the result does not depend on timing). No workspace, no second launch.
+// Two CTAs share an SM (about 100 KB of stages each), so one CTA's prologue and reduction run under the other's loads.
+// A's box in the tensor map is only as high as the rows there are, rounded up to 8: the MMA still reads 128 rows of shared
+// memory, and what the rows past the box hold ends up in accumulator rows that nobody reads. All of a CTA's A stages lie in
+// front of its B stages, so those reads stay inside its shared memory.
+// EPI 1 fuses SwiGLU: a tile is 64 gate rows and the 64 up rows that belong to them (B holds 128 gate rows, then their 128 up
+// rows, per 256).
+#include <cuda_bf16.h>
+
+#include <algorithm>
+#include <mutex>
+
+#include "mf_gemm.cuh"
+
+namespace mfk {
+
+constexpr int kSkBN = 128;
+constexpr int kSkThreads = 192;              // warp 0 TMA, warp 1 MMA, warps 2..5 read the accumulator, all six reduce
+constexpr int kSkMaxSplit = 8;               // portable cluster size
+constexpr int kSkStageArea = 100 * 1024;     // two CTAs per SM
+constexpr int kSkRowFloats = kSkBN + 4;      // 528-byte rows: eight lanes' 16-byte writes to eight rows hit all banks once
+constexpr int kSkMaxStages = 10;
+static_assert(BM * kSkRowFloats * 4 <= kSkStageArea, "the partial tile reuses the stages");
+
+struct SplitArgs {
+    TmaPair tm;
+    __nv_bfloat16 *C;
+    int64_t ldc;
+    int M, N, K;
+    int box_rows;   // rows of A per stage (multiple of 8, at most 128)
+    int stages;
+    int *status;
+};
+
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr)
+{
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+
+template <int EPI> __global__ void __launch_bounds__(kSkThreads, 2) k_gemm_bf16_splitk(const __grid_constant__ SplitArgs g)
+{
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *base = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    __shared__ __align__(8) uint64_t bar_full[kSkMaxStages], bar_empty[kSkMaxStages], bar_done;
+    __shared__ uint32_t tmem_slot;
+    __shared__ int abort_flag;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint32_t split, rank;
+    asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(split));
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const int m_tiles = (g.M + BM - 1) / BM;
+    const int tile = (int)(blockIdx.x / split);
+    const int mt = tile % m_tiles, nt = tile / m_tiles;   // CTAs running together share B tiles
+    const int k_iters = (g.K * 2 + KSPAN - 1) / KSPAN;
+    const int k0 = (int)((int64_t)k_iters * rank / split), k1 = (int)((int64_t)k_iters * (rank + 1) / split);
+    const int a_bytes = g.box_rows * KSPAN;
+    constexpr int kBBytes = kSkBN * KSPAN;
+    uint8_t *b_base = base + g.stages * a_bytes;
+    AbortCtl ac{&abort_flag, g.status};
+
+    if (threadIdx.x == 0) {
+        abort_flag = 0;
+        for (int s = 0; s < g.stages; s++) {
+            mbar_init(&bar_full[s], 1);
+            mbar_init(&bar_empty[s], 1);
+        }
+        mbar_init(&bar_done, 1);
+        mbar_fence_init();
+        tma_prefetch_desc(&g.tm.a);
+        tma_prefetch_desc(&g.tm.b);
+    }
+    if (warp == 1) {
+        tmem_alloc(&tmem_slot, kSkBN);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+
+    // rows of B of this tile: two runs of 64
+    int b0, b1;
+    if (EPI == 1) {
+        b0 = (nt >> 1) * 256 + (nt & 1) * 64;
+        b1 = b0 + 128;
+    } else {
+        b0 = nt * kSkBN;
+        b1 = b0 + 64;
+    }
+    bool have = false;
+    if (warp == 0) {
+        if (elect_one()) {
+            int s = 0;
+            uint32_t phase = 0;
+            for (int kb = k0; kb < k1; kb++) {
+                if (!mbar_wait(&bar_empty[s], phase ^ 1, ac, 0x311)) break;
+                mbar_expect_tx(&bar_full[s], (uint32_t)(a_bytes + kBBytes));
+                tma_load_2d(b_base + s * kBBytes, &g.tm.b, kb * (KSPAN / 2), b0, &bar_full[s]);
+                tma_load_2d(b_base + s * kBBytes + kBBytes / 2, &g.tm.b, kb * (KSPAN / 2), b1, &bar_full[s]);
+                tma_load_2d(base + s * a_bytes, &g.tm.a, kb * (KSPAN / 2), mt * BM, &bar_full[s]);
+                if (++s == g.stages) s = 0, phase ^= 1;
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        if (elect_one()) {
+            int s = 0;
+            uint32_t phase = 0;
+            bool fine = true;
+            const uint32_t idesc = umma_idesc(1, 1, BM, kSkBN);
+            for (int kb = k0; kb < k1; kb++) {
+                fine = mbar_wait(&bar_full[s], phase, ac, 0x312);
+                if (!fine) break;
+                tc_fence_after();
+                const uint64_t da = umma_desc_sw128(base + s * a_bytes);
+                const uint64_t db = umma_desc_sw128(b_base + s * kBBytes);
+#pragma unroll
+                for (int k = 0; k < KSPAN / 32; k++) umma_bf16(tmem, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb != k0) | (k != 0));
+                umma_commit(&bar_empty[s]);
+                if (++s == g.stages) s = 0, phase ^= 1;
+            }
+            if (fine) umma_commit(&bar_done);
+        }
+        __syncwarp();
+    } else {
+        // the four warps read one lane quadrant each and leave the partial sums as fp32 rows where the stages were: all
+        // loads have landed and all MMAs have read them once bar_done completes
+        const int quad = warp & 3;
+        const int row = quad * 32 + lane;
+        have = __all_sync(0xffffffffu, mbar_wait(&bar_done, 0, ac, 0x313));
+        if (have) {
+            tc_fence_after();
+            if (quad * 32 < g.M - mt * BM) {  // uniform over the warp: the reads below are collective
+                float *mine = reinterpret_cast<float *>(base) + row * kSkRowFloats;
+#pragma unroll
+                for (int c = 0; c < kSkBN / 32; c++) {
+                    uint32_t v[32];
+                    tmem_ld32(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(c * 32), v);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int q = 0; q < 8; q++)
+                        *reinterpret_cast<uint4 *>(mine + c * 32 + q * 4) = make_uint4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);
+                }
+            }
+            tc_fence_before();
+        }
+    }
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem, kSkBN);
+    }
+    cluster_sync_all();  // every CTA's partial tile is in its shared memory (every CTA arrives: the waits above are bounded)
+
+    const int rows = min(BM, g.M - mt * BM);
+    constexpr int kOutCols = EPI == 1 ? kSkBN / 2 : kSkBN;   // output columns of the tile
+    constexpr int kVecs = kOutCols / 8;
+    const int n_out = EPI == 1 ? g.N / 2 : g.N;
+    const bool vec_ok = (g.ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(g.C) & 15) == 0;
+    const uint32_t part0 = smem_u32(base);
+    for (int it = (int)(rank * kSkThreads + threadIdx.x); it < rows * kVecs; it += (int)split * kSkThreads) {
+        const int r = it / kVecs, c = (it % kVecs) * 8;
+        const uint32_t at = part0 + (uint32_t)(r * kSkRowFloats + c) * 4;
+        float acc[EPI == 1 ? 16 : 8];
+#pragma unroll
+        for (int e = 0; e < (EPI == 1 ? 16 : 8); e++) acc[e] = 0.f;
+        for (uint32_t p = 0; p < split; p++) {
+            const uint32_t from = mapa_u32(at, p);
+#pragma unroll
+            for (int h = 0; h < (EPI == 1 ? 4 : 2); h++) {
+                // SwiGLU: columns c.. are gate, c + 64.. the matching up projections
+                const float4 v = ld_cluster_f4(from + (uint32_t)((h & 1) * 16 + (h >> 1) * (kSkBN / 2) * 4));
+                acc[h * 4] += v.x;
+                acc[h * 4 + 1] += v.y;
+                acc[h * 4 + 2] += v.z;
+                acc[h * 4 + 3] += v.w;
+            }
+        }
+        float o[8];
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+            if (EPI == 1) {
+                const float gt = acc[e], up = acc[8 + e];
+                o[e] = gt / (1.f + __expf(-gt)) * up;
+            } else {
+                o[e] = acc[e];
+            }
+        }
+        const int col = nt * kOutCols + c;
+        __nv_bfloat16 *dst = g.C + (int64_t)(mt * BM + r) * g.ldc + col;
+        if (vec_ok && col + 8 <= n_out) {
+            uint4 pk;
+            __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(&pk);
+#pragma unroll
+            for (int e = 0; e < 4; e++) h[e] = __floats2bfloat162_rn(o[2 * e], o[2 * e + 1]);
+            *reinterpret_cast<uint4 *>(dst) = pk;
+        } else {
+#pragma unroll
+            for (int e = 0; e < 8; e++)
+                if (col + e < n_out) dst[e] = __float2bfloat16_rn(o[e]);
+        }
+    }
+    __syncwarp();
+    cluster_sync_all();  // nobody leaves while a peer still reads its partial tile
+}
+
+}  // namespace mfk
+
+using namespace mfk;
+
+namespace {
+
+constexpr int kSkDynBytes = kSkStageArea + 1024;
+
+template <int EPI> bool splitk_ready()
+{
+    static const bool ok = cudaFuncSetAttribute(k_gemm_bf16_splitk<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSkDynBytes) == cudaSuccess;
+    return ok;
+}
+
+void fill_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, int grid, int split, cudaStream_t s)
+{
+    cfg = cudaLaunchConfig_t{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(kSkThreads);
+    cfg.dynamicSmemBytes = kSkDynBytes;
+    cfg.stream = s;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)split;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+}
+
+// Clusters of `split` CTAs that the device holds at once (a property of the kernel and the device, asked once per size).
+int clusters_resident(int split)
+{
+    static std::mutex mu;
+    static int known[64][kSkMaxSplit + 1] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    std::lock_guard<std::mutex> lk(mu);
+    if (known[dev][split] == 0) {
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at[1];
+        fill_config(cfg, at, split, split, nullptr);
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, k_gemm_bf16_splitk<0>, &cfg) != cudaSuccess) {
+            (void)cudaGetLastError();
+            n = 0;
+        }
+        known[dev][split] = n > 0 ? n : -1;
+    }
+    return known[dev][split];
+}
+
+}  // namespace
+
+extern "C" {
+
+// Same contract as mf_gemm_bf16_one. split: CTAs per tile (1..8), 0: chosen here.
+int mf_gemm_bf16_splitk(const void *A, const void *B, void *C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc, int *status,
+                        int swiglu, int split, void *stream)
+{
+    if (M <= 0 || N <= 0 || K <= 0 || (K & 7) != 0 || split < 0 || split > kSkMaxSplit) return -1;
+    if (swiglu && (N % 256) != 0) return -3;
+    if (!(swiglu ? splitk_ready<1>() : splitk_ready<0>()) || !splitk_ready<0>()) {
+        (void)cudaGetLastError();
+        return -2;
+    }
+    SplitArgs g{};
+    g.box_rows = std::min(BM, (M + 7) / 8 * 8);
+    int rc = make_tmap_2d(&g.tm.a, A, 2, (uint64_t)M, (uint64_t)K, (uint64_t)lda * 2, (uint32_t)g.box_rows, false);
+    if (rc == 0) rc = make_tmap_2d(&g.tm.b, B, 2, (uint64_t)N, (uint64_t)K, (uint64_t)ldb * 2, kSkBN / 2, false);
+    if (rc != 0) return rc;
+    g.C = static_cast<__nv_bfloat16 *>(C);
+    g.ldc = ldc;
+    g.M = M;
+    g.N = N;
+    g.K = K;
+    g.status = status;
+    g.stages = std::min(kSkMaxStages, kSkStageArea / (g.box_rows * KSPAN + kSkBN * KSPAN));
+    const int tiles = ((M + BM - 1) / BM) * ((N + kSkBN - 1) / kSkBN);
+    const int k_iters = (K * 2 + KSPAN - 1) / KSPAN;
+    if (split == 0) {
+        // rounds of resident clusters x steps of K per CTA; a step is worth about 1/8 of the fixed cost of one more CTA per
+        // tile (exchange through distributed shared memory)
+        double best = 0;
+        for (int s = 1; s <= kSkMaxSplit && s <= k_iters; s++) {
+            const int res = clusters_resident(s);
+            if (res <= 0) continue;
+            const double cost = (double)((tiles + res - 1) / res) * ((k_iters + s - 1) / s + 8) + s;
+            if (split == 0 || cost < best) {
+                best = cost;
+                split = s;
+            }
+        }
+        if (split == 0) return -4;
+    }
+    if (split > k_iters) return -1;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute at[1];
+    fill_config(cfg, at, tiles * split, split, (cudaStream_t)stream);
+    cudaError_t e = swiglu ? cudaLaunchKernelEx(&cfg, k_gemm_bf16_splitk<1>, g) : cudaLaunchKernelEx(&cfg, k_gemm_bf16_splitk<0>, g);
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    return e == cudaSuccess ? 0 : (int)e;
+}
+
+}  // extern "C"

@@ -39,3 +39,41 @@ def test_gemm_bf16_swiglu_epilogue(M, F, K, pair):
     err = (c.float() - ref).abs().max().item()
     scale = ref.abs().max().item()
     assert err <= 1e-2 * scale + 1e-2, f"max abs err {err} vs scale {scale}"
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 128, 64), (8, 136, 72), (33, 520, 200), (64, 7168, 2048), (127, 1000, 512), (129, 256, 1024), (260, 384, 4096)])
+@pytest.mark.parametrize("split", [0, 1, 2, 5, 8])
+def test_gemm_bf16_split_over_a_cluster(M, N, K, split):
+    """Few rows: K split over the CTAs of a cluster, the partial tiles added through distributed shared memory. The result
+    is one bf16 rounding away from the exact product (2^-9 of the value) plus fp32 accumulation (K 2^-24 of the terms)."""
+    from memfabric_hybrid_b200.ops import gemm
+    if split > (K + 63) // 64:
+        pytest.skip("more CTAs than steps of K")
+    torch.manual_seed(M + N + K)
+    a = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    b = (torch.randn(N, K, device="cuda") * 0.05).to(torch.bfloat16)
+    ld = N + (8 if split % 2 else 3)   # rows of C that 16-byte stores reach, and rows that they do not
+    c = torch.full((M, ld), 7.0, device="cuda", dtype=torch.bfloat16)
+    assert gemm._cu().mf_gemm_bf16_splitk(a.data_ptr(), b.data_ptr(), c.data_ptr(), M, N, K, K, K, ld, gemm.status_word().data_ptr(), 0, split,
+                                          torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    gemm.check_status()
+    ref = a.double() @ b.double().t()
+    bound = ref.abs() * 2.0 ** -8 + (a.double().abs() @ b.double().abs().t()) * K * 2.0 ** -24
+    assert ((c[:, :N].double() - ref).abs() <= bound).all()
+    assert bool((c[:, N:] == 7.0).all()), "columns past N were written"
+
+
+@pytest.mark.parametrize("M,F,K", [(1, 128, 128), (32, 3584, 8192), (130, 256, 512)])
+def test_gemm_bf16_swiglu_few_rows(M, F, K):
+    """The library's own choice for few rows, next to the one-CTA kernel on the same operands."""
+    from memfabric_hybrid_b200.ops import gemm
+    torch.manual_seed(M + F + K)
+    a = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(2 * F, K, device="cuda") * 0.05).to(torch.bfloat16)
+    c = gemm.gemm_bf16(a, w, swiglu=True)
+    one = gemm.gemm_bf16(a, w, swiglu=True, pair=False)
+    torch.cuda.synchronize()
+    gemm.check_status()
+    # both round the same fp32 value once; the sums differ by K 2^-24 of their terms, which SwiGLU scales by about |up|
+    assert ((c.float() - one.float()).norm() / one.float().norm()).item() <= 2.0 ** -8
