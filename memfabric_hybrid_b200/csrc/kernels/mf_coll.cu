@@ -15,6 +15,7 @@
 #include <cooperative_groups.h>
 
 #include "mf_coll.cuh"
+#include "mf_shift.cuh"
 #include "mf_devtrace.cuh"
 
 namespace mfk {
@@ -99,26 +100,54 @@ __device__ __forceinline__ void cta_convert_copy(const TS *__restrict__ src, TD 
     }
 }
 
-// Raw copy of [beg, end) elements of T (no conversion).
+// Raw copy of [beg, end) elements of T (no conversion). Eight independent 16-byte loads are in flight per thread before the
+// first store: with one CTA of 512 threads per SM that is 64 KB per SM (four left HBM and NVLink waiting). Eight emulated ranks, 30 MB
+// of fp32 each: staged reduce-scatter 175 us with four, 134 us with eight and the rotation of by_rank below. Ends at different
+// offsets inside a 16-byte granule go through the shifting copy.
+constexpr int kRawUnroll = 8;
 template <typename T> __device__ __forceinline__ void cta_raw_copy(const T *src, T *dst, uint64_t beg, uint64_t end)
 {
     constexpr int VN = 16 / sizeof(T);
-    uint64_t vend = beg;
-    if (aligned16(src + beg) && aligned16(dst + beg)) {
-        vend = beg + (end - beg) / VN * VN;
+    if (beg >= end) return;
+    const uint64_t sa = reinterpret_cast<uint64_t>(src + beg), da = reinterpret_cast<uint64_t>(dst + beg);
+    uint64_t vbeg = beg, vend = beg;
+    if (((sa ^ da) & 15) == 0) {
+        vbeg = min(end, beg + ((16 - (sa & 15)) & 15) / sizeof(T));  // up to the first whole granule
+        vend = vbeg + (end - vbeg) / VN * VN;
         const uint64_t step = (uint64_t)blockDim.x * VN;
-        uint64_t i = beg + (uint64_t)threadIdx.x * VN;
-        // four independent 16-byte loads in flight per thread before the first store (NVLink latency)
-        for (; i + 3 * step < vend; i += 4 * step) {
-            uint4 v[4];
+        uint64_t i = vbeg + (uint64_t)threadIdx.x * VN;
+        for (; i + (kRawUnroll - 1) * step < vend; i += kRawUnroll * step) {
+            uint4 v[kRawUnroll];
 #pragma unroll
-            for (int u = 0; u < 4; u++) v[u] = __ldcg(reinterpret_cast<const uint4 *>(src + i + u * step));
+            for (int u = 0; u < kRawUnroll; u++) v[u] = __ldcg(reinterpret_cast<const uint4 *>(src + i + u * step));
 #pragma unroll
-            for (int u = 0; u < 4; u++) *reinterpret_cast<uint4 *>(dst + i + u * step) = v[u];
+            for (int u = 0; u < kRawUnroll; u++) *reinterpret_cast<uint4 *>(dst + i + u * step) = v[u];
         }
         for (; i < vend; i += step) *reinterpret_cast<uint4 *>(dst + i) = __ldcg(reinterpret_cast<const uint4 *>(src + i));
+    } else if ((blockDim.x & 31) == 0 && blockDim.x >= 64) {
+        cta_copy_shifted<false>(reinterpret_cast<const uint8_t *>(src + beg), reinterpret_cast<uint8_t *>(dst + beg), (end - beg) * sizeof(T));
+        return;
     }
+    for (uint64_t i = beg + threadIdx.x; i < vbeg; i += blockDim.x) dst[i] = src[i];
     for (uint64_t i = vend + threadIdx.x; i < end; i += blockDim.x) dst[i] = src[i];
+}
+
+// W values per rank in the order of the ranks, from the order in which they were loaded (rank me + k at place k): a barrel
+// rotation in log2(W) conditional steps. (Picking every value out of W with a chain of selects was 256 instructions per
+// vector at W = 8, more than unpacking and adding.)
+template <int W> __device__ __forceinline__ void by_rank(uint4 (&v)[W], uint32_t me)
+{
+    static_assert((W & (W - 1)) == 0, "a power of two");
+#pragma unroll
+    for (int s = 1; s < W; s <<= 1) {
+        if ((me & s) != 0) {  // uniform over the CTA
+            uint4 t[W];
+#pragma unroll
+            for (int k = 0; k < W; k++) t[(k + s) & (W - 1)] = v[k];
+#pragma unroll
+            for (int k = 0; k < W; k++) v[k] = t[k];
+        }
+    }
 }
 
 // One source range to several destinations (all-gather, broadcast): every 16-byte vector is loaded ONCE, four
@@ -175,11 +204,9 @@ __device__ __forceinline__ void reduce_ranks(const Team &t, uint32_t me, uint64_
 #pragma unroll
                 for (int k = 0; k < W; k++) {
                     const uint32_t r = (me + k) % W;
-                    const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(reinterpret_cast<const T *>(peer_ptr(t, r, stage_a)) + base + i));
-#pragma unroll
-                    for (int q = 0; q < W; q++)
-                        if (q == (int)r) raw[q] = v;  // static indexing keeps raw[] in registers
+                    raw[k] = __ldcg(reinterpret_cast<const uint4 *>(reinterpret_cast<const T *>(peer_ptr(t, r, stage_a)) + base + i));
                 }
+                by_rank<(W > 0 ? W : 1)>(raw, me);
 #pragma unroll
                 for (int r = 0; r < W; r++) {
                     float f[VN];
@@ -309,10 +336,12 @@ template <typename T, typename TO, bool INT, int W> __global__ void __launch_bou
     const uint64_t m = a.n / world;
     const Range sub = cta_range<8>(m);
     const uint64_t ps = a.part_stride ? a.part_stride : m;
+    // staged rows start on 16 bytes whatever m is (input that sits in the staging area already is packed)
+    const uint64_t mp = a.zero_copy ? m : (m + 7) / 8 * 8;
     if (!a.zero_copy)
-        for (uint32_t c = 0; c < world; c++) cta_raw_copy<T>(in + c * ps, myA + c * m, sub.beg, sub.end);
+        for (uint32_t c = 0; c < world; c++) cta_raw_copy<T>(in + c * ps, myA + c * mp, sub.beg, sub.end);
     if (!lane_sync(t, me, 0, a.epoch, 0x120)) return;
-    reduce_ranks<T, INT, W>(t, me, a.stage_a, (uint64_t)me * m, sub.beg, sub.end, a.op,
+    reduce_ranks<T, INT, W>(t, me, a.stage_a, (uint64_t)me * mp, sub.beg, sub.end, a.op,
                             [&](uint64_t i, float *acc, int cnt) { emit<TO, INT>(out, i, acc, cnt, a.scale); });
 }
 
@@ -326,15 +355,24 @@ template <typename T, typename TO> __global__ void __launch_bounds__(512) k_allg
     TO *out = reinterpret_cast<TO *>(a.out + (uint64_t)me * a.out_rank_stride);
     constexpr int VN = Vec<T>::N;
     const Range sub = cta_range<8>(a.n);
-    for (uint32_t k = 0; k < world; k++) {
-        const uint32_t r = (me + k) % world;
-        TO *dst = reinterpret_cast<TO *>(peer_ptr(t, r, a.stage_b)) + (uint64_t)me * a.n;
-        cta_convert_copy<T, TO>(in, dst, sub.beg, sub.end, a.scale);
+    const uint64_t np = (a.n + 7) / 8 * 8;  // staged rows start on 16 bytes whatever n is
+    if (sizeof(T) == sizeof(TO) && a.scale == 1.f) {
+        // same type, no scaling: the shard is read once and fanned out to every rank's staging area
+        __shared__ TO *dsts[kMaxRanks];
+        if (threadIdx.x < world) dsts[threadIdx.x] = reinterpret_cast<TO *>(peer_ptr(t, (me + threadIdx.x) % world, a.stage_b)) + (uint64_t)me * np;
+        __syncthreads();
+        cta_fanout_copy<TO>(reinterpret_cast<const TO *>(in), dsts, world, sub.beg, sub.end);
+    } else {
+        for (uint32_t k = 0; k < world; k++) {
+            const uint32_t r = (me + k) % world;
+            TO *dst = reinterpret_cast<TO *>(peer_ptr(t, r, a.stage_b)) + (uint64_t)me * np;
+            cta_convert_copy<T, TO>(in, dst, sub.beg, sub.end, a.scale);
+        }
     }
     if (!lane_sync(t, me, 0, a.epoch, 0x130)) return;
     const TO *myB = reinterpret_cast<const TO *>(peer_ptr(t, me, a.stage_b));
     const uint64_t ps = a.part_stride ? a.part_stride : a.n;
-    for (uint32_t c = 0; c < world; c++) cta_raw_copy<TO>(myB + (uint64_t)c * a.n, out + (uint64_t)c * ps, sub.beg, sub.end);
+    for (uint32_t c = 0; c < world; c++) cta_raw_copy<TO>(myB + (uint64_t)c * np, out + (uint64_t)c * ps, sub.beg, sub.end);
 }
 
 // broadcast of n elements from a.root
@@ -382,11 +420,9 @@ __device__ __forceinline__ void reduce_direct(const Team &t, uint32_t me, const 
 #pragma unroll
                 for (int k = 0; k < W; k++) {
                     const uint32_t r = (me + k) % W;
-                    const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(reinterpret_cast<const T *>(peer_ptr(t, r, src_off[r])) + base + i));
-#pragma unroll
-                    for (int q = 0; q < W; q++)
-                        if (q == (int)r) raw[q] = v;
+                    raw[k] = __ldcg(reinterpret_cast<const uint4 *>(reinterpret_cast<const T *>(peer_ptr(t, r, src_off[r])) + base + i));
                 }
+                by_rank<(W > 0 ? W : 1)>(raw, me);
 #pragma unroll
                 for (int r = 0; r < W; r++) {
                     float f[VN];

@@ -292,3 +292,23 @@ def test_collective_while_compute_occupies_the_sms():
     for outcomes, ok in res:
         assert ok and all(o in ("ok", "timeout") for o in outcomes), res
     assert any("ok" in o for o, _ in res), res   # 10 ms of queueing is far inside the waits' budget: it completes
+
+
+@pytest.mark.parametrize("world", [2, 4, 8])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("m", [1, 7, 33, 4099, 65_537])
+def test_parts_that_do_not_end_on_16_bytes(comms, world, dtype, m):
+    """Rows of the staging area start on 16 bytes whatever m is; what the user's buffers hold sits at any offset."""
+    c = comms[world]
+    torch.manual_seed(m + world)
+    x = torch.randn(world, world * m, device="cuda").to(dtype)
+    part = c.reduce_scatter(x, scale=1.0 / world)
+    full = c.all_gather(part)
+    torch.cuda.synchronize()
+    ref = (x.double().sum(0) / world).view(world, m)
+    # one rounding to the type of the fp32 sum of `world` terms
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -20
+    bound = ref.abs() * eps + x.double().abs().sum(0).view(world, m) / world * 2.0 ** -22
+    assert ((part.double() - ref).abs() <= bound).all()
+    for r in range(world):
+        assert torch.equal(full[r].view(world, m), part)
