@@ -96,6 +96,8 @@ struct XArgs {
     const int4 *recv_info;
     uint64_t comb_off;
     int topk;
+    uint32_t *done_count;  // EPI 2, optional: local counter of finished CTAs, zero between launches
+    uint64_t flag_off;     // EPI 2: slot offset of the flag row that the last CTA raises to `epoch` on every peer
     uint32_t epoch;        // flag value of this call (grows by one per call)
     uint32_t seq;          // number of fused calls so far on these counters, including this one
     // MODE 1
@@ -219,20 +221,36 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_g
         mbar_fence_init();
         tma_prefetch_desc(&g.tm.a);
         tma_prefetch_desc(&g.tm.b);
-        if (MODE == 0) {
-            int run = 0;
-            for (int i = 0; i <= g.G; i++) {
-                const int ro = min(g.row_off[i], g.max_rows);
-                s_row_off[i] = ro;
-                tile_start[i] = run;
-                if (i < g.G) run += ((min(g.row_off[i + 1], g.max_rows) - ro + BM - 1) / BM) * n_tiles;
-            }
-        } else {
+        if (MODE != 0) {
             s_row_off[0] = 0;
             s_row_off[1] = g.max_rows;
             tile_start[0] = 0;
             tile_start[1] = (g.max_rows / BM) * n_tiles;
         }
+    }
+    if (MODE == 0 && warp == 2) {
+        // first tile of every group, 32 groups per step (one thread walking them took over a microsecond at 32 groups)
+        int run = 0;
+        for (int i0 = 0; i0 < g.G; i0 += 32) {
+            const int i = i0 + lane;
+            int lo = 0, hi = 0;
+            if (i < g.G) {
+                lo = min(g.row_off[i], g.max_rows);
+                hi = min(g.row_off[i + 1], g.max_rows);
+                s_row_off[i] = lo;
+                if (i == g.G - 1) s_row_off[g.G] = hi;
+            }
+            const int n = ((hi - lo + BM - 1) / BM) * n_tiles;
+            int upto = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int below = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += below;
+            }
+            if (i < g.G) tile_start[i] = run + upto - n;
+            run += __shfl_sync(0xffffffffu, upto, 31);
+        }
+        if (lane == 0) tile_start[g.G] = run;
     }
     if (warp == 1) {
         tmem_alloc(sm.tmem_slot(), kXTmemCols);
@@ -607,9 +625,24 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_g
             raise(p);
         }
     }
-    if (EPI == 2) __threadfence_system();
     tc_fence_before();
     __syncthreads();
+    if (EPI == 2) {
+        // The CTA that finishes last tells every rank that all of this rank's rows are home: the CTA barrier orders the CTA's
+        // stores before thread 0, whose system fence covers them, and the counter links the CTAs' fences.
+        __shared__ int last_sh;
+        if (threadIdx.x == 0) {
+            __threadfence_system();
+            last_sh = g.done_count != nullptr && atomicAdd(g.done_count, 1u) + 1 == gridDim.x;
+            if (last_sh) {
+                *g.done_count = 0;
+                __threadfence_system();
+            }
+        }
+        __syncthreads();
+        if (last_sh && threadIdx.x < g.team.world)
+            st_release_sys(reinterpret_cast<uint32_t *>(peer_ptr(g.team, threadIdx.x, g.flag_off)) + me, g.epoch);
+    }
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem_base, kXTmemCols);
@@ -698,9 +731,12 @@ int mf_grouped_gemm_fp8_mx_supported(int G, int N, int K, int epi)
 
 // epi: 0 plain (out bf16 [rows, N]), 1 SwiGLU (out bf16 [rows, N/2]), 2 weighted push into the combine slots of the
 // tokens' home ranks, 3 SwiGLU + fp8 re-quantisation (out e4m3 [rows, N/2], out_scale fp32 [rows, N/256]).
-int mf_grouped_gemm_fp8_mx(const void *A, const float *a_scale, int max_rows, const void *B, const float *b_scale, const int *row_off, int G,
-                           int N, int K, void *out, int64_t ldo, float *out_scale, int epi, const Team *team, const void *recv_info,
-                           uint64_t comb_off, int topk, int *status, int sms, void *stream)
+// epi 2 with a done_count (a device word, zero between launches): the kernel's last CTA raises this rank's flag in the row at
+// flag_off of every slot to `epoch`.
+int mf_grouped_gemm_fp8_mx_signal(const void *A, const float *a_scale, int max_rows, const void *B, const float *b_scale, const int *row_off, int G,
+                                  int N, int K, void *out, int64_t ldo, float *out_scale, int epi, const Team *team, const void *recv_info,
+                                  uint64_t comb_off, int topk, uint32_t *done_count, uint64_t flag_off, uint32_t epoch, int *status, int sms,
+                                  void *stream)
 {
     if (!mf_grouped_gemm_fp8_mx_supported(G, N, K, epi) || max_rows <= 0) return -1;
     if (epi == 2 && (team == nullptr || recv_info == nullptr)) return -1;
@@ -724,6 +760,9 @@ int mf_grouped_gemm_fp8_mx(const void *A, const float *a_scale, int max_rows, co
     g.recv_info = static_cast<const int4 *>(recv_info);
     g.comb_off = comb_off;
     g.topk = topk;
+    g.done_count = done_count;
+    g.flag_off = flag_off;
+    g.epoch = epoch;
     cudaStream_t s = (cudaStream_t)stream;
     switch (epi) {
         case 0: return launch_mx<0, 0>(g, sms, s);
@@ -732,6 +771,14 @@ int mf_grouped_gemm_fp8_mx(const void *A, const float *a_scale, int max_rows, co
         case 3: return launch_mx<0, 3>(g, sms, s);
         default: return -1;
     }
+}
+
+int mf_grouped_gemm_fp8_mx(const void *A, const float *a_scale, int max_rows, const void *B, const float *b_scale, const int *row_off, int G,
+                           int N, int K, void *out, int64_t ldo, float *out_scale, int epi, const Team *team, const void *recv_info,
+                           uint64_t comb_off, int topk, int *status, int sms, void *stream)
+{
+    return mf_grouped_gemm_fp8_mx_signal(A, a_scale, max_rows, B, b_scale, row_off, G, N, K, out, ldo, out_scale, epi, team, recv_info, comb_off,
+                                         topk, nullptr, 0, 0, status, sms, stream);
 }
 
 // All-gather -> GEMM in fp8. x_local [shard_rows, K] bf16 is this rank's sequence shard; it is quantised (e4m3, one

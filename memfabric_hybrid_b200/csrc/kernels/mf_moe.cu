@@ -164,35 +164,46 @@ __device__ __forceinline__ bool notify_body(const Team &team, const MoeHeap &hp,
     }
     if (!team_barrier(team, me, channel, epoch)) return false;
     const int *tbl = reinterpret_cast<const int *>(peer_ptr(team, me, hp.counts));
-    __shared__ int per_expert[1024];  // totals of every expert over all sources
+    // totals of every expert over all sources, and where each expert's rows start inside its owner's buffer: one warp per
+    // owner scans its experts (a serial walk by one thread cost as much as the count exchange at 32 experts)
+    __shared__ int per_expert[1024], first[1024];
     for (int e = threadIdx.x; e < E; e += blockDim.x) {
         int s = 0;
         for (uint32_t r = 0; r < W; r++) s += __ldcg(tbl + r * E + e);
         per_expert[e] = s;
     }
     __syncthreads();
-    // 2. my receive layout
-    if (threadIdx.x == 0) {
+    const int lane = threadIdx.x & 31;
+    for (int d = (int)(threadIdx.x >> 5); d < (int)W; d += (int)(blockDim.x >> 5)) {
         int run = 0;
-        for (int le = 0; le < El; le++) {
-            row_off[le] = run;
-            recv_per_expert[le] = per_expert[me * El + le];
-            run += per_expert[me * El + le];
+        for (int l0 = 0; l0 < El; l0 += 32) {
+            const int v = l0 + lane < El ? per_expert[d * El + l0 + lane] : 0;
+            int upto = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int below = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += below;
+            }
+            if (l0 + lane < El) first[d * El + l0 + lane] = run + upto - v;
+            run += __shfl_sync(0xffffffffu, upto, 31);
         }
-        row_off[El] = run;
+        if (d == (int)me && lane == 0) row_off[El] = run;
     }
     __syncthreads();
+    // 2. my receive layout
+    for (int le = threadIdx.x; le < El; le += blockDim.x) {
+        row_off[le] = first[me * El + le];
+        recv_per_expert[le] = per_expert[me * El + le];
+    }
     for (int i = threadIdx.x; i < El * (int)W; i += blockDim.x) {
         const int le = i / (int)W, s = i % (int)W;
-        int off = row_off[le];
+        int off = first[me * El + le];
         for (int r = 0; r < s; r++) off += __ldcg(tbl + r * E + me * El + le);
         src_off[i] = off;
     }
     // 3. where my group for expert e starts in its owner's buffer
     for (int e = threadIdx.x; e < E; e += blockDim.x) {
-        const int d = e / El, le = e % El;
-        int off = 0;
-        for (int l2 = 0; l2 < le; l2++) off += per_expert[d * El + l2];
+        int off = first[e];
         for (uint32_t r = 0; r < me; r++) off += __ldcg(tbl + r * E + e);
         put_off[e] = off;
     }
@@ -202,6 +213,61 @@ __device__ __forceinline__ bool notify_body(const Team &team, const MoeHeap &hp,
 __global__ void __launch_bounds__(1024) k_moe_notify(Team team, MoeHeap hp, int E, const int *tokens_per_expert, int *recv_per_expert,
                                                      int *row_off, int *put_off, int *src_off, uint32_t epoch)
 {
+    notify_body(team, hp, E, tokens_per_expert, recv_per_expert, row_off, put_off, src_off, epoch);
+}
+
+// Layout and count exchange of a small batch in one launch of one CTA: at a few hundred tokens the six launches they take
+// otherwise (two fills, ranking, offsets, ranks, notify) cost more than the work. Entries are ranked 1024 at a time in token
+// order, as the chunked kernels do; a running count per expert takes the place of their second pass.
+constexpr int kPrepareMax = 4096;  // entries; a chunk costs about 2 us here and nothing in the grid-wide kernels
+__global__ void __launch_bounds__(1024) k_moe_prepare(Team team, MoeHeap hp, const int *__restrict__ topk_idx, int T, int K, int E,
+                                                      int *tokens_per_expert, int *tokens_per_rank, int *send_idx, uint8_t *is_token_in_rank,
+                                                      int *recv_per_expert, int *row_off, int *put_off, int *src_off, uint32_t epoch)
+{
+    extern __shared__ uint16_t warp_cnt[];  // [32 warps][E]: hits of expert e in warp w, then the position of that warp's first hit
+    __shared__ int running[1024], per_rank[kMaxRanks];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int n = T * K, W = (int)team.world, El = E / W;
+    for (int x = threadIdx.x; x < E; x += blockDim.x) running[x] = 0;
+    if (threadIdx.x < kMaxRanks) per_rank[threadIdx.x] = 0;
+    for (int base = 0; base < n; base += 1024) {
+        for (int i = threadIdx.x; i < 32 * E; i += blockDim.x) warp_cnt[i] = 0;
+        __syncthreads();
+        const int i = base + (int)threadIdx.x;
+        int e = i < n ? topk_idx[i] : -1;
+        if (e >= E) e = -1;
+        const unsigned peers = __match_any_sync(0xffffffffu, e);
+        const int rank_in_warp = __popc(peers & ((1u << lane) - 1));
+        if (e >= 0 && rank_in_warp == 0) warp_cnt[warp * E + e] = (uint16_t)__popc(peers);
+        __syncthreads();
+        for (int x = threadIdx.x; x < E; x += blockDim.x) {
+            int run = running[x];
+            for (int w = 0; w < 32; w++) {
+                const int c = warp_cnt[w * E + x];
+                warp_cnt[w * E + x] = (uint16_t)run;
+                run += c;
+            }
+            running[x] = run;
+        }
+        __syncthreads();
+        if (i < n) send_idx[i] = e >= 0 ? (int)warp_cnt[warp * E + e] + rank_in_warp : 0;
+        __syncthreads();
+    }
+    for (int t = threadIdx.x; t < T; t += blockDim.x) {
+        uint32_t mask = 0;
+        for (int k = 0; k < K; k++) {
+            const int e = topk_idx[t * K + k];
+            if (e >= 0) mask |= 1u << (e / El);
+        }
+        for (int r = 0; r < W; r++) {
+            const bool in = (mask >> r) & 1u;
+            is_token_in_rank[t * W + r] = in ? 1 : 0;
+            if (in) atomicAdd(&per_rank[r], 1);
+        }
+    }
+    for (int x = threadIdx.x; x < E; x += blockDim.x) tokens_per_expert[x] = running[x];
+    __syncthreads();
+    if ((int)threadIdx.x < W) tokens_per_rank[threadIdx.x] = per_rank[threadIdx.x];
     notify_body(team, hp, E, tokens_per_expert, recv_per_expert, row_off, put_off, src_off, epoch);
 }
 
@@ -238,9 +304,37 @@ __device__ __forceinline__ void dispatch_preload(const DispatchArgs &a, uint4 &l
     }
 }
 
+// End of a dispatch, all threads of every CTA: the CTA that finishes last raises this rank's flag on every peer (the CTA
+// barrier orders the CTA's stores before thread 0, whose system fence covers them; the counter links the CTAs' fences).
+// Returns whether this CTA was the last one. Nobody waits for the peers here: a waiting CTA of this kernel would keep an SM
+// from kernels on other streams (a launch that needs every SM among them), which the one-warp k_moe_wait_all does not.
+__device__ __forceinline__ bool finish_dispatch(const DispatchArgs &a, uint32_t me)
+{
+    const Team &t = a.team;
+    __shared__ int last_sh;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence_system();
+        const uint32_t done = atomicAdd(a.done_count, 1u) + 1;
+        // seq > 0: the counter only grows and the host numbers the calls; seq == 0: the last CTA puts it back
+        // to zero, so the same launch parameters work again (CUDA-graph replay)
+        const bool last = a.seq != 0 ? done == gridDim.x * a.seq : done == gridDim.x;
+        if (last) {
+            if (a.seq == 0) *a.done_count = 0;
+            __threadfence_system();
+        }
+        last_sh = last ? 1 : 0;
+    }
+    __syncthreads();
+    // (the fence by thread 0 and the CTA barrier order everything in front of these stores)
+    if (last_sh && threadIdx.x < t.world)
+        st_release_sys(reinterpret_cast<uint32_t *>(peer_ptr(t, threadIdx.x, a.hp.flags)) + me, a.epoch);
+    return last_sh != 0;
+}
+
 constexpr int kTokBatch = 32;  // tokens whose routing table a CTA resolves in one pass
 
-__device__ __forceinline__ void dispatch_body(const DispatchArgs &a, uint4 nxt_lo, uint4 nxt_hi)
+__device__ __forceinline__ bool dispatch_body(const DispatchArgs &a, uint4 nxt_lo, uint4 nxt_hi)
 {
     const Team &t = a.team;
     const uint32_t me = team_rank(t);
@@ -373,22 +467,7 @@ __device__ __forceinline__ void dispatch_body(const DispatchArgs &a, uint4 nxt_l
             }
         }
     }
-    // the CTA that finishes last tells every peer that all of this rank's rows have been stored (the barrier orders the
-    // CTA's stores before thread 0, whose system fence covers them; the counter links the CTAs' fences)
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence_system();
-        const uint32_t done = atomicAdd(a.done_count, 1u) + 1;
-        // seq > 0: the counter only grows and the host numbers the calls; seq == 0: the last CTA puts it back
-        // to zero, so the same launch parameters work again (CUDA-graph replay)
-        const bool last = a.seq != 0 ? done == gridDim.x * a.seq : done == gridDim.x;
-        if (last) {
-            if (a.seq == 0) *a.done_count = 0;
-            __threadfence_system();
-            for (uint32_t r = 0; r < t.world; r++)
-                st_release_sys(reinterpret_cast<uint32_t *>(peer_ptr(t, r, a.hp.flags)) + me, a.epoch);
-        }
-    }
+    return finish_dispatch(a, me);
 }
 
 // ---- warp-per-token dispatch ------------------------------------------------------------------------------
@@ -396,12 +475,13 @@ __device__ __forceinline__ void dispatch_body(const DispatchArgs &a, uint4 nxt_l
 // and for every destination its lane 0 hands the copy unit ONE bulk store of the whole row, the scales leave as one
 // 16-byte store per lane and the info record as one store from the lane that resolved the destination. Nothing in the
 // loop involves another warp, so there is no CTA barrier per token, and a row costs one copy instruction per destination
-// instead of one 16-byte store per thread per destination. Two buffers per warp: the copy unit reads the previous token's
-// buffer while the next row is quantised.
-constexpr int kDwWarps = 12;
-constexpr int kDwLoads = 14;  // independent 16-byte loads per lane in flight (256 elements per warp load)
+// instead of one 16-byte store per thread per destination. What bounds a token is its chain (routing, row, conversion, copy
+// unit), so as many tokens as shared memory holds are on their way at once: 24 warps with one 7.4 KB buffer each (H = 7168)
+// rather than 12 warps with two.
+constexpr int kDwWarps = 24;
+constexpr int kDwLoads = 7;  // independent 16-byte loads per lane in flight (256 elements per warp load)
 __host__ __device__ constexpr int dw_buf_bytes(int H) { return (H + (H / kQuantGroup) * 4 + 127) / 128 * 128; }  // e4m3 row + its scales
-__host__ __device__ constexpr int dw_smem_bytes(int H) { return kDwWarps * 2 * dw_buf_bytes(H); }
+__host__ __device__ constexpr int dw_smem_bytes(int H) { return kDwWarps * dw_buf_bytes(H); }
 
 __device__ __forceinline__ void bulk_store(void *gdst, const void *ssrc, uint32_t bytes)
 {
@@ -417,14 +497,12 @@ __global__ void __launch_bounds__(kDwWarps * 32) k_moe_dispatch_warp(DispatchArg
     const int H = a.sh.H, K = a.sh.K, El = a.sh.E / (int)t.world;
     const int groups = H / kQuantGroup;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int stride_buf = dw_buf_bytes(H);
-    uint8_t *bufs = dw_smem + (size_t)warp * 2 * stride_buf;
-    const int wid = (int)blockIdx.x * kDwWarps + warp, wtotal = (int)gridDim.x * kDwWarps;
+    uint8_t *buf = dw_smem + (size_t)warp * dw_buf_bytes(H);
+    float *sc = reinterpret_cast<float *>(buf + H);
+    // neighbouring tokens go to different SMs: a small batch uses every SM's path to memory
+    const int wid = warp * (int)gridDim.x + (int)blockIdx.x, wtotal = (int)gridDim.x * kDwWarps;
     const bool smoothed = a.smooth != nullptr;
-    int which = 0;
-    for (int tok = wid; tok < a.sh.T; tok += wtotal, which ^= 1) {
-        uint8_t *buf = bufs + which * stride_buf;
-        float *sc = reinterpret_cast<float *>(buf + H);
+    for (int tok = wid; tok < a.sh.T; tok += wtotal) {
         // routing of this token: lane k resolves destination k (two dependent loads, overlapped with the row loads below)
         int d_rank = -1, d_pos = 0;
         float d_w = 0.f;
@@ -441,12 +519,8 @@ __global__ void __launch_bounds__(kDwWarps * 32) k_moe_dispatch_warp(DispatchArg
                 }
             }
         }
-        // the copy unit must be done READING this buffer (the token before the previous one)
-        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-        __syncwarp();
-        // quantise: one warp load covers 256 elements = two 128-groups (lanes 0-15 and 16-31); half a row of 7168 elements
-        // is requested before the first conversion (14 independent 16-byte loads per lane), so a token costs two memory
-        // latencies, not one per chunk.
+        // quantise: one warp load covers 256 elements = two 128-groups (lanes 0-15 and 16-31); a quarter of a row of 7168
+        // elements is requested before the first conversion.
         const __nv_bfloat16 *row = a.x + (int64_t)tok * H;
         for (int c0 = 0; c0 < H; c0 += kDwLoads * 256) {
             uint4 raw[kDwLoads];
@@ -454,6 +528,11 @@ __global__ void __launch_bounds__(kDwWarps * 32) k_moe_dispatch_warp(DispatchArg
             for (int u = 0; u < kDwLoads; u++) {
                 const int col = c0 + u * 256 + lane * 8;
                 raw[u] = col < H ? __ldg(reinterpret_cast<const uint4 *>(row + col)) : make_uint4(0, 0, 0, 0);
+            }
+            if (c0 == 0) {
+                // the copy unit must be done READING this buffer (the previous token); the row's first loads are on their way
+                if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                __syncwarp();
             }
 #pragma unroll
             for (int u = 0; u < kDwLoads; u++) {
@@ -514,18 +593,8 @@ __global__ void __launch_bounds__(kDwWarps * 32) k_moe_dispatch_warp(DispatchArg
         asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
         asm volatile("fence.proxy.async;" ::: "memory");  // the copy unit's writes, as the generic proxy (the fences below) sees them
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence_system();
-        const uint32_t done = atomicAdd(a.done_count, 1u) + 1;
-        const bool last = a.seq != 0 ? done == gridDim.x * a.seq : done == gridDim.x;
-        if (last) {
-            if (a.seq == 0) *a.done_count = 0;
-            __threadfence_system();
-            for (uint32_t r = 0; r < t.world; r++)
-                st_release_sys(reinterpret_cast<uint32_t *>(peer_ptr(t, r, a.hp.flags)) + me, a.epoch);
-        }
-    }
+    __syncwarp();
+    finish_dispatch(a, me);
 }
 
 __global__ void __launch_bounds__(448) k_moe_dispatch(DispatchArgs a)
@@ -705,12 +774,13 @@ __device__ __forceinline__ void combine_reduce_body(const Team &t, const MoeHeap
 // One cooperative launch per direction instead of six: the launches, not the bytes, dominate at 128
 // tokens. Dispatch: CTA 0 builds the layout (shared-memory histogram; the order of rows inside an expert
 // group is the order in which the atomics land) and runs the count exchange, the grid then pushes the
-// tokens and CTA 0 waits for every peer's rows. Combine: the grid pushes the expert outputs home, CTA 0
-// signals and waits for all peers, the grid reduces the K slots of each token.
+// tokens and the CTA that finishes last waits for every peer's rows. Combine: the grid pushes the expert outputs
+// home, the last CTA signals, every CTA waits for all ranks' flags and the grid reduces the K slots of each token
+// (a cooperative launch: CTAs wait for the last one of their own grid).
 // The pair numbers its calls with a counter in device memory and uses flag rows and a barrier channel of
 // its own (the caller passes MoeHeap.flags advanced by two rows), so a captured launch can be replayed
 // as a CUDA graph and may be mixed with the multi-launch path on the same buffers.
-// A wait that runs out is recorded in the status word; the kernel still reaches every grid-wide
+// A wait that runs out is recorded in the status word; the kernel still reaches every
 // synchronisation and returns (the results of that call are then unspecified).
 struct LLDispatchArgs {
     DispatchArgs d;          // d.send_idx and d.put_off are OUTPUTS here (device scratch of T*K and E ints)
@@ -752,20 +822,19 @@ __global__ void __launch_bounds__(448) k_moe_ll_dispatch(LLDispatchArgs a)
     grid.sync();  // every CTA has read the call counter before this point
     if (blockIdx.x == 0 && threadIdx.x == 0) *a.epoch_dev = a.d.epoch;
     MF_PROF_START(PF_DISPATCH);
-    dispatch_body(a.d, pre_lo, pre_hi);
+    const bool last = dispatch_body(a.d, pre_lo, pre_hi);
     MF_PROF_STOP(PF_DISPATCH);
-    if (blockIdx.x == 0) MF_PROF_START(PF_WAIT_PEERS);
-    if (blockIdx.x == 0 && threadIdx.x < t.world) {
+    if (!last) return;  // uniform over the CTA
+    MF_PROF_START(PF_WAIT_PEERS);
+    if (threadIdx.x < t.world) {
         const uint32_t *f = reinterpret_cast<const uint32_t *>(peer_ptr(t, me, a.d.hp.flags)) + threadIdx.x;
         if (!wait_flag(f, a.d.epoch, t.spin_limit)) {
             report_timeout(t, me, 0x421, a.d.epoch);
             atomicCAS(a.d.status, 0, 0x421);
         }
     }
-    if (blockIdx.x == 0) {
-        __syncthreads();
-        MF_PROF_STOP(PF_WAIT_PEERS);
-    }
+    __syncthreads();
+    MF_PROF_STOP(PF_WAIT_PEERS);
 }
 
 struct LLCombineArgs {
@@ -777,33 +846,42 @@ struct LLCombineArgs {
     int *status;
     const float *topk_w;   // optional [T, K]: weights applied on the home side
     const uint32_t *epoch_dev;  // the call counter the matching k_moe_ll_dispatch left behind
+    uint32_t *done_count;       // counts this launch's CTAs, zero between launches (the dispatch's counter serves)
 };
 
 __global__ void __launch_bounds__(256) k_moe_ll_combine(LLCombineArgs a)
 {
-    cooperative_groups::grid_group grid = cooperative_groups::this_grid();
     const Team &t = a.p.team;
     const uint32_t me = team_rank(t);
     if (a.epoch_dev != nullptr) a.epoch = *reinterpret_cast<const volatile uint32_t *>(a.epoch_dev);
     MF_PROF_START(PF_PUSH);
     combine_push_body(a.p);
-    __threadfence_system();
     MF_PROF_STOP(PF_PUSH);
-    grid.sync();
+    // The last CTA to finish pushing raises this rank's flag on every peer; every CTA waits for the peers' flags itself (its
+    // own rank's among them, so nobody reduces before this rank's rows are stored): no grid-wide barrier on either side.
+    __shared__ int last_sh;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence_system();
+        const uint32_t done = atomicAdd(a.done_count, 1u) + 1;
+        last_sh = done == gridDim.x ? 1 : 0;
+        if (done == gridDim.x) {
+            *a.done_count = 0;
+            __threadfence_system();
+        }
+    }
+    __syncthreads();
     if (blockIdx.x == 0) MF_PROF_START(PF_WAIT_PEERS);
-    if (blockIdx.x == 0 && threadIdx.x < t.world) {
-        st_release_sys(reinterpret_cast<uint32_t *>(peer_ptr(t, threadIdx.x, a.p.hp.flags)) + kMaxRanks + me, a.epoch);
+    if (threadIdx.x < t.world) {
+        if (last_sh) st_release_sys(reinterpret_cast<uint32_t *>(peer_ptr(t, threadIdx.x, a.p.hp.flags)) + kMaxRanks + me, a.epoch);
         const uint32_t *f = reinterpret_cast<const uint32_t *>(peer_ptr(t, me, a.p.hp.flags)) + kMaxRanks + threadIdx.x;
         if (!wait_flag(f, a.epoch, t.spin_limit)) {
             report_timeout(t, me, 0x422, a.epoch);
             atomicCAS(a.status, 0, 0x422);
         }
     }
-    if (blockIdx.x == 0) {
-        __syncthreads();
-        MF_PROF_STOP(PF_WAIT_PEERS);
-    }
-    grid.sync();
+    __syncthreads();
+    if (blockIdx.x == 0) MF_PROF_STOP(PF_WAIT_PEERS);
     MF_PROF_START(PF_COMBINE);
     combine_reduce_body(t, a.p.hp, a.sh, a.topk_idx, a.out, a.topk_w);
     MF_PROF_STOP(PF_COMBINE);
@@ -858,6 +936,7 @@ int mf_moe_layout(const int *topk_idx, int T, int K, int E, int world, int *toke
         k_moe_layout_chunk_rank<<<chunks, kLayoutChunk, 32 * E * sizeof(uint16_t), s>>>(topk_idx, n, E, send_idx, chunk_cnt);
         k_moe_layout_chunk_offset<<<chunks, kLayoutChunk, E * sizeof(int), s>>>(topk_idx, n, E, send_idx, chunk_cnt, tokens_per_expert);
     } else {
+        cudaMemsetAsync(send_idx, 0, sizeof(int) * (size_t)n, s);  // unselected slots
         k_moe_layout_expert<<<E, 1024, 0, s>>>(topk_idx, T * K, tokens_per_expert, send_idx);
     }
     k_moe_layout_rank<<<(T + 255) / 256, 256, 0, s>>>(topk_idx, T, K, E / world, world, tokens_per_rank, is_token_in_rank);
@@ -870,6 +949,22 @@ int mf_moe_notify(const Team *team, const MoeHeap *hp, int E, const int *tokens_
 {
     if (team == nullptr || hp == nullptr || team->emu || E > 1024 || E % (int)team->world != 0) return -1;
     k_moe_notify<<<1, 1024, 0, (cudaStream_t)stream>>>(*team, *hp, E, tokens_per_expert, recv_per_expert, row_off, put_off, src_off, epoch);
+    cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? 0 : (int)e;
+}
+
+// mf_moe_layout and mf_moe_notify of up to kPrepareMax entries in one launch; -3: too many, make the two calls.
+int mf_moe_prepare(const Team *team, const MoeHeap *hp, const int *topk_idx, int T, int K, int E, int *tokens_per_expert, int *tokens_per_rank,
+                   int *send_idx, uint8_t *is_token_in_rank, int *recv_per_expert, int *row_off, int *put_off, int *src_off, uint32_t epoch,
+                   void *stream)
+{
+    if (team == nullptr || hp == nullptr || team->emu || T <= 0 || K <= 0 || K > 16 || E <= 0 || E > 1024 || E % (int)team->world != 0) return -1;
+    if (T * K > kPrepareMax) return -3;
+    static const bool ok = cudaFuncSetAttribute(k_moe_prepare, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * 1024 * 2) == cudaSuccess;
+    if (!ok) return -2;
+    k_moe_prepare<<<1, 1024, 32 * E * sizeof(uint16_t), (cudaStream_t)stream>>>(*team, *hp, topk_idx, T, K, E, tokens_per_expert, tokens_per_rank,
+                                                                                send_idx, is_token_in_rank, recv_per_expert, row_off, put_off,
+                                                                                src_off, epoch);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : (int)e;
 }
@@ -949,12 +1044,12 @@ int mf_moe_ll_dispatch(const DispatchArgs *d, int *tokens_per_expert, int *recv_
 }
 
 int mf_moe_ll_combine(const Team *team, const MoeHeap *hp, const MoeShape *sh, const void *y, int64_t ldy, const int *rows_dev, int weighted,
-                      const int *topk_idx, const float *topk_w, void *out, uint32_t epoch, const uint32_t *epoch_dev, int *status, int ctas,
-                      void *stream)
+                      const int *topk_idx, const float *topk_w, void *out, uint32_t epoch, const uint32_t *epoch_dev, uint32_t *done_count,
+                      int *status, int ctas, void *stream)
 {
-    if (team == nullptr || hp == nullptr || sh == nullptr || team->emu || sh->H % 8 != 0 || ctas <= 0) return -1;
+    if (team == nullptr || hp == nullptr || sh == nullptr || team->emu || sh->H % 8 != 0 || ctas <= 0 || done_count == nullptr) return -1;
     LLCombineArgs a{{*team, *hp, static_cast<const __nv_bfloat16 *>(y), ldy, rows_dev, sh->H, sh->K, weighted}, *sh, topk_idx,
-                    static_cast<__nv_bfloat16 *>(out), epoch, status, topk_w, epoch_dev};
+                    static_cast<__nv_bfloat16 *>(out), epoch, status, topk_w, epoch_dev, done_count};
     void *params[] = {&a};
     cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_moe_ll_combine), dim3(ctas), dim3(256), params, 0,
                                                 (cudaStream_t)stream);

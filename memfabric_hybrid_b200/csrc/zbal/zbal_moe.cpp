@@ -52,7 +52,7 @@ struct MoeLaunchers {
     int (*combinePush)(const MfTeam *, const MoeHeap *, const void *, int64_t, const int *, int, int, int, int, void *) = nullptr;
     int (*llDispatch)(const DispatchArgs *, int *, int *, int *, int *, uint32_t *, int, void *) = nullptr;
     int (*llCombine)(const MfTeam *, const MoeHeap *, const MoeShape *, const void *, int64_t, const int *, int, const int *, const float *,
-                     void *, uint32_t, const uint32_t *, int *, int, void *) = nullptr;
+                     void *, uint32_t, const uint32_t *, uint32_t *, int *, int, void *) = nullptr;
     int (*quantRows)(const void *, int64_t, const int *, int, void *, float *, int, void *) = nullptr;
     int (*groupedGemm)(const void *, const float *, int, const void *, const float *, const int *, int, int, int, void *, int64_t, int,
                        const MfTeam *, const void *, uint64_t, int, int *, int, void *) = nullptr;
@@ -347,7 +347,7 @@ int32_t zbal_combine_low_latency(zbal_moe_t moe, const void *expandX, int64_t ld
     if (!expandX || !rowsDev || !topkIndex || !xOut || tokens <= 0 || tokens > c->sh.T) return MF_FAIL(Z_INVALID_PARAM, "low-latency combine: NULL tensor or bad token count");
     MoeShape sh = c->sh;
     sh.T = (int)tokens;
-    return Launched(Moe()->llCombine(&c->comm->team, &c->hpLL, &sh, expandX, ld, rowsDev, weighted, topkIndex, homeWeights, xOut, 0, c->epochLL, c->status,
+    return Launched(Moe()->llCombine(&c->comm->team, &c->hpLL, &sh, expandX, ld, rowsDev, weighted, topkIndex, homeWeights, xOut, 0, c->epochLL, c->doneLL, c->status,
                                      c->llGrid, stream), "low-latency combine");
 }
 

@@ -43,6 +43,8 @@ class DispatchArgsC(C.Structure):
                 ("smooth", C.c_void_p)]
 
 
+_COMBINE_ROW = 16 * 4  # byte offset of the combine row in the flag area: 16 ranks x u32 per row (kMaxRanks in mf_team.cuh)
+_PREPARE_MAX = 4096  # (token, expert) entries up to which one CTA does the layout and the count exchange (kPrepareMax in mf_moe.cu)
 _lib = None
 
 
@@ -55,6 +57,8 @@ def _cu():
         l.mf_moe_layout.argtypes = [vp, ci, ci, ci, ci, vp, vp, vp, vp, vp]
         l.mf_moe_notify.restype = ci
         l.mf_moe_notify.argtypes = [P(TeamC), P(MoeHeapC), ci, vp, vp, vp, vp, vp, C.c_uint32, vp]
+        l.mf_moe_prepare.restype = ci
+        l.mf_moe_prepare.argtypes = [P(TeamC), P(MoeHeapC), vp, ci, ci, ci, vp, vp, vp, vp, vp, vp, vp, vp, C.c_uint32, vp]
         l.mf_moe_dispatch.restype = ci
         l.mf_moe_dispatch.argtypes = [P(DispatchArgsC), ci, vp]
         l.mf_moe_wait_all.restype = ci
@@ -68,13 +72,16 @@ def _cu():
         l.mf_moe_ll_dispatch.restype = ci
         l.mf_moe_ll_dispatch.argtypes = [P(DispatchArgsC), vp, vp, vp, vp, vp, ci, vp]
         l.mf_moe_ll_combine.restype = ci
-        l.mf_moe_ll_combine.argtypes = [P(TeamC), P(MoeHeapC), P(MoeShapeC), vp, C.c_int64, vp, ci, vp, vp, vp, C.c_uint32, vp, vp, ci, vp]
+        l.mf_moe_ll_combine.argtypes = [P(TeamC), P(MoeHeapC), P(MoeShapeC), vp, C.c_int64, vp, ci, vp, vp, vp, C.c_uint32, vp, vp, vp, ci, vp]
         l.mf_quant_rows_fp8.restype = ci
         l.mf_quant_rows_fp8.argtypes = [vp, C.c_int64, vp, ci, vp, vp, ci, vp]
         l.mf_grouped_gemm_fp8.restype = ci
         l.mf_grouped_gemm_fp8.argtypes = [vp, vp, ci, vp, vp, vp, ci, ci, ci, vp, C.c_int64, ci, P(TeamC), vp, C.c_uint64, ci, vp, ci, vp]
         l.mf_grouped_gemm_fp8_mx.restype = ci
         l.mf_grouped_gemm_fp8_mx.argtypes = [vp, vp, ci, vp, vp, vp, ci, ci, ci, vp, C.c_int64, vp, ci, P(TeamC), vp, C.c_uint64, ci, vp, ci, vp]
+        l.mf_grouped_gemm_fp8_mx_signal.restype = ci
+        l.mf_grouped_gemm_fp8_mx_signal.argtypes = [vp, vp, ci, vp, vp, vp, ci, ci, ci, vp, C.c_int64, vp, ci, P(TeamC), vp, C.c_uint64, ci, vp,
+                                                    C.c_uint64, C.c_uint32, vp, ci, vp]
         l.mf_grouped_gemm_fp8_mx_supported.restype = ci
         l.mf_grouped_gemm_fp8_mx_supported.argtypes = [ci, ci, ci, ci]
         _lib = l
@@ -228,6 +235,7 @@ class MoEComm:
         heap.view(hp.counts, (self.world * experts,), torch.int32).zero_()
         self._epoch = 0
         self._done = torch.zeros(1, dtype=torch.int32, device=self.dev)
+        self._push_done = torch.zeros(1, dtype=torch.int32, device=self.dev)  # finished CTAs of the down projection, zero between launches
         self._dispatches = 0
         self._ll_done = torch.zeros(1, dtype=torch.int32, device=self.dev)
         self._ll_grid = None
@@ -268,7 +276,7 @@ class MoEComm:
         idx = topk_idx.to(torch.int32).contiguous()
         tpe = torch.empty(self.E, dtype=torch.int32, device=self.dev)
         tpr = torch.empty(self.world, dtype=torch.int32, device=self.dev)
-        sidx = torch.zeros(T * self.K, dtype=torch.int32, device=self.dev)
+        sidx = torch.empty(T * self.K, dtype=torch.int32, device=self.dev)
         inr = torch.empty((T, self.world), dtype=torch.uint8, device=self.dev)
         _ok(_cu().mf_moe_layout(idx.data_ptr(), T, self.K, self.E, self.world, tpe.data_ptr(), tpr.data_ptr(), sidx.data_ptr(),
                                 inr.data_ptr(), _s()), "moe_layout")
@@ -281,15 +289,28 @@ class MoEComm:
         if smooth is not None:
             assert not self.raw_bf16 and smooth.dtype == torch.float32 and smooth.is_contiguous() and smooth.numel() == self.H
         T = x.shape[0]
-        idx, tpe, tpr, sidx, inr = self.get_dispatch_layout(topk_idx)
-        self._epoch += 1
         team = self.heap.team()
+        small = T * self.K <= _PREPARE_MAX
+        if small:
+            i32 = dict(dtype=torch.int32, device=self.dev)
+            idx = topk_idx.to(torch.int32).contiguous()
+            tpe, tpr, sidx = torch.empty(self.E, **i32), torch.empty(self.world, **i32), torch.empty(T * self.K, **i32)
+            inr = torch.empty((T, self.world), dtype=torch.uint8, device=self.dev)
+        else:
+            idx, tpe, tpr, sidx, inr = self.get_dispatch_layout(topk_idx)
+        self._epoch += 1
         rpe = torch.empty(self.El, dtype=torch.int32, device=self.dev)
         row_off = torch.empty(self.El + 1, dtype=torch.int32, device=self.dev)
         put_off = torch.empty(self.E, dtype=torch.int32, device=self.dev)
         src_off = torch.empty(self.El * self.world, dtype=torch.int32, device=self.dev)
-        _ok(_cu().mf_moe_notify(C.byref(team), C.byref(self.hp), self.E, tpe.data_ptr(), rpe.data_ptr(), row_off.data_ptr(),
-                                put_off.data_ptr(), src_off.data_ptr(), self._epoch, _s()), "moe_notify")
+        if small:
+            # layout and count exchange in one launch
+            _ok(_cu().mf_moe_prepare(C.byref(team), C.byref(self.hp), idx.data_ptr(), T, self.K, self.E, tpe.data_ptr(), tpr.data_ptr(),
+                                     sidx.data_ptr(), inr.data_ptr(), rpe.data_ptr(), row_off.data_ptr(), put_off.data_ptr(), src_off.data_ptr(),
+                                     self._epoch, _s()), "moe_prepare")
+        else:
+            _ok(_cu().mf_moe_notify(C.byref(team), C.byref(self.hp), self.E, tpe.data_ptr(), rpe.data_ptr(), row_off.data_ptr(),
+                                    put_off.data_ptr(), src_off.data_ptr(), self._epoch, _s()), "moe_notify")
         w = topk_w.to(torch.float32).contiguous()
         self._dispatches += 1
         a = DispatchArgsC(team, self.hp, self._shape(T), x.data_ptr(), idx.data_ptr(), w.data_ptr(), sidx.data_ptr(), put_off.data_ptr(),
@@ -334,15 +355,16 @@ class MoEComm:
         cu = _cu()
         if cu.mf_grouped_gemm_fp8_mx_supported(El, two_i, H, 3) and cu.mf_grouped_gemm_fp8_mx_supported(El, H, I, 2):
             # two launches: gate/up + SwiGLU + re-quantisation to fp8 in the first GEMM's epilogue, down projection +
-            # weighted push to the tokens' home ranks in the second's; w1q interleaved with tile 128
+            # weighted push to the tokens' home ranks in the second's, whose last CTA raises the combine flag; w1q interleaved
+            # with tile 128
             _ok(cu.mf_grouped_gemm_fp8_mx(self.heap.ptr(self.rank, self.hp.recv_x), self.heap.ptr(self.rank, self.hp.recv_scale), self.max_recv,
                                           w1q.data_ptr(), w1s.data_ptr(), st.row_off.data_ptr(), El, two_i, H, self._hq.data_ptr(), I,
                                           self._hs.data_ptr(), 3, None, None, 0, self.K, stw, self._grid, _s()), "grouped_gemm_fp8_mx (gate/up)")
-            _ok(cu.mf_grouped_gemm_fp8_mx(self._hq.data_ptr(), self._hs.data_ptr(), self.max_recv, w2q.data_ptr(), w2s.data_ptr(),
-                                          st.row_off.data_ptr(), El, H, I, None, 0, None, 2, C.byref(team),
-                                          self.heap.ptr(self.rank, self.hp.recv_info), self.hp.comb, self.K, stw, self._grid, _s()),
+            _ok(cu.mf_grouped_gemm_fp8_mx_signal(self._hq.data_ptr(), self._hs.data_ptr(), self.max_recv, w2q.data_ptr(), w2s.data_ptr(),
+                                                 st.row_off.data_ptr(), El, H, I, None, 0, None, 2, C.byref(team),
+                                                 self.heap.ptr(self.rank, self.hp.recv_info), self.hp.comb, self.K, self._push_done.data_ptr(),
+                                                 self.hp.flags + _COMBINE_ROW, st.epoch & 0xFFFFFFFF, stw, self._grid, _s()),
                 "grouped_gemm_fp8_mx (down+combine)")
-            _ok(cu.mf_moe_signal_all(C.byref(team), C.byref(self.hp), 1, st.epoch, _s()), "moe_signal")
             return
         # shapes the 128 x 256 kernel does not take (N not a multiple of 256): the 128 x 128 kernel that applies the
         # scales in registers, with w1q interleaved with tile 64 and a separate re-quantisation pass
@@ -422,6 +444,6 @@ class MoEComm:
         hw = home_weights.to(torch.float32).contiguous() if home_weights is not None else None
         _ok(_cu().mf_moe_ll_combine(C.byref(team), C.byref(self._ll_hp), C.byref(sh), y.data_ptr(), y.stride(0), st.row_off[self.El:].data_ptr(),
                                     1 if weighted else 0, st.topk_idx.data_ptr(), hw.data_ptr() if hw is not None else None, out.data_ptr(), 0, self._ll_epoch.data_ptr(),
-                                    status_word(self.dev).data_ptr(),
+                                    self._ll_done.data_ptr(), status_word(self.dev).data_ptr(),
                                     self._ll_grid or self._grid, _s()), "moe_ll_combine")
         return out

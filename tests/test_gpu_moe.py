@@ -220,3 +220,59 @@ def _canary_rank(rank, world, url, sync):
 def test_moe_receive_areas_are_guarded_by_canaries():
     url = f"127.0.0.1:{free_port()}"
     assert run_ranks(_canary_rank, 1, (url,), timeout=300, with_barrier=True, env={"MF_MOE_CANARY": "1"}) == [True]
+
+
+def _prepare_rank(rank, world, url, sync):
+    import torch
+    from memfabric_hybrid_b200.ops import gemm, moe as M
+    from memfabric_hybrid_b200.ops.heap import SymmetricHeap
+    H, E, K, Tmax = 512, 48, 4, 1300
+    heap = SymmetricHeap(url, 1, 0, 0, (2 << 20) + Tmax * K * (H + H // 128 * 4 + 16) + Tmax * K * H * 2 + (4 << 20))
+    comm = M.MoEComm(heap, Tmax, H, E, K, max_recv=Tmax * K)
+    bad = []
+    for T in (1, 7, 255, 256, 257, 1023, 1024, 1025, 1300):   # 4096 entries is where the one-launch layout ends
+        g = torch.Generator("cuda").manual_seed(T)
+        x = torch.randn(T, H, device="cuda", generator=g).to(torch.bfloat16)
+        idx = torch.rand(T, E, device="cuda", generator=g).topk(K, dim=-1).indices.to(torch.int32)
+        idx[torch.rand(T, K, device="cuda", generator=g) < 0.1] = -1    # unselected slots
+        w = torch.rand(T, K, device="cuda", generator=g)
+        st = comm.dispatch(x, idx, w)
+        torch.cuda.synchronize()
+        gemm.check_status()
+        flat = idx.view(-1).cpu().long()
+        on = flat >= 0
+        counts = torch.bincount(flat[on], minlength=E)
+        pos = torch.zeros_like(flat)
+        seen = [0] * E
+        for i, e in enumerate(flat.tolist()):
+            if e >= 0:
+                pos[i] = seen[e]
+                seen[e] += 1
+        first = torch.cat([torch.zeros(1, dtype=torch.long), counts.cumsum(0)])
+        ok = torch.equal(st.tokens_per_expert.cpu().long(), counts) and torch.equal(st.row_off.cpu().long(), first)
+        ok = ok and torch.equal(st.recv_per_expert.cpu().long(), counts) and torch.equal(st.put_off.cpu().long(), first[:-1])
+        ok = ok and torch.equal(st.src_off.cpu().long(), first[:-1])
+        ok = ok and torch.equal(st.send_idx.cpu().long()[on], pos[on]) and bool((st.send_idx.cpu()[~on] == 0).all())
+        any_on = (idx >= 0).any(1)
+        ok = ok and int(st.tokens_per_rank[0]) == int(any_on.sum()) and torch.equal(st.is_token_in_rank[:, 0].bool(), any_on)
+        # every row where the tables say, with its token's values, scales and origin
+        rows = (first[flat[on]] + pos[on]).cuda()
+        tok = torch.arange(T).repeat_interleave(K)[on].cuda()
+        got = (comm.recv_x()[rows].float().view(-1, H // 128, 128) * comm.recv_scale()[rows][:, :, None]).view(-1, H)
+        want = x[tok].float()
+        block = want.view(-1, H // 128, 128).abs().amax(2, keepdim=True).expand(-1, -1, 128).reshape(-1, H)
+        ok = ok and bool(((got - want).abs() <= want.abs() / 16 + block / 448).all())   # e4m3: half a step of 2^-3, 2^-9 at the bottom
+        info = comm.recv_info()[rows]
+        ok = ok and torch.equal(info[:, 1].long(), tok) and torch.equal(info[:, 3].contiguous().view(torch.float32), w.view(-1)[on.cuda()])
+        comm.combine_push(torch.zeros(int(first[-1]), H, dtype=torch.bfloat16, device="cuda"), st)
+        comm.combine(st)
+        if not ok:
+            bad.append(T)
+    heap.close()
+    SymmetricHeap.shutdown()
+    return bad
+
+
+def test_dispatch_tables_and_rows_around_the_one_launch_layout():
+    url = f"127.0.0.1:{free_port()}"
+    assert run_ranks(_prepare_rank, 1, (url,), timeout=300, with_barrier=True) == [[]]
