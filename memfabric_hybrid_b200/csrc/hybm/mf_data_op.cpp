@@ -333,8 +333,8 @@ KernelBatch::KernelBatch(ComposeDataOp &op, void *userStream, uint32_t flags, ui
     uint64_t sms = std::max(1, op_.dev_->Caps().smCount);
     uint64_t chunk = AlignUp(std::max<uint64_t>(totalBytes / (sms * 8), 1), 4096);
     chunk_ = std::min(std::max<uint64_t>(chunk, 16 * kKiB), op_.chunk_);
+    first_ = op_.ringHead_;  // before a wrap: what earlier batches left in the ring has been launched by them
     if (op_.ringHead_ >= op_.ringCap_) Wrap();
-    first_ = op_.ringHead_;
 }
 
 int KernelBatch::Launch()

@@ -208,3 +208,44 @@ def _rank_56(rank, world, url, sync):
 def test_fake_device_56_bit_addresses():
     url = f"tcp://127.0.0.1:{free_port()}"
     assert run_ranks(_rank_56, 2, (url,), timeout=180, env={"MF_DEVICE_BACKEND": "fake"}, with_barrier=True) == [True, True]
+
+
+def _ring_rank(rank, world, url):
+    import memfabric_hybrid as mf
+    from memfabric_hybrid import bm
+    assert mf.initialize() == 0
+    cfg = bm.BmConfig()
+    cfg.rank_id = 0
+    cfg.start_store = True
+    assert bm.initialize(url, 1, 0, cfg) == 0, mf.get_last_err_msg()
+    h = bm.create2(id=6, local_dram_size=0, max_dram_size=0, local_hbm_size=8 * MiB, max_hbm_size=8 * MiB)
+    assert h.join() == 0, mf.get_last_err_msg()
+    base = h.peer_rank_ptr(0, bm.BmMemType.DEVICE)
+    # a ring of 1 MiB holds 43690 descriptors of 24 bytes: ten batches of 4369 pieces fill it to the last slot
+    n = 4369
+    assert (1 << 20) // 24 == 10 * n
+    src = np.random.default_rng(0).integers(0, 256, n * 16, dtype=np.uint8)
+    old = src.copy()
+    off = np.arange(n, dtype=np.uint64) * np.uint64(16)   # 8 of every 16 bytes: neighbours do not merge
+    size = np.full(n, 8, dtype=np.uint64)
+    for _ in range(10):
+        assert h.copy_data_batch(off + np.uint64(src.ctypes.data), off + np.uint64(base), size, n, bm.BmCopyType.L2G, bm.ASYNC_COPY_FLAG) == 0
+    assert h.copy_stats()["kernel_chunks"] == 10 * n
+    src[:] = 0
+    # the next batch finds the ring full: it must launch its own piece only, not what is still written in the ring
+    assert h.copy_data_batch([src.ctypes.data], [base + 4 * MiB], [16], 1, bm.BmCopyType.L2G, bm.ASYNC_COPY_FLAG) == 0
+    assert h.copy_stats()["kernel_chunks"] == 10 * n + 1
+    assert h.wait() == 0
+    got = np.zeros(n * 16, dtype=np.uint8)
+    assert h.copy_data(base, got.ctypes.data, n * 16, bm.BmCopyType.G2H, 0) == 0
+    ok = bool(np.array_equal(got.reshape(n, 16)[:, :8], old.reshape(n, 16)[:, :8]))
+    h.leave()
+    h.destroy()
+    bm.uninitialize(0)
+    mf.uninitialize()
+    return ok
+
+
+def test_a_batch_that_finds_the_descriptor_ring_full_launches_its_own_pieces_only():
+    url = f"tcp://127.0.0.1:{free_port()}"
+    assert run_ranks(_ring_rank, 1, (url,), timeout=120, env={"MF_DEVICE_BACKEND": "fake", "MF_XCOPY_RING_MB": "1"}) == [True]
