@@ -534,13 +534,18 @@ public:
                 fast = (q0.src & 15) == 0 && (q0.dst & 7) == 0 && (q0.scale & 3) == 0 && (q0.elems % 128) == 0 && q0.elems != 0;
             }
             if (fast) {
-                dim3 g2((unsigned)std::min<uint64_t>({perItem, (maxUnits + 127) / 128, 65535ull}), n);  // a CTA takes 128 units per step
+                // blocks of kQuantBlockUnits units over a grid that is resident at once; no item is cut into more parts than it
+                // takes to give every CTA sixteen blocks
+                const uint32_t resident = (uint32_t)(std::max(1, caps_.smCount) * mfk::kQuantCtasPerSm);
+                const uint32_t parts = (uint32_t)std::max<uint64_t>(
+                    1, std::min<uint64_t>((maxUnits + mfk::kQuantBlockUnits - 1) / mfk::kQuantBlockUnits, 16ull * resident / n));
+                const unsigned g2 = std::min(n * parts, resident);
                 if (inputFp16) {
-                    if (mode == 0) mfk::mf_xcopy_quant128_kernel<__half, 0><<<g2, 256, 0, st>>>(q + off);
-                    else mfk::mf_xcopy_quant128_kernel<__half, 1><<<g2, 256, 0, st>>>(q + off);
+                    if (mode == 0) mfk::mf_xcopy_quant128_kernel<__half, 0><<<g2, 256, 0, st>>>(q + off, n, parts);
+                    else mfk::mf_xcopy_quant128_kernel<__half, 1><<<g2, 256, 0, st>>>(q + off, n, parts);
                 } else {
-                    if (mode == 0) mfk::mf_xcopy_quant128_kernel<__nv_bfloat16, 0><<<g2, 256, 0, st>>>(q + off);
-                    else mfk::mf_xcopy_quant128_kernel<__nv_bfloat16, 1><<<g2, 256, 0, st>>>(q + off);
+                    if (mode == 0) mfk::mf_xcopy_quant128_kernel<__nv_bfloat16, 0><<<g2, 256, 0, st>>>(q + off, n, parts);
+                    else mfk::mf_xcopy_quant128_kernel<__nv_bfloat16, 1><<<g2, 256, 0, st>>>(q + off, n, parts);
                 }
                 RT_CHECK(cudaGetLastError(), "xcopy quant launch");
                 continue;

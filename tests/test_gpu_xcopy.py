@@ -253,3 +253,59 @@ def _shifted_rank(rank, world, url):
 def test_pieces_at_every_pair_of_byte_offsets():
     url = f"tcp://127.0.0.1:{free_port()}"
     assert run_ranks(_shifted_rank, 1, (url,), timeout=180) == [True]
+
+
+def _quant_rank(rank, world, url):
+    import torch
+    import memfabric_hybrid as mf
+    from memfabric_hybrid import bm
+    torch.cuda.set_device(0)
+    assert mf.initialize() == 0
+    cfg = bm.BmConfig()
+    cfg.rank_id = 0
+    cfg.start_store = True
+    assert bm.initialize(url, 1, 0, cfg) == 0, mf.get_last_err_msg()
+    pool = 320 * MiB
+    h = bm.create2(id=5, local_dram_size=0, max_dram_size=0, local_hbm_size=pool, max_hbm_size=pool)
+    assert h.join() == 0, mf.get_last_err_msg()
+    base = h.peer_rank_ptr(0, bm.BmMemType.DEVICE)
+    # units per item: around a half-warp's eight, a CTA's step of 128, a block of 256; then so many items that none is cut into
+    # parts and an item of 257 units is walked by the CTA that has its first block
+    plans = [[1, 2, 8, 15, 16, 17, 127, 128, 129, 255, 256, 257, 600], [257] * 7200]
+    bad = []
+    for pi, units in enumerate(plans):
+        for fp8, fp16 in ((True, False), (False, True)):
+            n = sum(units) * 128
+            g = torch.Generator("cuda").manual_seed(pi)
+            x = torch.randn(n, device="cuda", generator=g).to(torch.float16 if fp16 else torch.bfloat16)
+            x[:128] = 0    # a unit without a largest value
+            torch.cuda.synchronize()
+            first = np.concatenate(([0], np.cumsum(units)))[:-1]
+            fac = base + (n + 255) // 256 * 256 + 4 * (pi == 0)   # factors that 16-byte stores do not reach in the first plan
+            assert h.quant_copy_batch([x.data_ptr() + int(f) * 256 for f in first], [base + int(f) * 128 for f in first], [u * 256 for u in units],
+                                      [fac + int(f) * 4 for f in first], 128, fp8=fp8, fp16_input=fp16) == 0, mf.get_last_err_msg()
+            q = torch.empty(n, dtype=torch.uint8, device="cuda")
+            f = torch.empty(n // 128, device="cuda")
+            assert h.copy_data(base, q.data_ptr(), n, bm.BmCopyType.G2L, 0) == 0
+            assert h.copy_data(fac, f.data_ptr(), n // 32, bm.BmCopyType.G2L, 0) == 0
+            top = 448.0 if fp8 else 127.0
+            v = x.float().view(-1, 128)
+            amax = v.abs().amax(1, keepdim=True)
+            one = torch.ones_like(amax)
+            top = torch.full_like(amax, top)   # tensor by tensor: a division by a Python number is a product with its reciprocal
+            y = v * torch.where(amax > 0, top / amax, one)
+            want = y.to(torch.float8_e4m3fn).view(torch.uint8) if fp8 else y.round().clamp(-127, 127).to(torch.int8).view(torch.uint8)
+            if not (torch.equal(q.view(-1, 128), want) and torch.equal(f.view(-1, 1), torch.where(amax > 0, amax / top, one))):
+                bad.append((pi, fp8))
+            del x, q, v, y, want
+    h.leave()
+    h.destroy()
+    bm.uninitialize(0)
+    mf.uninitialize()
+    return bad
+
+
+def test_quantising_copy_of_items_around_its_block_sizes():
+    """The same bytes and factors as the formula in fp32 (x * (top / amax), amax / top)."""
+    url = f"tcp://127.0.0.1:{free_port()}"
+    assert run_ranks(_quant_rank, 1, (url,), timeout=300) == [[]]
