@@ -102,7 +102,8 @@ __device__ __forceinline__ void cta_convert_copy(const TS *__restrict__ src, TD 
 
 // Raw copy of [beg, end) elements of T (no conversion). Eight independent 16-byte loads are in flight per thread before the
 // first store: with one CTA of 512 threads per SM that is 64 KB per SM (four left HBM and NVLink waiting). Eight emulated ranks, 30 MB
-// of fp32 each: staged reduce-scatter 175 us with four, 134 us with eight and the rotation of by_rank below. Ends at different
+// of fp32 each: staged reduce-scatter 175 us with four, 134 us with eight and the rotation of by_rank below, 130 us
+// with a last round as wide as the others (staged all-gather of the bf16 shards 92, 84, 72 us). Ends at different
 // offsets inside a 16-byte granule go through the shifting copy.
 constexpr int kRawUnroll = 8;
 template <typename T> __device__ __forceinline__ void cta_raw_copy(const T *src, T *dst, uint64_t beg, uint64_t end)
@@ -116,14 +117,15 @@ template <typename T> __device__ __forceinline__ void cta_raw_copy(const T *src,
         vend = vbeg + (end - vbeg) / VN * VN;
         const uint64_t step = (uint64_t)blockDim.x * VN;
         uint64_t i = vbeg + (uint64_t)threadIdx.x * VN;
-        for (; i + (kRawUnroll - 1) * step < vend; i += kRawUnroll * step) {
+        for (; i < vend; i += kRawUnroll * step) {  // the last round is as wide as the others: a CTA's range is only a few rounds
             uint4 v[kRawUnroll];
 #pragma unroll
-            for (int u = 0; u < kRawUnroll; u++) v[u] = __ldcg(reinterpret_cast<const uint4 *>(src + i + u * step));
+            for (int u = 0; u < kRawUnroll; u++)
+                if (i + u * step < vend) v[u] = __ldcg(reinterpret_cast<const uint4 *>(src + i + u * step));
 #pragma unroll
-            for (int u = 0; u < kRawUnroll; u++) *reinterpret_cast<uint4 *>(dst + i + u * step) = v[u];
+            for (int u = 0; u < kRawUnroll; u++)
+                if (i + u * step < vend) *reinterpret_cast<uint4 *>(dst + i + u * step) = v[u];
         }
-        for (; i < vend; i += step) *reinterpret_cast<uint4 *>(dst + i) = __ldcg(reinterpret_cast<const uint4 *>(src + i));
     } else if ((blockDim.x & 31) == 0 && blockDim.x >= 64) {
         cta_copy_shifted<false>(reinterpret_cast<const uint8_t *>(src + beg), reinterpret_cast<uint8_t *>(dst + beg), (end - beg) * sizeof(T));
         return;
@@ -164,18 +166,16 @@ template <typename T> __device__ __forceinline__ void cta_fanout_copy(const T *s
         vend = beg + (end - beg) / VN * VN;
         const uint64_t step = (uint64_t)blockDim.x * VN;
         uint64_t i = beg + (uint64_t)threadIdx.x * VN;
-        for (; i + 3 * step < vend; i += 4 * step) {
+        for (; i < vend; i += 4 * step) {
             uint4 v[4];
 #pragma unroll
-            for (int u = 0; u < 4; u++) v[u] = __ldcs(reinterpret_cast<const uint4 *>(src + i + u * step));
+            for (int u = 0; u < 4; u++)
+                if (i + u * step < vend) v[u] = __ldcs(reinterpret_cast<const uint4 *>(src + i + u * step));
             for (uint32_t k = 0; k < ndst; k++) {
 #pragma unroll
-                for (int u = 0; u < 4; u++) *reinterpret_cast<uint4 *>(dsts[k] + i + u * step) = v[u];
+                for (int u = 0; u < 4; u++)
+                    if (i + u * step < vend) *reinterpret_cast<uint4 *>(dsts[k] + i + u * step) = v[u];
             }
-        }
-        for (; i < vend; i += step) {
-            const uint4 v = __ldcs(reinterpret_cast<const uint4 *>(src + i));
-            for (uint32_t k = 0; k < ndst; k++) *reinterpret_cast<uint4 *>(dsts[k] + i) = v;
         }
     }
     for (uint64_t i = vend + threadIdx.x; i < end; i += blockDim.x) {
