@@ -36,6 +36,7 @@
 
 #include "mf_fp8.cuh"
 #include "mf_gemm.cuh"
+#include "mf_launch.cuh"
 #include "mf_team.cuh"
 
 namespace mfk {
@@ -227,6 +228,10 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_g
             tile_start[0] = 0;
             tile_start[1] = (g.max_rows / BM) * n_tiles;
         }
+    }
+    if (MODE == 0) {
+        after_predecessor();  // barriers and descriptors were set up under the kernel in front of this one
+        start_successor();
     }
     if (MODE == 0 && warp == 2) {
         // first tile of every group, 32 groups per step (one thread walking them took over a microsecond at 32 groups)
@@ -632,11 +637,11 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_g
         // stores before thread 0, whose system fence covers them, and the counter links the CTAs' fences.
         __shared__ int last_sh;
         if (threadIdx.x == 0) {
-            __threadfence_system();
+            fence_sys();
             last_sh = g.done_count != nullptr && atomicAdd(g.done_count, 1u) + 1 == gridDim.x;
             if (last_sh) {
                 *g.done_count = 0;
-                __threadfence_system();
+                __threadfence();  // acquires what the other CTAs' fences released; the flag stores below release it to the system
             }
         }
         __syncthreads();
@@ -714,6 +719,11 @@ template <int MODE, int EPI> int launch_mx(const XArgs &g, int grid, cudaStream_
         }
         attr_set = true;
     }
+    if (MODE == 0) {
+        const cudaError_t e = launch_overlapped(kern, dim3((unsigned)grid), dim3(kXThreads), XSmem::kDynBytes, s, 1, g);
+        return e == cudaSuccess ? 0 : (int)e;
+    }
+    // a grid whose CTAs wait for the peers' (MODE 1, 2) starts when the kernel in front of it has left the SMs
     kern<<<grid, kXThreads, XSmem::kDynBytes, s>>>(g);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : (int)e;

@@ -2,7 +2,7 @@
 //
 // What bounds it: reading B once from memory. The persistent kernel of mf_gemm.cu gives one SM a whole 128 x 256 tile over all
 // of K, so a layer with N = 7168 keeps 28 SMs busy and the other 120 idle. Measured with B from memory (us, the persistent kernel's
-// better tiling / this kernel): 32 x 7168 x 8192 SwiGLU 51.3 / 28.8, 32 x 8192 x 3584 24.7 / 16.6, 16 x 1024 x 8192 43.1 / 12.4. Here a tile is 128 x 128 and the S CTAs of a cluster
+// better tiling / this kernel): 32 x 7168 x 8192 SwiGLU 51.3 / 26.0, 32 x 8192 x 3584 24.7 / 14.7, 16 x 1024 x 8192 43.1 / 10.0. Here a tile is 128 x 128 and the S CTAs of a cluster
 // each take 1/S of K into their own tensor memory; the partial sums meet through distributed shared memory (every CTA adds up
 // and stores 1/S of the tile, in CTA order: the result does not depend on timing). No workspace, no second launch.
 // Two CTAs share an SM (about 100 KB of stages each), so one CTA's prologue and reduction run under the other's loads.
@@ -14,9 +14,10 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
-#include <mutex>
+#include <cmath>
 
 #include "mf_gemm.cuh"
+#include "mf_launch.cuh"
 
 namespace mfk {
 
@@ -85,6 +86,8 @@ template <int EPI> __global__ void __launch_bounds__(kSkThreads, 2) k_gemm_bf16_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
+    after_predecessor();  // everything above ran under the kernel in front of this one
+    start_successor();
 
     // rows of B of this tile: two runs of 64
     int b0, b1;
@@ -222,45 +225,11 @@ constexpr int kSkDynBytes = kSkStageArea + 1024;
 
 template <int EPI> bool splitk_ready()
 {
-    static const bool ok = cudaFuncSetAttribute(k_gemm_bf16_splitk<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSkDynBytes) == cudaSuccess;
+    // with the carve-out that holds two CTAs per SM
+    static const bool ok = cudaFuncSetAttribute(k_gemm_bf16_splitk<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSkDynBytes) == cudaSuccess &&
+                           cudaFuncSetAttribute(k_gemm_bf16_splitk<EPI>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                                cudaSharedmemCarveoutMaxShared) == cudaSuccess;
     return ok;
-}
-
-void fill_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, int grid, int split, cudaStream_t s)
-{
-    cfg = cudaLaunchConfig_t{};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(kSkThreads);
-    cfg.dynamicSmemBytes = kSkDynBytes;
-    cfg.stream = s;
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)split;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-}
-
-// Clusters of `split` CTAs that the device holds at once (a property of the kernel and the device, asked once per size).
-int clusters_resident(int split)
-{
-    static std::mutex mu;
-    static int known[64][kSkMaxSplit + 1] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-    std::lock_guard<std::mutex> lk(mu);
-    if (known[dev][split] == 0) {
-        cudaLaunchConfig_t cfg;
-        cudaLaunchAttribute at[1];
-        fill_config(cfg, at, split, split, nullptr);
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, k_gemm_bf16_splitk<0>, &cfg) != cudaSuccess) {
-            (void)cudaGetLastError();
-            n = 0;
-        }
-        known[dev][split] = n > 0 ? n : -1;
-    }
-    return known[dev][split];
 }
 
 }  // namespace
@@ -269,7 +238,7 @@ extern "C" {
 
 // Same contract as mf_gemm_bf16_one. split: CTAs per tile (1..8), 0: chosen here.
 int mf_gemm_bf16_splitk(const void *A, const void *B, void *C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc, int *status,
-                        int swiglu, int split, void *stream)
+                        int sms, int swiglu, int split, void *stream)
 {
     if (M <= 0 || N <= 0 || K <= 0 || (K & 7) != 0 || split < 0 || split > kSkMaxSplit) return -1;
     if (swiglu && (N % 256) != 0) return -3;
@@ -292,26 +261,28 @@ int mf_gemm_bf16_splitk(const void *A, const void *B, void *C, int M, int N, int
     const int tiles = ((M + BM - 1) / BM) * ((N + kSkBN - 1) / kSkBN);
     const int k_iters = (K * 2 + KSPAN - 1) / KSPAN;
     if (split == 0) {
-        // rounds of resident clusters x steps of K per CTA; a step is worth about 1/8 of the fixed cost of one more CTA per
-        // tile (exchange through distributed shared memory)
+        // Cost in steps of K (64 elements of a 128 x 128 tile), for rounds of resident clusters (two CTAs per SM, a tenth lost to
+        // clusters that do not fit a GPC's rest): a round takes K / s steps, or what memory takes for all tiles' steps (about 1.2
+        // steps per SM at a time); every CTA of a tile adds its exchange, which grows with the rows and with how many CTAs
+        // exchange at once. Measured (us for s = 1, 2, 4, 8): 32 x 7168 x 8192 35.8, 27.3, 26.0, 37.7; 16 x 1024 x 8192 31.5, 18.7,
+        // 12.1, 10.0; 256 x 7168 x 8192 52.4, 38.6, 54.6; 1024 x 1024 x 4096 25.4, 16.8, 19.5, 40.2.
+        const int n = sms > 0 ? sms : 148;
+        const double memory = (double)tiles * k_iters / (1.2 * n);
         double best = 0;
-        for (int s = 1; s <= kSkMaxSplit && s <= k_iters; s++) {
-            const int res = clusters_resident(s);
-            if (res <= 0) continue;
-            const double cost = (double)((tiles + res - 1) / res) * ((k_iters + s - 1) / s + 8) + s;
+        for (int s = 1; s <= kSkMaxSplit && s <= k_iters; s *= 2) {  // clusters of 3, 5, 6 leave more of a GPC unused: slower throughout
+            const double resident = s == 1 ? 2.0 * n : 1.8 * n / s;
+            const double rounds = std::ceil(tiles / std::max(1.0, std::floor(resident)));
+            const double busy = std::min(1.0, (double)tiles * s / (2.0 * n));
+            const double cost = std::max(rounds * ((k_iters + s - 1) / s), memory) + 8 + s * (1 + 4.0 * g.box_rows / BM * busy);
             if (split == 0 || cost < best) {
                 best = cost;
                 split = s;
             }
         }
-        if (split == 0) return -4;
     }
     if (split > k_iters) return -1;
-    cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute at[1];
-    fill_config(cfg, at, tiles * split, split, (cudaStream_t)stream);
-    cudaError_t e = swiglu ? cudaLaunchKernelEx(&cfg, k_gemm_bf16_splitk<1>, g) : cudaLaunchKernelEx(&cfg, k_gemm_bf16_splitk<0>, g);
-    if (e != cudaSuccess) (void)cudaGetLastError();
+    const cudaError_t e = launch_overlapped(swiglu ? k_gemm_bf16_splitk<1> : k_gemm_bf16_splitk<0>, dim3((unsigned)(tiles * split)), dim3(kSkThreads),
+                                            kSkDynBytes, (cudaStream_t)stream, (unsigned)split, g);
     return e == cudaSuccess ? 0 : (int)e;
 }
 

@@ -1,0 +1,43 @@
+// Launches whose start overlaps the end of the kernel in front of them on the stream (programmatic dependent launch): the
+// CTAs set up barriers, tensor memory and descriptors while the predecessor drains, then call after_predecessor() in front
+// of the first access to memory that an earlier kernel may have written or may still read. The call returns when the
+// predecessor has completed and its writes are visible. start_successor() afterwards lets the next kernel launched this way
+// do the same; a kernel that never calls it is simply not overlapped, and a launch without the attribute makes both no-ops.
+// Every kernel launched like this calls after_predecessor() before it ends (by every thread that touches global memory), so
+// the end of a kernel still means the end of everything in front of it.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <utility>
+
+namespace mfk {
+
+__device__ __forceinline__ void after_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void start_successor() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... A>
+cudaError_t launch_overlapped(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, unsigned cluster, A &&...args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = 1;
+    if (cluster > 1) {
+        at[1].id = cudaLaunchAttributeClusterDimension;
+        at[1].val.clusterDim.x = cluster;
+        at[1].val.clusterDim.y = 1;
+        at[1].val.clusterDim.z = 1;
+        cfg.numAttrs = 2;
+    }
+    cfg.attrs = at;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    return e;
+}
+
+}  // namespace mfk

@@ -23,6 +23,7 @@
 
 #include "mf_devtrace.cuh"
 #include "mf_fp8.cuh"
+#include "mf_launch.cuh"
 #include "mf_team.cuh"
 
 namespace mfk {
@@ -228,6 +229,8 @@ __global__ void __launch_bounds__(1024) k_moe_prepare(Team team, MoeHeap hp, con
     __shared__ int running[1024], per_rank[kMaxRanks];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int n = T * K, W = (int)team.world, El = E / W;
+    after_predecessor();
+    start_successor();
     for (int x = threadIdx.x; x < E; x += blockDim.x) running[x] = 0;
     if (threadIdx.x < kMaxRanks) per_rank[threadIdx.x] = 0;
     for (int base = 0; base < n; base += 1024) {
@@ -314,19 +317,18 @@ __device__ __forceinline__ bool finish_dispatch(const DispatchArgs &a, uint32_t 
     __shared__ int last_sh;
     __syncthreads();
     if (threadIdx.x == 0) {
-        __threadfence_system();
+        fence_sys();
         const uint32_t done = atomicAdd(a.done_count, 1u) + 1;
         // seq > 0: the counter only grows and the host numbers the calls; seq == 0: the last CTA puts it back
         // to zero, so the same launch parameters work again (CUDA-graph replay)
         const bool last = a.seq != 0 ? done == gridDim.x * a.seq : done == gridDim.x;
         if (last) {
             if (a.seq == 0) *a.done_count = 0;
-            __threadfence_system();
+            __threadfence();  // acquires what the other CTAs' fences released; the flag stores below release it to the system
         }
         last_sh = last ? 1 : 0;
     }
     __syncthreads();
-    // (the fence by thread 0 and the CTA barrier order everything in front of these stores)
     if (last_sh && threadIdx.x < t.world)
         st_release_sys(reinterpret_cast<uint32_t *>(peer_ptr(t, threadIdx.x, a.hp.flags)) + me, a.epoch);
     return last_sh != 0;
@@ -502,6 +504,8 @@ __global__ void __launch_bounds__(kDwWarps * 32) k_moe_dispatch_warp(DispatchArg
     // neighbouring tokens go to different SMs: a small batch uses every SM's path to memory
     const int wid = warp * (int)gridDim.x + (int)blockIdx.x, wtotal = (int)gridDim.x * kDwWarps;
     const bool smoothed = a.smooth != nullptr;
+    after_predecessor();
+    start_successor();
     for (int tok = wid; tok < a.sh.T; tok += wtotal) {
         // routing of this token: lane k resolves destination k (two dependent loads, overlapped with the row loads below)
         int d_rank = -1, d_pos = 0;
@@ -600,6 +604,8 @@ __global__ void __launch_bounds__(kDwWarps * 32) k_moe_dispatch_warp(DispatchArg
 __global__ void __launch_bounds__(448) k_moe_dispatch(DispatchArgs a)
 {
     uint4 lo, hi;
+    after_predecessor();
+    start_successor();
     dispatch_preload(a, lo, hi);
     dispatch_body(a, lo, hi);
 }
@@ -607,6 +613,8 @@ __global__ void __launch_bounds__(448) k_moe_dispatch(DispatchArgs a)
 // Waits until every rank raised flag row `which` (0 dispatch, 1 combine) to `epoch`.
 __global__ void k_moe_wait_all(Team t, MoeHeap hp, int which, uint32_t epoch, int *status)
 {
+    after_predecessor();
+    start_successor();
     const uint32_t me = team_rank(t);
     if (threadIdx.x < t.world) {
         const uint32_t *f = reinterpret_cast<const uint32_t *>(peer_ptr(t, me, hp.flags)) + which * kMaxRanks + threadIdx.x;
@@ -633,6 +641,8 @@ __device__ __forceinline__ void combine_reduce_body(const Team &t, const MoeHeap
                                                     const float *topk_w);
 __global__ void __launch_bounds__(256, 4) k_moe_combine_reduce(Team t, MoeHeap hp, MoeShape sh, const int *topk_idx, __nv_bfloat16 *out)
 {
+    after_predecessor();
+    start_successor();
     combine_reduce_body(t, hp, sh, topk_idx, out, nullptr);
 }
 
@@ -862,12 +872,12 @@ __global__ void __launch_bounds__(256) k_moe_ll_combine(LLCombineArgs a)
     __shared__ int last_sh;
     __syncthreads();
     if (threadIdx.x == 0) {
-        __threadfence_system();
+        fence_sys();
         const uint32_t done = atomicAdd(a.done_count, 1u) + 1;
         last_sh = done == gridDim.x ? 1 : 0;
         if (done == gridDim.x) {
             *a.done_count = 0;
-            __threadfence_system();
+            __threadfence();  // as in finish_dispatch
         }
     }
     __syncthreads();
@@ -962,10 +972,9 @@ int mf_moe_prepare(const Team *team, const MoeHeap *hp, const int *topk_idx, int
     if (T * K > kPrepareMax) return -3;
     static const bool ok = cudaFuncSetAttribute(k_moe_prepare, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * 1024 * 2) == cudaSuccess;
     if (!ok) return -2;
-    k_moe_prepare<<<1, 1024, 32 * E * sizeof(uint16_t), (cudaStream_t)stream>>>(*team, *hp, topk_idx, T, K, E, tokens_per_expert, tokens_per_rank,
-                                                                                send_idx, is_token_in_rank, recv_per_expert, row_off, put_off,
-                                                                                src_off, epoch);
-    cudaError_t e = cudaGetLastError();
+    const cudaError_t e = launch_overlapped(k_moe_prepare, dim3(1), dim3(1024), 32 * E * sizeof(uint16_t), (cudaStream_t)stream, 1, *team, *hp, topk_idx, T,
+                                            K, E, tokens_per_expert, tokens_per_rank, send_idx, is_token_in_rank, recv_per_expert, row_off,
+                                            put_off, src_off, epoch);
     return e == cudaSuccess ? 0 : (int)e;
 }
 
@@ -987,19 +996,16 @@ int mf_moe_dispatch(const DispatchArgs *a, int ctas, void *stream)
             }
             attr_for = smem;
         }
-        k_moe_dispatch_warp<<<ctas, kDwWarps * 32, smem, (cudaStream_t)stream>>>(*a);
-        cudaError_t e = cudaGetLastError();
+        const cudaError_t e = launch_overlapped(k_moe_dispatch_warp, dim3((unsigned)ctas), dim3(kDwWarps * 32), (size_t)smem, (cudaStream_t)stream, 1, *a);
         return e == cudaSuccess ? 0 : (int)e;
     }
-    k_moe_dispatch<<<ctas, 448, 0, (cudaStream_t)stream>>>(*a);
-    cudaError_t e = cudaGetLastError();
+    const cudaError_t e = launch_overlapped(k_moe_dispatch, dim3((unsigned)ctas), dim3(448), 0, (cudaStream_t)stream, 1, *a);
     return e == cudaSuccess ? 0 : (int)e;
 }
 
 int mf_moe_wait_all(const Team *team, const MoeHeap *hp, int which, uint32_t epoch, int *status, void *stream)
 {
-    k_moe_wait_all<<<1, 32, 0, (cudaStream_t)stream>>>(*team, *hp, which, epoch, status);
-    cudaError_t e = cudaGetLastError();
+    const cudaError_t e = launch_overlapped(k_moe_wait_all, dim3(1), dim3(32), 0, (cudaStream_t)stream, 1, *team, *hp, which, epoch, status);
     return e == cudaSuccess ? 0 : (int)e;
 }
 
@@ -1013,8 +1019,8 @@ int mf_moe_signal_all(const Team *team, const MoeHeap *hp, int which, uint32_t e
 int mf_moe_combine_reduce(const Team *team, const MoeHeap *hp, const MoeShape *sh, const int *topk_idx, void *out, int ctas, void *stream)
 {
     if (sh->H % 8 != 0) return -1;
-    k_moe_combine_reduce<<<ctas, 256, 0, (cudaStream_t)stream>>>(*team, *hp, *sh, topk_idx, static_cast<__nv_bfloat16 *>(out));
-    cudaError_t e = cudaGetLastError();
+    const cudaError_t e = launch_overlapped(k_moe_combine_reduce, dim3((unsigned)ctas), dim3(256), 0, (cudaStream_t)stream, 1, *team, *hp, *sh, topk_idx,
+                                            static_cast<__nv_bfloat16 *>(out));
     return e == cudaSuccess ? 0 : (int)e;
 }
 

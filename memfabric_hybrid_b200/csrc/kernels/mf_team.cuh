@@ -72,6 +72,10 @@ __device__ __forceinline__ uint32_t ld_relaxed_sys(const uint32_t *p)
     return v;
 }
 
+// Orders this thread's (and, behind a CTA barrier, its CTA's) accesses for observers on every GPU: release and acquire, which is
+// all that a counter or a flag behind it needs. (__threadfence_system() is the sequentially consistent fence.)
+__device__ __forceinline__ void fence_sys() { asm volatile("fence.acq_rel.sys;" ::: "memory"); }
+
 __device__ __forceinline__ void report_timeout(const Team &t, uint32_t me, uint32_t where, uint32_t epoch)
 {
     uint32_t *st = reinterpret_cast<uint32_t *>(peer_ptr(t, me, kStatusOff));

@@ -28,7 +28,7 @@ def _cu():
             fn.argtypes = l.mf_gemm_bf16.argtypes
         l.mf_gemm_bf16_splitk.restype = C.c_int
         l.mf_gemm_bf16_splitk.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int64, C.c_int64, C.c_int64,
-                                          C.c_void_p, C.c_int, C.c_int, C.c_void_p]
+                                          C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p]
         _lib = l
     return _lib
 

@@ -54,7 +54,7 @@ def test_gemm_bf16_split_over_a_cluster(M, N, K, split):
     b = (torch.randn(N, K, device="cuda") * 0.05).to(torch.bfloat16)
     ld = N + (8 if split % 2 else 3)   # rows of C that 16-byte stores reach, and rows that they do not
     c = torch.full((M, ld), 7.0, device="cuda", dtype=torch.bfloat16)
-    assert gemm._cu().mf_gemm_bf16_splitk(a.data_ptr(), b.data_ptr(), c.data_ptr(), M, N, K, K, K, ld, gemm.status_word().data_ptr(), 0, split,
+    assert gemm._cu().mf_gemm_bf16_splitk(a.data_ptr(), b.data_ptr(), c.data_ptr(), M, N, K, K, K, ld, gemm.status_word().data_ptr(), gemm.sm_count(), 0, split,
                                           torch.cuda.current_stream().cuda_stream) == 0
     torch.cuda.synchronize()
     gemm.check_status()
@@ -77,3 +77,30 @@ def test_gemm_bf16_swiglu_few_rows(M, F, K):
     gemm.check_status()
     # both round the same fp32 value once; the sums differ by K 2^-24 of their terms, which SwiGLU scales by about |up|
     assert ((c.float() - one.float()).norm() / one.float().norm()).item() <= 2.0 ** -8
+
+
+@pytest.mark.parametrize("M", [32, 4096])
+def test_gemm_bf16_in_a_cuda_graph(M):
+    """Two products in a row, captured: the second may start under the end of the first (few rows) and must still see all of it."""
+    from memfabric_hybrid_b200.ops import gemm
+    torch.manual_seed(M)
+    a = torch.randn(M, 2048, device="cuda").to(torch.bfloat16)
+    w1 = (torch.randn(4096, 2048, device="cuda") * 0.05).to(torch.bfloat16)
+    w2 = (torch.randn(2048, 4096, device="cuda") * 0.05).to(torch.bfloat16)
+    h, y = torch.empty(M, 4096, device="cuda", dtype=torch.bfloat16), torch.empty(M, 2048, device="cuda", dtype=torch.bfloat16)
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        gemm.gemm_bf16(gemm.gemm_bf16(a, w1, out=h), w2, out=y)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        gemm.gemm_bf16(gemm.gemm_bf16(a, w1, out=h), w2, out=y)
+    for i in range(3):
+        a.copy_(torch.randn(M, 2048, device="cuda").to(torch.bfloat16))
+        g.replay()
+        torch.cuda.synchronize()
+        gemm.check_status()
+        ref = h.float() @ w2.float().t()
+        assert ((h.float() - a.float() @ w1.float().t()).norm() / h.float().norm()).item() <= 2.0 ** -8
+        assert ((y.float() - ref).norm() / ref.norm()).item() <= 2.0 ** -8
