@@ -666,38 +666,9 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_g
             __syncthreads();
             if (!ok_sh) break;
             const int ml = t / n_tiles, nt = t % n_tiles;
-            constexpr int kVecRow = XBN / 8;
-            for (int v = threadIdx.x; v < BM * kVecRow; v += blockDim.x) {
-                const int lr = ml * BM + v / kVecRow;
-                const int col = nt * XBN + (v % kVecRow) * 8;
-                float accv[8];
-#pragma unroll
-                for (int e = 0; e < 8; e++) accv[e] = 0.f;
-                // partials are fetched eight at a time (independent loads in flight), added in rank order
-                for (uint32_t s0 = 0; s0 < g.team.world; s0 += 8) {
-                    uint4 raw[8];
-#pragma unroll
-                    for (int u = 0; u < 8; u++)
-                        if (s0 + u < g.team.world)
-                            raw[u] = __ldcg(reinterpret_cast<const uint4 *>(land + ((int64_t)(s0 + u) * g.rows_per_rank + lr) * g.N + col));
-#pragma unroll
-                    for (int u = 0; u < 8; u++) {
-                        if (s0 + u >= g.team.world) continue;
-                        const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&raw[u]);
-#pragma unroll
-                        for (int e = 0; e < 4; e++) {
-                            const float2 f = __bfloat1622float2(h[e]);
-                            accv[2 * e] += f.x;
-                            accv[2 * e + 1] += f.y;
-                        }
-                    }
-                }
-                uint4 pk;
-                __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(&pk);
-#pragma unroll
-                for (int e = 0; e < 4; e++) h[e] = __floats2bfloat162_rn(accv[2 * e] * g.scale, accv[2 * e + 1] * g.scale);
-                *reinterpret_cast<uint4 *>(g.y_out + (int64_t)lr * g.ldy + col) = pk;
-            }
+            const int64_t at = (int64_t)ml * BM * g.N + nt * XBN;
+            add_partials(land + at, (int64_t)g.rows_per_rank * g.N, g.N, XBN / 8, (int)g.team.world, g.scale,
+                         g.y_out + (int64_t)ml * BM * g.ldy + nt * XBN, g.ldy);
             __syncthreads();
         }
     }

@@ -134,3 +134,24 @@ def test_tp_mlp_fp8_multi_gpu():
     res = run_ranks(_ranks_fp8, n, (url, 1024, 1024, 2048), timeout=300, with_barrier=True)
     for worst, st in res:
         assert st == 0 and worst < 3e-2, res
+
+
+@pytest.mark.parametrize("world", [1, 2, 3, 4, 8, 11, 16])
+@pytest.mark.parametrize("vec_row,threads", [(32, 384), (32, 192), (1, 192), (13, 384)])
+def test_partial_tiles_are_added_in_rank_order(world, vec_row, threads):
+    """The reduction behind GEMM -> reduce-scatter for every number of ranks: fp32 sums in rank order, one rounding at the end."""
+    import ctypes as C
+    from memfabric_hybrid_b200 import _native as N
+    torch.manual_seed(world * 100 + vec_row)
+    f = N.cuda().mf_gemm_rs_reduce_probe
+    f.restype, f.argtypes = C.c_int, [C.c_void_p, C.c_int64, C.c_int64, C.c_int, C.c_int, C.c_float, C.c_void_p, C.c_int64, C.c_int, C.c_void_p]
+    cols, ld, ldo = vec_row * 8, vec_row * 8 + 16, vec_row * 8 + 8
+    land = torch.randn(world, 128, ld, device="cuda").to(torch.bfloat16)
+    out = torch.full((128, ldo), 5.0, device="cuda", dtype=torch.bfloat16)
+    assert f(land.data_ptr(), 128 * ld, ld, vec_row, world, 0.375, out.data_ptr(), ldo, threads, torch.cuda.current_stream().cuda_stream) == 0
+    acc = torch.zeros(128, cols, device="cuda")
+    for r in range(world):
+        acc += land[r, :, :cols].float()
+    torch.cuda.synchronize()
+    assert torch.equal(out[:, :cols], (acc * 0.375).to(torch.bfloat16))
+    assert bool((out[:, cols:] == 5.0).all())
