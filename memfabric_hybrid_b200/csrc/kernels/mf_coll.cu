@@ -154,28 +154,28 @@ template <int W> __device__ __forceinline__ void by_rank(uint4 (&v)[W], uint32_t
 
 // One source range to several destinations (all-gather, broadcast): every 16-byte vector is loaded ONCE, four
 // independent loads in flight per thread, and stored to each destination in turn, so that all peers fill at the same
-// time and the source is not re-read per peer. Same element type on both sides, no scaling; falls back to
-// element-wise copies when an address is not 16-byte aligned.
+// time and the source is not re-read per peer. Same element type on both sides, no scaling; where an address is not 16-byte
+// aligned every destination is a copy of its own (whole vectors, shifted).
 template <typename T> __device__ __forceinline__ void cta_fanout_copy(const T *src, T *const *dsts, uint32_t ndst, uint64_t beg, uint64_t end)
 {
     constexpr int VN = 16 / sizeof(T);
     bool al = aligned16(src + beg);
     for (uint32_t k = 0; k < ndst; k++) al = al && aligned16(dsts[k] + beg);
-    uint64_t vend = beg;
-    if (al) {
-        vend = beg + (end - beg) / VN * VN;
-        const uint64_t step = (uint64_t)blockDim.x * VN;
-        uint64_t i = beg + (uint64_t)threadIdx.x * VN;
-        for (; i < vend; i += 4 * step) {
-            uint4 v[4];
+    if (!al) {
+        for (uint32_t k = 0; k < ndst; k++) cta_raw_copy<T>(src, dsts[k], beg, end);
+        return;
+    }
+    const uint64_t vend = beg + (end - beg) / VN * VN;
+    const uint64_t step = (uint64_t)blockDim.x * VN;
+    for (uint64_t i = beg + (uint64_t)threadIdx.x * VN; i < vend; i += 4 * step) {
+        uint4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (i + u * step < vend) v[u] = __ldcs(reinterpret_cast<const uint4 *>(src + i + u * step));
+        for (uint32_t k = 0; k < ndst; k++) {
 #pragma unroll
             for (int u = 0; u < 4; u++)
-                if (i + u * step < vend) v[u] = __ldcs(reinterpret_cast<const uint4 *>(src + i + u * step));
-            for (uint32_t k = 0; k < ndst; k++) {
-#pragma unroll
-                for (int u = 0; u < 4; u++)
-                    if (i + u * step < vend) *reinterpret_cast<uint4 *>(dsts[k] + i + u * step) = v[u];
-            }
+                if (i + u * step < vend) *reinterpret_cast<uint4 *>(dsts[k] + i + u * step) = v[u];
         }
     }
     for (uint64_t i = vend + threadIdx.x; i < end; i += blockDim.x) {
