@@ -134,4 +134,8 @@ __device__ __forceinline__ void add_partials(const __nv_bfloat16 *land, int64_t 
 int make_tmap_2d(CUtensorMap *out, const void *base, int elem_bytes, uint64_t rows, uint64_t cols, uint64_t row_stride_bytes,
                  uint32_t box_rows, bool is_fp8);
 
+// Host: 5-D tensor map over a row-major fp8 [rows, cols] matrix whose rows alternate in runs of 128 of two kinds (gate, up). A box is 64
+// rows of each kind in turns of 16: coordinates (column, 0, 0, first 16-row run inside the 128, block of 256 rows), 128B swizzle.
+int make_tmap_runs16(CUtensorMap *out, const void *base, uint64_t rows, uint64_t cols);
+
 }  // namespace mfk

@@ -1,9 +1,8 @@
-// Grouped expert GEMM in fp8 e4m3 whose block scales are applied by the tensor core itself
+// The two tensor-parallel fusions in fp8 e4m3, whose block scales are applied by the tensor core itself
 // (tcgen05.mma kind::mxf8f6f4.block_scale): the whole K loop of a tile accumulates in ONE TMEM buffer and
-// nothing is pulled out of TMEM per K block.
+// nothing is pulled out of TMEM per K block. (The grouped expert GEMM is in mf_gemm_fp8_pair.cu.)
 //   activations A [rows, K] fp8, one power-of-two fp32 scale per row per 128 elements of K      (1 x 128)
-//   weights     B [experts, N, K] fp8, one power-of-two fp32 scale per 128 x 128 block          (128 x 128)
-//   rows grouped by expert: group g owns rows [row_off[g], row_off[g+1]) (device array, no host sync)
+//   weights     B [N, K] fp8, one power-of-two fp32 scale per 128 x 128 block                   (128 x 128)
 // The scales must be powers of two (every quantiser of this library produces such scales): a producer
 // warp turns them into UE8M0 bytes (the fp32 exponent) in the tensor core's scale layout in shared
 // memory, four K blocks per 32-bit word; the MMA thread copies a group of them into TMEM (tcgen05.cp)
@@ -14,14 +13,12 @@
 // The epilogue warps first move their part of the accumulator into registers and hand TMEM back, so the
 // next tile's MMAs overlap the epilogue arithmetic and stores.
 // Epilogues:
-//   EPI 0  plain            : bf16 rows to local memory
+//   EPI 0  plain            : bf16 rows (MODE 2: to the owner's landing zone)
 //   EPI 1  gate/up + SwiGLU : B is tile-interleaved (128 gate rows, 128 up rows per 256); out[row, 128 cols] bf16
-//   EPI 2  down + combine   : row x routing weight stored straight into the combine slot of the token's home
-//                             rank (peer stores over NVLink)
 //   EPI 3  gate/up + SwiGLU + re-quantisation: the 128 outputs of a tile row are one 1 x 128 block of the next
 //                             GEMM's fp8 input: amax, power-of-two scale, e4m3 bytes and the scale are written
 //                             here, so the activation never exists in bf16 in memory
-// The same mainloop also runs the two tensor-parallel fusions on dense operands (MODE 1 / MODE 2):
+// Modes:
 //   MODE 1  all-gather -> GEMM : warps 3..11 of every CTA quantise its rows of this rank's bf16 sequence shard to
 //                                fp8 + 1 x 128 scales into the rank's own gather buffer (first, so the first
 //                                tiles can start), then warp 3 copies those bytes into every peer's gather buffer,
@@ -30,13 +27,10 @@
 //   MODE 2  GEMM -> reduce-scatter : the epilogue stores each partial tile (bf16) into the landing zone of the
 //                                rank that owns the rows and counts it there; after its tiles a CTA adds up
 //                                the landed partials of the tiles it owns.
-// Parity of role: app/zbal/doc/fused_deep_moe.md:106-127,213-281 (GMM1 -> dequant + SwiGLU + dynamic re-quant
-// -> GMM2 -> combine) of the reference.
 #include <cuda_bf16.h>
 
 #include "mf_fp8.cuh"
 #include "mf_gemm.cuh"
-#include "mf_launch.cuh"
 #include "mf_team.cuh"
 
 namespace mfk {
@@ -45,7 +39,6 @@ constexpr int XBN = 256;
 constexpr int XSTAGES = 4;
 constexpr int XSFBUFS = 4;
 constexpr int kXThreads = 384;
-constexpr int kXMaxGroups = 64;
 constexpr int kXTmemCols = 512;
 constexpr uint32_t kXSfaCol = 256;  // TMEM columns [256, 260): scales of A; [260, 268): scales of B
 constexpr uint32_t kXSfbCol = 260;
@@ -83,22 +76,16 @@ struct XSmem {
 static_assert(XSmem::kDynBytes <= 227 * 1024, "shared memory of the block-scaled fp8 GEMM");
 
 struct XArgs {
-    TmaPair tm;            // A: [rows, K] fp8; B: [G * N, K] fp8
+    TmaPair tm;            // A: [rows, K] fp8; B: [N, K] fp8
     const float *a_scale;  // [rows, K/128]
-    const float *b_scale;  // [G, N/128, K/128]  (N in ORIGINAL row order: for EPI 1/3 gate rows then up rows)
-    const int *row_off;    // [G + 1] device
-    int G, N, K;
+    const float *b_scale;  // [N/128, K/128]  (N in ORIGINAL row order: for EPI 1/3 gate rows then up rows)
+    int N, K;
     int max_rows;
     void *out;             // EPI 0/1: bf16; EPI 3: e4m3 bytes
     int64_t ldo;           // elements per output row
     float *out_scale;      // EPI 3: [rows, N/256]
     int *status;
-    Team team;             // EPI 2, MODE 1, MODE 2
-    const int4 *recv_info;
-    uint64_t comb_off;
-    int topk;
-    uint32_t *done_count;  // EPI 2, optional: local counter of finished CTAs, zero between launches
-    uint64_t flag_off;     // EPI 2: slot offset of the flag row that the last CTA raises to `epoch` on every peer
+    Team team;
     uint32_t epoch;        // flag value of this call (grows by one per call)
     uint32_t seq;          // MODE 1: number of fused calls so far on these counters, including this one
     // MODE 1
@@ -195,12 +182,10 @@ __device__ __noinline__ void ag_quant_rows(const XArgs &g, uint32_t me, int wq, 
     }
 }
 
-template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_grouped_fp8_mx(const __grid_constant__ XArgs g)
+template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_tp_fp8_mx(const __grid_constant__ XArgs g)
 {
     extern __shared__ uint8_t smem_raw[];
     XSmem sm(smem_raw);
-    __shared__ int tile_start[kXMaxGroups + 1];
-    __shared__ int s_row_off[kXMaxGroups + 1];
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int n_tiles = g.N / XBN;
@@ -223,41 +208,6 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_g
         mbar_fence_init();
         tma_prefetch_desc(&g.tm.a);
         tma_prefetch_desc(&g.tm.b);
-        if (MODE != 0) {
-            s_row_off[0] = 0;
-            s_row_off[1] = g.max_rows;
-            tile_start[0] = 0;
-            tile_start[1] = (g.max_rows / BM) * n_tiles;
-        }
-    }
-    // Barriers and descriptors were set up under the kernel in front of this one. The kernel behind it gets no early start, which gains
-    // nothing in a decode batch and costs in a prefill batch (its CTAs would take SMs in the order in which these become free;
-    // presumably neighbouring tiles then share less in the L2). MoE layer, early start / none, us: 128 tokens 303.5 / 303.4, 512:
-    // 388 / 385, 1024: 575 / 559, 4096: 1634 / 1578.
-    if (MODE == 0) after_predecessor();
-    if (MODE == 0 && warp == 2) {
-        // first tile of every group, 32 groups per step (one thread walking them took over a microsecond at 32 groups)
-        int run = 0;
-        for (int i0 = 0; i0 < g.G; i0 += 32) {
-            const int i = i0 + lane;
-            int lo = 0, hi = 0;
-            if (i < g.G) {
-                lo = min(g.row_off[i], g.max_rows);
-                hi = min(g.row_off[i + 1], g.max_rows);
-                s_row_off[i] = lo;
-                if (i == g.G - 1) s_row_off[g.G] = hi;
-            }
-            const int n = ((hi - lo + BM - 1) / BM) * n_tiles;
-            int upto = n;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int below = __shfl_up_sync(0xffffffffu, upto, o);
-                if (lane >= o) upto += below;
-            }
-            if (i < g.G) tile_start[i] = run + upto - n;
-            run += __shfl_sync(0xffffffffu, upto, 31);
-        }
-        if (lane == 0) tile_start[g.G] = run;
     }
     if (warp == 1) {
         tmem_alloc(sm.tmem_slot(), kXTmemCols);
@@ -267,34 +217,20 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_g
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *sm.tmem_slot();
-    const int total = tile_start[MODE == 0 ? g.G : 1];
+    const int total = (g.max_rows / BM) * n_tiles;
     const uint32_t me = g.team.rank;
 
-    // linear tile -> (group, first row, row limit, column tile); inside a group the row tile varies fastest
-    auto locate = [&](int t, int &grp, int &row0, int &row_end, int &nt) {
-        if (MODE != 0) {
-            // blocks of rows owned by one rank, visited starting with this rank (MODE 1: the order in which the shards
-            // arrive) or with the next rank (MODE 2: remote owners first, own rows last)
-            const int rows = MODE == 1 ? g.shard_rows : g.rows_per_rank;
-            const int mt_per = rows / BM;
-            const int per_block = mt_per * n_tiles;
-            const int i = t / per_block;
-            const int owner = (int)((me + (MODE == 2 ? 1 : 0) + i) % g.team.world);
-            const int r = t - i * per_block;
-            grp = 0;
-            nt = r / mt_per;
-            row0 = (owner * mt_per + r % mt_per) * BM;
-            row_end = g.max_rows;
-            return;
-        }
-        int lo = 0;
-        while (lo + 1 < g.G && tile_start[lo + 1] <= t) lo++;
-        grp = lo;
-        const int local = t - tile_start[lo];
-        const int mt_cnt = (s_row_off[lo + 1] - s_row_off[lo] + BM - 1) / BM;
-        nt = local / mt_cnt;
-        row0 = s_row_off[lo] + (local % mt_cnt) * BM;
-        row_end = s_row_off[lo + 1];
+    // linear tile -> (first row, column tile): blocks of rows owned by one rank, visited starting with this rank (MODE 1: the order in
+    // which the shards arrive) or with the next rank (MODE 2: remote owners first, own rows last); inside a block the row tile varies fastest
+    auto locate = [&](int t, int &row0, int &nt) {
+        const int rows = MODE == 1 ? g.shard_rows : g.rows_per_rank;
+        const int mt_per = rows / BM;
+        const int per_block = mt_per * n_tiles;
+        const int i = t / per_block;
+        const int owner = (int)((me + (MODE == 2 ? 1 : 0) + i) % g.team.world);
+        const int r = t - i * per_block;
+        nt = r / mt_per;
+        row0 = (owner * mt_per + r % mt_per) * BM;
     };
 
     if (MODE == 1 && warp >= 3) {
@@ -307,8 +243,8 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_g
             PipeState ps;
             bool fine = true;
             for (int t = blockIdx.x; t < total && fine; t += gridDim.x) {
-                int grp, row0, row_end, nt;
-                locate(t, grp, row0, row_end, nt);
+                int row0, nt;
+                locate(t, row0, nt);
                 if (MODE == 1) {
                     // the shard holding this tile's rows must have landed in this GPU's gather buffer
                     const uint32_t *ready = reinterpret_cast<const uint32_t *>(peer_ptr(g.team, me, g.ag_ready_off)) + row0 / g.shard_rows;
@@ -324,7 +260,7 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_g
                     if (!fine) break;
                     mbar_expect_tx(sm.full(ps.stage), XSmem::kStageBytes);
                     tma_load_2d(sm.a(ps.stage), &g.tm.a, kb * 128, row0, sm.full(ps.stage));
-                    tma_load_2d(sm.b(ps.stage), &g.tm.b, kb * 128, grp * g.N + nt * XBN, sm.full(ps.stage));
+                    tma_load_2d(sm.b(ps.stage), &g.tm.b, kb * 128, nt * XBN, sm.full(ps.stage));
                     ps.advance<XSTAGES>();
                 }
             }
@@ -375,8 +311,8 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_g
         const int nblocks = g.N / 128;
         bool fine = true;
         for (int t = blockIdx.x; t < total && fine; t += gridDim.x) {
-            int grp, row0, row_end, nt;
-            locate(t, grp, row0, row_end, nt);
+            int row0, nt;
+            locate(t, row0, nt);
             int nb0, nb1;
             if (EPI == 1 || EPI == 3) {
                 nb0 = nt;                  // gate rows nt * 128 .. + 128
@@ -385,8 +321,8 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_g
                 nb0 = 2 * nt;
                 nb1 = 2 * nt + 1;
             }
-            const float *bs0 = g.b_scale + ((int64_t)grp * nblocks + nb0) * k_blocks;
-            const float *bs1 = g.b_scale + ((int64_t)grp * nblocks + nb1) * k_blocks;
+            const float *bs0 = g.b_scale + (int64_t)nb0 * k_blocks;
+            const float *bs1 = g.b_scale + (int64_t)nb1 * k_blocks;
             if (MODE == 1) {
                 // the scales of a shard arrive with its rows
                 int ok = 1;
@@ -428,8 +364,7 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_g
 #pragma unroll
                     for (int j = 0; j < 4; j++) {
                         const int kb = gq * 4 + j;
-                        // MODE 1: written by peers during this kernel, so past L1. MODE 0: complete since after_predecessor(), but
-                        // this kernel may have been there before that (mf_launch.cuh), so not through the read-only path either
+                        // MODE 1: written by peers during this kernel, so past L1
                         w |= (kb < k_blocks ? ue8m0_byte(MODE == 1 ? __ldcg(as + kb) : as[kb]) : 127u) << (8 * j);
                     }
                     wa[r1] = w;
@@ -452,10 +387,10 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_g
         uint8_t *stg = sm.out_stage(warp - 4);
         constexpr int kRowB = XSmem::kOutRowB;
         for (int t = blockIdx.x; t < total; t += gridDim.x) {
-            int grp, row0, row_end, nt;
-            locate(t, grp, row0, row_end, nt);
+            int row0, nt;
+            locate(t, row0, nt);
             const int row = row0 + quad * 32 + lane;
-            const bool row_ok = row < row_end;
+            const bool row_ok = row < g.max_rows;
             if (!__all_sync(0xffffffffu, mbar_wait(sm.tfull(), tphase, ac, 0x605))) break;
             tc_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16);
@@ -527,14 +462,8 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_g
             } else {
                 // rows leave through shared memory: lane = row on the way in, 16 lanes x 16 bytes per row on the way out
                 unsigned long long dst = 0;
-                float w = 1.f;
                 if (row_ok) {
-                    if (EPI == 2) {
-                        const int4 info = g.recv_info[row];
-                        w = __int_as_float(info.w);
-                        dst = reinterpret_cast<unsigned long long>(reinterpret_cast<__nv_bfloat16 *>(peer_ptr(g.team, (uint32_t)info.x, g.comb_off)) +
-                                                                   ((int64_t)info.y * g.topk + info.z) * g.N + nt * XBN + half * 128);
-                    } else if (MODE == 2) {
+                    if (MODE == 2) {
                         // the partial tile goes to the landing zone of the rank that owns these rows
                         const int owner = row0 / g.rows_per_rank;
                         dst = reinterpret_cast<unsigned long long>(reinterpret_cast<__nv_bfloat16 *>(peer_ptr(g.team, (uint32_t)owner, g.rs_land_off)) +
@@ -561,7 +490,7 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_g
                                 __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(&pk);
 #pragma unroll
                                 for (int e = 0; e < 4; e++)
-                                    h[e] = __floats2bfloat162_rn(__uint_as_float(v[c][q * 8 + 2 * e]) * w, __uint_as_float(v[c][q * 8 + 2 * e + 1]) * w);
+                                    h[e] = __floats2bfloat162_rn(__uint_as_float(v[c][q * 8 + 2 * e]), __uint_as_float(v[c][q * 8 + 2 * e + 1]));
                                 *reinterpret_cast<uint4 *>(mine + c * 64 + q * 16) = pk;
                             }
                         }
@@ -638,22 +567,6 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_g
     if (MODE == 2 && threadIdx.x == 0 && (int)blockIdx.x < (g.rows_per_rank / BM) * n_tiles) uses = g.tile_uses[blockIdx.x];
     tc_fence_before();
     __syncthreads();
-    if (EPI == 2) {
-        // The CTA that finishes last tells every rank that all of this rank's rows are home: the CTA barrier orders the CTA's
-        // stores before thread 0, whose system fence covers them, and the counter links the CTAs' fences.
-        __shared__ int last_sh;
-        if (threadIdx.x == 0) {
-            fence_sys();
-            last_sh = g.done_count != nullptr && atomicAdd(g.done_count, 1u) + 1 == gridDim.x;
-            if (last_sh) {
-                *g.done_count = 0;
-                __threadfence();  // acquires what the other CTAs' fences released; the flag stores below release it to the system
-            }
-        }
-        __syncthreads();
-        if (last_sh && threadIdx.x < g.team.world)
-            st_release_sys(reinterpret_cast<uint32_t *>(peer_ptr(g.team, threadIdx.x, g.flag_off)) + me, g.epoch);
-    }
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem_base, kXTmemCols);
@@ -692,7 +605,7 @@ using namespace mfk;
 namespace {
 template <int MODE, int EPI> int launch_mx(const XArgs &g, int grid, cudaStream_t s)
 {
-    auto kern = k_grouped_fp8_mx<MODE, EPI>;
+    auto kern = k_tp_fp8_mx<MODE, EPI>;
     static bool attr_set = false;
     if (!attr_set) {
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, XSmem::kDynBytes) != cudaSuccess) {
@@ -701,11 +614,7 @@ template <int MODE, int EPI> int launch_mx(const XArgs &g, int grid, cudaStream_
         }
         attr_set = true;
     }
-    if (MODE == 0) {
-        const cudaError_t e = launch_overlapped(kern, dim3((unsigned)grid), dim3(kXThreads), XSmem::kDynBytes, s, 1, g);
-        return e == cudaSuccess ? 0 : (int)e;
-    }
-    // a grid whose CTAs wait for the peers' (MODE 1, 2) starts when the kernel in front of it has left the SMs
+    // a grid whose CTAs wait for the peers' starts when the kernel in front of it has left the SMs
     kern<<<grid, kXThreads, XSmem::kDynBytes, s>>>(g);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : (int)e;
@@ -714,64 +623,7 @@ template <int MODE, int EPI> int launch_mx(const XArgs &g, int grid, cudaStream_
 
 extern "C" {
 
-// 1 when the block-scaled kernel takes this shape (the caller guarantees power-of-two scales).
-int mf_grouped_gemm_fp8_mx_supported(int G, int N, int K, int epi)
-{
-    if (G <= 0 || G > kXMaxGroups || N <= 0 || K <= 0 || (N % XBN) != 0 || (K % 128) != 0) return 0;
-    return epi >= 0 && epi <= 3;
-}
-
-// epi: 0 plain (out bf16 [rows, N]), 1 SwiGLU (out bf16 [rows, N/2]), 2 weighted push into the combine slots of the
-// tokens' home ranks, 3 SwiGLU + fp8 re-quantisation (out e4m3 [rows, N/2], out_scale fp32 [rows, N/256]).
-// epi 2 with a done_count (a device word, zero between launches): the kernel's last CTA raises this rank's flag in row `which` of
-// the flag area at `flags` of every slot to `epoch`, as mf_moe_signal_all does.
-int mf_grouped_gemm_fp8_mx_signal(const void *A, const float *a_scale, int max_rows, const void *B, const float *b_scale, const int *row_off, int G,
-                                  int N, int K, void *out, int64_t ldo, float *out_scale, int epi, const Team *team, const void *recv_info,
-                                  uint64_t comb_off, int topk, uint32_t *done_count, uint64_t flags, int which, uint32_t epoch, int *status,
-                                  int sms, void *stream)
-{
-    if (!mf_grouped_gemm_fp8_mx_supported(G, N, K, epi) || max_rows <= 0) return -1;
-    if (epi == 2 && (team == nullptr || recv_info == nullptr)) return -1;
-    if (epi == 3 && (out_scale == nullptr || (ldo & 15) != 0)) return -1;
-    XArgs g{};
-    int rc = make_tmap_2d(&g.tm.a, A, 1, (uint64_t)max_rows, (uint64_t)K, (uint64_t)K, BM, true);
-    if (rc == 0) rc = make_tmap_2d(&g.tm.b, B, 1, (uint64_t)G * N, (uint64_t)K, (uint64_t)K, XBN, true);
-    if (rc != 0) return rc;
-    g.a_scale = a_scale;
-    g.b_scale = b_scale;
-    g.row_off = row_off;
-    g.G = G;
-    g.N = N;
-    g.K = K;
-    g.max_rows = max_rows;
-    g.out = out;
-    g.ldo = ldo;
-    g.out_scale = out_scale;
-    g.status = status;
-    if (team != nullptr) g.team = *team;
-    g.recv_info = static_cast<const int4 *>(recv_info);
-    g.comb_off = comb_off;
-    g.topk = topk;
-    g.done_count = done_count;
-    g.flag_off = flags + (uint64_t)which * kMaxRanks * sizeof(uint32_t);
-    g.epoch = epoch;
-    cudaStream_t s = (cudaStream_t)stream;
-    switch (epi) {
-        case 0: return launch_mx<0, 0>(g, sms, s);
-        case 1: return launch_mx<0, 1>(g, sms, s);
-        case 2: return launch_mx<0, 2>(g, sms, s);
-        case 3: return launch_mx<0, 3>(g, sms, s);
-        default: return -1;
-    }
-}
-
-int mf_grouped_gemm_fp8_mx(const void *A, const float *a_scale, int max_rows, const void *B, const float *b_scale, const int *row_off, int G,
-                           int N, int K, void *out, int64_t ldo, float *out_scale, int epi, const Team *team, const void *recv_info,
-                           uint64_t comb_off, int topk, int *status, int sms, void *stream)
-{
-    return mf_grouped_gemm_fp8_mx_signal(A, a_scale, max_rows, B, b_scale, row_off, G, N, K, out, ldo, out_scale, epi, team, recv_info, comb_off,
-                                         topk, nullptr, 0, 0, 0, status, sms, stream);
-}
+int mf_grouped_gemm_fp8_mx_supported(int G, int N, int K, int epi);  // mf_gemm_fp8_pair.cu
 
 // All-gather -> GEMM in fp8. x_local [shard_rows, K] bf16 is this rank's sequence shard; it is quantised (e4m3, one
 // power-of-two scale per 128 elements) on its way into the gather buffers ([world * shard_rows, K] bytes at ag_buf_off,
@@ -794,7 +646,6 @@ int mf_ag_gemm_fp8(const Team *team, const void *x_local, int64_t ldx, int shard
     if (rc != 0) return rc;
     g.a_scale = reinterpret_cast<const float *>(slot + ag_scale_off);
     g.b_scale = b_scale;
-    g.G = 1;
     g.N = N;
     g.K = K;
     g.max_rows = M;
@@ -838,7 +689,6 @@ int mf_gemm_rs_fp8(const Team *team, const void *A, const float *a_scale, const 
     if (rc != 0) return rc;
     g.a_scale = a_scale;
     g.b_scale = b_scale;
-    g.G = 1;
     g.N = N;
     g.K = K;
     g.max_rows = M;

@@ -187,6 +187,26 @@ __device__ __forceinline__ void tma_load_2d_pair(void *smem_dst, const CUtensorM
                  "l"(m), "r"(x), "r"(y), "r"(bar_cluster)
                  : "memory");
 }
+// The same over a 5-D tensor map.
+__device__ __forceinline__ void tma_load_5d_pair(void *smem_dst, const CUtensorMap *m, int c0, int c1, int c2, int c3, int c4, uint32_t bar_cluster)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(
+            smem_u32(smem_dst)),
+        "l"(m), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar_cluster)
+        : "memory");
+}
+// Arrives on the barrier at `cluster_addr` without ordering generic memory accesses for the other CTA (tensor memory hand-over).
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr)
+{
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// Stores a float into the shared memory of another CTA of the cluster; its 4 bytes are counted on `bar_cluster`, in that CTA too.
+__device__ __forceinline__ void st_async_f32(uint32_t cluster_addr, float v, uint32_t bar_cluster)
+{
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(cluster_addr), "r"(__float_as_uint(v)), "r"(bar_cluster)
+                 : "memory");
+}
 // Both CTAs' allocating warps execute these; the pair gets the same columns in both tensor memories.
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t *smem_result, uint32_t cols)
 {
@@ -246,6 +266,24 @@ __device__ __forceinline__ void tmem_cp_sf(uint32_t tmem_col, uint64_t desc)
     asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(tmem_col), "l"(desc) : "memory");
 }
 
+// The same for a CTA pair: rows of A from both CTAs (each CTA's tensor memory holds the scales of its own 128 rows), columns from
+// both CTAs' halves of B (each CTA's tensor memory holds the scales of ALL columns).
+__device__ __forceinline__ void umma_fp8_bs_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate,
+                                                 uint32_t tmem_sfa, uint32_t tmem_sfb)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}" ::"r"(tmem_d),
+        "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(tmem_sfa), "r"(tmem_sfb)
+        : "memory");
+}
+// Issued by the leader: each CTA of the pair copies the chunk at this offset of its own shared memory into its own tensor memory.
+__device__ __forceinline__ void tmem_cp_sf_pair(uint32_t tmem_col, uint64_t desc)
+{
+    asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(tmem_col), "l"(desc) : "memory");
+}
+
 // 32 lanes x 32 consecutive 32-bit columns -> 32 registers per thread (thread i holds lane i of the
 // warp's quadrant). taddr = (lane << 16) | column.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32])
@@ -260,6 +298,24 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32])
           "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr)
         : "memory");
+}
+// 16 lanes x 32 consecutive 32-bit columns -> 16 registers per thread, in the layout of 8 x 8 matrix fragments: r[4i + 2h + e] is lane
+// thread / 4 + 8h of the 16, column 8i + 2 (thread % 4) + e. The 16 lanes are the lower or the upper half of the warp's quadrant.
+__device__ __forceinline__ void tmem_ld_frag(uint32_t taddr, uint32_t (&r)[16])
+{
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
+// Stores four 8 x 8 matrices of 16-bit values, each transposed: lane 8m + k passes the (16-byte aligned) address of row k of matrix m
+// as it lies in memory, which holds column k of the fragments (two values per thread: row thread / 4, columns 2 (thread % 4), + 1).
+__device__ __forceinline__ void stmatrix_x4_trans(const void *row, uint32_t m0, uint32_t m1, uint32_t m2, uint32_t m3)
+{
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(smem_u32(row)), "r"(m0), "r"(m1), "r"(m2), "r"(m3)
+                 : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 

@@ -1,4 +1,4 @@
-"""tcgen05 / TMEM GEMMs (csrc/kernels/mf_gemm.cu, mf_gemm_fp8.cu, mf_gemm_fp8_mx.cu).
+"""tcgen05 / TMEM GEMMs (csrc/kernels/mf_gemm.cu, mf_gemm_fp8.cu, mf_gemm_fp8_mx.cu, mf_gemm_fp8_pair.cu).
 
     gemm_bf16(a, b)                  C[M,N] = A[M,K] . B[N,K]^T   (bf16 in, fp32 accumulate in TMEM, bf16 out)
 

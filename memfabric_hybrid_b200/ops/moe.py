@@ -8,7 +8,7 @@ GEMMs (tcgen05, fp8 block-scaled) with SwiGLU and combine fused into their epilo
 
 Calls must alternate dispatch ... combine on every rank: the wait inside combine is what guarantees that
 peers finished reading the receive buffers before the next dispatch overwrites them.
-Kernels: csrc/kernels/mf_moe.cu, csrc/kernels/mf_gemm_fp8.cu.
+Kernels: csrc/kernels/mf_moe.cu, csrc/kernels/mf_gemm_fp8_pair.cu, csrc/kernels/mf_gemm_fp8.cu.
 """
 from __future__ import annotations
 
@@ -111,7 +111,7 @@ def quantize_weight_fp8(w: torch.Tensor):
 
 
 def gate_up_tile(experts: int, intermediate: int, hidden: int) -> int:
-    """Rows per gate / up run that ``expert_ffn`` expects in the first GEMM's weights: 128 when the 128 x 256
+    """Rows per gate / up run that ``expert_ffn`` expects in the first GEMM's weights: 128 when the
     block-scaled kernel takes the layer's shapes, else 64 (the 128 x 128 kernel that applies the scales in registers)."""
     try:
         cu = _cu()
@@ -365,7 +365,7 @@ class MoEComm:
                                                  self.hp.flags, 1, st.epoch & 0xFFFFFFFF, stw, self._grid, _s()),
                 "grouped_gemm_fp8_mx (down+combine)")
             return
-        # shapes the 128 x 256 kernel does not take (N not a multiple of 256): the 128 x 128 kernel that applies the
+        # shapes the block-scaled kernel does not take (N not a multiple of 256): the 128 x 128 kernel that applies the
         # scales in registers, with w1q interleaved with tile 64 and a separate re-quantisation pass
         if self._h is None:
             self._h = torch.empty((self.max_recv, I), dtype=torch.bfloat16, device=self.dev)

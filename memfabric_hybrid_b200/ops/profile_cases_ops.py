@@ -126,7 +126,7 @@ def case_moe(args) -> None:
 
 def case_gemm_fp8(args) -> None:
     """Grouped fp8 GEMMs of the DeepSeek-V3 expert FFN (gate/up: N 4096, K 7168; down: N 7168, K 2048) on --tokens rows per
-    expert and 8 experts (operands 290 MB / 130 MB: larger than L2): the 128 x 256 kernel with tensor-core block scaling
+    expert and 8 experts (operands 290 MB / 130 MB: larger than L2): the CTA-pair kernel with tensor-core block scaling
     (SwiGLU + re-quantisation epilogue, plain epilogue) next to the 128 x 128 kernel that applies the scales in registers.
     A band of rows is checked against an fp32 reference of the dequantised operands."""
     from . import gemm, moe as M

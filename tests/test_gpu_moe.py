@@ -118,6 +118,63 @@ def test_grouped_gemm_fp8_block_scaled(G, N, K, counts):
     assert torch.equal(hs, hs2) and torch.equal(hq, hq2)
 
 
+@pytest.mark.parametrize("N,K,counts", [(256, 128, [1]), (256, 640, [31, 0, 32, 33, 223]), (512, 2176, [224, 225, 0, 449]), (256, 2048, [0] * 33 + [65] + [0] * 29 + [3]),
+                                        (768, 512, [1000, 1, 448])])
+def test_grouped_gemm_fp8_tile_widths(N, K, counts):
+    """Row counts around the steps (32) and the largest width (224) of a tile, empty groups, 64 groups, K of one block, of a group of scales
+    that is not full (5, 17 blocks) and of whole spans (16): plain and re-quantised results, rows behind the last one untouched, and
+    a row of NaN and infinities that changes no other row."""
+    from memfabric_hybrid_b200.ops import gemm, moe as M
+    cu = M._cu()
+    torch.manual_seed(sum(counts) + N + K)
+    s = torch.cuda.current_stream().cuda_stream
+    G, R, spare = len(counts), sum(counts), 40
+    off = torch.tensor([0] + list(torch.tensor(counts).cumsum(0)), dtype=torch.int32, device="cuda")
+    x = torch.randn(R, K, device="cuda").to(torch.bfloat16)
+    xq, xs = torch.zeros(R + spare, K, dtype=torch.uint8, device="cuda"), torch.ones(R + spare, K // 128, device="cuda")
+    assert cu.mf_quant_rows_fp8(x.data_ptr(), K, off[G:].data_ptr(), K, xq.data_ptr(), xs.data_ptr(), 64, s) == 0
+    w = (torch.randn(G, N, K, device="cuda") * 0.05).to(torch.bfloat16)
+    wq, ws = M.quantize_weight_fp8(w)
+    xd, wd = _deq(xq[:R].view(torch.float8_e4m3fn), xs[:R]).double(), _deq_w(wq, ws).double()
+    ref = torch.cat([xd[off[g]:off[g + 1]] @ wd[g].t() for g in range(G)])
+    # one rounding to bf16, and the fp32 accumulation of K terms
+    bound = ref.abs() * 2.0 ** -8 + torch.cat([xd[off[g]:off[g + 1]].abs() @ wd[g].abs().t() for g in range(G)]) * K * 2.0 ** -24
+    st = gemm.status_word()
+
+    def run(epi, b, ldo, dt, scales=None):
+        out = torch.full((R + spare, ldo), 7.0, device="cuda").to(dt)
+        assert cu.mf_grouped_gemm_fp8_mx(xq.data_ptr(), xs.data_ptr(), R + spare, b.data_ptr(), ws.data_ptr(), off.data_ptr(), G, N, K, out.data_ptr(), ldo,
+                                         scales.data_ptr() if scales is not None else None, epi, None, None, 0, 1, st.data_ptr(), gemm.sm_count(), s) == 0
+        torch.cuda.synchronize()
+        gemm.check_status()
+        assert bool((out[R:] == 7).all())
+        return out[:R]
+
+    out = run(0, wq, N, torch.bfloat16)
+    assert bool(((out.double() - ref).abs() <= bound).all())
+    wi = M.interleave_gate_up_fp8(wq, tile=128)
+    h = run(1, wi, N // 2, torch.bfloat16)
+    gate, up = ref[:, :N // 2], ref[:, N // 2:]
+    want = torch.nn.functional.silu(gate) * up
+    # silu' <= 1.1: the accumulation errors of both factors, one rounding to bf16, a few units of fp32 of the exponential and the quotient
+    bg, bu = (bound - ref.abs() * 2.0 ** -8).split(N // 2, 1)
+    assert bool(((h.double() - want).abs() <= want.abs() * 2.0 ** -7.9 + 1.1 * bg * up.abs() + bu * gate.abs() + 1e-6).all())
+    hs, hs2, hq2 = torch.zeros(R + spare, N // 256, device="cuda"), torch.zeros(R, N // 256, device="cuda"), torch.zeros(R, N // 2, dtype=torch.uint8, device="cuda")
+    hq = run(3, wi, N // 2, torch.uint8, hs)
+    assert cu.mf_quant_rows_fp8(h.data_ptr(), N // 2, off[G:].data_ptr(), N // 2, hq2.data_ptr(), hs2.data_ptr(), 64, s) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(hq, hq2) and torch.equal(hs[:R], hs2) and bool((hs[R:] == 0).all())
+    bad = R // 2
+    xq[bad, ::5] = 0x7F  # NaN
+    again = run(0, wq, N, torch.bfloat16)
+    keep = torch.arange(R, device="cuda") != bad
+    assert torch.equal(again[keep], out[keep]) and bool(torch.isnan(again[bad]).all())
+    hs3 = torch.zeros_like(hs)
+    hq3 = run(3, wi, N // 2, torch.uint8, hs3)
+    assert torch.equal(hq3[keep], hq[keep]) and torch.equal(hs3[:R][keep], hs[:R][keep])
+    assert bool((hq3[bad] & 0x7F == 0x7F).all()) and bool((hs3[bad] == 1).all())
+
+
 def _moe_ranks(rank, world, url, T, H, I, E, K, sync):
     import torch
     from memfabric_hybrid_b200.ops import gemm
