@@ -6,6 +6,13 @@ import enum
 import threading
 from typing import Callable, Sequence
 
+try:
+    import numpy as np
+except ImportError:   # batches need it, single copies do not
+    np = None
+else:
+    _U64, _I64 = np.dtype(np.uint64), np.dtype(np.int64)
+
 from .. import _native as N
 
 
@@ -99,9 +106,9 @@ def _u64_view(values, n: int):
     """Address of ``values`` as an array of ``n`` 64-bit words plus the object that keeps it alive. A contiguous numpy array
     of 64-bit integers is passed as it is (no copy: the cost of a call on a large descriptor list is then the C call
     alone); any other sequence is converted once."""
-    import numpy as np
     a = values if isinstance(values, np.ndarray) else np.asarray(values[:n], dtype=np.uint64)
-    if a.dtype not in (np.uint64, np.int64) or not a.flags.c_contiguous:
+    d = a.dtype
+    if (d is not _U64 and d is not _I64 and d != _U64 and d != _I64) or not a.flags.c_contiguous:
         a = np.ascontiguousarray(a, dtype=np.uint64)
     if a.shape[0] < n:
         raise ValueError(f"batch of {n} items but only {a.shape[0]} values")
@@ -182,8 +189,18 @@ class BigMemory:
     def copy_data_batch(self, src_addrs, dst_addrs, sizes, count, type: BmCopyType, flags: int = 0, stream: int = 0) -> int:
         """``smem_bm_copy_batch``. The three lists may be any sequences of integers; contiguous numpy arrays of
         uint64 / int64 are handed to the C call without conversion."""
-        p, _keep = self._batch(src_addrs, dst_addrs, sizes, count, stream)
-        return N.lib().smem_bm_copy_batch(self._h, C.byref(p), int(type), flags)
+        tl = _TLS
+        p = getattr(tl, "batch_params", None)
+        if p is None:     # as in copy_data: one parameter block per thread
+            p = tl.batch_params = N.BatchCopyParamsC()
+            tl.batch_ref = C.byref(p)
+            tl.batch_fn = N.lib().smem_bm_copy_batch
+        n = int(count)
+        p.sources, _k0 = _u64_view(src_addrs, n)
+        p.destinations, _k1 = _u64_view(dst_addrs, n)
+        p.dataSizes, _k2 = _u64_view(sizes, n)
+        p.batchSize, p.stream = n, stream or None
+        return tl.batch_fn(self._h, tl.batch_ref, int(type), flags)
 
     def prepare_batch(self, src_addrs, dst_addrs, sizes, count=None):
         """Extension: marshals a batch once so that repeated submissions skip the Python-side conversion (every submission

@@ -599,18 +599,23 @@ int Entity::BatchCopyData(const hybm_batch_copy_params &p, hybm_data_copy_direct
         const uint64_t end = base + slot * opt_.rankCount;
         const bool srcPool = dir != HYBM_LOCAL_DEVICE_TO_GLOBAL_DEVICE, dstPool = dir != HYBM_GLOBAL_DEVICE_TO_LOCAL_DEVICE;
         Segment *seg = hbm_.get();
-        auto poolOk = [&](uint64_t a, uint64_t len) {
-            if (a < base || a >= end) return false;
-            uint64_t rel = a - base;
-            uint32_t r = (uint32_t)(rel / slot);
-            const uint64_t mapped = seg->MappedBytes(r);
-            return len <= mapped && rel - (uint64_t)r * slot <= mapped - len;  // no sum that a huge len could wrap
+        // slot of the last address on each side: a batch mostly stays with one rank, and the division took a third of the pass
+        struct Last {
+            uint64_t lo, mapped;
+        } srcLast{base, seg->MappedBytes(0)}, dstLast = srcLast;
+        auto poolOk = [&](uint64_t a, uint64_t len, Last &at) {
+            if (a - at.lo >= slot) {
+                if (a < base || a >= end) return false;
+                const uint32_t r = (uint32_t)((a - base) / slot);
+                at = Last{base + r * slot, seg->MappedBytes(r)};
+            }
+            return len <= at.mapped && a - at.lo <= at.mapped - len;  // no sum that a huge len could wrap
         };
         uint64_t total = 0;
         for (uint32_t i = 0; i < p.batchSize; i++) {
             uint64_t s = reinterpret_cast<uint64_t>(p.sources[i]), d = reinterpret_cast<uint64_t>(p.destinations[i]);
             uint64_t len = p.dataSizes[i];
-            if (s == 0 || d == 0 || len == 0 || (srcPool && !poolOk(s, len)) || (dstPool && !poolOk(d, len)))
+            if (s == 0 || d == 0 || len == 0 || (srcPool && !poolOk(s, len, srcLast)) || (dstPool && !poolOk(d, len, dstLast)))
                 return MF_FAIL(ERR_INVALID_PARAM, "batch copy item %u (%p -> %p, %lu bytes): null, empty or outside the mapped pool",
                                i, p.sources[i], p.destinations[i], (unsigned long)len);
             total += len;

@@ -18,7 +18,7 @@ import ctypes as C
 import torch
 
 from .. import _native as N
-from .heap import TeamC, _HeapBase
+from .heap import TeamC, _HeapBase, current_stream_ptr as _stream
 
 DT = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2, torch.int32: 3}
 OPS = {"sum": 0, "max": 1, "min": 2, "prod": 3}
@@ -67,10 +67,6 @@ def _cu():
         assert l.mf_coll_args_size() == C.sizeof(CollArgsC), "CollArgs layout differs between Python and CUDA"
         _lib = l
     return _lib
-
-
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
 
 
 def _check(rc: int, what: str) -> None:
@@ -153,11 +149,12 @@ class Communicator:
         assert t.is_cuda and t.is_contiguous(), "collective tensors must be contiguous CUDA tensors"
         if self.heap.emu:
             assert t.shape[0] == self.world, "emulated collectives take tensors with a leading world dimension"
-            return t.data_ptr(), t.stride(0) * t.element_size(), t[0].numel()
+            n = t.numel() // self.world
+            return t.data_ptr(), n * t.element_size(), n
         return t.data_ptr(), 0, t.numel()
 
-    def _args(self, x, out, n, epoch, stage, scale=1.0, op="sum", root=0, algo=0) -> CollArgsC:
-        xin, xs, _ = self._local(x)
+    def _args(self, x, out, n, epoch, stage, scale=1.0, op="sum", root=0, algo=0, x_local=None) -> CollArgsC:
+        xin, xs, _ = x_local or self._local(x)
         xo, os_, _ = self._local(out)
         return CollArgsC(self.heap.team(), xin, xo, xs, os_, n, stage[0], stage[1], float(scale), OPS[op], epoch, 0, root, algo, 0)
 
@@ -170,9 +167,7 @@ class Communicator:
         return lo <= p and p + t.numel() * t.element_size() <= lo + getattr(self.heap, "usable", self.heap.stride)
 
     def _empty_like(self, x: torch.Tensor, per_rank_numel: int, dtype: torch.dtype) -> torch.Tensor:
-        if self.heap.emu:
-            return torch.empty((self.world, per_rank_numel), dtype=dtype, device=x.device)
-        return torch.empty((per_rank_numel,), dtype=dtype, device=x.device)
+        return x.new_empty((self.world, per_rank_numel) if self.heap.emu else (per_rank_numel,), dtype=dtype)
 
     # ------------------------------------------------------------------ collectives
     def barrier(self, channel: int = 0) -> None:
@@ -183,7 +178,8 @@ class Communicator:
     def all_reduce(self, x: torch.Tensor, out: torch.Tensor | None = None, op: str = "sum", scale: float = 1.0,
                    out_dtype: torch.dtype | None = None, algo: str | None = None) -> torch.Tensor:
         od = out_dtype or x.dtype
-        _, _, n = self._local(x)
+        xl = self._local(x)
+        n = xl[2]
         if out is None:
             out = self._empty_like(x, n, od)
         es = x.element_size()
@@ -204,7 +200,7 @@ class Communicator:
             cnt = min(piece, n - done)
             use = a if a is not None else (0 if cnt * es <= ONE_SHOT_MAX else 1)
             epoch, stage = self._next()
-            args = self._args(x, out, cnt, epoch, stage, scale, op, 0, use)
+            args = self._args(x, out, cnt, epoch, stage, scale, op, 0, use, xl)
             args.inp += done * es
             args.out += done * out.element_size()
             _check(_cu().mf_coll_launch(0, DT[x.dtype], DT[od], C.byref(args), self._ctas(cnt * es), 512, _stream()), "all_reduce")

@@ -7,10 +7,12 @@ The status word is a device int that a kernel sets when one of its bounded pipel
 from __future__ import annotations
 
 import ctypes as C
+import functools
 
 import torch
 
 from .. import _native as N
+from .heap import current_stream_ptr
 
 _lib = None
 _status = {}
@@ -50,8 +52,13 @@ def check_status(device=None) -> None:
         raise RuntimeError(f"a GEMM pipeline wait gave up (code {v:#x})")
 
 
+@functools.lru_cache(maxsize=64)
+def _sms(device) -> int:
+    return torch.cuda.get_device_properties(device).multi_processor_count
+
+
 def sm_count(device=None) -> int:
-    return torch.cuda.get_device_properties(device if device is not None else torch.cuda.current_device()).multi_processor_count
+    return _sms(device if device is not None else torch.cuda.current_device())
 
 
 def interleave_gate_up(w_gate: torch.Tensor, w_up: torch.Tensor, tile: int = 128) -> torch.Tensor:
@@ -76,7 +83,7 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None,
     fn = _cu().mf_gemm_bf16 if pair is None else (_cu().mf_gemm_bf16_pair if pair else _cu().mf_gemm_bf16_one)
     rc = fn(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, Nn, K, a.stride(0), b.stride(0), out.stride(0),
             status_word(a.device).data_ptr(), sms or sm_count(a.device), 1 if swiglu else 0,
-            torch.cuda.current_stream().cuda_stream)
+            current_stream_ptr())
     if rc != 0:
         raise RuntimeError(f"mf_gemm_bf16 failed to launch ({rc})")
     return out

@@ -20,7 +20,7 @@ import torch
 
 from .. import _native as N
 from .gemm import sm_count, status_word
-from .heap import TeamC, _HeapBase
+from .heap import TeamC, _HeapBase, current_stream_ptr as _s
 
 
 _CANARY_BYTES = 4096
@@ -86,10 +86,6 @@ def _cu():
         l.mf_grouped_gemm_fp8_mx_supported.argtypes = [ci, ci, ci, ci]
         _lib = l
     return _lib
-
-
-def _s() -> int:
-    return torch.cuda.current_stream().cuda_stream
 
 
 def _ok(rc: int, what: str) -> None:

@@ -22,7 +22,7 @@ import torch
 from .. import _native as N
 from . import gemm
 from .gemm import status_word, sm_count
-from .heap import TeamC, _HeapBase
+from .heap import TeamC, _HeapBase, current_stream_ptr
 
 _lib = None
 
@@ -96,7 +96,7 @@ class TensorParallel:
         rc = _cu().mf_ag_gemm_bf16(C.byref(team), x_shard.data_ptr(), x_shard.stride(0), rows, w.data_ptr(), w.stride(0), out.data_ptr(),
                                    out.stride(0), Nn, K, self._ag[b], self._ready[b], self._push[b].data_ptr(), self._epoch,
                                    self._ag_calls[b], status_word(x_shard.device).data_ptr(), sm_count(x_shard.device),
-                                   1 if swiglu else 0, torch.cuda.current_stream().cuda_stream)
+                                   1 if swiglu else 0, current_stream_ptr())
         if rc != 0:
             raise RuntimeError(f"mf_ag_gemm_bf16 failed to launch ({rc})")
         return out
@@ -117,7 +117,7 @@ class TensorParallel:
         team = self.heap.team()
         rc = _cu().mf_gemm_rs_bf16(C.byref(team), a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), rows,
                                    Nn, K, self._land[b], self._cnt[b], self._tile_uses[b].data_ptr(), self._epoch, float(scale),
-                                   status_word(a.device).data_ptr(), sm_count(a.device), torch.cuda.current_stream().cuda_stream)
+                                   status_word(a.device).data_ptr(), sm_count(a.device), current_stream_ptr())
         if rc != 0:
             raise RuntimeError(f"mf_gemm_rs_bf16 failed to launch ({rc})")
         return out
@@ -149,7 +149,7 @@ class TensorParallel:
         rc = _cu().mf_ag_gemm_fp8(C.byref(team), x_shard.data_ptr(), x_shard.stride(0), rows, wq.data_ptr(), ws.data_ptr(), out.data_ptr(),
                                   out.stride(0), out_s.data_ptr() if out_s is not None else None, Nn, K, self._ag[b], self._ags[b], self._ready[b],
                                   self._push[b].data_ptr(), self._epoch, self._ag_calls[b], status_word(dev).data_ptr(), sm_count(dev), code,
-                                  torch.cuda.current_stream().cuda_stream)
+                                  current_stream_ptr())
         if rc != 0:
             raise RuntimeError(f"mf_ag_gemm_fp8 failed to launch ({rc})")
         return (out.view(torch.float8_e4m3fn), out_s) if code == 3 else out
@@ -170,7 +170,7 @@ class TensorParallel:
         team = self.heap.team()
         rc = _cu().mf_gemm_rs_fp8(C.byref(team), aq.data_ptr(), a_scale.data_ptr(), wq.data_ptr(), ws.data_ptr(), out.data_ptr(), out.stride(0), rows,
                                   Nn, K, self._land[b], self._cnt[b], self._tile_uses[b].data_ptr(), self._epoch, float(scale),
-                                  status_word(aq.device).data_ptr(), sm_count(aq.device), torch.cuda.current_stream().cuda_stream)
+                                  status_word(aq.device).data_ptr(), sm_count(aq.device), current_stream_ptr())
         if rc != 0:
             raise RuntimeError(f"mf_gemm_rs_fp8 failed to launch ({rc})")
         return out

@@ -91,6 +91,49 @@ def test_fake_device_two_ranks():
     assert sorted(ranks) == [0, 1]
 
 
+def _alternating_rank(rank, world, url, sync):
+    import memfabric_hybrid as mf
+    from memfabric_hybrid import bm
+    assert mf.initialize() == 0
+    cfg = bm.BmConfig()
+    cfg.rank_id = rank
+    cfg.start_store = rank == 0
+    assert bm.initialize(url, world, 0, cfg) == 0, mf.get_last_err_msg()
+    h = bm.create2(id=8, local_dram_size=0, max_dram_size=0, local_hbm_size=8 * MiB, max_hbm_size=16 * MiB)
+    assert h.join() == 0, mf.get_last_err_msg()
+    sync.wait(60)
+    base = [h.peer_rank_ptr(r, bm.BmMemType.DEVICE) for r in range(world)]
+    if rank == 0:
+        n, seg = 64, 4096
+        src = np.random.default_rng(3).integers(0, 256, n * seg, dtype=np.uint8)
+        a = src.ctypes.data + np.arange(n, dtype=np.uint64) * np.uint64(seg)
+        d = np.array([base[i % 2] + 2 * MiB + i * seg for i in range(n)], dtype=np.uint64)   # a slot that changes with every item
+        size = np.full(n, seg, dtype=np.int64)
+        assert h.copy_data_batch(a, d, size, n, bm.BmCopyType.L2G, 0) == 0, mf.get_last_err_msg()
+        back = np.zeros_like(src)
+        b = back.ctypes.data + np.arange(n, dtype=np.uint64) * np.uint64(seg)
+        assert h.copy_data_batch(d, b, size, n, bm.BmCopyType.G2L, 0) == 0, mf.get_last_err_msg()
+        assert np.array_equal(back, src)
+        assert h.copy_data_batch(list(map(int, d)), list(map(int, d + np.uint64(MiB))), list(map(int, size)), n, bm.BmCopyType.G2G, 0) == 0
+        # behind good items of the same slot: past the mapped 8 MiB, across their end, in front of the window, behind it, and a length that wraps
+        for bad, length in [(base[1] + 8 * MiB, 1), (base[1] + 8 * MiB - 8, 16), (base[0] + 16 * MiB - 1, 1), (base[0] - 8, 8), (base[1] + 16 * MiB, 8),
+                            (base[1] + 64, (1 << 64) - 32)]:
+            for last in (base[0], base[1]):
+                rc = h.copy_data_batch([src.ctypes.data] * 2, [last + 4096, bad], [64, length], 2, bm.BmCopyType.L2G, 0)
+                assert rc != 0, (hex(bad), length)
+                mf.get_and_clear_last_err_msg()
+    sync.wait(60)
+    h.destroy()
+    bm.uninitialize(0)
+    mf.uninitialize()
+    return True
+
+
+def test_batch_whose_items_change_slots_and_ranges_that_leave_them():
+    url = f"tcp://127.0.0.1:{free_port()}"
+    assert run_ranks(_alternating_rank, 2, (url,), timeout=180, env={"MF_DEVICE_BACKEND": "fake"}, with_barrier=True) == [True, True]
+
+
 def _quant_rank(rank, world, url):
     import torch
     import memfabric_hybrid as mf
