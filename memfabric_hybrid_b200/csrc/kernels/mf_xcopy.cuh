@@ -260,12 +260,17 @@ template <typename In> __device__ __forceinline__ void unpack8(const uint4 &raw,
     for (int k = 0; k < 8; k++) f[k] = to_f32<In>(h[k]);
 }
 
+// int8: adding 1.5 * 2^23 rounds to an integer (to nearest, ties to even, as rintf) and leaves it in the low bits of the sum; the clamp, whose
+// bounds are integers, comes first and takes a NaN to -127. Round and convert instructions run at a quarter of the rate: 512 items
+// of 128 Ki fp16 elements, units of 128, took 54.2 us with them, 41.8 so.
+__device__ __forceinline__ uint32_t round_int8(float x, float mul)
+{
+    return __float_as_uint(fminf(127.f, fmaxf(-127.f, x * mul)) + 12582912.f);  // the low byte
+}
+
 template <int MODE> __device__ __forceinline__ uint8_t quant1(float x, float mul)
 {
-    if (MODE == 0) {
-        const float q = fminf(127.f, fmaxf(-127.f, rintf(x * mul)));
-        return (uint8_t)(int8_t)q;
-    }
+    if (MODE == 0) return (uint8_t)round_int8(x, mul);
     return (uint8_t)__nv_cvt_float_to_fp8(x * mul, __NV_SATFINITE, __NV_E4M3);
 }
 
@@ -281,12 +286,12 @@ template <int MODE> __device__ __forceinline__ uint2 quant8(const float *f, floa
         }
         return make_uint2(lo, hi);
     }
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        lo |= (uint32_t)quant1<MODE>(f[k], mul) << (8 * k);
-        hi |= (uint32_t)quant1<MODE>(f[4 + k], mul) << (8 * k);
-    }
-    return make_uint2(lo, hi);
+    // the low bytes of four sums in three byte permutations
+    auto four = [&](const float *g) {
+        return __byte_perm(__byte_perm(round_int8(g[0], mul), round_int8(g[1], mul), 0x0040),
+                           __byte_perm(round_int8(g[2], mul), round_int8(g[3], mul), 0x0040), 0x5410);
+    };
+    return make_uint2(four(f), four(f + 4));
 }
 
 template <typename In, int MODE>

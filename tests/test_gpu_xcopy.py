@@ -316,3 +316,53 @@ def test_quantising_copy_of_items_around_its_block_sizes():
     """The same bytes and factors as the formula in fp32 (x * (top / amax), amax / top)."""
     url = f"tcp://127.0.0.1:{free_port()}"
     assert run_ranks(_quant_rank, 1, (url,), timeout=300) == [[]]
+
+
+def _int8_rank(rank, world, url):
+    import torch
+    import memfabric_hybrid as mf
+    from memfabric_hybrid import bm
+    torch.cuda.set_device(0)
+    torch.zeros(1, device="cuda")
+    assert mf.initialize() == 0
+    cfg = bm.BmConfig()
+    cfg.rank_id = 0
+    cfg.start_store = True
+    assert bm.initialize(url, 1, 0, cfg) == 0, mf.get_last_err_msg()
+    h = bm.create2(id=12, local_dram_size=0, max_dram_size=0, local_hbm_size=64 << 20, max_hbm_size=64 << 20)
+    assert h.join() == 0, mf.get_last_err_msg()
+    base = h.peer_rank_ptr(0, bm.BmMemType.DEVICE)
+    from memfabric_hybrid_b200.ops.heap import tensor_at
+    bad = []
+    for dt in (torch.bfloat16, torch.float16):
+        # every 16-bit pattern (NaN, infinities and subnormal values among them), shuffled so that units mix them, and the finite ones
+        # in order, so that units hold one magnitude; then values half-way between two integers
+        bits = torch.arange(65536, dtype=torch.int32).to(torch.int16)
+        mixed = bits[torch.randperm(65536, generator=torch.Generator().manual_seed(1))]
+        half = (torch.arange(65536) % 255 - 127.5).clamp(-127, 127).to(dt).view(torch.int16)
+        for pi, pattern in enumerate((mixed, bits, half)):
+            for unit, off in ((128, 0), (1024, 0), (64, 0), (128, 1)):
+                n = 65536 - (unit if off else 0)
+                x = pattern.cuda().view(dt)[off:off + n]
+                q, f = tensor_at(base, (n,), torch.uint8), tensor_at(base + (1 << 20), (n // unit,), torch.float32)
+                torch.cuda.synchronize()
+                assert h.quant_copy_batch([x.data_ptr()], [base], [2 * n], [base + (1 << 20)], unit, fp16_input=dt == torch.float16) == 0
+                v = x.float().view(-1, unit)
+                amax = torch.where(torch.isnan(v), torch.zeros_like(v), v.abs()).amax(1, keepdim=True)   # a NaN counts as nothing
+                one, top = torch.ones_like(amax), torch.full_like(amax, 127.0)
+                y = v * torch.where(amax > 0, top / amax, one)
+                want = torch.where(torch.isnan(y), torch.full_like(y, -127.0), y.round().clamp(-127, 127)).to(torch.int8).view(torch.uint8)
+                if not torch.equal(q.view(-1, unit), want) or not torch.equal(f.view(-1, 1), torch.where(amax > 0, amax / top, one)):
+                    bad.append((str(dt), pi, unit, off, int((q.view(-1, unit) != want).sum())))
+    h.leave()
+    h.destroy()
+    bm.uninitialize(0)
+    mf.uninitialize()
+    return bad
+
+
+def test_int8_rounding_of_every_16_bit_value():
+    """Round to nearest even and the clamp, as the formula in fp32 gives them; a NaN becomes -127. Units of the fast path and of the general one,
+    source addresses on and off 16 bytes."""
+    url = f"tcp://127.0.0.1:{free_port()}"
+    assert run_ranks(_int8_rank, 1, (url,), timeout=300) == [[]]
