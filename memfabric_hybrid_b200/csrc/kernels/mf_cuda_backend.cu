@@ -510,6 +510,34 @@ public:
         if (clear && v != 0) *reinterpret_cast<volatile uint32_t *>(copyStatus_) = 0;
         return v;
     }
+    // Lanes per unit, vectors per lane and units per step (at most nine loads per lane in flight) by the vectors of a unit: few lanes,
+    // of whose places few stay empty, but four at least (two read 32 bytes each at 256-byte distances: units of 128 47.9 us for 35.6).
+    void LaunchQuantUnits(const mfk::QuantItem *q, uint32_t n, uint32_t vecs, uint64_t maxUnits, bool fp16, int mode, cudaStream_t st)
+    {
+        // Blocks of one step of a CTA where all steps fit a grid that is resident at once (few items: 4 x 300 units of 128, int8, 11.1 us
+        // with two, 7.4 with one), else of two; no item is cut into more parts than it takes to give every CTA sixteen blocks.
+        auto go = [&](auto kern, uint32_t step, int perSm) {
+            const uint32_t resident = (uint32_t)(std::max(1, caps_.smCount) * perSm);
+            const uint64_t steps = (maxUnits + step - 1) / step;
+            const uint32_t parts = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(steps * n <= resident ? steps : (steps + 1) / 2, 16ull * resident / n));
+            kern<<<std::min(n * parts, resident), 256, 0, st>>>(q, n, parts, vecs);
+        };
+#define MF_QUANT_GO(MODE, W, R, J, V)                                                                                                       \
+    (fp16 ? go(mfk::mf_xcopy_quant_units_kernel<__half, MODE, W, R, J, V>, mfk::quant_step<W, J>(), mfk::kQuantCtasPerSm)                   \
+          : go(mfk::mf_xcopy_quant_units_kernel<__nv_bfloat16, MODE, W, R, J, V>, mfk::quant_step<W, J>(), mfk::kQuantCtasPerSm))
+        if (mode == 1) MF_QUANT_GO(1, 4, 4, 2, 16);  // units of 128 only
+        else if (vecs <= 8) MF_QUANT_GO(0, 4, 2, 4, 0);
+        else if (vecs == 16) MF_QUANT_GO(0, 4, 4, 2, 16);
+        else if (vecs <= 16) MF_QUANT_GO(0, 4, 4, 2, 0);
+        else if (vecs <= 24) MF_QUANT_GO(0, 8, 3, 3, 0);
+        else if (vecs <= 32) MF_QUANT_GO(0, 8, 4, 2, 0);
+        else if (vecs <= 72) MF_QUANT_GO(0, 8, 9, 1, 0);
+        else if (vecs <= 128) MF_QUANT_GO(0, 32, 4, 2, 0);
+        else if (vecs <= 256) MF_QUANT_GO(0, 32, 8, 1, 0);
+        else if (fp16) go(mfk::mf_xcopy_quant_wide_kernel<__half>, 1, 4);
+        else go(mfk::mf_xcopy_quant_wide_kernel<__nv_bfloat16>, 1, 4);
+#undef MF_QUANT_GO
+    }
     int LaunchQuantCopy(const QuantItem *items, uint32_t count, uint32_t unit, int inputFp16, int mode, void *s) override
     {
         if (count == 0) return OK;
@@ -526,27 +554,15 @@ public:
             const uint64_t perItem = std::max<uint64_t>(1, (2ull * (uint64_t)std::max(1, grid_) + n - 1) / n);
             dim3 grid((unsigned)std::min<uint64_t>({perItem, (maxUnits + 15) / 16, 65535ull}), n);  // a CTA takes at least 16 units per step
             cudaStream_t st = (cudaStream_t)s;
-            // units of 128 elements on aligned addresses (the fp8 1 x 128 format, and int8 with that unit): the kernel
-            // that keeps eight loads per lane in flight
-            bool fast = unit == 128;
+            // whole vectors per unit, whole units per item, aligned addresses: the kernels that read a unit once with many loads in flight
+            const uint32_t vecs = unit / 8;
+            bool fast = unit % 8 == 0 && vecs <= 1024;
             for (uint32_t i = 0; i < n && fast; i++) {
                 const QuantItem &q0 = items[off + i];
-                fast = (q0.src & 15) == 0 && (q0.dst & 7) == 0 && (q0.scale & 3) == 0 && (q0.elems % 128) == 0 && q0.elems != 0;
+                fast = (q0.src & 15) == 0 && (q0.dst & 7) == 0 && (q0.scale & 3) == 0 && q0.elems != 0 && q0.elems % unit == 0;
             }
             if (fast) {
-                // blocks of one step of a CTA where all steps fit a grid that is resident at once (few items: 4 x 300 units, int8, 11.1 us
-                // with two, 7.4 with one), else of two; no item is cut into more parts than it takes to give every CTA sixteen blocks
-                const uint32_t resident = (uint32_t)(std::max(1, caps_.smCount) * mfk::kQuantCtasPerSm);
-                const uint64_t steps = (maxUnits + mfk::kQuantStep - 1) / mfk::kQuantStep;
-                const uint32_t parts = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(steps * n <= resident ? steps : (steps + 1) / 2, 16ull * resident / n));
-                const unsigned g2 = std::min(n * parts, resident);
-                if (inputFp16) {
-                    if (mode == 0) mfk::mf_xcopy_quant128_kernel<__half, 0><<<g2, 256, 0, st>>>(q + off, n, parts);
-                    else mfk::mf_xcopy_quant128_kernel<__half, 1><<<g2, 256, 0, st>>>(q + off, n, parts);
-                } else {
-                    if (mode == 0) mfk::mf_xcopy_quant128_kernel<__nv_bfloat16, 0><<<g2, 256, 0, st>>>(q + off, n, parts);
-                    else mfk::mf_xcopy_quant128_kernel<__nv_bfloat16, 1><<<g2, 256, 0, st>>>(q + off, n, parts);
-                }
+                LaunchQuantUnits(q + off, n, vecs, maxUnits, inputFp16 != 0, mode, st);
                 RT_CHECK(cudaGetLastError(), "xcopy quant launch");
                 continue;
             }

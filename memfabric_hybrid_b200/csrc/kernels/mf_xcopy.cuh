@@ -369,17 +369,20 @@ __global__ void __launch_bounds__(256) mf_xcopy_quant_kernel(const QuantItem *__
     }
 }
 
-// Fast path of the quantising copy for the common shape: units of 128 elements, source 16-byte aligned, destination
-// 8-byte aligned, element count a multiple of 128. A half-warp (16 lanes x 16 bytes = one unit per load instruction)
-// takes EIGHT consecutive units per step: eight independent loads per lane are in flight before the first reduction,
-// the maxima are taken two at a time and every division is done once. The kernel above keeps two loads per lane in flight and
-// is bound by the latency of each step; here, memory (201 MB in 41 us: 4.9 TB/s) and instruction issue are about even.
+// Fast path of the quantising copy: units that are whole 16-byte vectors of the source, whole units per item; source 16-byte,
+// destination 8-byte aligned. W lanes share a unit, R vectors each, and take J consecutive units per step: J x R (eight or nine)
+// independent loads per lane are in flight before the first reduction, and a unit is read once. Few lanes per unit: what they hold
+// is reduced without shuffles, and fewer lanes repeat a unit's divisions. The kernel above keeps two loads per lane in flight and is bound
+// by the latency of each step, and reads a unit of more than 512 elements twice; here memory and the latencies of the arithmetic are about
+// even. 512 items of 128 Ki 16-bit values (201 MB), us, before / now: units of 128 -> fp8 39.7 / 35.6 (5.6 TB/s; 16 lanes per unit that
+// traded units while they reduced, 2 lanes: 47.9), -> int8 40.0 / 36.1; -> int8 by the kernel above / here: 64 198 / 40.5, 192 145 / 40.6,
+// 256 112 / 36.8, 576 95 / 39.3, 1024 75 / 38.2, 2048 86 / 35.6. (Loads of the next steps by cp.async into shared memory, two CTAs
+// per SM: 48.9 for 38.4; the warps that hide the arithmetic are worth more.)
 //
 // Blocks are dealt out over a grid that fits the GPU at once: block v takes steps v % parts, v % parts + parts, .. of item
-// v / parts, a step being the kQuantStep units that a CTA converts at once. The descriptors sit in pinned host memory (a PCIe
+// v / parts, a step being the units that a CTA converts at once. The descriptors sit in pinned host memory (a PCIe
 // read of more than a microsecond), so a CTA fetches those of its next 32 blocks together and its warps then run through these
-// blocks without another barrier. (One CTA per item and part, each with its own read before the first load, and both divisions in
-// all sixteen lanes of a unit: 46.7 us for 512 items of 128 Ki bf16 elements; 41.3 us now.)
+// blocks without another barrier.
 template <typename In> struct PairOf;
 template <> struct PairOf<__nv_bfloat16> { using type = __nv_bfloat162; };
 template <> struct PairOf<__half> { using type = __half2; };
@@ -391,19 +394,23 @@ template <typename In> struct Pair16 {  // two 16-bit values in a register
     __device__ static type xchg(type a, int lane_mask) { return __shfl_xor_sync(0xffffffffu, a, lane_mask); }
     __device__ static float fold(type a) { return fmaxf(__low2float(a), __high2float(a)); }
 };
-constexpr uint32_t kQuantStep = 128;           // units that the 8 warps of a CTA take at once, 16 each
 constexpr uint32_t kQuantList = 32;
 constexpr int kQuantCtasPerSm = 3;             // 80 registers a thread, 96 KB of loads in flight per SM
-template <typename In, int MODE>
-__global__ void __launch_bounds__(256, kQuantCtasPerSm) mf_xcopy_quant128_kernel(const QuantItem *__restrict__ items, uint32_t count, uint32_t parts)
+// Units that the 8 warps of a CTA take at once.
+template <int W, int J> constexpr uint32_t quant_step() { return 8u * (32u / W) * J; }
+
+// V: 16-byte vectors per unit, 0: unit_vecs of them, at most W * R
+template <typename In, int MODE, int W, int R, int J, int V>
+__global__ void __launch_bounds__(256, kQuantCtasPerSm) mf_xcopy_quant_units_kernel(const QuantItem *__restrict__ items, uint32_t count, uint32_t parts,
+                                                                                    uint32_t unit_vecs)
 {
+    const uint32_t vecs = V > 0 ? (uint32_t)V : unit_vecs;
     __shared__ QuantItem list[kQuantList];
-    constexpr int J = 8;
+    constexpr uint32_t kStep = quant_step<W, J>();
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t sub = lane >> 4, sl = lane & 15;
+    const uint32_t sub = lane / W, sl = lane % W;
     const float qmax = MODE == 0 ? 127.f : 448.f;
     const uint32_t blocks = count * parts;  // the launch keeps this far below 2^32
-    static_assert(kQuantStep == 8u * 2u * J, "warps x half-warps x units");
     for (uint32_t v0 = blockIdx.x; v0 < blocks; v0 += gridDim.x * kQuantList) {
         __syncthreads();  // the previous list is no longer read
         if (threadIdx.x < kQuantList * 4) {
@@ -416,57 +423,121 @@ __global__ void __launch_bounds__(256, kQuantCtasPerSm) mf_xcopy_quant128_kernel
             const uint32_t v = v0 + l * gridDim.x;
             if (v >= blocks) break;
             const QuantItem it = list[l];
-            const uint64_t units = it.elems / 128;
-            const uint4 *src = reinterpret_cast<const uint4 *>(it.src);   // 16 vectors per unit
-            uint2 *dst = reinterpret_cast<uint2 *>(it.dst);               // 16 x 8 bytes per unit
+            const uint64_t units = it.elems / 8 / vecs;
+            const uint4 *src = reinterpret_cast<const uint4 *>(it.src);
+            uint2 *dst = reinterpret_cast<uint2 *>(it.dst);
             float *scales = reinterpret_cast<float *>(it.scale);
-            // the loop bounds are the same for the whole warp (the shuffles below), its second half-warp may have fewer units left
-            for (uint64_t step = (uint64_t)(v % parts) * kQuantStep + warp * 2 * J; step < units; step += (uint64_t)parts * kQuantStep) {
+            // the loop bounds are the same for the whole warp (the shuffles below), its last lanes may have fewer units left
+            for (uint64_t step = (uint64_t)(v % parts) * kStep + warp * (32 / W) * J; step < units; step += (uint64_t)parts * kStep) {
                 const uint64_t base = step + sub * J;
-                uint4 raw[J];
+                uint4 raw[J][R];
 #pragma unroll
-                for (int j = 0; j < J; j++) {
-                    const uint64_t u = base + j;
-                    raw[j] = u < units ? __ldcs(src + u * 16 + sl) : make_uint4(0, 0, 0, 0);
-                }
-                // Largest magnitude of each of the eight units, two 16-bit values per register (a maximum needs no rounding).
-                // Lanes trade halves of their units at every step, so that eight shuffles instead of thirty-two leave lane l
-                // with the maximum of ONE unit, (l >> 1) & 7 in the order 8, 4, 2 of its bits; it alone does that unit's two
-                // divisions, which all sixteen lanes did before.
+                for (int j = 0; j < J; j++)
+#pragma unroll
+                    for (int r = 0; r < R; r++)
+                        raw[j][r] = base + j < units && sl + r * W < vecs ? __ldcs(src + (base + j) * vecs + sl + r * W) : make_uint4(0, 0, 0, 0);
+                // Largest magnitude of each unit, two 16-bit values per register (a maximum needs no rounding).
                 typename Pair16<In>::type m[J];
 #pragma unroll
-                for (int j = 0; j < J; j++) m[j] = Pair16<In>::absmax(raw[j]);
+                for (int j = 0; j < J; j++) {
+                    m[j] = Pair16<In>::absmax(raw[j][0]);
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const bool up = (sl & 8) != 0;
-                    const auto give = up ? m[i] : m[i + 4];
-                    m[i] = Pair16<In>::max2(up ? m[i + 4] : m[i], Pair16<In>::xchg(give, 8));
+                    for (int r = 1; r < R; r++) m[j] = Pair16<In>::max2(m[j], Pair16<In>::absmax(raw[j][r]));
                 }
-#pragma unroll
-                for (int i = 0; i < 2; i++) {
-                    const bool up = (sl & 4) != 0;
-                    const auto give = up ? m[i] : m[i + 2];
-                    m[i] = Pair16<In>::max2(up ? m[i + 2] : m[i], Pair16<In>::xchg(give, 4));
-                }
-                {
-                    const bool up = (sl & 2) != 0;
-                    const auto give = up ? m[0] : m[1];
-                    m[0] = Pair16<In>::max2(up ? m[1] : m[0], Pair16<In>::xchg(give, 2));
-                }
-                m[0] = Pair16<In>::max2(m[0], Pair16<In>::xchg(m[0], 1));
-                const float amax = Pair16<In>::fold(m[0]);
-                const float mul1 = amax > 0.f ? qmax / amax : 1.f;
-                const uint32_t mine = (sl >> 3 & 1) * 4 + (sl >> 2 & 1) * 2 + (sl >> 1 & 1);
-                if ((sl & 1) == 0 && base + mine < units) scales[base + mine] = amax > 0.f ? amax / qmax : 1.f;
+                float mul[J];
 #pragma unroll
                 for (int j = 0; j < J; j++) {
-                    const float mul = __shfl_sync(0xffffffffu, mul1, (int)(sub * 16) + (j >> 2 & 1) * 8 + (j >> 1 & 1) * 4 + (j & 1) * 2);
-                    const uint64_t u = base + j;
-                    if (u < units) {
-                        float f[8];
-                        unpack8<In>(raw[j], f);
-                        __stcs(dst + u * 16 + sl, quant8<MODE>(f, mul));
-                    }
+#pragma unroll
+                    for (int o = W / 2; o >= 1; o /= 2) m[j] = Pair16<In>::max2(m[j], Pair16<In>::xchg(m[j], o));
+                    const float amax = Pair16<In>::fold(m[j]);
+                    mul[j] = amax > 0.f ? qmax / amax : 1.f;
+                    if (sl == 0 && base + j < units) scales[base + j] = amax > 0.f ? amax / qmax : 1.f;
+                }
+#pragma unroll
+                for (int j = 0; j < J; j++)
+#pragma unroll
+                    for (int r = 0; r < R; r++)
+                        if (base + j < units && sl + r * W < vecs) {
+                            float f[8];
+                            unpack8<In>(raw[j][r], f);
+                            __stcs(dst + (base + j) * vecs + sl + r * W, quant8<MODE>(f, mul[j]));
+                        }
+            }
+        }
+    }
+}
+
+// Units of more vectors than a warp holds, up to 1024: the CTA shares a unit, four vectors per thread; the next unit's vectors are on
+// their way while this one is reduced and stored. 512 items of 126 Ki values, units of 7168 -> int8: 113 us above, 46 here.
+template <typename In>
+__global__ void __launch_bounds__(256, 4) mf_xcopy_quant_wide_kernel(const QuantItem *__restrict__ items, uint32_t count, uint32_t parts, uint32_t vecs)
+{
+    __shared__ QuantItem list[kQuantList];
+    __shared__ float top[2][8];
+    constexpr int R = 4;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t blocks = count * parts;
+    uint32_t parity = 0;
+    for (uint32_t v0 = blockIdx.x; v0 < blocks; v0 += gridDim.x * kQuantList) {
+        __syncthreads();
+        if (threadIdx.x < kQuantList * 4) {
+            const uint32_t v = v0 + (threadIdx.x >> 2) * gridDim.x;
+            if (v < blocks)
+                reinterpret_cast<uint64_t *>(list)[threadIdx.x] = reinterpret_cast<const uint64_t *>(items + v / parts)[threadIdx.x & 3];
+        }
+        __syncthreads();
+        const uint32_t have = min(kQuantList, (blocks - v0 + gridDim.x - 1) / gridDim.x);
+        // unit u of block l of the list; behind the last unit of a block comes the next block that has one
+        uint32_t l = 0;
+        uint64_t u = 0;
+        auto settle = [&]() {
+            for (; l < have; l++) {
+                u = (v0 + l * gridDim.x) % parts;
+                if (u < list[l].elems / 8 / vecs) return;
+            }
+        };
+        auto load = [&](uint4 (&raw)[R]) {
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const uint32_t at = threadIdx.x + r * 256;
+                raw[r] = l < have && at < vecs ? __ldcs(reinterpret_cast<const uint4 *>(list[l].src) + u * vecs + at) : make_uint4(0, 0, 0, 0);
+            }
+        };
+        settle();
+        uint4 next[R];
+        load(next);
+        while (l < have) {
+            uint4 raw[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) raw[r] = next[r];
+            uint2 *dst = reinterpret_cast<uint2 *>(list[l].dst) + u * vecs;
+            float *scale = reinterpret_cast<float *>(list[l].scale) + u;
+            u += parts;
+            if (u >= list[l].elems / 8 / vecs) {
+                l++;
+                settle();
+            }
+            load(next);
+            typename Pair16<In>::type m = Pair16<In>::absmax(raw[0]);
+#pragma unroll
+            for (int r = 1; r < R; r++) m = Pair16<In>::max2(m, Pair16<In>::absmax(raw[r]));
+#pragma unroll
+            for (int o = 16; o >= 1; o /= 2) m = Pair16<In>::max2(m, Pair16<In>::xchg(m, o));
+            if (lane == 0) top[parity][warp] = fmaxf(Pair16<In>::fold(m), 0.f);
+            __syncthreads();  // the other half of top is written by warps that have passed the next barrier
+            float amax = 0.f;
+#pragma unroll
+            for (int w = 0; w < 8; w++) amax = fmaxf(amax, top[parity][w]);
+            parity ^= 1;
+            const float mul = amax > 0.f ? 127.f / amax : 1.f;
+            if (threadIdx.x == 0) *scale = amax > 0.f ? amax / 127.f : 1.f;
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const uint32_t at = threadIdx.x + r * 256;
+                if (at < vecs) {
+                    float f[8];
+                    unpack8<In>(raw[r], f);
+                    __stcs(dst + at, quant8<0>(f, mul));
                 }
             }
         }

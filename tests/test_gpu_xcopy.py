@@ -366,3 +366,65 @@ def test_int8_rounding_of_every_16_bit_value():
     source addresses on and off 16 bytes."""
     url = f"tcp://127.0.0.1:{free_port()}"
     assert run_ranks(_int8_rank, 1, (url,), timeout=300) == [[]]
+
+
+def _units_rank(rank, world, url):
+    import torch
+    import memfabric_hybrid as mf
+    from memfabric_hybrid import bm
+    from memfabric_hybrid_b200.ops.heap import tensor_at
+    torch.cuda.set_device(0)
+    torch.zeros(1, device="cuda")
+    assert mf.initialize() == 0
+    cfg = bm.BmConfig()
+    cfg.rank_id = 0
+    cfg.start_store = True
+    assert bm.initialize(url, 1, 0, cfg) == 0, mf.get_last_err_msg()
+    pool = 256 * MiB
+    h = bm.create2(id=13, local_dram_size=0, max_dram_size=0, local_hbm_size=pool, max_hbm_size=pool)
+    assert h.join() == 0, mf.get_last_err_msg()
+    base = h.peer_rank_ptr(0, bm.BmMemType.DEVICE)
+    bad = []
+    # units on both sides of every line of the rule, the largest of each lane layout and sizes that leave places empty; 8200 and 100
+    # (not whole vectors) are the general kernel's, and so is an item whose last unit is not full (tail)
+    for unit in (8, 56, 64, 72, 128, 136, 192, 200, 256, 264, 576, 584, 1024, 1032, 2048, 2056, 7168, 8192, 8200, 100):
+        for units, tail in (([1, 2, 3, 7, 8, 9, 31, 64, 65], 0), ([33] * 700 if unit <= 1024 else [5] * 700, 0), ([4, 9], unit // 2)):
+            dt = torch.float16 if unit % 16 == 8 else torch.bfloat16
+            sizes = [u * unit + tail for u in units]
+            n, nf = sum(sizes), sum(-(-e // unit) for e in sizes)
+            x = torch.randn(n, device="cuda", generator=torch.Generator("cuda").manual_seed(unit)).to(dt)
+            x[:unit] = 0
+            first = np.concatenate(([0], np.cumsum(sizes)))
+            f0 = np.concatenate(([0], np.cumsum([-(-e // unit) for e in sizes])))
+            fac = base + (n + 64 + 255) // 256 * 256
+            q, f = tensor_at(base, (n + 64,), torch.uint8), tensor_at(fac, (nf + 1,), torch.float32)
+            q.fill_(77)
+            f.fill_(-5)
+            torch.cuda.synchronize()
+            assert h.quant_copy_batch([x.data_ptr() + int(a) * 2 for a in first[:-1]], [base + int(a) for a in first[:-1]], [e * 2 for e in sizes],
+                                      [fac + int(a) * 4 for a in f0[:-1]], unit, fp16_input=dt == torch.float16) == 0, mf.get_last_err_msg()
+            if len(units) > 100 and tail == 0:
+                v = x.float().view(-1, unit)
+                want_amax = v.abs().amax(1)
+            else:
+                v, want_amax = None, torch.cat([x[a + k:min(b, a + k + unit)].float().abs().amax().view(1) for a, b in zip(first[:-1], first[1:])
+                                                for k in range(0, int(b - a), unit)])
+            one, top = torch.ones_like(want_amax), torch.full_like(want_amax, 127.0)
+            mul = torch.where(want_amax > 0, top / want_amax, one)
+            lens = torch.tensor([min(int(b - a) - k, unit) for a, b in zip(first[:-1], first[1:]) for k in range(0, int(b - a), unit)], device="cuda")
+            y = x.float() * torch.repeat_interleave(mul, lens)
+            want = y.round().clamp(-127, 127).to(torch.int8).view(torch.uint8)
+            if not (torch.equal(q[:n], want) and torch.equal(f[:nf], torch.where(want_amax > 0, want_amax / top, one)) and bool((q[n:] == 77).all())
+                    and float(f[nf]) == -5):
+                bad.append((unit, units[:2], tail, int((q[:n] != want).sum())))
+    h.leave()
+    h.destroy()
+    bm.uninitialize(0)
+    mf.uninitialize()
+    return bad
+
+
+def test_quantising_copy_of_units_of_any_size():
+    """int8 bytes and factors as the formula in fp32 gives them, nothing written behind them."""
+    url = f"tcp://127.0.0.1:{free_port()}"
+    assert run_ranks(_units_rank, 1, (url,), timeout=300) == [[]]
