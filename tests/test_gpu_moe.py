@@ -175,6 +175,28 @@ def test_grouped_gemm_fp8_tile_widths(N, K, counts):
     assert bool((hq3[bad] & 0x7F == 0x7F).all()) and bool((hs3[bad] == 1).all())
 
 
+def test_swiglu_of_the_expert_kernels_is_the_same():
+    """Small whole numbers: both kernels' sums are exact (14 bits), so that every bf16 activation has to be the same one, and with it
+    every byte of a layer that changes its kernel with its shape. 2 M activations: a quotient one unit of fp32 off moves a few dozen."""
+    from memfabric_hybrid_b200.ops import gemm, moe as M
+    cu = M._cu()
+    G, R, N, K = 2, 4096, 1024, 256
+    gen = torch.Generator("cuda").manual_seed(5)
+    x = torch.randint(-8, 9, (R, K), generator=gen, device="cuda").float().to(torch.float8_e4m3fn)
+    w = torch.randint(-8, 9, (G, N, K), generator=gen, device="cuda").float().to(torch.float8_e4m3fn)
+    xs, ws = torch.full((R, K // 128), 2.0 ** -3, device="cuda"), torch.full((G, N // 128, K // 128), 2.0 ** -3, device="cuda")
+    off = torch.tensor([0, 1500, R], dtype=torch.int32, device="cuda")
+    st, s = gemm.status_word(), torch.cuda.current_stream().cuda_stream
+    got, want = (torch.zeros(R, N // 2, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    assert cu.mf_grouped_gemm_fp8_mx(x.data_ptr(), xs.data_ptr(), R, M.interleave_gate_up_fp8(w, tile=128).data_ptr(), ws.data_ptr(), off.data_ptr(), G, N, K,
+                                     got.data_ptr(), N // 2, None, 1, None, None, 0, 1, st.data_ptr(), gemm.sm_count(), s) == 0
+    assert cu.mf_grouped_gemm_fp8(x.data_ptr(), xs.data_ptr(), R, M.interleave_gate_up_fp8(w, tile=64).data_ptr(), ws.data_ptr(), off.data_ptr(), G, N, K,
+                                  want.data_ptr(), N // 2, 1, None, None, 0, 1, st.data_ptr(), gemm.sm_count(), s) == 0
+    torch.cuda.synchronize()
+    gemm.check_status()
+    assert int((got != want).sum()) == 0 and float(got.abs().max()) > 100
+
+
 def _moe_ranks(rank, world, url, T, H, I, E, K, sync):
     import torch
     from memfabric_hybrid_b200.ops import gemm
