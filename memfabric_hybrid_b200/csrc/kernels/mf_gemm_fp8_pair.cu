@@ -148,6 +148,15 @@ struct RingState {
     }
 };
 
+// Cut of a group's `steps` runs of 32 rows into `cnt` tiles whose widths differ by one run at most: tile mi starts at run `first` and is `gran`
+// runs wide. No product of a tile's number and the runs: in 32 bits that overflows at 3.9 M rows.
+__host__ __device__ inline void p_tile_cut(int steps, int cnt, int mi, int &first, int &gran)
+{
+    const int each = steps / cnt, wider = steps - each * cnt;
+    first = mi * each + (mi < wider ? mi : wider);
+    gran = each + (mi < wider ? 1 : 0);
+}
+
 struct PTile {
     int grp = 0;    // walks forward with the tiles
     int row0, row_end, gran, nt;
@@ -256,9 +265,9 @@ template <int EPI> __global__ void __launch_bounds__(kPThreads, 1) k_grouped_fp8
         const int steps = (hi - lo + kGran - 1) / kGran;
         p.nt = local / cnt;
         const int mi = local - p.nt * cnt;
-        const int g0 = mi * steps / cnt, g1 = (mi + 1) * steps / cnt;
-        p.row0 = lo + g0 * kGran;
-        p.gran = g1 - g0;
+        int first;
+        p_tile_cut(steps, cnt, mi, first, p.gran);
+        p.row0 = lo + first * kGran;
         p.row_end = hi;
     };
 
@@ -641,6 +650,9 @@ int mf_grouped_gemm_fp8_mx_supported(int G, int N, int K, int epi)
     if (G <= 0 || G > kPMaxGroups || N <= 0 || K <= 0 || (N % kPTileN) != 0 || (K % 128) != 0) return 0;
     return epi >= 0 && epi <= 3;
 }
+
+// The cut of a group's rows into tiles, as the kernels make it: tile `mi` of `cnt` starts at run `*first` of 32 rows and takes `*gran` of them.
+void mf_grouped_gemm_fp8_mx_cut(int steps, int cnt, int mi, int *first, int *gran) { p_tile_cut(steps, cnt, mi, *first, *gran); }
 
 // epi: 0 plain (out bf16 [rows, N]), 1 SwiGLU (out bf16 [rows, N/2]), 2 weighted push into the combine slots of the
 // tokens' home ranks, 3 SwiGLU + fp8 re-quantisation (out e4m3 [rows, N/2], out_scale fp32 [rows, N/256]).

@@ -46,3 +46,23 @@ def test_a_product_that_the_split_kernel_cannot_take_goes_to_the_persistent_ones
 
     assert rc("mf_gemm_bf16_one") == rc("mf_gemm_bf16_pair") != rc("mf_gemm_bf16_splitk", 0)
     assert rc("mf_gemm_bf16") == rc("mf_gemm_bf16_one")
+
+
+@pytest.mark.parametrize("steps", [1, 6, 7, 8, 48, 1000, 65_536, 122_606, 122_607, 122_608, 1 << 20, (1 << 26) - 1, 1 << 26])
+@pytest.mark.parametrize("widest", [1, 3, 7])
+def test_rows_of_a_group_are_cut_into_tiles_without_gaps(steps, widest):
+    """Runs of 32 rows, up to the 2^31 rows that the entry takes: every run belongs to one tile and no tile is wider than the others need.
+    A 32-bit product of the tile's number and the runs left its range at 122 607 runs (3.9 M rows) in tiles of seven."""
+    cut = N.cuda().mf_grouped_gemm_fp8_mx_cut
+    cut.restype, cut.argtypes = None, [C.c_int] * 3 + [C.POINTER(C.c_int)] * 2
+    cnt = -(-steps // widest)
+    first, gran = C.c_int(), C.c_int()
+    many = cnt > 2000
+    for lo, hi in ([(0, 500), (cnt // 2, cnt // 2 + 500), (cnt - 500, cnt)] if many else [(0, cnt)]):
+        end = None
+        for mi in range(lo, hi):
+            cut(steps, cnt, mi, C.byref(first), C.byref(gran))
+            assert 1 <= gran.value <= -(-steps // cnt) and (end is None or first.value == end), mi
+            assert mi > 0 or first.value == 0
+            end = first.value + gran.value
+        assert hi < cnt or end == steps
