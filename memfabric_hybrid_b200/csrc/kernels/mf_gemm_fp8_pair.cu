@@ -312,14 +312,14 @@ template <int EPI> __global__ void __launch_bounds__(kPThreads, 1) k_grouped_fp8
             const uint32_t sfa = tmem_base + kPSfaCol, sfb = tmem_base + kPSfbCol;
             for (int t = walker; t < total && fine; t += walkers) {
                 locate(t, p);
-                fine = mbar_wait(sm.tempty(acc), acc_phase ^ 1, ac, 0x603);  // both CTAs' epilogues have taken this accumulator out of TMEM
+                fine = mbar_wait<true>(sm.tempty(acc), acc_phase ^ 1, ac, 0x603);  // both CTAs' epilogues have taken this accumulator out of TMEM
                 if (!fine) break;
                 tc_fence_after();
                 const uint32_t d = tmem_base + (uint32_t)(acc * kMaxWidth);
                 const uint32_t width = (uint32_t)(p.gran * kGran);
                 for (int kb = 0; kb < k_blocks; kb++) {
                     if (kb % kSfSpan == 0) {
-                        fine = mbar_wait(sm.sf_full(sf.slot), sf.phase, ac, 0x606);
+                        fine = mbar_wait<true>(sm.sf_full(sf.slot), sf.phase, ac, 0x606);
                         if (!fine) break;
                         tc_fence_after();
                     }
@@ -359,10 +359,10 @@ template <int EPI> __global__ void __launch_bounds__(kPThreads, 1) k_grouped_fp8
         }
     } else if (warp == 2) {
         // scale producer: one 32-bit word of four K-block scale bytes per operand row. Lane l writes the 16 bytes of rows l, l + 32, l + 64,
-        // l + 96 of a chunk: this CTA's 128 rows of W, and all rows of X. The scales of 16 K blocks go over at once. Nobody in the other
-        // CTA reads them: each CTA's tensor core copies its own chunks, so the proxy fence is all the ordering they need, and the arrive on the
-        // leader's barrier carries none for the cluster (a cluster-scope release there waits until the SM's outstanding loads are home:
-        // 32 experts of about 32 rows, 4096 x 7168: 150 us without, 163-175 with one per 16 K blocks, 227 with one per four).
+        // l + 96 of a chunk: this CTA's 128 rows of W, and all rows of X. The scales of 16 K blocks go over at once. Each CTA's tensor
+        // core copies its own chunks, but the leader has both do it, so the other CTA's bytes are released to the cluster: the
+        // proxy fence, then a release of shared memory alone. A full release waits for the SM's outstanding loads as well: 32 experts of about
+        // 32 rows, 4096 x 7168: 161 us with it, 149.4 so (148.4 without any order), 227 with a full release per four K blocks.
         RingState sf;
         PTile p;
         const int nblocks = g.N / 128;
@@ -399,6 +399,7 @@ template <int EPI> __global__ void __launch_bounds__(kPThreads, 1) k_grouped_fp8
                 int ok = 1;
                 if (lane == 0) ok = mbar_wait(sm.sf_empty(sf.slot), sf.phase ^ 1, ac, 0x607) ? 1 : 0;
                 ok = __shfl_sync(0xffffffffu, ok, 0);
+                __syncwarp();  // what lane 0 has waited for holds for all lanes
                 if (!ok) {
                     fine = false;
                     break;
@@ -412,7 +413,10 @@ template <int EPI> __global__ void __launch_bounds__(kPThreads, 1) k_grouped_fp8
                 }
                 fence_proxy_async_smem();  // the tensor core's copy unit reads these bytes through the async proxy
                 __syncwarp();
-                if (lane == 0) mbar_arrive_remote(mapa_u32(smem_u32(sm.sf_full(sf.slot)), 0));
+                if (lane == 0) {
+                    if (crank == 0) mbar_arrive(sm.sf_full(sf.slot));
+                    else mbar_arrive_cluster_smem(mapa_u32(smem_u32(sm.sf_full(sf.slot)), 0));
+                }
                 sf.advance(kPSfBufs);
             }
         }
@@ -458,7 +462,10 @@ template <int EPI> __global__ void __launch_bounds__(kPThreads, 1) k_grouped_fp8
             auto release = [&]() {  // this warp has read its part of the accumulator
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive_remote(mapa_u32(smem_u32(sm.tempty(acc)), 0));
+                if (lane == 0) {
+                    if (crank == 0) mbar_arrive(sm.tempty(acc));
+                    else mbar_arrive_cluster_smem(mapa_u32(smem_u32(sm.tempty(acc)), 0));
+                }
             };
             const int last = p.gran > set ? (p.gran - 1 - set) / 2 : -1;  // index of this set's last chunk
             if (last < 0) release();
@@ -553,9 +560,9 @@ template <int EPI> __global__ void __launch_bounds__(kPThreads, 1) k_grouped_fp8
                         // four floats (a lane quadrant each) for every row come from the peer
                         if (set == 0 && quad == 0) mbar_expect_tx(sm.amax_full(acc), (uint32_t)(p.gran * kGran * 16));
                         else mbar_arrive(sm.amax_full(acc));
-                        mbar_arrive_remote(mapa_u32(smem_u32(sm.amax_full(acc)), crank ^ 1));
+                        mbar_arrive_cluster_smem(mapa_u32(smem_u32(sm.amax_full(acc)), crank ^ 1));
                     }
-                    if (!p_bar_all(1 + set, 128, mbar_wait(sm.amax_full(acc), acc_phase, ac, 0x60A))) break;
+                    if (!p_bar_all(1 + set, 128, mbar_wait<true>(sm.amax_full(acc), acc_phase, ac, 0x60A))) break;
                     // The buffer of this parity is written again for the tile after the next, by warps that have passed the next tile's barrier:
                     // every warp of the pair has contributed to that one after it has read this tile's maxima.
 #pragma unroll

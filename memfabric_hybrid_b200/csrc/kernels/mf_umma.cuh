@@ -41,16 +41,26 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar)
 {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity)
+// CLUSTER: what threads of the other CTAs of the cluster released with their arrivals is visible too.
+template <bool CLUSTER = false> __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity)
 {
     uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred P;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, P;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
+    if (CLUSTER)
+        asm volatile(
+            "{\n\t.reg .pred P;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P, [%1], %2;\n\t"
+            "selp.b32 %0, 1, 0, P;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred P;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+            "selp.b32 %0, 1, 0, P;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
     return ok != 0;
 }
 
@@ -60,10 +70,10 @@ struct AbortCtl {
 };
 
 // Returns false when the wait ran out or another role aborted.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, const AbortCtl &ac, int where)
+template <bool CLUSTER = false> __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, const AbortCtl &ac, int where)
 {
     for (uint32_t i = 0; i < kMbarSpinLimit; i++) {
-        if (mbar_try_wait(bar, parity)) return true;
+        if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
         if ((i & 1023) == 1023 && *ac.abort_smem) return false;
     }
     *ac.abort_smem = 1;
@@ -178,6 +188,15 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr)
 {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
+// The same for what this thread has done, or has seen done, in its own CTA's shared memory alone: mbar_arrive_cluster() also waits for the
+// loads and stores to global memory that are under way.
+__device__ __forceinline__ void mbar_arrive_cluster_smem(uint32_t cluster_addr)
+{
+    asm volatile(
+        "fence.release.sync_restrict::shared::cta.cluster;\n\t"
+        "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr)
+        : "memory");
+}
 // 2-D tile load of the CTA-pair form into this CTA's shared memory; the bytes are counted on the barrier at cluster address
 // `bar_cluster` (the leader's). Every CTA fetches its own tiles.
 __device__ __forceinline__ void tma_load_2d_pair(void *smem_dst, const CUtensorMap *m, int x, int y, uint32_t bar_cluster)
@@ -195,11 +214,6 @@ __device__ __forceinline__ void tma_load_5d_pair(void *smem_dst, const CUtensorM
             smem_u32(smem_dst)),
         "l"(m), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar_cluster)
         : "memory");
-}
-// Arrives on the barrier at `cluster_addr` without ordering generic memory accesses for the other CTA (tensor memory hand-over).
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr)
-{
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // Stores a float into the shared memory of another CTA of the cluster; its 4 bytes are counted on `bar_cluster`, in that CTA too.
 __device__ __forceinline__ void st_async_f32(uint32_t cluster_addr, float v, uint32_t bar_cluster)

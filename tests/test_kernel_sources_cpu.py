@@ -56,3 +56,21 @@ def test_overlapped_kernels_read_nothing_through_the_read_only_path(src, kernel,
     for name, (sig, body) in reach.items():
         assert "__ldg(" not in body, f"{src}: {name} (reached from {kernel}) reads through the read-only path"
         assert not re.search(r"const\b[^,()]*__restrict__", sig), f"{src}: {name} (reached from {kernel}) takes a read-only pointer"
+
+
+def test_what_crosses_a_cluster_is_ordered_for_the_cluster():
+    """An arrival or a wait without a scope orders the memory of one CTA. An arrival on another CTA's barrier names the cluster, with a release of its own
+    or right behind a fence; a barrier that another CTA's threads arrive on is waited for with an acquire of the same scope."""
+    text = {p.name: re.sub(r"//[^\n]*", "", p.read_text()) for p in sorted(KERNELS.glob("*.cu*"))}
+    arrivals = [(n, m.group(0)) for n, t in text.items() for m in re.finditer(r"mbarrier\.arrive[\w.:]*shared::cluster[\w.]*", t)]
+    assert len(arrivals) >= 2
+    for name, a in arrivals:
+        assert ".release.cluster" in a or ".relaxed.cluster" in a, (name, a)
+        if ".relaxed.cluster" in a:
+            assert re.search(r"fence\.release\.sync_restrict::shared::cta\.cluster;[\s\\nt\"]*" + re.escape(a), text[name]), (name, a)
+    pair = text["mf_gemm_fp8_pair.cu"]
+    shared = set(re.findall(r"mbar_arrive_cluster(?:_smem)?\(mapa_u32\(smem_u32\(sm\.(\w+)\(", pair))
+    assert shared == {"sf_full", "tempty", "amax_full"}
+    for bar in shared:
+        waits = re.findall(r"mbar_wait(<true>)?\(sm\." + bar + r"\(", pair)
+        assert waits and all(waits), bar
