@@ -51,7 +51,20 @@ class BmGroupEvent(enum.IntEnum):
     LEAVE_EVENT = 1
 
 
-_TLS = threading.local()
+class _Blocks(threading.local):
+    """Parameter blocks (block, reference to it, C function), kept per thread from call to call: the calls release the GIL, so threads must not
+    share one. A call takes its block away while it uses it: a copy that runs inside it on the same thread, from a finaliser or a
+    signal handler, finds none and makes its own instead of overwriting this one."""
+    copy = None
+    batch = None
+
+
+_TLS = _Blocks()
+
+
+def _block(struct, fn: str):
+    p = struct()
+    return p, C.byref(p), getattr(N.lib(), fn)
 
 ASYNC_COPY_FLAG = 1 << 0
 COPY_EXTEND_FLAG = 1 << 1
@@ -170,13 +183,14 @@ class BigMemory:
         ``randn``, the output of a layer) must be complete first (synchronise its stream), or pass that stream
         with the flag so that the copy is enqueued behind the producer."""
         tl = _TLS
-        p = getattr(tl, "copy_params", None)
-        if p is None:     # one parameter block per thread: the call releases the GIL, so threads must not share one
-            p = tl.copy_params = N.CopyParamsC()
-            tl.copy_ref = C.byref(p)
-            tl.copy_fn = N.lib().smem_bm_copy
+        block, tl.copy = tl.copy, None
+        if block is None:
+            block = _block(N.CopyParamsC, "smem_bm_copy")
+        p, ref, fn = block
         p.src, p.dest, p.dataSize, p.stream = src_ptr, dst_ptr, size, stream or None
-        return tl.copy_fn(self._h, tl.copy_ref, int(type), flags)
+        rc = fn(self._h, ref, int(type), flags)
+        tl.copy = block
+        return rc
 
     def _batch(self, src_addrs, dst_addrs, sizes, count, stream):
         n = int(count)
@@ -189,18 +203,19 @@ class BigMemory:
     def copy_data_batch(self, src_addrs, dst_addrs, sizes, count, type: BmCopyType, flags: int = 0, stream: int = 0) -> int:
         """``smem_bm_copy_batch``. The three lists may be any sequences of integers; contiguous numpy arrays of
         uint64 / int64 are handed to the C call without conversion."""
-        tl = _TLS
-        p = getattr(tl, "batch_params", None)
-        if p is None:     # as in copy_data: one parameter block per thread
-            p = tl.batch_params = N.BatchCopyParamsC()
-            tl.batch_ref = C.byref(p)
-            tl.batch_fn = N.lib().smem_bm_copy_batch
         n = int(count)
-        p.sources, _k0 = _u64_view(src_addrs, n)
-        p.destinations, _k1 = _u64_view(dst_addrs, n)
-        p.dataSizes, _k2 = _u64_view(sizes, n)
-        p.batchSize, p.stream = n, stream or None
-        return tl.batch_fn(self._h, tl.batch_ref, int(type), flags)
+        srcs, _k0 = _u64_view(src_addrs, n)
+        dsts, _k1 = _u64_view(dst_addrs, n)
+        lens, _k2 = _u64_view(sizes, n)
+        tl = _TLS
+        block, tl.batch = tl.batch, None
+        if block is None:
+            block = _block(N.BatchCopyParamsC, "smem_bm_copy_batch")
+        p, ref, fn = block
+        p.sources, p.destinations, p.dataSizes, p.batchSize, p.stream = srcs, dsts, lens, n, stream or None
+        rc = fn(self._h, ref, int(type), flags)
+        tl.batch = block
+        return rc
 
     def prepare_batch(self, src_addrs, dst_addrs, sizes, count=None):
         """Extension: marshals a batch once so that repeated submissions skip the Python-side conversion (every submission

@@ -145,3 +145,88 @@ def _rank_56(rank, world, url, sync):
 
 def test_56_bit_addresses_for_a_window_larger_than_the_address_space(store_url):
     assert run_ranks(_rank_56, 2, (store_url,), timeout=120, with_barrier=True) == [True, True]
+
+
+class _Inside:
+    """An integer whose conversion runs ``inner`` once, as a finaliser or a signal handler could at the same place."""
+
+    def __init__(self, value, inner):
+        self.value, self.inner = value, inner
+
+    def __int__(self):
+        inner, self.inner = self.inner, None
+        if inner is not None:
+            inner()
+        return int(self.value)
+
+    __index__ = __int__
+
+
+def _copies_inside_copies(rank, world, url):
+    import memfabric_hybrid as mf
+    from memfabric_hybrid import bm
+    assert mf.initialize() == 0
+    cfg = bm.BmConfig()
+    cfg.rank_id, cfg.start_store = 0, True
+    assert bm.initialize(url, 1, 0, cfg) == 0, mf.get_last_err_msg()
+    h = bm.create2(id=0, local_dram_size=4 * MiB, max_dram_size=4 * MiB, data_op_type=bm.BmDataOpType.HOST_SHM)
+    assert h.join() == 0, mf.get_last_err_msg()
+    pool = h.peer_rank_ptr(0, bm.BmMemType.HOST)
+    n, seg = 8, 4096
+    outer, inner = (np.random.default_rng(k).integers(0, 256, n * seg, dtype=np.uint8) for k in (1, 2))
+    step = np.arange(n, dtype=np.uint64) * np.uint64(seg)
+    size = np.full(n, seg, dtype=np.uint64)
+
+    def at(base):
+        return np.uint64(base) + step
+
+    def batch_inside():
+        assert h.copy_data_batch(at(inner.ctypes.data), at(pool + MiB), size, n, bm.BmCopyType.H2GH, 0) == 0, mf.get_last_err_msg()
+
+    def copy_inside():
+        assert h.copy_data(inner.ctypes.data, pool + MiB, inner.size, bm.BmCopyType.H2GH, 0) == 0, mf.get_last_err_msg()
+
+    def got(base):
+        out = np.zeros(n * seg, dtype=np.uint8)
+        assert h.copy_data(base, out.ctypes.data, out.size, bm.BmCopyType.GH2H, 0) == 0, mf.get_last_err_msg()
+        return out
+
+    def both_arrived():
+        ok = np.array_equal(got(pool), outer) and np.array_equal(got(pool + MiB), inner)
+        zero = np.zeros(2 * MiB, dtype=np.uint8)
+        assert h.copy_data(zero.ctypes.data, pool, zero.size, bm.BmCopyType.H2GH, 0) == 0
+        return ok
+
+    bad = []
+    src, kind = at(outer.ctypes.data), int(bm.BmCopyType.H2GH)
+    for case in range(6):
+        keep = [at(outer.ctypes.data), at(inner.ctypes.data), at(pool), at(pool + MiB)]
+        if case == 0:      # while the destinations are read, the sources have been
+            rc = h.copy_data_batch(src, [_Inside(v, batch_inside if i == 3 else None) for i, v in enumerate(keep[2])], size, n, kind, 0)
+        elif case == 1:    # while the sizes are read
+            rc = h.copy_data_batch(src, keep[2], [_Inside(seg, batch_inside if i == 0 else None) for i in range(n)], n, kind, 0)
+        elif case == 2:    # in front of the C call
+            rc = h.copy_data_batch(src, keep[2], size, n, _Inside(kind, batch_inside), 0)
+        elif case == 3:
+            rc = h.copy_data(outer.ctypes.data, pool, outer.size, _Inside(kind, copy_inside), 0)
+        elif case == 4:
+            rc = h.copy_data_batch(src, keep[2], size, n, _Inside(kind, copy_inside), 0)
+        else:              # a conversion that fails leaves nothing behind for the next call
+            try:
+                h.copy_data_batch(src, keep[2][:2], size, n, kind, 0)
+                bad.append("short list taken")
+            except ValueError:
+                pass
+            batch_inside()
+            rc = h.copy_data_batch(src, keep[2], size, n, kind, 0)
+        if rc != 0 or not both_arrived():
+            bad.append((case, rc))
+    h.destroy()
+    bm.uninitialize(0)
+    mf.uninitialize()
+    return bad
+
+
+def test_a_copy_issued_inside_another_one_on_the_same_thread(store_url):
+    """The outer call keeps its own lists and pointers."""
+    assert run_ranks(_copies_inside_copies, 1, (store_url,), timeout=120) == [[]]
