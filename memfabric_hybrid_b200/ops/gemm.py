@@ -58,6 +58,10 @@ def _sms(device) -> int:
 
 
 def sm_count(device=None) -> int:
+    if device is not None and not isinstance(device, int):
+        device = torch.device(device)
+        if device.type == "cuda" and device.index is None:   # the current device, which may be another one at the next call
+            device = None
     return _sms(device if device is not None else torch.cuda.current_device())
 
 

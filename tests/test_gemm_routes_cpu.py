@@ -66,3 +66,30 @@ def test_rows_of_a_group_are_cut_into_tiles_without_gaps(steps, widest):
             assert mi > 0 or first.value == 0
             end = first.value + gran.value
         assert hi < cnt or end == steps
+
+
+def test_sm_count_of_a_device_without_an_index_follows_the_current_device(monkeypatch):
+    import types
+
+    import torch
+    from memfabric_hybrid_b200.ops import gemm
+
+    def props(device):
+        d = torch.device(device) if not isinstance(device, int) else torch.device("cuda", device)
+        if d.type != "cuda":
+            raise ValueError(f"Expected a cuda device, but got: {d}")
+        return types.SimpleNamespace(multi_processor_count=100 + (d.index if d.index is not None else torch.cuda.current_device()))
+
+    current = [0]
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: current[0])
+    monkeypatch.setattr(torch.cuda, "get_device_properties", props)
+    gemm._sms.cache_clear()
+    try:
+        for current[0] in (0, 1, 0):
+            want = 100 + current[0]
+            assert [gemm.sm_count(d) for d in (None, "cuda", torch.device("cuda"))] == [want] * 3
+            assert [gemm.sm_count(d) for d in (1, "cuda:1", torch.device("cuda", 1))] == [101] * 3
+            with pytest.raises(ValueError):
+                gemm.sm_count("cpu")
+    finally:
+        gemm._sms.cache_clear()
