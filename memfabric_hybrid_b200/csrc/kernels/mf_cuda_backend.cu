@@ -510,21 +510,25 @@ public:
         if (clear && v != 0) *reinterpret_cast<volatile uint32_t *>(copyStatus_) = 0;
         return v;
     }
-    // Lanes per unit, vectors per lane and units per step (at most nine loads per lane in flight) by the vectors of a unit: few lanes,
-    // of whose places few stay empty, but four at least (two read 32 bytes each at 256-byte distances: units of 128 47.9 us for 35.6).
+    // Lanes per unit, vectors per lane and units per step (at most nine loads per lane in flight) by the vectors of a unit: the fewest
+    // lanes that hold it, but four at least (two read 32 bytes each at 256-byte distances: units of 128 47.9 us for 35.6). Units just
+    // above a line leave up to half of the places empty, and still take less than in the general kernel; 512 items of 128 Ki bf16 values
+    // to int8, us, general kernel / here: 8 1603 / 198, 136 210 / 60, 264 136 / 54, 320 114 / 47, 584 93 / 55, 640 95 / 52, 1032 93 / 51.
     void LaunchQuantUnits(const mfk::QuantItem *q, uint32_t n, uint32_t vecs, uint64_t maxUnits, bool fp16, int mode, cudaStream_t st)
     {
-        // Blocks of one step of a CTA where all steps fit a grid that is resident at once (few items: 4 x 300 units of 128, int8, 11.1 us
-        // with two, 7.4 with one), else of two; no item is cut into more parts than it takes to give every CTA sixteen blocks.
-        auto go = [&](auto kern, uint32_t step, int perSm) {
-            const uint32_t resident = (uint32_t)(std::max(1, caps_.smCount) * perSm);
+        // Blocks of one step of a CTA where all steps fit three CTAs per SM (few items: 4 x 300 units of 128, int8, 11.1 us with two, 7.4 with
+        // one), else of two; no item is cut into more parts than it takes to give every CTA `each` blocks. A block costs a read of
+        // its descriptor from host memory, about 8 ns of the bus: with 16 blocks for each of the wide kernel's CTAs the descriptors of
+        // 512 items of 63 units of 2056 held the copy up (128 us; four 68, two 62).
+        auto go = [&](auto kern, uint32_t step, uint32_t perSm, uint32_t threads, uint64_t each) {
+            const uint32_t sms = (uint32_t)std::max(1, caps_.smCount), resident = sms * perSm;
             const uint64_t steps = (maxUnits + step - 1) / step;
-            const uint32_t parts = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(steps * n <= resident ? steps : (steps + 1) / 2, 16ull * resident / n));
-            kern<<<std::min(n * parts, resident), 256, 0, st>>>(q, n, parts, vecs);
+            const uint32_t parts = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(steps * n <= std::min(resident, 3 * sms) ? steps : (steps + 1) / 2, each * resident / n));
+            kern<<<std::min(n * parts, resident), threads, 0, st>>>(q, n, parts, vecs);
         };
 #define MF_QUANT_GO(MODE, W, R, J, V)                                                                                                       \
-    (fp16 ? go(mfk::mf_xcopy_quant_units_kernel<__half, MODE, W, R, J, V>, mfk::quant_step<W, J>(), mfk::kQuantCtasPerSm)                   \
-          : go(mfk::mf_xcopy_quant_units_kernel<__nv_bfloat16, MODE, W, R, J, V>, mfk::quant_step<W, J>(), mfk::kQuantCtasPerSm))
+    (fp16 ? go(mfk::mf_xcopy_quant_units_kernel<__half, MODE, W, R, J, V>, mfk::quant_step<W, J>(), mfk::kQuantCtasPerSm, 256, 16)          \
+          : go(mfk::mf_xcopy_quant_units_kernel<__nv_bfloat16, MODE, W, R, J, V>, mfk::quant_step<W, J>(), mfk::kQuantCtasPerSm, 256, 16))
         if (mode == 1) MF_QUANT_GO(1, 4, 4, 2, 16);  // units of 128 only
         else if (vecs <= 8) MF_QUANT_GO(0, 4, 2, 4, 0);
         else if (vecs == 16) MF_QUANT_GO(0, 4, 4, 2, 16);
@@ -534,8 +538,11 @@ public:
         else if (vecs <= 72) MF_QUANT_GO(0, 8, 9, 1, 0);
         else if (vecs <= 128) MF_QUANT_GO(0, 32, 4, 2, 0);
         else if (vecs <= 256) MF_QUANT_GO(0, 32, 8, 1, 0);
-        else if (fp16) go(mfk::mf_xcopy_quant_wide_kernel<__half>, 1, 4);
-        else go(mfk::mf_xcopy_quant_wide_kernel<__nv_bfloat16>, 1, 4);
+        else {
+            const uint32_t threads = mfk::quant_wide_threads(vecs);
+            if (fp16) go(mfk::mf_xcopy_quant_wide_kernel<__half>, 1, 1024 / threads, threads, 2);
+            else go(mfk::mf_xcopy_quant_wide_kernel<__nv_bfloat16>, 1, 1024 / threads, threads, 2);
+        }
 #undef MF_QUANT_GO
     }
     int LaunchQuantCopy(const QuantItem *items, uint32_t count, uint32_t unit, int inputFp16, int mode, void *s) override

@@ -467,23 +467,27 @@ __global__ void __launch_bounds__(256, kQuantCtasPerSm) mf_xcopy_quant_units_ker
     }
 }
 
-// Units of more vectors than a warp holds, up to 1024: the CTA shares a unit, four vectors per thread; the next unit's vectors are on
-// their way while this one is reduced and stored. 512 items of 126 Ki values, units of 7168 -> int8: 113 us above, 46 here.
+// Units of more vectors than a warp holds, up to 1024: the CTA shares a unit, four vectors per thread, and has the warps that takes
+// (quant_wide_threads); the next unit's vectors are on their way while this one is reduced and stored.
+// 512 items of 128 Ki bf16 values to int8, us, general kernel / 256 threads for every unit / so: 2056 100 / 126 / 62, 3072 101 / 105 / 50,
+// 4096 97 / 88 / 46, 5120 115 / 72 / 50, 7168 131 / 53 / 48, 8192 142 / 49 / 46.
+constexpr uint32_t kQuantWideVecs = 4;
+inline uint32_t quant_wide_threads(uint32_t vecs) { return (vecs + 32 * kQuantWideVecs - 1) / (32 * kQuantWideVecs) * 32; }
+
 template <typename In>
 __global__ void __launch_bounds__(256, 4) mf_xcopy_quant_wide_kernel(const QuantItem *__restrict__ items, uint32_t count, uint32_t parts, uint32_t vecs)
 {
     __shared__ QuantItem list[kQuantList];
     __shared__ float top[2][8];
-    constexpr int R = 4;
+    constexpr int R = kQuantWideVecs;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t blocks = count * parts;
     uint32_t parity = 0;
     for (uint32_t v0 = blockIdx.x; v0 < blocks; v0 += gridDim.x * kQuantList) {
         __syncthreads();
-        if (threadIdx.x < kQuantList * 4) {
-            const uint32_t v = v0 + (threadIdx.x >> 2) * gridDim.x;
-            if (v < blocks)
-                reinterpret_cast<uint64_t *>(list)[threadIdx.x] = reinterpret_cast<const uint64_t *>(items + v / parts)[threadIdx.x & 3];
+        for (uint32_t i = threadIdx.x; i < kQuantList * 4; i += blockDim.x) {
+            const uint32_t v = v0 + (i >> 2) * gridDim.x;
+            if (v < blocks) reinterpret_cast<uint64_t *>(list)[i] = reinterpret_cast<const uint64_t *>(items + v / parts)[i & 3];
         }
         __syncthreads();
         const uint32_t have = min(kQuantList, (blocks - v0 + gridDim.x - 1) / gridDim.x);
@@ -499,7 +503,7 @@ __global__ void __launch_bounds__(256, 4) mf_xcopy_quant_wide_kernel(const Quant
         auto load = [&](uint4 (&raw)[R]) {
 #pragma unroll
             for (int r = 0; r < R; r++) {
-                const uint32_t at = threadIdx.x + r * 256;
+                const uint32_t at = threadIdx.x + r * blockDim.x;
                 raw[r] = l < have && at < vecs ? __ldcs(reinterpret_cast<const uint4 *>(list[l].src) + u * vecs + at) : make_uint4(0, 0, 0, 0);
             }
         };
@@ -527,13 +531,14 @@ __global__ void __launch_bounds__(256, 4) mf_xcopy_quant_wide_kernel(const Quant
             __syncthreads();  // the other half of top is written by warps that have passed the next barrier
             float amax = 0.f;
 #pragma unroll
-            for (int w = 0; w < 8; w++) amax = fmaxf(amax, top[parity][w]);
+            for (int w = 0; w < 8; w++)
+                if (w < (int)(blockDim.x >> 5)) amax = fmaxf(amax, top[parity][w]);
             parity ^= 1;
             const float mul = amax > 0.f ? 127.f / amax : 1.f;
             if (threadIdx.x == 0) *scale = amax > 0.f ? amax / 127.f : 1.f;
 #pragma unroll
             for (int r = 0; r < R; r++) {
-                const uint32_t at = threadIdx.x + r * 256;
+                const uint32_t at = threadIdx.x + r * blockDim.x;
                 if (at < vecs) {
                     float f[8];
                     unpack8<In>(raw[r], f);

@@ -428,3 +428,61 @@ def test_quantising_copy_of_units_of_any_size():
     """int8 bytes and factors as the formula in fp32 gives them, nothing written behind them."""
     url = f"tcp://127.0.0.1:{free_port()}"
     assert run_ranks(_units_rank, 1, (url,), timeout=300) == [[]]
+
+
+def _wide_rank(rank, world, url):
+    import torch
+    import memfabric_hybrid as mf
+    from memfabric_hybrid import bm
+    from memfabric_hybrid_b200.ops.heap import tensor_at
+    torch.cuda.set_device(0)
+    torch.zeros(1, device="cuda")
+    assert mf.initialize() == 0
+    cfg = bm.BmConfig()
+    cfg.rank_id = 0
+    cfg.start_store = True
+    assert bm.initialize(url, 1, 0, cfg) == 0, mf.get_last_err_msg()
+    pool = 256 * MiB
+    h = bm.create2(id=14, local_dram_size=0, max_dram_size=0, local_hbm_size=pool, max_hbm_size=pool)
+    assert h.join() == 0, mf.get_last_err_msg()
+    base = h.peer_rank_ptr(0, bm.BmMemType.DEVICE)
+    bad = []
+    # units that a CTA shares, three warps to eight, both sides of each step, in items of one, two and many units; then more items than 32 for every
+    # CTA of the grid, so that a CTA fetches a second list of descriptors: 444 CTAs, 1480 of three warps, 592 of eight
+    cases = [(u, per, n) for u in (2056, 3072, 3080, 4096, 4104, 5128, 6152, 7176, 8192) for per, n in ((1, 5), (2, 700), (37, 3), (400, 2))]
+    cases += [(64, 1, 15000), (2056, 1, 47500), (8192, 1, 19500)]
+    for unit, per, n in cases:
+        dt = torch.float16 if unit % 16 == 8 else torch.bfloat16
+        each = unit * per
+        x = torch.randn(n * per, unit, device="cuda", generator=torch.Generator("cuda").manual_seed(unit + n)).to(dt)
+        x[n * per // 2] = 0
+        fac = base + (n * each + 64 + 255) // 256 * 256
+        q, f = tensor_at(base, (n * each + 64,), torch.uint8), tensor_at(fac, (n * per + 1,), torch.float32)
+        q.fill_(77)
+        f.fill_(-5)
+        torch.cuda.synchronize()
+        at = range(n)
+        assert h.quant_copy_batch([x.data_ptr() + i * each * 2 for i in at], [base + i * each for i in at], [each * 2] * n, [fac + i * per * 4 for i in at], unit,
+                                  fp16_input=dt == torch.float16) == 0, mf.get_last_err_msg()
+        amax = x.abs().amax(1).float()
+        one, top = torch.ones_like(amax), torch.full_like(amax, 127.0)
+        mul = torch.where(amax > 0, top / amax, one)
+        ok = torch.equal(f[:n * per], torch.where(amax > 0, amax / top, one)) and bool((q[n * each:] == 77).all()) and float(f[n * per]) == -5
+        got = q[:n * each].view(n * per, unit)
+        for lo in range(0, n * per, 4096):   # in bands: the fp32 values of all items would be 2.5 times the pool
+            want = (x[lo:lo + 4096].float() * mul[lo:lo + 4096, None]).round().clamp(-127, 127).to(torch.int8).view(torch.uint8)
+            ok = ok and torch.equal(got[lo:lo + 4096], want)
+        if not ok:
+            bad.append((unit, per, n))
+        del x
+    h.leave()
+    h.destroy()
+    bm.uninitialize(0)
+    mf.uninitialize()
+    return bad
+
+
+def test_quantising_copy_of_wide_units_and_of_more_items_than_a_list_holds():
+    """int8 bytes and factors as the formula in fp32 gives them, nothing written behind them."""
+    url = f"tcp://127.0.0.1:{free_port()}"
+    assert run_ranks(_wide_rank, 1, (url,), timeout=300) == [[]]
