@@ -56,6 +56,14 @@ template <int VN> __device__ __forceinline__ Range cta_range(uint64_t count)
 
 __device__ __forceinline__ bool aligned16(const void *p) { return (reinterpret_cast<uint64_t>(p) & 15) == 0; }
 
+// Whether the caller's input and output (all ranks', when emulating) share no memory. Where they do, a rank's own part goes through its staging area
+// like the others: it is then read in front of the exchange and written behind it.
+__device__ __forceinline__ bool apart(const CollArgs &a, uint64_t in_bytes, uint64_t out_bytes)
+{
+    const uint64_t more = a.team.emu ? a.team.world - 1 : 0;
+    return a.in + more * a.in_rank_stride + in_bytes <= a.out || a.out + more * a.out_rank_stride + out_bytes <= a.in;
+}
+
 // dst[i] = (TD)(src[i] * scale) for i in [beg, end): 16-byte vectors where both ends allow it
 template <typename TS, typename TD>
 __device__ __forceinline__ void cta_convert_copy(const TS *__restrict__ src, TD *__restrict__ dst, uint64_t beg, uint64_t end, float scale)
@@ -294,7 +302,8 @@ template <typename T, typename TO, bool INT, int W> __global__ void __launch_bou
     uint64_t C = (a.n + world - 1) / world;
     C = (C + 7) / 8 * 8;
     const Range sub = cta_range<8>(C);
-    const bool own = !a.zero_copy && aligned16(in);  // nobody else reads the part that this rank reduces
+    // nobody else reads the part that this rank reduces, and nobody writes to any output before all ranks have read theirs (second exchange)
+    const bool own = !a.zero_copy && aligned16(in);
     MF_PROF_START(PF_STAGE_IN);
     if (!a.zero_copy) {
         for (uint32_t c = 0; c < world; c++) {
@@ -354,7 +363,9 @@ template <typename T, typename TO, bool INT, int W> __global__ void __launch_bou
     const uint64_t ps = a.part_stride ? a.part_stride : m;
     // staged rows start on 16 bytes whatever m is (input that sits in the staging area already is packed)
     const uint64_t mp = a.zero_copy ? m : (m + 7) / 8 * 8;
-    const bool own = !a.zero_copy && aligned16(in + (uint64_t)me * ps);  // nobody else reads the part that this rank reduces
+    // Nobody else reads the part that this rank reduces. In place, an element is read and written by the same thread.
+    const bool in_place = sizeof(T) == sizeof(TO) && !a.team.emu && (uint64_t)out == (uint64_t)(in + (uint64_t)me * ps);
+    const bool own = !a.zero_copy && aligned16(in + (uint64_t)me * ps) && (in_place || apart(a, ((world - 1) * ps + m) * sizeof(T), m * sizeof(TO)));
     if (!a.zero_copy)
         for (uint32_t c = 0; c < world; c++)
             if (!own || c != me) cta_raw_copy<T>(in + c * ps, myA + c * mp, sub.beg, sub.end);
@@ -376,7 +387,9 @@ template <typename T, typename TO> __global__ void __launch_bounds__(512) k_allg
     const uint64_t np = (a.n + 7) / 8 * 8;  // staged rows start on 16 bytes whatever n is
     const uint64_t ps = a.part_stride ? a.part_stride : a.n;
     // the rank's own shard goes straight to its place, where that is as well aligned as a staged row
-    const bool own = sizeof(T) == sizeof(TO) && a.scale == 1.f && aligned16(out + (uint64_t)me * ps);
+    const bool in_place = !a.team.emu && (uint64_t)in == (uint64_t)(out + (uint64_t)me * ps);
+    const bool own = sizeof(T) == sizeof(TO) && a.scale == 1.f && aligned16(out + (uint64_t)me * ps) &&
+                     (in_place || apart(a, a.n * sizeof(T), ((world - 1) * ps + a.n) * sizeof(TO)));
     if (sizeof(T) == sizeof(TO) && a.scale == 1.f) {
         // same type, no scaling: the shard is read once and fanned out to every rank's staging area
         __shared__ TO *dsts[kMaxRanks];

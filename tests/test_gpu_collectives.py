@@ -86,6 +86,72 @@ def test_reduce_scatter_all_gather(comms, world, dtype, m):
         assert torch.equal(agc[0].view(world, m), shard.to(torch.bfloat16))
 
 
+def _rank_order_sum(x):
+    """fp32 sum of the ranks' rows in rank order, rounded once: what every rank has to hold, bit for bit."""
+    acc = x[0].float()
+    for r in range(1, x.shape[0]):
+        acc = acc + x[r].float()
+    return acc.to(x.dtype)
+
+
+@pytest.mark.parametrize("world", [2, 8])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n", [8, 1001, 4096, 70_001, 1_500_001])
+def test_two_shot_all_reduce_in_place_and_off_16_bytes(comms, world, dtype, n):
+    """A rank's own part is read from the input behind the first exchange, where it lies on 16 bytes; odd rows put some ranks' inputs off them. The
+    largest size takes several pieces."""
+    c = comms[world]
+    x = torch.randn(world, n, device="cuda", generator=torch.Generator("cuda").manual_seed(n)).to(dtype)
+    want = _rank_order_sum(x).expand(world, n)
+    assert torch.equal(c.all_reduce(x, algo="twoshot"), want)
+    y = x.clone()
+    assert c.all_reduce(y, out=y, algo="twoshot") is y and torch.equal(y, want)
+    shifted = torch.empty(world * n + 3, dtype=dtype, device="cuda")[3:].view(world, n)
+    shifted.copy_(x)
+    assert torch.equal(c.all_reduce(shifted, out=shifted, algo="twoshot"), want)
+
+
+@pytest.mark.parametrize("world", [2, 8])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("m", [8, 125, 1001, 60_001])
+def test_reduce_scatter_and_all_gather_of_odd_parts(comms, world, dtype, m):
+    """Parts that start on and off 16 bytes, next to outputs that nothing else may be written to."""
+    c = comms[world]
+    gen = torch.Generator("cuda").manual_seed(m)
+    x = torch.randn(world, world * m, device="cuda", generator=gen).to(dtype)
+    assert torch.equal(c.reduce_scatter(x), _rank_order_sum(x).view(world, m))
+    shard = torch.randn(world, m, device="cuda", generator=gen).to(dtype)
+    room = torch.full((world * world * m + 8,), 7.0, device="cuda").to(dtype)
+    out = room[3:3 + world * world * m].view(world, world * m)
+    c.all_gather(shard, out=out)
+    assert torch.equal(out, shard.reshape(1, -1).expand(world, -1))
+    assert bool((room[:3] == 7).all()) and bool((room[3 + world * world * m:] == 7).all())
+
+
+@pytest.mark.parametrize("world", [2, 8])
+def test_reduce_scatter_and_all_gather_whose_output_lies_in_the_input(comms, world):
+    """One CTA per rank: the exchange stands between the last read of any input and the first write to any output, so that every overlap is fine,
+    of another type too."""
+    c = comms[world]
+    m = 4096 // world // world
+    x0 = torch.randn(world, world * m, device="cuda", generator=torch.Generator("cuda").manual_seed(world))
+    want = _rank_order_sum(x0).view(world, m)
+    for off in (0, 4, 5, m, (world - 1) * (world * m)):
+        x = x0.clone()
+        assert torch.equal(c.reduce_scatter(x, out=x.view(-1)[off:off + world * m].view(world, m)), want), off
+        x = x0.clone()
+        out = x.view(-1).view(torch.bfloat16)[off * 2:off * 2 + world * m].view(world, m)
+        assert torch.equal(c.reduce_scatter(x, out=out, out_dtype=torch.bfloat16), want.to(torch.bfloat16)), off
+    m = 8192 // world
+    shard = torch.randn(world, m, device="cuda", generator=torch.Generator("cuda").manual_seed(world)).to(torch.bfloat16)
+    for off in (0, 3, 8, m, (world - 1) * world * m):
+        out = torch.zeros(world, world * m, device="cuda", dtype=torch.bfloat16)
+        x = out.view(-1)[off:off + world * m].view(world, m)
+        x.copy_(shard)
+        c.all_gather(x, out=out)
+        assert torch.equal(out, shard.reshape(1, -1).expand(world, -1)), off
+
+
 @pytest.mark.parametrize("world", [2, 8])
 def test_broadcast_scatter_alltoallv(comms, world):
     c = comms[world]
