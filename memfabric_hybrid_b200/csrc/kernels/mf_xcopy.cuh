@@ -98,7 +98,9 @@ __device__ __forceinline__ void cta_copy(const uint8_t *__restrict__ src, uint8_
 // and nothing but the list's end holds its warps back: a warp that has no vectors left in one chunk is already in the next. With a
 // descriptor and a barrier per chunk (one descriptor ahead), us before / now: 700 pieces of 256 B - 512 KiB at 2-byte offsets 26.2 / 24.5,
 // 1500 of up to 16 KiB at any offset 15.0 / 12.2, 200 of up to 512 KiB at 8-byte offsets 11.9 / 10.1. (Warps that take pieces of 2 to
-// 16 KiB by themselves: 9.7 for the 1500, but 26.6 for the 700.)
+// 16 KiB by themselves: 9.7 for the 1500, but 26.6 for the 700.) Where no CTA has more than one chunk a list
+// and its barriers are in the way: replayed from a graph, one piece of up to 1 KiB takes 2.4 us with the single descriptor, 2.7 to 2.9 with a
+// list; 20 pieces of up to 16 KiB 3.8 and 4.2, 100 of them 4.1 and 4.4.
 __global__ void __launch_bounds__(kCopyThreads) mf_xcopy_batch_kernel(const CopyItem *__restrict__ items, uint32_t count,
                                                                       const CopyWindow *__restrict__ window, uint32_t *status)
 {
@@ -110,9 +112,16 @@ __global__ void __launch_bounds__(kCopyThreads) mf_xcopy_batch_kernel(const Copy
         const uint64_t i = first + (uint64_t)slot * gridDim.x;
         return slot < kCopyList && i < count ? reinterpret_cast<const uint64_t *>(items + i)[word] : 0;
     };
+    if (blockIdx.x >= count) return;
+    if (count <= gridDim.x) {
+        const CopyItem it = items[blockIdx.x];
+        if (window == nullptr || xc_check(window, it.src, it.dst, it.len, status))
+            cta_copy(reinterpret_cast<const uint8_t *>(it.src), reinterpret_cast<uint8_t *>(it.dst), it.len);
+        return;
+    }
     uint64_t next = fetch(blockIdx.x);
     for (uint64_t first = blockIdx.x; first < count; first += round) {
-        __syncthreads();  // the previous list is no longer read
+        if (first != blockIdx.x) __syncthreads();  // the previous list is no longer read
         if (slot < kCopyList) list[threadIdx.x] = next;
         __syncthreads();
         next = fetch(first + round);  // arrives while this list's chunks are copied

@@ -486,3 +486,74 @@ def test_quantising_copy_of_wide_units_and_of_more_items_than_a_list_holds():
     """int8 bytes and factors as the formula in fp32 gives them, nothing written behind them."""
     url = f"tcp://127.0.0.1:{free_port()}"
     assert run_ranks(_wide_rank, 1, (url,), timeout=300) == [[]]
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 63, 64, 65, 129, 1000])
+def test_register_copy_takes_one_list_of_descriptors_after_another(n):
+    """Two CTAs, 32 descriptors in a list: a CTA without any, one descriptor each, part of a list, a full one, several; pieces at odd offsets, nothing
+    written between them."""
+    import ctypes as C
+    import torch
+    from memfabric_hybrid_b200 import _native as N
+    cu = N.cuda()
+    cu.mf_xcopy_debug_probe.restype = C.c_int
+    cu.mf_xcopy_debug_probe.argtypes = [C.POINTER(C.c_uint64), C.c_uint32, C.c_uint64, C.c_uint64, C.c_uint32, C.POINTER(C.c_uint64), C.c_int]
+    r = np.random.default_rng(n)
+    size = r.integers(1, 3000, n)
+    s_off = np.concatenate(([0], np.cumsum(size + r.integers(1, 40, n))))
+    d_off = np.concatenate(([0], np.cumsum(size + r.integers(1, 40, n))))
+    src = torch.randint(1, 256, (int(s_off[-1]),), dtype=torch.uint8, device="cuda")
+    dst = torch.zeros(int(d_off[-1]) + 64, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    trip = np.stack([src.data_ptr() + s_off[:-1], dst.data_ptr() + d_off[:-1], size], 1).reshape(-1)
+    assert cu.mf_xcopy_debug_probe((C.c_uint64 * (3 * n))(*map(int, trip)), n, 0, 0, 0, None, 0) == 0
+    torch.cuda.synchronize()
+    a, got, want = src.cpu().numpy(), dst.cpu().numpy(), np.zeros(dst.numel(), dtype=np.uint8)
+    for s, d, k in zip(s_off, d_off, size):
+        want[d:d + k] = a[s:s + k]
+    assert np.array_equal(got, want)
+
+
+def _many_pieces_rank(rank, world, url):
+    import torch
+    import memfabric_hybrid as mf
+    from memfabric_hybrid import bm
+    from memfabric_hybrid_b200.ops.heap import tensor_at
+    torch.cuda.set_device(0)
+    torch.zeros(1, device="cuda")
+    assert mf.initialize() == 0
+    cfg = bm.BmConfig()
+    cfg.rank_id = 0
+    cfg.start_store = True
+    assert bm.initialize(url, 1, 0, cfg) == 0, mf.get_last_err_msg()
+    h = bm.create2(id=15, local_dram_size=0, max_dram_size=0, local_hbm_size=64 * MiB, max_hbm_size=64 * MiB)
+    assert h.join() == 0, mf.get_last_err_msg()
+    base = h.peer_rank_ptr(0, bm.BmMemType.DEVICE)
+    bad = []
+    # the register copy's grid is 296 CTAs here: one chunk each, a second one for a few, a full list each, and a second and third list
+    for n in (1, 200, 296, 297, 9472, 9473, 20000):
+        r = np.random.default_rng(n)
+        size = r.integers(1, 1500, n)
+        s_off = np.concatenate(([1], 1 + np.cumsum(size + r.integers(1, 40, n))))
+        d_off = np.concatenate(([2], 2 + np.cumsum(size + r.integers(1, 40, n))))
+        src = torch.randint(1, 256, (int(s_off[-1]),), dtype=torch.uint8, device="cuda")
+        pool = tensor_at(base, (int(d_off[-1]) + 64,), torch.uint8)
+        pool.zero_()
+        torch.cuda.synchronize()
+        lists = [src.data_ptr() + s_off[:-1].astype(np.uint64), base + d_off[:-1].astype(np.uint64), size.astype(np.uint64)]
+        assert h.copy_data_batch(*lists, n, bm.BmCopyType.L2G, 0) == 0, mf.get_last_err_msg()
+        a, got, want = src.cpu().numpy(), pool.cpu().numpy(), np.zeros(pool.numel(), dtype=np.uint8)
+        for s, d, k in zip(s_off, d_off, size):
+            want[d:d + k] = a[s:s + k]
+        if not np.array_equal(got, want):
+            bad.append(n)
+    h.leave()
+    h.destroy()
+    bm.uninitialize(0)
+    mf.uninitialize()
+    return bad
+
+
+def test_batches_of_more_pieces_than_the_ctas_lists_hold():
+    url = f"tcp://127.0.0.1:{free_port()}"
+    assert run_ranks(_many_pieces_rank, 1, (url,), timeout=300) == [[]]
