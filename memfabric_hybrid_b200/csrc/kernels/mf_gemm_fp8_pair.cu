@@ -18,7 +18,7 @@
 // The scales must be powers of two (every quantiser of this library produces such scales): a producer warp turns them into UE8M0 bytes
 // (the fp32 exponent) in the tensor core's layout in shared memory, four K blocks per 32-bit word; the leader's MMA thread
 // copies a group of them into both CTAs' tensor memory (tcgen05.cp) and picks the byte of the K block through the instruction descriptor.
-// Warps: 0 TMA, 1 MMA (leader; + TMEM allocation), 2 scale producer, 4..11 epilogue (two per TMEM lane quadrant, alternate 32-row chunks).
+// Warps: 0 TMA, 1 MMA (leader; + TMEM allocation), 2 and 3 scale producers, 4..11 epilogue (two per TMEM lane quadrant, alternate 32-row chunks).
 // Accumulators are transposed: a TMEM lane is an output column (a row of W), a TMEM column is a row of X.
 // Epilogues (rows leave through shared memory, so that a row's columns are stored in contiguous pieces):
 //   EPI 0  plain            : bf16 rows to local memory
@@ -135,6 +135,36 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) { return as_u3
 // 3 * 10^4 rounds to another bf16 value.)
 __device__ __forceinline__ float swiglu(float gate, float up) { return gate / (1.f + __expf(-gate)) * up; }
 
+// The first `have` (at most four) of the scales at s as they lie in memory, 1.0 for the others. `vec`: s is 16-byte aligned and `have` a multiple of
+// four. Predicated loads: with a branch around each, the next one waited for the one in front of it.
+__device__ __forceinline__ void load_scales(const float *s, int have, bool vec, uint32_t (&f)[4])
+{
+    asm volatile(
+        "{\n\t.reg .pred v, p0, p1, p2, p3;\n\t.reg .b32 m;\n\t"
+        "mov.b32 %0, 0x3f800000;\n\tmov.b32 %1, 0x3f800000;\n\tmov.b32 %2, 0x3f800000;\n\tmov.b32 %3, 0x3f800000;\n\t"
+        "setp.ne.s32 v, %6, 0;\n\t"
+        "setp.gt.and.s32 p0, %5, 0, v;\n\t"
+        "@p0 ld.global.v4.b32 {%0, %1, %2, %3}, [%4];\n\t"
+        "selp.b32 m, 0, %5, v;\n\t"
+        "setp.gt.s32 p0, m, 0;\n\t"
+        "setp.gt.s32 p1, m, 1;\n\t"
+        "setp.gt.s32 p2, m, 2;\n\t"
+        "setp.gt.s32 p3, m, 3;\n\t"
+        "@p0 ld.global.b32 %0, [%4];\n\t"
+        "@p1 ld.global.b32 %1, [%4 + 4];\n\t"
+        "@p2 ld.global.b32 %2, [%4 + 8];\n\t"
+        "@p3 ld.global.b32 %3, [%4 + 12];\n\t}"
+        : "=&r"(f[0]), "=&r"(f[1]), "=&r"(f[2]), "=&r"(f[3])
+        : "l"(s), "r"(have), "r"((int)vec)
+        : "memory");
+}
+
+// The exponent bytes (UE8M0) of four floats.
+__device__ __forceinline__ uint32_t exponents(const uint32_t (&f)[4])
+{
+    return __byte_perm(__byte_perm(f[0] << 1, f[1] << 1, 0x0073), __byte_perm(f[2] << 1, f[3] << 1, 0x0073), 0x5410);
+}
+
 // Ring position for a number of slots known at run time.
 struct RingState {
     int slot = 0;
@@ -186,7 +216,7 @@ template <int EPI> __global__ void __launch_bounds__(kPThreads, 1) k_grouped_fp8
             mbar_init(sm.empty(s), 1);
         }
         for (int i = 0; i < kPSfBufs; i++) {
-            mbar_init(sm.sf_full(i), 2);   // the scale producers of both CTAs (counted in the leader)
+            mbar_init(sm.sf_full(i), 4);   // the scale producers of both CTAs (counted in the leader)
             mbar_init(sm.sf_empty(i), 1);
         }
         for (int i = 0; i < 2; i++) {
@@ -357,45 +387,42 @@ template <int EPI> __global__ void __launch_bounds__(kPThreads, 1) k_grouped_fp8
                 if (acc == 0) acc_phase ^= 1;
             }
         }
-    } else if (warp == 2) {
-        // scale producer: one 32-bit word of four K-block scale bytes per operand row. Lane l writes the 16 bytes of rows l, l + 32, l + 64,
-        // l + 96 of a chunk: this CTA's 128 rows of W, and all rows of X. The scales of 16 K blocks go over at once. Each CTA's tensor
-        // core copies its own chunks, but the leader has both do it, so the other CTA's bytes are released to the cluster: the
-        // proxy fence, then a release of shared memory alone. A full release waits for the SM's outstanding loads as well: 32 experts of about
-        // 32 rows, 4096 x 7168: 161 us with it, 149.4 so (148.4 without any order), 227 with a full release per four K blocks.
+    } else if (warp < 4) {
+        // scale producers: one 32-bit word of four K-block scale bytes per operand row; the two warps take alternate words. Lane l writes the
+        // 16 bytes of rows l, l + 32, l + 64, l + 96 of a chunk: this CTA's 128 rows of W, and all rows of X. The scales of 16 K blocks go
+        // over at once. Each CTA's tensor core copies its own chunks, but the leader has both do it, so the other CTA's bytes are
+        // released to the cluster: the proxy fence, then a release of shared memory alone. A full release waits for the SM's outstanding
+        // loads as well: 32 experts of about 32 rows, 4096 x 7168: 161 us with it, 149.4 so (148.4 without any order), 227 with a full release
+        // per four K blocks.
+        // A tile of few K blocks takes as long as its scales: two warps, and all loads of a span issued before the first is used, without
+        // branches between them. 32 experts of about 512 rows, N 4096, EPI 0, us, one warp that branches between aligned and single loads /
+        // so: K 128 77 / 49, 384 87 / 52, 512 56 / 54, 768 120 / 66, 1024 79 / 78 (tiles of 128 x 256 on single CTAs: 56, 61, 62, 73, 86).
+        const int part = warp - 2;
         RingState sf;
         PTile p;
         const int nblocks = g.N / 128;
         const bool vec = (k_blocks & 3) == 0 && ((reinterpret_cast<uintptr_t>(g.x_scale) | reinterpret_cast<uintptr_t>(g.w_scale)) & 15) == 0;
         bool fine = true;
-        // scales of K blocks kb .. kb + 3 as one word; past the end of K: 1.0
-        auto word = [&](const float *s, int kb) -> uint32_t {
-            if (kb >= k_blocks) return 0x7f7f7f7fu;
-            if (vec) {
-                const float4 f = *reinterpret_cast<const float4 *>(s + kb);
-                return ue8m0_byte(f.x) | ue8m0_byte(f.y) << 8 | ue8m0_byte(f.z) << 16 | ue8m0_byte(f.w) << 24;
-            }
-            uint32_t w = 0;
-#pragma unroll
-            for (int j = 0; j < 4; j++) w |= (kb + j < k_blocks ? ue8m0_byte(s[kb + j]) : 127u) << (8 * j);
-            return w;
-        };
         for (int t = walker; t < total && fine; t += walkers) {
             locate(t, p);
             // the 128-row block of W: SwiGLU: gate rows nt * 128 .. in lanes 0-15, up rows N/2 + nt * 128 .. in lanes 16-31
             const int nb = kSwiGLU ? (lane < 16 ? p.nt : nblocks / 2 + p.nt) : 2 * p.nt + (int)crank;
             const float *ws = g.w_scale + ((int64_t)p.grp * nblocks + nb) * k_blocks;
-            const float *xs[kMaxGran + 1];
+            const float *xs[kMaxGran];
 #pragma unroll
-            for (int i = 0; i <= kMaxGran; i++) xs[i] = g.x_scale + (int64_t)min(p.row0 + i * kGran + lane, g.max_rows - 1) * k_blocks;
+            for (int i = 0; i < kMaxGran; i++) xs[i] = g.x_scale + (int64_t)min(p.row0 + i * kGran + lane, g.max_rows - 1) * k_blocks;
             for (int sp = 0; sp < sf_spans; sp++) {
-                uint32_t ww[kSfSpan / 4], wx[kSfSpan / 4][kMaxGran + 1];
+                uint32_t raw[kSfSpan / 8][kMaxGran + 1][4], wrd[kSfSpan / 8][kMaxGran + 1];  // [..][kMaxGran]: W
 #pragma unroll
-                for (int q = 0; q < kSfSpan / 4; q++) {
-                    ww[q] = word(ws, sp * kSfSpan + q * 4);
+                for (int h = 0; h < kSfSpan / 8; h++) {
+                    const int kb = sp * kSfSpan + (2 * h + part) * 4;
 #pragma unroll
-                    for (int i = 0; i <= kMaxGran; i++) wx[q][i] = i < p.gran ? word(xs[i], sp * kSfSpan + q * 4) : 0x7f7f7f7fu;
+                    for (int i = 0; i <= kMaxGran; i++) load_scales((i < kMaxGran ? xs[i] : ws) + kb, i < kMaxGran && i >= p.gran ? 0 : k_blocks - kb, vec, raw[h][i]);
                 }
+#pragma unroll
+                for (int h = 0; h < kSfSpan / 8; h++)
+#pragma unroll
+                    for (int i = 0; i <= kMaxGran; i++) wrd[h][i] = exponents(raw[h][i]);
                 int ok = 1;
                 if (lane == 0) ok = mbar_wait(sm.sf_empty(sf.slot), sf.phase ^ 1, ac, 0x607) ? 1 : 0;
                 ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -405,11 +432,12 @@ template <int EPI> __global__ void __launch_bounds__(kPThreads, 1) k_grouped_fp8
                     break;
                 }
 #pragma unroll
-                for (int q = 0; q < kSfSpan / 4; q++) {
-                    uint8_t *chunk = sm.sf(sf.slot) + q * PSmem::kSfChunk;
-                    *reinterpret_cast<uint4 *>(chunk + lane * 16) = make_uint4(ww[q], ww[q], ww[q], ww[q]);
-                    *reinterpret_cast<uint4 *>(chunk + 512 + lane * 16) = make_uint4(wx[q][0], wx[q][1], wx[q][2], wx[q][3]);
-                    *reinterpret_cast<uint4 *>(chunk + 1024 + lane * 16) = make_uint4(wx[q][4], wx[q][5], wx[q][6], wx[q][7]);
+                for (int h = 0; h < kSfSpan / 8; h++) {
+                    uint8_t *chunk = sm.sf(sf.slot) + (2 * h + part) * PSmem::kSfChunk;
+                    const uint32_t w = wrd[h][kMaxGran];
+                    *reinterpret_cast<uint4 *>(chunk + lane * 16) = make_uint4(w, w, w, w);
+                    *reinterpret_cast<uint4 *>(chunk + 512 + lane * 16) = make_uint4(wrd[h][0], wrd[h][1], wrd[h][2], wrd[h][3]);
+                    *reinterpret_cast<uint4 *>(chunk + 1024 + lane * 16) = make_uint4(wrd[h][4], wrd[h][5], wrd[h][6], 0x7f7f7f7fu);
                 }
                 fence_proxy_async_smem();  // the tensor core's copy unit reads these bytes through the async proxy
                 __syncwarp();

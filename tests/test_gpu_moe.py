@@ -175,6 +175,35 @@ def test_grouped_gemm_fp8_tile_widths(N, K, counts):
     assert bool((hq3[bad] & 0x7F == 0x7F).all()) and bool((hs3[bad] == 1).all())
 
 
+@pytest.mark.parametrize("K", [128, 384, 512, 2560])
+def test_grouped_gemm_fp8_scales_on_and_off_16_bytes(K):
+    """Rows of scales that start on 16 bytes are read four at a time, others one by one: the same bytes, with scales that differ from row to row and
+    block to block, in front of a last span of 16 blocks that is not full (2560: 20 blocks)."""
+    from memfabric_hybrid_b200.ops import gemm, moe as M
+    cu = M._cu()
+    G, N, counts = 3, 512, [300, 1, 95]
+    R, kb = sum(counts), K // 128
+    gen = torch.Generator("cuda").manual_seed(K)
+    off = torch.tensor([0, 300, 301, R], dtype=torch.int32, device="cuda")
+    x = torch.randint(-8, 9, (R, K), generator=gen, device="cuda").float().to(torch.float8_e4m3fn)
+    w = torch.randint(-8, 9, (G, N, K), generator=gen, device="cuda").float().to(torch.float8_e4m3fn)
+    xs = 2.0 ** torch.randint(-3, 4, (R, kb), generator=gen, device="cuda").float()
+    ws = 2.0 ** torch.randint(-3, 4, (G, N // 128, kb), generator=gen, device="cuda").float()
+    ref = torch.cat([_deq(x[off[g]:off[g + 1]], xs[off[g]:off[g + 1]]).double() @ _deq_w(w[g], ws[g]).double().t() for g in range(G)])
+    st, s = gemm.status_word(), torch.cuda.current_stream().cuda_stream
+    for shift in (0, 1):   # floats by which both arrays of scales are moved off 16 bytes
+        xo, wo = (torch.full((t.numel() + 8,), float("nan"), device="cuda")[shift:shift + t.numel()].view(t.shape) for t in (xs, ws))
+        xo.copy_(xs)
+        wo.copy_(ws)
+        out = torch.zeros(R, N, dtype=torch.bfloat16, device="cuda")
+        assert cu.mf_grouped_gemm_fp8_mx(x.data_ptr(), xo.data_ptr(), R, w.data_ptr(), wo.data_ptr(), off.data_ptr(), G, N, K, out.data_ptr(), N, None, 0, None,
+                                         None, 0, 1, st.data_ptr(), gemm.sm_count(), s) == 0
+        torch.cuda.synchronize()
+        gemm.check_status()
+        # whole numbers times powers of two that span 2^12: 13 + 12 bits, up to one unit of fp32 in the sum, and one rounding to bf16
+        assert bool(((out.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + ref.abs().max() * 2.0 ** -22).all()), shift
+
+
 def test_swiglu_of_the_expert_kernels_is_the_same():
     """Small whole numbers: both kernels' sums are exact (14 bits), so that every bf16 activation has to be the same one, and with it
     every byte of a layer that changes its kernel with its shape. 2 M activations: a quotient one unit of fp32 off moves a few dozen."""
