@@ -130,10 +130,37 @@ __device__ __forceinline__ __nv_bfloat162 as_bf162(uint32_t v) { return *reinter
 __device__ __forceinline__ uint32_t as_u32(__nv_bfloat162 v) { return *reinterpret_cast<const uint32_t *>(&v); }
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) { return as_u32(__floats2bfloat162_rn(lo, hi)); }
 
-// silu(gate) * up, with the division that every other SwiGLU epilogue of the library has: the same activations round to the same bytes
-// whichever kernel takes a layer's shape. (With the hardware's approximate reciprocal 0.7 to 2.4 us of 106 to 742 less, and one activation in
-// 3 * 10^4 rounds to another bf16 value.)
+// silu(gate) * up as every other SwiGLU epilogue of the library has it, with its division: the same activations round to the same bytes whichever
+// kernel takes a layer's shape.
 __device__ __forceinline__ float swiglu(float gate, float up) { return gate / (1.f + __expf(-gate)) * up; }
+
+// The same value for |gate| < 80, where the divisor lies in [1, 2^116) and nothing overflows, without the branches that the general division has:
+// a reciprocal with one Newton step, a quotient, and the quotient corrected by its exact remainder, which rounds it as the division
+// does (P. Markstein, Computation of elementary functions on the IBM RISC System/6000 processor, 1990). The quotient depends on the gate alone and
+// has been compared with the division for every float (mf_swiglu_debug_probe). A warp divides where one of its gates is out of the range.
+// Re-quantising epilogue, 32 experts of about 512 rows, N 4096, us, division / so / approximate reciprocal: K 512 140 / 110 / 104, 2048 163 / 143 /
+// 141, 4096 258 / 252 / 251 (tiles of 128 x 256 rows on single CTAs: 110, 147, 261).
+__device__ __forceinline__ bool swiglu_in_range(float gate) { return fabsf(gate) < 80.f; }
+__device__ __forceinline__ float swiglu_fast(float gate, float up)
+{
+    const float d = 1.f + __expf(-gate);
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    r = __fmaf_rn(__fmaf_rn(-d, r, 1.f), r, r);
+    const float q = __fmul_rn(gate, r);
+    return __fmaf_rn(-__fmaf_rn(d, q, -gate), r, q) * up;  // the remainder as d * q - gate: a gate of -0 keeps its sign
+}
+
+// Debug aid: counts the gates among `count` bit patterns from `first` on whose two quotients differ.
+__global__ void k_swiglu_probe(uint32_t first, uint64_t count, unsigned long long *differ)
+{
+    unsigned long long bad = 0;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < count; i += (uint64_t)gridDim.x * blockDim.x) {
+        const float gate = __uint_as_float(first + (uint32_t)i);
+        if (swiglu_in_range(gate) && __float_as_uint(swiglu_fast(gate, 1.f)) != __float_as_uint(swiglu(gate, 1.f))) bad++;
+    }
+    if (bad != 0) atomicAdd(differ, bad);
+}
 
 // The first `have` (at most four) of the scales at s as they lie in memory, 1.0 for the others. `vec`: s is 16-byte aligned and `have` a multiple of
 // four. Predicated loads: with a branch around each, the next one waited for the one in front of it.
@@ -542,10 +569,20 @@ template <int EPI> __global__ void __launch_bounds__(kPThreads, 1) k_grouped_fp8
                     tmem_ld_frag(taddr + (16u << 16) + (uint32_t)((set + 2 * i) * kGran), up);
                     tmem_ld_wait();
                     if (i == last) release();
+                    bool in_range = true;
 #pragma unroll
-                    for (int j = 0; j < 8; j++)
-                        ob[i][j] = pack_bf16(swiglu(__uint_as_float(gt[2 * j]), __uint_as_float(up[2 * j])),
-                                             swiglu(__uint_as_float(gt[2 * j + 1]), __uint_as_float(up[2 * j + 1])));
+                    for (int j = 0; j < 16; j++) in_range = in_range && swiglu_in_range(__uint_as_float(gt[j]));
+                    if (__all_sync(0xffffffffu, in_range)) {
+#pragma unroll
+                        for (int j = 0; j < 8; j++)
+                            ob[i][j] = pack_bf16(swiglu_fast(__uint_as_float(gt[2 * j]), __uint_as_float(up[2 * j])),
+                                                 swiglu_fast(__uint_as_float(gt[2 * j + 1]), __uint_as_float(up[2 * j + 1])));
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 8; j++)
+                            ob[i][j] = pack_bf16(swiglu(__uint_as_float(gt[2 * j]), __uint_as_float(up[2 * j])),
+                                                 swiglu(__uint_as_float(gt[2 * j + 1]), __uint_as_float(up[2 * j + 1])));
+                    }
                     if (EPI == 1) {
 #pragma unroll
                         for (int c = 0; c < 4; c += 2)
@@ -688,6 +725,14 @@ int mf_grouped_gemm_fp8_mx_supported(int G, int N, int K, int epi)
 
 // The cut of a group's rows into tiles, as the kernels make it: tile `mi` of `cnt` starts at run `*first` of 32 rows and takes `*gran` of them.
 void mf_grouped_gemm_fp8_mx_cut(int steps, int cnt, int mi, int *first, int *gran) { p_tile_cut(steps, cnt, mi, *first, *gran); }
+
+// Debug aid: how many of `count` floats, by their bits from `first` on, get another quotient from the SwiGLU epilogue's own division than from the
+// general one; `differ` is a device word that the count is added to.
+int mf_swiglu_debug_probe(uint32_t first, uint64_t count, void *differ, void *stream)
+{
+    k_swiglu_probe<<<1184, 256, 0, (cudaStream_t)stream>>>(first, count, static_cast<unsigned long long *>(differ));
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
 
 // epi: 0 plain (out bf16 [rows, N]), 1 SwiGLU (out bf16 [rows, N/2]), 2 weighted push into the combine slots of the
 // tokens' home ranks, 3 SwiGLU + fp8 re-quantisation (out e4m3 [rows, N/2], out_scale fp32 [rows, N/256]).
