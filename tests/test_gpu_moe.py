@@ -175,6 +175,50 @@ def test_grouped_gemm_fp8_tile_widths(N, K, counts):
     assert bool((hq3[bad] & 0x7F == 0x7F).all()) and bool((hs3[bad] == 1).all())
 
 
+@pytest.mark.parametrize("sms", [148, 147, 1])
+@pytest.mark.parametrize("N,K,counts", [(256, 128, [1]), (256, 640, [31, 0, 32, 33, 223]), (512, 2176, [224, 225, 0, 449]), (256, 384, [0] * 33 + [65] + [0] * 29 + [3])])
+def test_grouped_gemm_fp8_push_of_weighted_rows(N, K, counts, sms):
+    """The combine epilogue around the steps and the largest width of a tile, with empty groups and with numbers of CTAs that are no whole pairs: every row
+    times its weight in its token's slot, no other slot touched, the flag raised by the last CTA and its counter back at zero."""
+    import ctypes as C
+    from memfabric_hybrid_b200.ops import gemm, moe as M
+    cu = M._cu()
+    gen = torch.Generator("cuda").manual_seed(sum(counts) + K)
+    G, R, spare, topk = len(counts), sum(counts), 40, 3
+    off = torch.tensor([0] + list(torch.tensor(counts).cumsum(0)), dtype=torch.int32, device="cuda")
+    x = torch.randn(R + spare, K, generator=gen, device="cuda").to(torch.float8_e4m3fn)
+    xs = 2.0 ** torch.randint(-4, 1, (R + spare, K // 128), generator=gen, device="cuda").float()
+    w = torch.randn(G, N, K, generator=gen, device="cuda").to(torch.float8_e4m3fn)
+    ws = 2.0 ** torch.randint(-7, -3, (G, N // 128, K // 128), generator=gen, device="cuda").float()
+    xd, wd = _deq(x[:R], xs[:R]).double(), _deq_w(w, ws).double()
+    ref = torch.cat([xd[off[g]:off[g + 1]] @ wd[g].t() for g in range(G)])
+    room = torch.cat([xd[off[g]:off[g + 1]].abs() @ wd[g].abs().t() for g in range(G)]) * K * 2.0 ** -24
+    weight = torch.rand(R + spare, generator=gen, device="cuda")
+    slots = (R + spare + topk - 1) // topk * topk
+    place = torch.randperm(slots, generator=gen, device="cuda")[:R + spare]   # slot token * topk + k of every row; the spare rows' slots stay as they are
+    info = torch.stack([torch.zeros_like(place), place // topk, place % topk, weight.view(torch.int32).long()], 1).to(torch.int32).contiguous()
+    flags_at, comb_at = 256, 4096
+    heap = torch.zeros(comb_at + slots * N * 2, dtype=torch.uint8, device="cuda")
+    flags, comb = heap[flags_at:flags_at + 4 * 64].view(torch.int32), heap[comb_at:].view(torch.bfloat16).view(slots, N)
+    comb.fill_(7)
+    done = torch.zeros(1, dtype=torch.int32, device="cuda")
+    team = M.TeamC(heap.data_ptr(), heap.numel(), 0, 0, 1, 0, 1 << 20)
+    st, s = gemm.status_word(), torch.cuda.current_stream().cuda_stream
+    for epoch in (5, 6):
+        assert cu.mf_grouped_gemm_fp8_mx_signal(x.data_ptr(), xs.data_ptr(), R + spare, w.data_ptr(), ws.data_ptr(), off.data_ptr(), G, N, K, None, 0, None, 2,
+                                                C.byref(team), info.data_ptr(), comb_at, topk, done.data_ptr(), flags_at, 1, epoch, st.data_ptr(), sms, s) == 0
+        torch.cuda.synchronize()
+        gemm.check_status()
+        assert int(done) == 0 and int(flags[16]) == epoch and int(flags.abs().sum()) == epoch
+    want = ref * weight[:R, None].double()
+    # the accumulation, the product in fp32, one rounding to bf16
+    bound = want.abs() * (2.0 ** -8 + 2.0 ** -23) + room * weight[:R, None]
+    assert bool(((comb[place[:R]].double() - want).abs() <= bound).all())
+    rest = torch.ones(slots, dtype=torch.bool, device="cuda")
+    rest[place[:R]] = False
+    assert bool((comb[rest] == 7).all())
+
+
 def test_swiglu_quotient_of_every_float():
     """The grouped GEMM's own division gives the general division's quotient for all 2^32 gates, bit for bit."""
     import ctypes as C
