@@ -260,9 +260,8 @@ template <int EPI> __global__ void __launch_bounds__(kPThreads, 1) k_grouped_fp8
         tmem_relinquish_pair();
     }
     // Barriers, tensor memory and descriptors were set up under the kernel in front of this one. The kernel behind it gets no early
-    // start, which gains nothing in a decode batch and costs in a prefill batch (its CTAs would take SMs in the order in which these
-    // become free; presumably neighbouring tiles then share less in the L2). MoE layer, early start / none, us, measured with tiles of 128 x 256:
-    // 128 tokens 303.5 / 303.4, 512: 388 / 385, 1024: 575 / 559, 4096: 1634 / 1578.
+    // start, which costs (its CTAs would take SMs in the order in which these become free; presumably neighbouring tiles then share less
+    // in the L2). MoE layer, early start / none, us: 128 tokens 272 / 268, 512: 328 / 317, 1024: 508 / 498, 4096: 1363 / 1330.
     after_predecessor();
     if (warp == 2) {
         for (int i = lane; i <= g.G; i += 32) s_row_off[i] = min(g.row_off[i], g.max_rows);
