@@ -11,9 +11,11 @@
 // at most 14 KiB of X per CTA (48 KiB before), so six stages fit, ten when no tile is wider than 32; two accumulators of
 // 224 columns fit beside the scales in tensor memory, so a tile's epilogue runs under the next tile's MMAs.
 //
-// What bounds it: few rows per expert, the weights from HBM (6.3 TB/s); many, the power limit (tensor pipe and operand traffic).
-// 32 experts, N x K 4096 x 7168 (EPI 3) and 7168 x 2048 (EPI 0), us, tiles of 128 rows x 256 on single CTAs / this kernel: about 32 rows per
-// expert 165 / 148 and 86 / 83, 128 rows 182 / 175 and 126 / 107, 256 rows 282 / 281 and 178 / 168, 1024 rows 840 / 785 and 532 / 429.
+// What bounds it: few rows per expert, the weights from HBM (6.5 TB/s); many, the power limit (tensor pipe and operand traffic); few K
+// blocks, the epilogue. 32 experts, N x K 4096 x 7168 (EPI 3) and 7168 x 2048 (EPI 0), us, tiles of 128 rows x 256 on single CTAs / this kernel:
+// about 32 rows per expert 166 / 144 and 86 / 82, 128 rows 201 / 172 and 104 / 93, 256 rows 261 / 257 and 150 / 143, 1024 rows 760 / 730 and
+// 438 / 390. Slower than those tiles: one expert of about 1 024 rows (4096 x 7168: 28.7 / 33.5; 128 tiles are one round of single CTAs, but two
+// of pairs, each of half a tile's work), and 75 to 148 tiles of few rows (5 experts of 20 rows, 4096 x 2048, EPI 0: 13.6 / 15.1).
 //
 // The scales must be powers of two (every quantiser of this library produces such scales): a producer warp turns them into UE8M0 bytes
 // (the fp32 exponent) in the tensor core's layout in shared memory, four K blocks per 32-bit word; the leader's MMA thread
