@@ -231,37 +231,36 @@ def test_swiglu_quotient_of_every_float():
     assert int(differ) == 0
 
 
-@pytest.mark.parametrize("big", [79.0, 81.0, 200.0, float("inf"), float("nan")])
-def test_swiglu_of_gates_that_leave_the_fast_divisions_range(big):
-    """One gate of a tile at either end of the range, infinite or not a number: its row's and its neighbours' activations are the other kernel's."""
+@pytest.mark.parametrize("gate", ["79", "80", "200", "inf", "nan"])
+@pytest.mark.parametrize("sign", [1, -1])
+def test_swiglu_of_gates_that_leave_the_fast_divisions_range(gate, sign):
+    """One column of gates on either side of the range's end (80), and one row's gate infinite or not a number: the bytes are the other kernel's."""
     from memfabric_hybrid_b200.ops import gemm, moe as M
     cu = M._cu()
     R, N, K = 96, 256, 128
     gen = torch.Generator("cuda").manual_seed(9)
-    x = torch.zeros(R, K, device="cuda")
+    x, w = torch.zeros(R, K, device="cuda"), torch.zeros(N, K, device="cuda")
     x[:, :2] = 1
-    w = torch.zeros(N, K, device="cuda")
     w[:, 0] = torch.randint(-8, 9, (N,), generator=gen, device="cuda").float()
     xs, ws = torch.ones(R, 1, device="cuda"), torch.ones(1, N // 128, 1, device="cuda")
-    for sign in (1, -1):
-        if big == big and big != float("inf"):
-            w[37, 0], w[37, 1] = 64 * sign, {79.0: 15, 81.0: 17 - 1, 200.0: 128 + 8}[big] * sign   # sums that e4m3 holds
-            x[50, 0] = 2 if big == 81.0 else 1
-        else:
-            w[37, 0] = 448 * sign
-            xs[50] = 2.0 ** 127 if big != big else 2.0 ** 120   # 448 * 2^127 overflows; times another infinity below: not a number
-            w[128 + 37, 0] = 448 if big != big else 1
-        xq, wq = x.to(torch.float8_e4m3fn), w.to(torch.float8_e4m3fn)[None]
-        off = torch.tensor([0, R], dtype=torch.int32, device="cuda")
-        st, s = gemm.status_word(), torch.cuda.current_stream().cuda_stream
-        got, want = (torch.full((R, N // 2), 7.0, device="cuda").to(torch.bfloat16) for _ in range(2))
-        assert cu.mf_grouped_gemm_fp8_mx(xq.data_ptr(), xs.data_ptr(), R, M.interleave_gate_up_fp8(wq, tile=128).data_ptr(), ws.data_ptr(), off.data_ptr(), 1, N, K,
-                                         got.data_ptr(), N // 2, None, 1, None, None, 0, 1, st.data_ptr(), gemm.sm_count(), s) == 0
-        assert cu.mf_grouped_gemm_fp8(xq.data_ptr(), xs.data_ptr(), R, M.interleave_gate_up_fp8(wq, tile=64).data_ptr(), ws.data_ptr(), off.data_ptr(), 1, N, K,
-                                      want.data_ptr(), N // 2, 1, None, None, 0, 1, st.data_ptr(), gemm.sm_count(), s) == 0
-        torch.cuda.synchronize()
-        gemm.check_status()
-        assert torch.equal(got.view(torch.int16), want.view(torch.int16)), sign
+    a, b = {"79": (64, 15), "80": (64, 16), "200": (128, 72), "inf": (448, 0), "nan": (1, 0)}[gate]   # values that e4m3 has
+    w[37, 0], w[37, 1] = sign * a, sign * b
+    if gate == "inf":
+        xs[50] = 2.0 ** 127   # 448 * 2^127 and most other sums of that row leave fp32
+    if gate == "nan":
+        x[50, 0] = float("nan")
+    xq, wq = x.to(torch.float8_e4m3fn), w.to(torch.float8_e4m3fn)[None]
+    off = torch.tensor([0, R], dtype=torch.int32, device="cuda")
+    st, s = gemm.status_word(), torch.cuda.current_stream().cuda_stream
+    got, want = (torch.full((R, N // 2), 7.0, device="cuda").to(torch.bfloat16) for _ in range(2))
+    assert cu.mf_grouped_gemm_fp8_mx(xq.data_ptr(), xs.data_ptr(), R, M.interleave_gate_up_fp8(wq, tile=128).data_ptr(), ws.data_ptr(), off.data_ptr(), 1, N, K,
+                                     got.data_ptr(), N // 2, None, 1, None, None, 0, 1, st.data_ptr(), gemm.sm_count(), s) == 0
+    assert cu.mf_grouped_gemm_fp8(xq.data_ptr(), xs.data_ptr(), R, M.interleave_gate_up_fp8(wq, tile=64).data_ptr(), ws.data_ptr(), off.data_ptr(), 1, N, K,
+                                  want.data_ptr(), N // 2, 1, None, None, 0, 1, st.data_ptr(), gemm.sm_count(), s) == 0
+    torch.cuda.synchronize()
+    gemm.check_status()
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+    assert gate not in ("inf", "nan") or not bool(torch.isfinite(want[50].float()).all())
 
 
 @pytest.mark.parametrize("K", [128, 384, 512, 2560])
