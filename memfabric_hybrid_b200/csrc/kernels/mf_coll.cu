@@ -3,9 +3,9 @@
 // pass. One launch per collective; CTA b of every rank works on the same element ranges as CTA b of
 // every other rank and synchronises only with those (lane flags), so no grid-wide barrier is needed.
 //   allreduce  one-shot : stage -> sync -> every rank reads all W copies, reduces, writes its output
-//   allreduce  two-shot : stage -> sync -> reduce own 1/W -> push result to all -> sync -> unstage
+//   allreduce  two-shot : stage -> sync -> reduce own 1/W into own staging -> sync -> pull every rank's part
 //   reduce_scatter      : stage -> sync -> reduce own 1/W straight into the output
-//   allgather           : push own shard into every peer's gather buffer -> sync -> unstage
+//   allgather           : stage own shard -> sync -> pull every rank's shard straight into the output
 //   broadcast, all-to-all-v, send / recv
 // Staging buffers A (inputs) and B (results) live in the slot; the host alternates between two sets
 // per call so that no trailing synchronisation is needed (a rank can only start call k+2 after every
@@ -205,6 +205,46 @@ template <typename T> __device__ __forceinline__ void cta_fanout_copy(const T *s
     }
 }
 
+// Several sources, one destination each (all-gather, second half of the two-shot all-reduce): part k is cnt[k] elements from srcs[k] to dsts[k]. The
+// vectors of all parts are numbered through, so that eight loads are in flight per thread however short a part is: part by part,
+// every part of a small message cost a memory latency of its own (over NVLink a round trip to the peer). The stores are streaming ones: outputs
+// as large as the L2 otherwise push the staged parts out (8 ranks, all-gather of 983 040 bf16 values each 46 us, 40 so).
+template <typename T> __device__ __forceinline__ void cta_gather_copy(const T *const *srcs, T *const *dsts, const uint32_t *cnt, uint32_t parts)
+{
+    constexpr uint32_t VN = 16 / sizeof(T);
+    bool al = true;
+    uint32_t nv = 0;
+    for (uint32_t k = 0; k < parts; k++) {
+        al = al && aligned16(srcs[k]) && aligned16(dsts[k]);
+        nv = max(nv, cnt[k] / VN);
+    }
+    if (!al) {
+        for (uint32_t k = 0; k < parts; k++) cta_raw_copy<T>(srcs[k], dsts[k], 0, cnt[k]);
+        return;
+    }
+    const uint32_t total = parts * nv;
+    for (uint32_t i = threadIdx.x; i < total; i += kRawUnroll * blockDim.x) {
+        uint4 v[kRawUnroll];
+        uint4 *to[kRawUnroll];
+#pragma unroll
+        for (int u = 0; u < kRawUnroll; u++) {
+            const uint32_t j = i + u * blockDim.x, k = j / nv, at = j - k * nv;
+            to[u] = nullptr;
+            if (j < total && at < cnt[k] / VN) {
+                v[u] = __ldcg(reinterpret_cast<const uint4 *>(srcs[k]) + at);
+                to[u] = reinterpret_cast<uint4 *>(dsts[k]) + at;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kRawUnroll; u++)
+            if (to[u] != nullptr) __stcs(to[u], v[u]);
+    }
+    for (uint32_t i = threadIdx.x; i < parts * VN; i += blockDim.x) {  // what is left of every part, less than a vector
+        const uint32_t k = i / VN, at = cnt[k] / VN * VN + i % VN;
+        if (at < cnt[k]) dsts[k][at] = __ldcg(srcs[k] + at);
+    }
+}
+
 // Reduces element range [beg, end) of staging A across all ranks (offset `base` elements into A) and
 // hands each result vector to `sink(i, values, count)`. Loads are issued in an order rotated by the
 // rank to spread the traffic over the peers; the accumulation order is fixed (rank 0 first) so that
@@ -316,20 +356,13 @@ template <typename T, typename TO, bool INT, int W> __global__ void __launch_bou
     if (!lane_sync(t, me, 0, a.epoch, 0x110)) return;
     MF_PROF_STOP(PF_SYNC);
     MF_PROF_START(PF_REDUCE);
+    TO *myB = reinterpret_cast<TO *>(peer_ptr(t, me, a.stage_b));
     {
         const uint64_t b = min(a.n, me * C + sub.beg), e = min(a.n, me * C + sub.end);
         reduce_ranks<T, INT, W>(t, me, a.stage_a, 0, b, e, a.op, own ? in : nullptr, [&](uint64_t i, float *acc, int cnt) {
             if (!INT && a.scale != 1.f)
                 for (int k = 0; k < cnt; k++) acc[k] *= a.scale;
-            // push the finished values into every rank's result buffer (own included)
-            for (uint32_t k = 0; k < world; k++) {
-                const uint32_t r = (me + k) % world;
-                TO *dst = reinterpret_cast<TO *>(peer_ptr(t, r, a.stage_b));
-                float tmp[VN];
-#pragma unroll
-                for (int q = 0; q < VN; q++) tmp[q] = acc[q];
-                emit<TO, true>(dst, i, tmp, cnt, 1.f);
-            }
+            emit<TO, true>(myB, i, acc, cnt, 1.f);
         });
     }
     MF_PROF_STOP(PF_REDUCE);
@@ -337,18 +370,28 @@ template <typename T, typename TO, bool INT, int W> __global__ void __launch_bou
     if (!lane_sync(t, me, 1, a.epoch, 0x111)) return;
     MF_PROF_STOP(PF_SYNC);
     MF_PROF_START(PF_COPY_OUT);
-    const TO *myB = reinterpret_cast<const TO *>(peer_ptr(t, me, a.stage_b));
-    for (uint32_t c = 0; c < world; c++) {
+    // Every rank fetches the finished parts from their owners: as many bytes cross NVLink as when the owners push them, but a part is written to
+    // memory once instead of once per rank and copied out of nobody's staging area. 8 emulated ranks, us, pushed / so: 983 040 bf16 27.5 / 24,
+    // fp32 40 / 34.5.
+    __shared__ const TO *srcs[kMaxRanks];
+    __shared__ TO *dsts[kMaxRanks];
+    __shared__ uint32_t cnts[kMaxRanks];
+    if (threadIdx.x < world) {
+        const uint32_t c = (me + 1 + threadIdx.x) % world;
         const uint64_t b = min(a.n, c * C + sub.beg), e = min(a.n, c * C + sub.end);
-        cta_raw_copy<TO>(myB, out, b, e);
+        srcs[threadIdx.x] = reinterpret_cast<const TO *>(peer_ptr(t, c, a.stage_b)) + b;
+        dsts[threadIdx.x] = out + b;
+        cnts[threadIdx.x] = (uint32_t)(e - b);
     }
+    __syncthreads();
+    cta_gather_copy<TO>(srcs, dsts, cnts, world);
     MF_PROF_STOP(PF_COPY_OUT);
 }
 
 // reduce_scatter: input n = W * m elements, output m elements (rank r gets the reduction of chunk r)
 // The part that a rank reduces itself is read where it is: nobody else needs it, and staging it moved an eighth more at 8 ranks. What bounds
 // the staged collectives of large ranges is memory: emulated ranks on one GPU, 8 x 30 MB of fp32: reduce-scatter 707 MB in 124 us (135 with
-// its own part staged), all-gather of the bf16 shards 71 (76), two-shot all-reduce 189 (198).
+// its own part staged).
 template <typename T, typename TO, bool INT, int W> __global__ void __launch_bounds__(512) k_reduce_scatter(CollArgs a)
 {
     const Team &t = a.team;
@@ -374,7 +417,11 @@ template <typename T, typename TO, bool INT, int W> __global__ void __launch_bou
                             [&](uint64_t i, float *acc, int cnt) { emit<TO, INT>(out, i, acc, cnt, a.scale); });
 }
 
-// allgather: every rank contributes n elements; output W * n. Shards are pushed (one NVLink crossing).
+// allgather: every rank contributes n elements; output W * n. A shard is written once, into its owner's staging area, and fetched from there by
+// every rank straight into its output. As many bytes cross NVLink as when the owners push, and memory sees n written + (W - 1) n read and
+// written per rank where it saw W n written, read and written again; the fetched lines of a staged shard come out of its owner's L2. What
+// bounds it is then the writing of the output. 8 emulated ranks, us, pushed / so: bf16 shards of 64 values 8.6 / 6.1, 32 768 10.3 / 7.7,
+// 983 040 68 / 40 (126 MB of output; filling as much takes 37), fp32 134 / 78; off 16 bytes (1 000 001 bf16) 84 / 41.
 template <typename T, typename TO> __global__ void __launch_bounds__(512) k_allgather(CollArgs a)
 {
     const Team &t = a.team;
@@ -382,33 +429,37 @@ template <typename T, typename TO> __global__ void __launch_bounds__(512) k_allg
     const uint32_t world = t.world;
     const T *in = reinterpret_cast<const T *>(a.in + (uint64_t)me * a.in_rank_stride);
     TO *out = reinterpret_cast<TO *>(a.out + (uint64_t)me * a.out_rank_stride);
-    constexpr int VN = Vec<T>::N;
     const Range sub = cta_range<8>(a.n);
-    const uint64_t np = (a.n + 7) / 8 * 8;  // staged rows start on 16 bytes whatever n is
     const uint64_t ps = a.part_stride ? a.part_stride : a.n;
-    // the rank's own shard goes straight to its place, where that is as well aligned as a staged row
-    const bool in_place = !a.team.emu && (uint64_t)in == (uint64_t)(out + (uint64_t)me * ps);
-    const bool own = sizeof(T) == sizeof(TO) && a.scale == 1.f && aligned16(out + (uint64_t)me * ps) &&
-                     (in_place || apart(a, a.n * sizeof(T), ((world - 1) * ps + a.n) * sizeof(TO)));
-    if (sizeof(T) == sizeof(TO) && a.scale == 1.f) {
-        // same type, no scaling: the shard is read once and fanned out to every rank's staging area
-        __shared__ TO *dsts[kMaxRanks];
-        if (threadIdx.x < world)
-            dsts[threadIdx.x] = threadIdx.x == 0 && own ? out + (uint64_t)me * ps
-                                                        : reinterpret_cast<TO *>(peer_ptr(t, (me + threadIdx.x) % world, a.stage_b)) + (uint64_t)me * np;
-        __syncthreads();
-        cta_fanout_copy<TO>(reinterpret_cast<const TO *>(in), dsts, world, sub.beg, sub.end);
-    } else {
-        for (uint32_t k = 0; k < world; k++) {
-            const uint32_t r = (me + k) % world;
-            TO *dst = reinterpret_cast<TO *>(peer_ptr(t, r, a.stage_b)) + (uint64_t)me * np;
-            cta_convert_copy<T, TO>(in, dst, sub.beg, sub.end, a.scale);
+    TO *myB = reinterpret_cast<TO *>(peer_ptr(t, me, a.stage_b));
+    TO *mine = out + (uint64_t)me * ps;
+    const bool raw = sizeof(T) == sizeof(TO) && a.scale == 1.f;
+    // the rank's own shard goes straight to its place while it is read, where that is as well aligned as a staged row
+    const bool in_place = !a.team.emu && (uint64_t)in == (uint64_t)mine;
+    const bool own = raw && (in_place || (aligned16(mine) && apart(a, a.n * sizeof(T), ((world - 1) * ps + a.n) * sizeof(TO))));
+    if (raw) {
+        __shared__ TO *to[2];
+        if (threadIdx.x == 0) {
+            to[0] = myB;
+            to[1] = mine;
         }
+        __syncthreads();
+        cta_fanout_copy<TO>(reinterpret_cast<const TO *>(in), to, own && !in_place ? 2 : 1, sub.beg, sub.end);
+    } else {
+        cta_convert_copy<T, TO>(in, myB, sub.beg, sub.end, a.scale);
     }
     if (!lane_sync(t, me, 0, a.epoch, 0x130)) return;
-    const TO *myB = reinterpret_cast<const TO *>(peer_ptr(t, me, a.stage_b));
-    for (uint32_t c = 0; c < world; c++)
-        if (!own || c != me) cta_raw_copy<TO>(myB + (uint64_t)c * np, out + (uint64_t)c * ps, sub.beg, sub.end);
+    __shared__ const TO *srcs[kMaxRanks];
+    __shared__ TO *dsts[kMaxRanks];
+    __shared__ uint32_t cnts[kMaxRanks];
+    if (threadIdx.x < world) {
+        const uint32_t c = (me + 1 + threadIdx.x) % world;  // the own shard last
+        srcs[threadIdx.x] = reinterpret_cast<const TO *>(peer_ptr(t, c, a.stage_b)) + sub.beg;
+        dsts[threadIdx.x] = out + (uint64_t)c * ps + sub.beg;
+        cnts[threadIdx.x] = (uint32_t)(sub.end - sub.beg);
+    }
+    __syncthreads();
+    cta_gather_copy<TO>(srcs, dsts, cnts, own ? world - 1 : world);
 }
 
 // broadcast of n elements from a.root
