@@ -17,6 +17,7 @@
 #include "mf_coll.cuh"
 #include "mf_shift.cuh"
 #include "mf_devtrace.cuh"
+#include "mf_umma.cuh"
 
 namespace mfk {
 
@@ -53,6 +54,9 @@ template <int VN> __device__ __forceinline__ Range cta_range(uint64_t count)
     r.end = min(count, r.beg + per);
     return r;
 }
+
+// elements of a rank's part of the two-shot all-reduce
+__host__ __device__ __forceinline__ uint64_t part_of_two_shot(uint64_t n, uint32_t world) { return ((n + world - 1) / world + 7) / 8 * 8; }
 
 __device__ __forceinline__ bool aligned16(const void *p) { return (reinterpret_cast<uint64_t>(p) & 15) == 0; }
 
@@ -320,6 +324,25 @@ template <typename TO, bool INT> __device__ __forceinline__ void emit(TO *dst, u
     }
 }
 
+// Second half of the two-shot all-reduce: every rank fetches the finished parts from their owners. As many bytes cross NVLink as when the owners
+// push them, but a part is written to memory once instead of once per rank and copied out of nobody's staging area. 8 emulated ranks, us, pushed /
+// so: 983 040 bf16 27.5 / 24, fp32 40 / 34.5.
+template <typename TO> __device__ __forceinline__ void fetch_parts(const Team &t, uint32_t me, uint64_t stage_b, uint64_t n, uint64_t C, const Range &sub, TO *out)
+{
+    __shared__ const TO *srcs[kMaxRanks];
+    __shared__ TO *dsts[kMaxRanks];
+    __shared__ uint32_t cnts[kMaxRanks];
+    if (threadIdx.x < t.world) {
+        const uint32_t c = (me + 1 + threadIdx.x) % t.world;
+        const uint64_t b = min(n, c * C + sub.beg), e = min(n, c * C + sub.end);
+        srcs[threadIdx.x] = reinterpret_cast<const TO *>(peer_ptr(t, c, stage_b)) + b;
+        dsts[threadIdx.x] = out + b;
+        cnts[threadIdx.x] = (uint32_t)(e - b);
+    }
+    __syncthreads();
+    cta_gather_copy<TO>(srcs, dsts, cnts, t.world);
+}
+
 // ------------------------------------------------------------------------------------------------
 template <typename T, typename TO, bool INT, int W> __global__ void __launch_bounds__(512) k_allreduce(CollArgs a)
 {
@@ -339,8 +362,7 @@ template <typename T, typename TO, bool INT, int W> __global__ void __launch_bou
         return;
     }
     // two-shot: chunk c = elements [c * C, (c + 1) * C) belongs to rank c
-    uint64_t C = (a.n + world - 1) / world;
-    C = (C + 7) / 8 * 8;
+    const uint64_t C = part_of_two_shot(a.n, world);
     const Range sub = cta_range<8>(C);
     // nobody else reads the part that this rank reduces, and nobody writes to any output before all ranks have read theirs (second exchange)
     const bool own = !a.zero_copy && aligned16(in);
@@ -370,21 +392,7 @@ template <typename T, typename TO, bool INT, int W> __global__ void __launch_bou
     if (!lane_sync(t, me, 1, a.epoch, 0x111)) return;
     MF_PROF_STOP(PF_SYNC);
     MF_PROF_START(PF_COPY_OUT);
-    // Every rank fetches the finished parts from their owners: as many bytes cross NVLink as when the owners push them, but a part is written to
-    // memory once instead of once per rank and copied out of nobody's staging area. 8 emulated ranks, us, pushed / so: 983 040 bf16 27.5 / 24,
-    // fp32 40 / 34.5.
-    __shared__ const TO *srcs[kMaxRanks];
-    __shared__ TO *dsts[kMaxRanks];
-    __shared__ uint32_t cnts[kMaxRanks];
-    if (threadIdx.x < world) {
-        const uint32_t c = (me + 1 + threadIdx.x) % world;
-        const uint64_t b = min(a.n, c * C + sub.beg), e = min(a.n, c * C + sub.end);
-        srcs[threadIdx.x] = reinterpret_cast<const TO *>(peer_ptr(t, c, a.stage_b)) + b;
-        dsts[threadIdx.x] = out + b;
-        cnts[threadIdx.x] = (uint32_t)(e - b);
-    }
-    __syncthreads();
-    cta_gather_copy<TO>(srcs, dsts, cnts, world);
+    fetch_parts<TO>(t, me, a.stage_b, a.n, C, sub, out);
     MF_PROF_STOP(PF_COPY_OUT);
 }
 
@@ -415,6 +423,274 @@ template <typename T, typename TO, bool INT, int W> __global__ void __launch_bou
     if (!lane_sync(t, me, 0, a.epoch, 0x120)) return;
     reduce_ranks<T, INT, W>(t, me, a.stage_a, (uint64_t)me * mp, sub.beg, sub.end, a.op, own ? in + (uint64_t)me * ps : nullptr,
                             [&](uint64_t i, float *acc, int cnt) { emit<TO, INT>(out, i, acc, cnt, a.scale); });
+}
+
+// ------------------------------------------------------------------------------------------------
+// Pipelined reduce (reduce-scatter and first half of the two-shot all-reduce, large parts). A CTA's range of every part is cut into chunks; seven warps
+// push chunk after chunk of the input into the staging areas of the ranks that reduce them, one warp tells these
+// ranks how many chunks have arrived, eight warps reduce the chunks that the peers have pushed here. A chunk is read a few microseconds after it
+// was written, out of the L2, and no rank waits for the whole of another's input.
+// Staging at a rank: one row of `row` elements per source rank (16-byte aligned).
+// What bounds it is the L2: 8 emulated ranks of 30 MB fp32 move 252 MB in, 220 into staging and 252 out of it, 16 out, in 105 us (7 TB/s; memory sees
+// 272 MB read and 190 written), staging everything first 121. Chunks of 28 pieces of 4 KiB and 7 + 8 warps, us: 14 or 56 pieces 109, 116 (28: 107); 15 + 16 warps
+// 126, 10 + 8 126, 5 + 5 146, 7 + 4 165, 7 + 16 113; one vector of all ranks in flight per lane 105, two 103; plain loads of the input or of the staged rows +2 to +4.
+constexpr int kPushWarps = 7, kReduceWarps = 8, kPipeThreads = (kPushWarps + 1 + kReduceWarps) * 32;
+constexpr int kMaxChunks = 64;
+constexpr int kPieceBytes = 4096;  // what a warp moves at once: eight vectors per lane
+constexpr int kPiecesPerChunk = 28;
+
+struct PipeArgs {
+    const void *in;      // this rank's parts: part c starts at in + c * part_stride
+    uint64_t part_stride;
+    uint64_t total;      // elements behind `in` that belong to the parts: part c holds those of [c * part_stride, ...) up to `total`, at most `len`
+    uint64_t len;        // elements of a whole part
+    uint64_t row;        // elements between staged rows
+    uint64_t stage;
+    bool own;            // this rank's own part is reduced where it lies; else it is staged like the others
+    bool apart;          // the output may be written while the input is still read
+};
+
+// n elements (at most a piece) to dst (16-byte aligned); src anywhere. [lo, hi): memory that may be read in whole granules.
+template <int Q> __device__ __forceinline__ uint4 cut_neighbours(const uint4 &v, const uint4 &next, uint32_t bits, int lane)
+{
+    const uint4 give = lane == 0 ? next : v;
+    uint4 hi;
+    hi.x = __shfl_sync(0xffffffffu, give.x, (lane + 1) & 31);
+    hi.y = __shfl_sync(0xffffffffu, give.y, (lane + 1) & 31);
+    hi.z = __shfl_sync(0xffffffffu, give.z, (lane + 1) & 31);
+    hi.w = __shfl_sync(0xffffffffu, give.w, (lane + 1) & 31);
+    return cut16<Q>(v, hi, bits);
+}
+template <typename T> __device__ __forceinline__ void warp_push_piece(const T *src, T *dst, uint32_t n, uint64_t lo, uint64_t hi)
+{
+    constexpr uint32_t VN = 16 / sizeof(T), U = kPieceBytes / 512;
+    const int lane = threadIdx.x & 31;
+    const uint32_t nv = n / VN;
+    const uint32_t off = (uint32_t)(reinterpret_cast<uint64_t>(src) & 15);
+    uint4 *d = reinterpret_cast<uint4 *>(dst);
+    if (off == 0) {
+        const uint4 *sv = reinterpret_cast<const uint4 *>(src);
+        uint4 v[U];
+#pragma unroll
+        for (uint32_t u = 0; u < U; u++)
+            if (u * 32 + lane < nv) v[u] = __ldcs(sv + u * 32 + lane);
+#pragma unroll
+        for (uint32_t u = 0; u < U; u++)
+            if (u * 32 + lane < nv) d[u * 32 + lane] = v[u];
+        const uint32_t i = nv * VN + lane;
+        if (i < n) dst[i] = src[i];
+        return;
+    }
+    // vector i is cut out of granules i and i + 1
+    const uint64_t g0 = reinterpret_cast<uint64_t>(src) - off;
+    auto granule = [&](uint32_t i) {
+        const uint64_t at = g0 + (uint64_t)i * 16;
+        return i <= nv && at >= lo && at + 16 <= hi ? __ldcs(reinterpret_cast<const uint4 *>(at)) : make_uint4(0, 0, 0, 0);
+    };
+    uint4 v[U + 1];
+#pragma unroll
+    for (uint32_t u = 0; u < U; u++) v[u] = granule(u * 32 + lane);
+    v[U] = lane == 0 ? granule(U * 32) : make_uint4(0, 0, 0, 0);
+    const uint32_t bits = (off & 3) * 8, first = g0 < lo ? 1 : 0;                         // the first vector's granule starts in front of the input
+    const uint32_t last = nv > 0 && g0 + ((uint64_t)nv + 1) * 16 > hi ? nv - 1 : nv;      // the last one's ends behind it
+#pragma unroll
+    for (uint32_t u = 0; u < U; u++) {
+        uint4 o;
+        switch (off >> 2) {  // uniform over the warp
+            case 0: o = cut_neighbours<0>(v[u], v[u + 1], bits, lane); break;
+            case 1: o = cut_neighbours<1>(v[u], v[u + 1], bits, lane); break;
+            case 2: o = cut_neighbours<2>(v[u], v[u + 1], bits, lane); break;
+            default: o = cut_neighbours<3>(v[u], v[u + 1], bits, lane); break;
+        }
+        const uint32_t i = u * 32 + lane;
+        if (i >= first && i < last) d[i] = o;
+    }
+    // what no vector covered, element by element: the first vector, the last one, the rest behind them
+    if (first != 0 && lane < VN && lane < n) dst[lane] = src[lane];
+    for (uint32_t i = max(last * VN, first * VN) + lane; i < n; i += 32) dst[i] = src[i];
+}
+
+__device__ __forceinline__ uint64_t ld_acquire_sys_u64(const uint64_t *p)
+{
+    uint64_t v;
+    asm volatile("ld.acquire.sys.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// sink(i, values, count): element i of this rank's part. All threads of a CTA of kPipeThreads. False: a wait gave up (uniform over the CTA).
+template <typename T, bool INT, int W, typename Sink>
+__device__ __forceinline__ bool pipe_reduce(const Team &t, uint32_t me, const PipeArgs &p, const Range &sub, uint32_t epoch, int op, uint32_t where, Sink sink)
+{
+    constexpr uint32_t VN = Vec<T>::N, kPiece = kPieceBytes / sizeof(T);
+    __shared__ uint64_t done[kMaxChunks];
+    __shared__ int ok_sh;
+    const uint32_t world = W > 0 ? (uint32_t)W : t.world;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t parts = p.own ? world - 1 : world;
+    const uint64_t span = sub.end > sub.beg ? sub.end - sub.beg : 0;
+    // pieces of a part per chunk, the same on every rank
+    uint32_t per = max(1u, kPiecesPerChunk / max(1u, world - 1));
+    per = max(per, (uint32_t)((span + (uint64_t)kPiece * kMaxChunks - 1) / ((uint64_t)kPiece * kMaxChunks)));
+    const uint64_t chunk = (uint64_t)per * kPiece;
+    const uint32_t chunks = (uint32_t)((span + chunk - 1) / chunk);
+    for (uint32_t i = threadIdx.x; i < chunks; i += blockDim.x) mbar_init(done + i, kPushWarps);
+    if (threadIdx.x == 0) ok_sh = 1;
+    __syncthreads();
+    auto part_end = [&](uint32_t c) { return min(min(sub.end, p.len), p.total > c * p.part_stride ? p.total - c * p.part_stride : 0); };  // of the range in part c
+    const uint64_t flag_off = kChunkOff + (uint64_t)blockIdx.x * kMaxRanks * sizeof(uint64_t);
+    const T *in = static_cast<const T *>(p.in);
+    if (warp < kPushWarps) {
+        const uint64_t lo = reinterpret_cast<uint64_t>(in), hi = lo + p.total * sizeof(T);
+        MF_PROF_START(PF_STAGE_IN);
+        for (uint32_t q = 0; q < chunks; q++) {
+            for (uint32_t x = warp; x < parts * per; x += kPushWarps) {
+                const uint32_t k = x / per;
+                const uint32_t c = (me + 1 + k) % world;
+                const uint64_t b = sub.beg + q * chunk + (uint64_t)(x - k * per) * kPiece, e = part_end(c);
+                if (b >= e) continue;
+                T *row = reinterpret_cast<T *>(peer_ptr(t, c, p.stage)) + (uint64_t)me * p.row;
+                warp_push_piece<T>(in + c * p.part_stride + b, row + b, (uint32_t)min(e - b, (uint64_t)kPiece), lo, hi);
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(done + q);
+        }
+        MF_PROF_STOP(PF_STAGE_IN);
+        MF_PROF_START(PF_REDUCE);  // what is left of it
+    } else if (warp == kPushWarps) {
+        for (uint32_t q = 0; q < chunks; q++) {
+            uint32_t i = 0;
+            while (i < kMbarSpinLimit && !mbar_try_wait(done + q, 0)) i++;
+            if (i == kMbarSpinLimit) break;  // not to be expected: the pushing warps wait for nobody
+            const uint32_t c = (me + 1 + lane) % world;
+            if ((uint32_t)lane < parts)
+                asm volatile("st.release.sys.global.u64 [%0], %1;" ::"l"(reinterpret_cast<uint64_t *>(peer_ptr(t, c, flag_off)) + me),
+                             "l"((uint64_t)epoch << 32 | (q + 1)) : "memory");
+        }
+    } else {
+        const uint32_t tid = threadIdx.x - (kPushWarps + 1) * 32;
+        const uint64_t *flags = reinterpret_cast<const uint64_t *>(peer_ptr(t, me, flag_off));
+        const T *stage = reinterpret_cast<const T *>(peer_ptr(t, me, p.stage));
+        auto row = [&](uint32_t r) { return p.own && r == me ? in + me * p.part_stride : stage + (uint64_t)r * p.row; };
+        const uint64_t end = part_end(me);
+        for (uint32_t q = 0; q < chunks; q++) {
+            bool ok = true;
+            if ((uint32_t)lane < world && !(p.own && (uint32_t)lane == me)) {
+                const uint64_t want = (uint64_t)epoch << 32 | (p.apart ? q + 1 : chunks);
+                uint32_t i = 0;
+                while ((int64_t)(ld_acquire_sys_u64(flags + lane) - want) < 0 && i < t.spin_limit) {
+                    if (i > 64) __nanosleep(i > 4096 ? 256 : 32);
+                    i++;
+                }
+                ok = i < t.spin_limit;
+                if (!ok && warp == kPushWarps + 1) report_timeout(t, me, where, epoch);
+            }
+            if (!__all_sync(0xffffffffu, ok)) {
+                ok_sh = 0;
+                break;
+            }
+            __syncwarp();  // what a lane has seen arrive, all lanes may read
+            const uint64_t b = sub.beg + q * chunk, e = min(end, b + chunk);
+            if (b >= e) continue;
+            const uint64_t vend = b + (e - b) / VN * VN;
+            constexpr int U = W == 0 ? 1 : 2;
+            for (uint64_t i = b + (uint64_t)tid * VN; i < vend; i += (uint64_t)U * kReduceWarps * 32 * VN) {
+                if (W > 0) {
+                    uint4 raw[U][W > 0 ? W : 1];
+#pragma unroll
+                    for (int u = 0; u < U; u++)
+#pragma unroll
+                        for (int r = 0; r < W; r++)
+                            if (u == 0 || i + u * kReduceWarps * 32 * VN < vend)
+                                raw[u][r] = __ldcs(reinterpret_cast<const uint4 *>(row(r) + i + u * kReduceWarps * 32 * VN));
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        if (u != 0 && i + u * kReduceWarps * 32 * VN >= vend) continue;
+                        float acc[VN];
+#pragma unroll
+                        for (int r = 0; r < W; r++) {
+                            float f[VN];
+                            Vec<T>::unpack(raw[u][r], f);
+#pragma unroll
+                            for (uint32_t k = 0; k < VN; k++) acc[k] = r == 0 ? f[k] : red_apply<INT>(acc[k], f[k], op);
+                        }
+                        sink(i + u * kReduceWarps * 32 * VN, acc, VN);
+                    }
+                } else {
+                    float acc[VN];
+                    for (uint32_t r = 0; r < world; r++) {
+                        float f[VN];
+                        Vec<T>::load(row(r) + i, f);
+#pragma unroll
+                        for (uint32_t k = 0; k < VN; k++) acc[k] = r == 0 ? f[k] : red_apply<INT>(acc[k], f[k], op);
+                    }
+                    sink(i, acc, VN);
+                }
+            }
+            for (uint64_t i = vend + tid; i < e; i += kReduceWarps * 32) {
+                float acc[VN];
+                for (uint32_t r = 0; r < world; r++) {
+                    const float f = Vec<T>::to_f(__ldcg(row(r) + i));
+                    acc[0] = r == 0 ? f : red_apply<INT>(acc[0], f, op);
+                }
+                sink(i, acc, 1);
+            }
+        }
+    }
+    __syncthreads();
+    MF_PROF_STOP(PF_REDUCE);
+    return ok_sh != 0;
+}
+
+template <typename T, typename TO, bool INT, int W> __global__ void __launch_bounds__(kPipeThreads) k_reduce_scatter_pipe(CollArgs a)
+{
+    const Team &t = a.team;
+    const uint32_t me = team_rank(t);
+    const uint32_t world = t.world;
+    const T *in = reinterpret_cast<const T *>(a.in + (uint64_t)me * a.in_rank_stride);
+    TO *out = reinterpret_cast<TO *>(a.out + (uint64_t)me * a.out_rank_stride);
+    const uint64_t m = a.n / world;
+    const uint64_t ps = a.part_stride ? a.part_stride : m;
+    const bool in_place = sizeof(T) == sizeof(TO) && !a.team.emu && (uint64_t)out == (uint64_t)(in + (uint64_t)me * ps);
+    PipeArgs p;
+    p.in = in;
+    p.part_stride = ps;
+    p.total = (world - 1) * ps + m;
+    p.len = m;
+    p.row = (m + 7) / 8 * 8;
+    p.stage = a.stage_a;
+    p.apart = in_place || apart(a, p.total * sizeof(T), m * sizeof(TO));
+    p.own = p.apart && aligned16(in + (uint64_t)me * ps);
+    pipe_reduce<T, INT, W>(t, me, p, cta_range<8>(m), a.epoch, a.op, 0x128,
+                           [&](uint64_t i, float *acc, int cnt) { emit<TO, INT>(out, i, acc, cnt, a.scale); });
+}
+
+template <typename T, typename TO, bool INT, int W> __global__ void __launch_bounds__(kPipeThreads) k_allreduce_pipe(CollArgs a)
+{
+    const Team &t = a.team;
+    const uint32_t me = team_rank(t);
+    const T *in = reinterpret_cast<const T *>(a.in + (uint64_t)me * a.in_rank_stride);
+    TO *out = reinterpret_cast<TO *>(a.out + (uint64_t)me * a.out_rank_stride);
+    const uint64_t C = part_of_two_shot(a.n, t.world);
+    const Range sub = cta_range<8>(C);
+    PipeArgs p;
+    p.in = in;
+    p.part_stride = C;
+    p.total = a.n;
+    p.len = C;
+    p.row = C;
+    p.stage = a.stage_a;
+    p.apart = true;  // the sums go to staging B; the output is written behind the second exchange
+    p.own = aligned16(in);
+    TO *myB = reinterpret_cast<TO *>(peer_ptr(t, me, a.stage_b)) + me * C;
+    const bool ok = pipe_reduce<T, INT, W>(t, me, p, sub, a.epoch, a.op, 0x118,
+                                           [&](uint64_t i, float *acc, int cnt) { emit<TO, INT>(myB, i, acc, cnt, a.scale); });
+    if (!ok) return;
+    MF_PROF_START(PF_SYNC);
+    if (!lane_sync(t, me, 1, a.epoch, 0x111)) return;
+    MF_PROF_STOP(PF_SYNC);
+    MF_PROF_START(PF_COPY_OUT);
+    fetch_parts<TO>(t, me, a.stage_b, a.n, C, sub, out);
+    MF_PROF_STOP(PF_COPY_OUT);
 }
 
 // allgather: every rank contributes n elements; output W * n. A shard is written once, into its owner's staging area, and fetched from there by
@@ -1100,8 +1376,29 @@ template <typename K, typename A> int launch(K kernel, const A &args, int ctas, 
     return e == cudaSuccess ? 0 : (int)e;
 }
 
+// Whether the pipelined kernels take a reduction; the same on every rank. They pay where the staged parts of all ranks do not stay in the L2 between
+// the two passes of the others. Emulated ranks, fp32, us, two passes / pipelined by the bytes of all ranks: reduce-scatter of 32 MB 18.2 / 21.0 (4
+// ranks), 63 MB 36.4 / 32.6, 64 MB 36.2 / 35.3 (8 ranks), 128 MB 66 / 60, 252 MB 125 / 107; two-shot all-reduce of 33 MB 36.8 / 38.9 (2 ranks), 67 MB 62.6 /
+// 60.4, 8 ranks of 32 MB 207 / 185. Real ranks, not measured here, follow the same line (8 ranks: 7.5 MB each): there the copy into the own staging area
+// in front of the exchange goes away as well. Parts off 16 bytes have to be shifted, which the two passes do with more warps (139 / 143).
+constexpr uint64_t kPipeMinBytes = 60ull << 20;
+bool pipe_pays(const CollArgs &a, uint64_t part_stride, uint64_t es, int threads)
+{
+    return !a.zero_copy && threads == kPipeThreads && a.team.world > 1 && a.team.world * a.n * es >= kPipeMinBytes && part_stride * es % 16 == 0;
+}
+
 template <typename T, typename TO, bool INT> int launch_allreduce(const CollArgs &a, int ctas, int threads, cudaStream_t s)
 {
+    const uint64_t C = part_of_two_shot(a.n, a.team.world);
+    // a row per rank has to fit the staging area, which ends in front of the results'
+    if (a.algo == 1 && pipe_pays(a, C, sizeof(T), threads) && a.stage_b >= a.stage_a + a.team.world * C * sizeof(T)) {
+        switch (a.team.world) {
+            case 2: return launch(k_allreduce_pipe<T, TO, INT, 2>, a, ctas, threads, s, false);
+            case 4: return launch(k_allreduce_pipe<T, TO, INT, 4>, a, ctas, threads, s, false);
+            case 8: return launch(k_allreduce_pipe<T, TO, INT, 8>, a, ctas, threads, s, false);
+            default: return launch(k_allreduce_pipe<T, TO, INT, 0>, a, ctas, threads, s, false);
+        }
+    }
     switch (a.team.world) {
         case 2: return launch(k_allreduce<T, TO, INT, 2>, a, ctas, threads, s, false);
         case 4: return launch(k_allreduce<T, TO, INT, 4>, a, ctas, threads, s, false);
@@ -1147,6 +1444,14 @@ template <typename T, typename TO> int launch_rs_mc(const CollArgs &a, int ctas,
 }
 template <typename T, typename TO, bool INT> int launch_rs(const CollArgs &a, int ctas, int threads, cudaStream_t s)
 {
+    if (pipe_pays(a, a.part_stride ? a.part_stride : a.n / a.team.world, sizeof(T), threads)) {
+        switch (a.team.world) {
+            case 2: return launch(k_reduce_scatter_pipe<T, TO, INT, 2>, a, ctas, threads, s, false);
+            case 4: return launch(k_reduce_scatter_pipe<T, TO, INT, 4>, a, ctas, threads, s, false);
+            case 8: return launch(k_reduce_scatter_pipe<T, TO, INT, 8>, a, ctas, threads, s, false);
+            default: return launch(k_reduce_scatter_pipe<T, TO, INT, 0>, a, ctas, threads, s, false);
+        }
+    }
     switch (a.team.world) {
         case 2: return launch(k_reduce_scatter<T, TO, INT, 2>, a, ctas, threads, s, false);
         case 4: return launch(k_reduce_scatter<T, TO, INT, 4>, a, ctas, threads, s, false);

@@ -35,6 +35,8 @@ constexpr uint32_t kLaneOff = 128 * 1024;
 constexpr int kPhases = 4;
 //   [256 KiB, 256 KiB + 128 KiB) address exchange [cta 0..255][rank 0..15] x 4 words {epoch, 32 bits of payload}
 constexpr uint32_t kXchgOff = 256 * 1024;
+//   [384 KiB, 384 KiB + 32 KiB)  chunk progress  [cta 0..255][rank 0..15] x u64 {epoch, chunks delivered}
+constexpr uint32_t kChunkOff = 384 * 1024;
 
 enum MfStatus : uint32_t { ST_OK = 0, ST_TIMEOUT = 1, ST_BAD_ARG = 2 };
 

@@ -152,6 +152,43 @@ def test_reduce_scatter_and_all_gather_whose_output_lies_in_the_input(comms, wor
         assert torch.equal(out, shard.reshape(1, -1).expand(world, -1)), off
 
 
+@pytest.mark.parametrize("world,stage_mb", [(2, 32), (3, 21), (4, 16), (8, 8)])
+def test_large_reductions_whose_parts_are_pushed_in_chunks(world, stage_mb):
+    """From 60 MiB over all ranks on, the parts travel in chunks while they are reduced: ends of chunks and of CTA ranges, inputs on and off 16 bytes, an
+    output in the input's memory, every rank's sum in rank order bit for bit; just below, the two passes."""
+    from memfabric_hybrid_b200.ops.heap import EmulatedHeap
+    from memfabric_hybrid_b200.ops.collectives import Communicator
+    heap = EmulatedHeap(world, (1 << 20) + 4 * (stage_mb << 20) + (1 << 20))
+    c = Communicator(heap, stage_bytes=stage_mb << 20)
+    line = (60 << 20) // world // world     # bytes of a part
+    for dtype, shift, more in ((torch.float32, 0, 0), (torch.float32, 1, 36), (torch.bfloat16, 0, 8), (torch.bfloat16, 5, 1000), (torch.int32, 0, 4), (torch.float32, 0, -16)):
+        es = 2 if dtype == torch.bfloat16 else 4
+        m = -(-line // es) // 8 * 8 + 8 + more
+        g = torch.Generator("cuda").manual_seed(m)
+        flat = torch.empty(world * world * m + 8, dtype=dtype, device="cuda")
+        x = flat[shift:shift + world * world * m].view(world, world * m)
+        if dtype == torch.int32:
+            x.copy_(torch.randint(-1000, 1000, x.shape, device="cuda", dtype=dtype, generator=g))
+            want = x.sum(0).to(dtype)
+        else:
+            x.copy_(torch.randn(x.shape, device="cuda", generator=g).to(dtype))
+            want = _rank_order_sum(x)
+        room = torch.full((world * m + 16,), 7, device="cuda", dtype=dtype)
+        c.reduce_scatter(x, out=room[8:8 + world * m].view(world, m))
+        assert torch.equal(room[8:8 + world * m], want) and bool((room[:8] == 7).all()) and bool((room[8 + world * m:] == 7).all()), (dtype, shift)
+        y = x.clone()
+        assert torch.equal(c.all_reduce(y, out=y, algo="twoshot"), want.expand(world, -1)), (dtype, shift)
+        z = y[:, :world * m - 3].contiguous().zero_() + x[:, :world * m - 3]     # a last part that is shorter
+        assert torch.equal(c.all_reduce(z), want[:world * m - 3].expand(world, -1)), (dtype, shift)
+        if dtype == torch.float32:
+            assert torch.equal(c.reduce_scatter(x, scale=0.5, out_dtype=torch.bfloat16).view(-1), (want * 0.5).to(torch.bfloat16))
+            assert torch.equal(c.reduce_scatter(x, op="max").view(-1), x.max(0).values)
+        y = x.clone()
+        assert torch.equal(c.reduce_scatter(y, out=y.view(-1)[:world * m].view(world, m)).reshape(-1), want), (dtype, shift)
+    torch.cuda.synchronize()
+    assert heap.status()[0] == 0
+
+
 @pytest.mark.parametrize("world", [2, 8])
 def test_broadcast_scatter_alltoallv(comms, world):
     c = comms[world]
