@@ -676,20 +676,18 @@ template <int EPI> __global__ void __launch_bounds__(kPThreads, 1) k_grouped_fp8
     __syncthreads();
     cluster_sync_all();  // nobody signals a barrier of a CTA that has left, and both halves of the tensor memory are freed together
     if (EPI == 2) {
-        // The CTA that finishes last tells every rank that all of this rank's rows are home: the CTA barrier orders the CTA's
-        // stores before thread 0, whose system fence covers them, and the counter links the CTAs' fences.
-        __shared__ int last_sh;
-        if (threadIdx.x == 0) {
-            fence_sys();
-            last_sh = g.done_count != nullptr && atomicAdd(g.done_count, 1u) + 1 == gridDim.x;
-            if (last_sh) {
+        // The CTA that finishes last tells every rank that all of this rank's rows are home: the CTA barrier orders the CTA's stores before thread 0, whose fence
+        // and count hand them to the last CTA's, whose system fence covers all of them; the flags need no order of their own.
+        if (threadIdx.x == 0 && g.done_count != nullptr) {
+            __threadfence();
+            if (atomicAdd(g.done_count, 1u) + 1 == gridDim.x) {
                 *g.done_count = 0;
-                __threadfence();  // acquires what the other CTAs' fences released; the flag stores below release it to the system
+                fence_sys();
+                for (uint32_t r = 0; r < g.team.world; r++)
+                    asm volatile("st.relaxed.sys.global.u32 [%0], %1;" ::"l"(reinterpret_cast<uint32_t *>(peer_ptr(g.team, r, g.flag_off)) + g.team.rank), "r"(g.epoch)
+                                 : "memory");
             }
         }
-        __syncthreads();
-        if (last_sh && threadIdx.x < g.team.world)
-            st_release_sys(reinterpret_cast<uint32_t *>(peer_ptr(g.team, threadIdx.x, g.flag_off)) + g.team.rank, g.epoch);
     }
     if (warp == 1) {
         tc_fence_after();

@@ -319,54 +319,47 @@ __device__ __forceinline__ void dispatch_preload(const DispatchArgs &a, uint4 &l
     }
 }
 
-// End of a dispatch, all threads of every CTA: the CTA that finishes last raises this rank's flag on every peer (the CTA
-// barrier orders the CTA's stores before thread 0, whose system fence covers them; the counter links the CTAs' fences).
+// By the thread that has counted the last CTA of a grid: this rank's flag of the row at `flags` on every rank. A CTA's barrier orders its stores before its
+// counting thread, whose fence for this GPU hands them to the last one, whose fence hands all of them to the system (release is cumulative, whatever
+// the scope of the steps in front); the stores behind that fence need no order of their own. A fence for the system waits about 3 us here:
+// with one in every CTA and a release store per flag the low-latency pair of 128 tokens took 14.2 + 15.6 us, so 10.3 + 12.4.
+__device__ __forceinline__ void raise_flags(const Team &t, uint64_t flags, uint32_t me, uint32_t epoch)
+{
+    fence_sys();
+    for (uint32_t r = 0; r < t.world; r++)
+        asm volatile("st.relaxed.sys.global.u32 [%0], %1;" ::"l"(reinterpret_cast<uint32_t *>(peer_ptr(t, r, flags)) + me), "r"(epoch) : "memory");
+}
+
+// End of a dispatch, all threads of every CTA: the CTA that finishes last raises this rank's flag on every peer.
 // Returns whether this CTA was the last one. Nobody waits for the peers here: a waiting CTA of this kernel would keep an SM
 // from kernels on other streams (a launch that needs every SM among them), which the one-warp k_moe_wait_all does not; that
 // kernel lets its own successor start only when the flags are there.
-__device__ __forceinline__ bool finish_dispatch(const DispatchArgs &a, uint32_t me)
+// epoch_dev: the call counter in device memory, if the last CTA is to advance it (all CTAs have read it by then).
+__device__ __forceinline__ bool finish_dispatch(const DispatchArgs &a, uint32_t me, uint32_t *epoch_dev = nullptr)
 {
     const Team &t = a.team;
     __shared__ int last_sh;
     __syncthreads();
     if (threadIdx.x == 0) {
-        fence_sys();
+        __threadfence();  // to the CTA that finishes last
         const uint32_t done = atomicAdd(a.done_count, 1u) + 1;
         // seq > 0: the counter only grows and the host numbers the calls; seq == 0: the last CTA puts it back
         // to zero, so the same launch parameters work again (CUDA-graph replay)
         const bool last = a.seq != 0 ? done == gridDim.x * a.seq : done == gridDim.x;
         if (last) {
             if (a.seq == 0) *a.done_count = 0;
-            __threadfence();  // acquires what the other CTAs' fences released; the flag stores below release it to the system
+            if (epoch_dev != nullptr) *epoch_dev = a.epoch;
+            raise_flags(t, a.hp.flags, me, a.epoch);
         }
         last_sh = last ? 1 : 0;
     }
     __syncthreads();
-    if (last_sh && threadIdx.x < t.world)
-        st_release_sys(reinterpret_cast<uint32_t *>(peer_ptr(t, threadIdx.x, a.hp.flags)) + me, a.epoch);
     return last_sh != 0;
 }
 
-constexpr int kTokBatch = 32;  // tokens whose routing table a CTA resolves in one pass
-
-__device__ __forceinline__ bool dispatch_body(const DispatchArgs &a, uint4 nxt_lo, uint4 nxt_hi)
+// Smooth-quant factors of this thread's 16 columns: the same for every token.
+__device__ __forceinline__ bool load_smooth(const DispatchArgs &a, int vec, int vecs, float (&smooth)[16])
 {
-    const Team &t = a.team;
-    const uint32_t me = team_rank(t);
-    const int H = a.sh.H, K = a.sh.K, El = a.sh.E / (int)t.world;
-    const int groups = H / kQuantGroup;
-    const int vec = threadIdx.x;          // 16-element vector index inside the row
-    const int vecs = H / 16;
-    // Routing table of the next kTokBatch tokens of this CTA (destination rank, row there, weight), resolved by all
-    // threads at once: the chain expert id -> put offset -> position is two dependent global loads, which would
-    // otherwise sit in front of every single token.
-    __shared__ int dst_rank[kTokBatch][16];
-    __shared__ int dst_pos[kTokBatch][16];
-    __shared__ float dst_w[kTokBatch][16];
-    __shared__ __align__(16) float s_scale[2][64];  // the row's 1 x 128 scales, leaving as one burst per destination
-    const int stride = (int)gridDim.x;
-    // smooth-quant factors of this thread's 16 columns: the same for every token
-    float smooth[16];
 #pragma unroll
     for (int i = 0; i < 16; i++) smooth[i] = 1.f;
     const bool smoothed = a.smooth != nullptr && !a.raw_bf16;
@@ -377,6 +370,101 @@ __device__ __forceinline__ bool dispatch_body(const DispatchArgs &a, uint4 nxt_l
             smooth[4 * i] = s4.x, smooth[4 * i + 1] = s4.y, smooth[4 * i + 2] = s4.z, smooth[4 * i + 3] = s4.w;
         }
     }
+    return smoothed;
+}
+
+// This thread's 16 elements of a row as e4m3; the 128-group's scale goes to sc.
+__device__ __forceinline__ uint4 quantise_16(const DispatchArgs &a, const uint4 &lo, const uint4 &hi, const float (&smooth)[16], bool smoothed, int vec, int vecs, float *sc)
+{
+    float f[16];
+    const __nv_bfloat162 *h0 = reinterpret_cast<const __nv_bfloat162 *>(&lo);
+    const __nv_bfloat162 *h1 = reinterpret_cast<const __nv_bfloat162 *>(&hi);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        float2 p = __bfloat1622float2(h0[i]);
+        f[2 * i] = p.x;
+        f[2 * i + 1] = p.y;
+        p = __bfloat1622float2(h1[i]);
+        f[8 + 2 * i] = p.x;
+        f[8 + 2 * i + 1] = p.y;
+    }
+    if (smoothed) {
+#pragma unroll
+        for (int i = 0; i < 16; i++) f[i] *= smooth[i];
+    }
+    float amax = 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; i++) amax = fmaxf(amax, fabsf(f[i]));
+    // the 8 threads of a 128-group are consecutive lanes of one warp; every lane takes part
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
+    const float scale = pow2_scale_e4m3(amax);   // a power of two: the expert GEMM feeds it to the tensor core as a UE8M0 byte
+    const float mul = 1.f / scale;
+    uint4 q;
+    q.x = pack4_e4m3(f[0], f[1], f[2], f[3], mul);
+    q.y = pack4_e4m3(f[4], f[5], f[6], f[7], mul);
+    q.z = pack4_e4m3(f[8], f[9], f[10], f[11], mul);
+    q.w = pack4_e4m3(f[12], f[13], f[14], f[15], mul);
+    if (!a.raw_bf16 && vec < vecs && (vec & 7) == 0) sc[vec >> 3] = scale;
+    return q;
+}
+
+// One token's row to the K ranks and rows of d_rank / d_pos (rank -1: nowhere), by all threads of the CTA.
+__device__ __forceinline__ void push_row(const DispatchArgs &a, uint32_t me, int tok, int vec, int vecs, const uint4 &q, const uint4 &raw_lo, const uint4 &raw_hi,
+                                         const float *sc, const int *d_rank, const int *d_pos, const float *d_w)
+{
+    const Team &t = a.team;
+    const int H = a.sh.H, groups = H / kQuantGroup;
+    for (int k = 0; k < a.sh.K; k++) {
+        const int d = d_rank[k];
+        if (d < 0) continue;
+        const int64_t pos = d_pos[k];
+        if (vec < vecs) {
+            if (a.raw_bf16) {
+                uint4 *row = reinterpret_cast<uint4 *>(peer_ptr(t, d, a.hp.recv_x) + pos * H * 2 + vec * 32);
+                row[0] = raw_lo;
+                row[1] = raw_hi;
+            } else {
+                *reinterpret_cast<uint4 *>(peer_ptr(t, d, a.hp.recv_x) + pos * H + vec * 16) = q;
+            }
+        }
+        if (!a.raw_bf16) {
+            // scales: groups * 4 bytes, contiguous in the receiver's array: 16-byte stores from the last warp's lanes
+            // (one or two NVLink packets per row instead of one partial write per 128-group)
+            const int sv = threadIdx.x - ((int)blockDim.x - 32);
+            float *srow = reinterpret_cast<float *>(peer_ptr(t, d, a.hp.recv_scale)) + pos * groups;
+            if (sv >= 0) {
+                if (((pos * groups) & 3) == 0 && (groups & 3) == 0) {
+                    if (sv < groups / 4) reinterpret_cast<float4 *>(srow)[sv] = reinterpret_cast<const float4 *>(sc)[sv];
+                } else {
+                    for (int g = sv; g < groups; g += 32) srow[g] = sc[g];
+                }
+            }
+        }
+        if (threadIdx.x == 0) reinterpret_cast<int4 *>(peer_ptr(t, d, a.hp.recv_info))[pos] = make_int4((int)me, tok, k, __float_as_int(d_w[k]));
+    }
+}
+
+constexpr int kTokBatch = 32;  // tokens whose routing table a CTA resolves in one pass
+
+__device__ __forceinline__ bool dispatch_body(const DispatchArgs &a, uint4 nxt_lo, uint4 nxt_hi)
+{
+    const Team &t = a.team;
+    const uint32_t me = team_rank(t);
+    const int H = a.sh.H, K = a.sh.K, El = a.sh.E / (int)t.world;
+    const int vec = threadIdx.x;          // 16-element vector index inside the row
+    const int vecs = H / 16;
+    // Routing table of the next kTokBatch tokens of this CTA (destination rank, row there, weight), resolved by all
+    // threads at once: the chain expert id -> put offset -> position is two dependent global loads, which would
+    // otherwise sit in front of every single token.
+    __shared__ int dst_rank[kTokBatch][16];
+    __shared__ int dst_pos[kTokBatch][16];
+    __shared__ float dst_w[kTokBatch][16];
+    __shared__ __align__(16) float s_scale[2][64];  // the row's 1 x 128 scales, leaving as one burst per destination
+    const int stride = (int)gridDim.x;
+    float smooth[16];
+    const bool smoothed = load_smooth(a, vec, vecs, smooth);
     for (int base = blockIdx.x; base < a.sh.T; base += stride * kTokBatch) {
         __syncthreads();  // the previous batch's table is no longer read
         for (int e = threadIdx.x; e < kTokBatch * K; e += blockDim.x) {
@@ -401,86 +489,17 @@ __device__ __forceinline__ bool dispatch_body(const DispatchArgs &a, uint4 nxt_l
         for (int j = 0; j < kTokBatch; j++) {
             const int tok = base + j * stride;
             if (tok >= a.sh.T) break;
-            uint4 q;
-            uint4 raw_lo = make_uint4(0, 0, 0, 0), raw_hi = make_uint4(0, 0, 0, 0);
+            const uint4 lo = nxt_lo, hi = nxt_hi;
+            const int nxt = tok + stride;
+            if (vec < vecs && nxt < a.sh.T) {
+                const uint4 *src = reinterpret_cast<const uint4 *>(a.x + (int64_t)nxt * H + vec * 16);
+                nxt_lo = __ldcg(src);
+                nxt_hi = __ldcg(src + 1);
+            }
             float *sc = s_scale[j & 1];
-            {
-                float f[16];
-#pragma unroll
-                for (int i = 0; i < 16; i++) f[i] = 0.f;
-                if (vec < vecs) {
-                    const uint4 lo = nxt_lo, hi = nxt_hi;
-                    raw_lo = lo;
-                    raw_hi = hi;
-                    const int nxt = tok + stride;
-                    if (nxt < a.sh.T) {
-                        const uint4 *src = reinterpret_cast<const uint4 *>(a.x + (int64_t)nxt * H + vec * 16);
-                        nxt_lo = __ldcg(src);
-                        nxt_hi = __ldcg(src + 1);
-                    }
-                    const __nv_bfloat162 *h0 = reinterpret_cast<const __nv_bfloat162 *>(&lo);
-                    const __nv_bfloat162 *h1 = reinterpret_cast<const __nv_bfloat162 *>(&hi);
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        float2 p = __bfloat1622float2(h0[i]);
-                        f[2 * i] = p.x;
-                        f[2 * i + 1] = p.y;
-                        p = __bfloat1622float2(h1[i]);
-                        f[8 + 2 * i] = p.x;
-                        f[8 + 2 * i + 1] = p.y;
-                    }
-                }
-                if (smoothed) {
-#pragma unroll
-                    for (int i = 0; i < 16; i++) f[i] *= smooth[i];
-                }
-                float amax = 0.f;
-#pragma unroll
-                for (int i = 0; i < 16; i++) amax = fmaxf(amax, fabsf(f[i]));
-                // the 8 threads of a 128-group are consecutive lanes of one warp; every lane takes part
-                amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-                amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-                amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-                const float scale = pow2_scale_e4m3(amax);   // a power of two: the expert GEMM feeds it to the tensor core as a UE8M0 byte
-                const float mul = 1.f / scale;
-                q.x = pack4_e4m3(f[0], f[1], f[2], f[3], mul);
-                q.y = pack4_e4m3(f[4], f[5], f[6], f[7], mul);
-                q.z = pack4_e4m3(f[8], f[9], f[10], f[11], mul);
-                q.w = pack4_e4m3(f[12], f[13], f[14], f[15], mul);
-                if (!a.raw_bf16 && vec < vecs && (vec & 7) == 0) sc[vec >> 3] = scale;
-            }
+            const uint4 q = quantise_16(a, lo, hi, smooth, smoothed, vec, vecs, sc);
             if (!a.raw_bf16) __syncthreads();  // the row's scales are complete (the buffers alternate: one barrier per token)
-            for (int k = 0; k < K; k++) {
-                const int d = dst_rank[j][k];
-                if (d < 0) continue;
-                const int64_t pos = dst_pos[j][k];
-                if (vec < vecs) {
-                    if (a.raw_bf16) {
-                        uint4 *row = reinterpret_cast<uint4 *>(peer_ptr(t, d, a.hp.recv_x) + pos * H * 2 + vec * 32);
-                        row[0] = raw_lo;
-                        row[1] = raw_hi;
-                    } else {
-                        *reinterpret_cast<uint4 *>(peer_ptr(t, d, a.hp.recv_x) + pos * H + vec * 16) = q;
-                    }
-                }
-                if (!a.raw_bf16) {
-                    // scales: groups * 4 bytes, contiguous in the receiver's array: 16-byte stores from the last warp's lanes
-                    // (one or two NVLink packets per row instead of one partial write per 128-group)
-                    const int sv = threadIdx.x - ((int)blockDim.x - 32);
-                    float *srow = reinterpret_cast<float *>(peer_ptr(t, d, a.hp.recv_scale)) + pos * groups;
-                    if (sv >= 0) {
-                        if (((pos * groups) & 3) == 0 && (groups & 3) == 0) {
-                            if (sv < groups / 4) reinterpret_cast<float4 *>(srow)[sv] = reinterpret_cast<const float4 *>(sc)[sv];
-                        } else {
-                            for (int g = sv; g < groups; g += 32) srow[g] = sc[g];
-                        }
-                    }
-                }
-                if (threadIdx.x == 0) {
-                    int4 info = make_int4((int)me, tok, k, __float_as_int(dst_w[j][k]));
-                    reinterpret_cast<int4 *>(peer_ptr(t, d, a.hp.recv_info))[pos] = info;
-                }
-            }
+            push_row(a, me, tok, vec, vecs, q, lo, hi, sc, dst_rank[j], dst_pos[j], dst_w[j]);
         }
     }
     return finish_dispatch(a, me);
@@ -713,35 +732,36 @@ __device__ __forceinline__ void combine_push_body(const CombinePushArgs &a)
     const int rows = *a.rows_dev;
     const int vecs = a.H / 8;
     const int4 *info = reinterpret_cast<const int4 *>(peer_ptr(t, me, a.hp.recv_info));
-    // one warp per row, four 16-byte loads in flight per lane before the first store: at decode sizes the
-    // push is bound by NVLink latency, so rows must overlap rather than queue behind one another
+    // A warp takes a piece of a row, at most eight 16-byte loads per lane, all in flight before the first store: at decode sizes the push is bound by
+    // latencies, so the pieces of a row overlap rather than queue behind one another. (A row of 7168 per warp, four loads at a time, seven times over:
+    // the low-latency combine of 1024 rows 17.8 us; a quarter of a row per warp and 512 threads per CTA 15.6, 768 or 1024 threads 18.)
     const int lane = threadIdx.x & 31;
     const int warps = gridDim.x * (blockDim.x >> 5);
-    for (int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < rows; r += warps) {
+    const int pieces = (vecs + 255) / 256, per = ((vecs + pieces - 1) / pieces + 31) / 32 * 32;
+    for (int64_t x = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); x < (int64_t)rows * pieces; x += warps) {
+        const int r = (int)(x / pieces), beg = (int)(x - (int64_t)r * pieces) * per, end = min(beg + per, vecs);
+        const uint4 *src = reinterpret_cast<const uint4 *>(a.y + (int64_t)r * a.ldy);
+        uint4 raw[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            if (beg + u * 32 + lane < end) raw[u] = __ldg(src + beg + u * 32 + lane);
         const int4 in = __ldcg(info + r);
         const uint32_t home = (uint32_t)in.x;
         if (home >= t.world) continue;
         const float w = a.weighted ? __int_as_float(in.w) : 1.f;
         uint4 *dst = reinterpret_cast<uint4 *>(reinterpret_cast<__nv_bfloat16 *>(peer_ptr(t, home, a.hp.comb)) + ((int64_t)in.y * a.K + in.z) * a.H);
-        const uint4 *src = reinterpret_cast<const uint4 *>(a.y + (int64_t)r * a.ldy);
-        for (int v0 = lane; v0 < vecs; v0 += 128) {
-            uint4 raw[4];
 #pragma unroll
-            for (int u = 0; u < 4; u++)
-                if (v0 + 32 * u < vecs) raw[u] = __ldg(src + v0 + 32 * u);
+        for (int u = 0; u < 8; u++) {
+            if (beg + u * 32 + lane >= end) continue;
+            if (w != 1.f) {
+                __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(&raw[u]);
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-                if (v0 + 32 * u >= vecs) continue;
-                if (w != 1.f) {
-                    __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(&raw[u]);
-#pragma unroll
-                    for (int e = 0; e < 4; e++) {
-                        float2 f = __bfloat1622float2(h[e]);
-                        h[e] = __floats2bfloat162_rn(f.x * w, f.y * w);
-                    }
+                for (int e = 0; e < 4; e++) {
+                    float2 f = __bfloat1622float2(h[e]);
+                    h[e] = __floats2bfloat162_rn(f.x * w, f.y * w);
                 }
-                dst[v0 + 32 * u] = raw[u];
             }
+            dst[beg + u * 32 + lane] = raw[u];
         }
     }
 }
@@ -820,6 +840,22 @@ struct LLDispatchArgs {
                              // end, so a captured launch can be replayed (d.epoch is ignored, d.seq must be 0)
 };
 
+// The last CTA of a low-latency dispatch waits for every peer's rows.
+__device__ __forceinline__ void ll_wait_rows(const LLDispatchArgs &a, uint32_t me)
+{
+    const Team &t = a.d.team;
+    MF_PROF_START(PF_WAIT_PEERS);
+    if (threadIdx.x < t.world && threadIdx.x != me) {  // its own rank's rows are stored: that is what made it the last one
+        const uint32_t *f = reinterpret_cast<const uint32_t *>(peer_ptr(t, me, a.d.hp.flags)) + threadIdx.x;
+        if (!wait_flag(f, a.d.epoch, t.spin_limit)) {
+            report_timeout(t, me, 0x421, a.d.epoch);
+            atomicCAS(a.d.status, 0, 0x421);
+        }
+    }
+    __syncthreads();
+    MF_PROF_STOP(PF_WAIT_PEERS);
+}
+
 __global__ void __launch_bounds__(448) k_moe_ll_dispatch(LLDispatchArgs a)
 {
     cooperative_groups::grid_group grid = cooperative_groups::this_grid();
@@ -852,17 +888,165 @@ __global__ void __launch_bounds__(448) k_moe_ll_dispatch(LLDispatchArgs a)
     MF_PROF_START(PF_DISPATCH);
     const bool last = dispatch_body(a.d, pre_lo, pre_hi);
     MF_PROF_STOP(PF_DISPATCH);
-    if (!last) return;  // uniform over the CTA
-    MF_PROF_START(PF_WAIT_PEERS);
-    if (threadIdx.x < t.world) {
-        const uint32_t *f = reinterpret_cast<const uint32_t *>(peer_ptr(t, me, a.d.hp.flags)) + threadIdx.x;
-        if (!wait_flag(f, a.d.epoch, t.spin_limit)) {
-            report_timeout(t, me, 0x421, a.d.epoch);
-            atomicCAS(a.d.status, 0, 0x421);
+    if (last) ll_wait_rows(a, me);  // uniform over the CTA
+}
+
+// The same call for a batch of a few tokens per CTA, without the chain layout -> count exchange -> grid-wide barrier -> routing table: every CTA reads all
+// of the routing (a few KB) and counts it by itself, finds the places of its own entries in token order, and takes the other ranks' counts from
+// this rank's table as soon as their flags are up (CTA 0 has sent this rank's). Its first row is quantised by then. One rank waits for
+// nothing in front of its stores. What bounds it are the latencies that are left: routing and rows from memory, the stores' way to
+// memory, the counter of finished CTAs, the flag. The ranks need not take the same kernel: the exchange is the other one's.
+// Tokens of 7168, 8 of 32 experts, one rank, us, the other kernel / this one (the fences of finish_dispatch not counted): 1 token 16.3 / 11.0, 128 19.5 / 14.2,
+// 256 24.1 / 18.3. A pass of the pair with a stand-in expert, 128 tokens: 81 before this kernel and the present combine, 66.
+constexpr int kLLTokens = 4;        // tokens of a CTA
+constexpr int kLLEntries = 4096;    // entries in all: a CTA looks at every entry once for each of its own
+__global__ void __launch_bounds__(448) k_moe_ll_dispatch_few(LLDispatchArgs a)
+{
+    const Team &t = a.d.team;
+    const uint32_t me = team_rank(t), W = t.world;
+    const int T = a.d.sh.T, K = a.d.sh.K, E = a.d.sh.E, H = a.d.sh.H, n = T * K, El = E / (int)W;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (int)(blockDim.x >> 5);
+    __shared__ uint16_t ids[kLLEntries];
+    __shared__ int cnt[1024];    // this rank's entries per expert; then all ranks'
+    __shared__ int put[1024];    // lower ranks' entries per expert; then where this rank's group starts in the owner's buffer
+    __shared__ int dst_rank[kLLTokens][16], dst_pos[kLLTokens][16];
+    __shared__ float dst_w[kLLTokens][16];
+    __shared__ __align__(16) float s_scale[2][64];
+    __shared__ int ok_sh;
+    MF_PROF_START(PF_LAYOUT);
+    a.d.epoch = *reinterpret_cast<volatile uint32_t *>(a.epoch_dev) + 1;
+    const int vec = threadIdx.x, vecs = H / 16;
+    uint4 lo, hi;
+    dispatch_preload(a.d, lo, hi);
+    for (int e = threadIdx.x; e < E; e += blockDim.x) {
+        cnt[e] = 0;
+        put[e] = 0;
+    }
+    if (threadIdx.x == 0) ok_sh = 1;
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const int e = a.d.topk_idx[i];
+        const bool on = e >= 0 && e < E;
+        ids[i] = on ? (uint16_t)e : (uint16_t)0xffff;
+        if (on) atomicAdd(&cnt[e], 1);
+    }
+    float smooth[16];
+    const bool smoothed = load_smooth(a.d, vec, vecs, smooth);
+    uint4 q = quantise_16(a.d, lo, hi, smooth, smoothed, vec, vecs, s_scale[0]);
+    __syncthreads();
+    const uint64_t bar = kBarrierOff + 9 * 256;  // the channel of the pair's count exchange
+    if (W > 1) {
+        if (blockIdx.x == 0) {
+            for (int e = threadIdx.x; e < E; e += blockDim.x)
+                for (uint32_t k = 0; k < W; k++) reinterpret_cast<int *>(peer_ptr(t, (me + k) % W, a.d.hp.counts))[me * E + e] = cnt[e];
+            __syncthreads();
+            if (threadIdx.x < W) st_release_sys(reinterpret_cast<uint32_t *>(peer_ptr(t, threadIdx.x, bar)) + me, a.d.epoch);
         }
     }
+    // places of this CTA's entries: how many entries in front of them name the same expert
+    const int own = T > (int)blockIdx.x ? (T - (int)blockIdx.x - 1) / (int)gridDim.x + 1 : 0;  // tokens blockIdx.x + j * gridDim.x
+    for (int x = warp; x < own * K; x += warps) {
+        const int j = x / K, k = x - j * K, i = ((int)blockIdx.x + j * (int)gridDim.x) * K + k;
+        const int e = ids[i];
+        int before = 0;
+        for (int o = lane; o < i; o += 32) before += ids[o] == e;
+        before = __reduce_add_sync(0xffffffffu, before);
+        if (lane == 0) {
+            const_cast<int *>(a.d.send_idx)[i] = e != 0xffff ? before : 0;
+            dst_rank[j][k] = e != 0xffff ? e : -1;  // for now the expert
+            dst_pos[j][k] = before;
+            dst_w[j][k] = e != 0xffff ? a.d.topk_w[i] : 0.f;
+        }
+    }
+    const int *tbl = reinterpret_cast<const int *>(peer_ptr(t, me, a.d.hp.counts));
+    const bool tables = blockIdx.x == gridDim.x - 1;  // this CTA leaves the tables for the caller
+    if (tables)
+        for (int e = threadIdx.x; e < E; e += blockDim.x) a.tokens_per_expert[e] = cnt[e];
+    if (W > 1) {
+        if (threadIdx.x < W && !wait_flag(reinterpret_cast<const uint32_t *>(peer_ptr(t, me, bar)) + threadIdx.x, a.d.epoch, t.spin_limit)) {
+            ok_sh = 0;
+            report_timeout(t, me, 0x1009, a.d.epoch);
+            atomicCAS(a.d.status, 0, 0x420);
+        }
+        __syncthreads();
+        if (ok_sh) {
+            for (int e = threadIdx.x; e < E; e += blockDim.x) {
+                int all = 0, lower = 0;
+                for (uint32_t r = 0; r < W; r++) {
+                    if (r == me) lower = all;
+                    all += __ldcg(tbl + r * E + e);
+                }
+                cnt[e] = all;
+                put[e] = lower;
+            }
+        }
+        __syncthreads();
+    }
+    const bool ok = ok_sh != 0;
+    // where every expert's rows start in its owner's buffer: a warp per owner
+    for (int d = warp; d < (int)W; d += warps) {
+        int run = 0;
+        for (int l0 = 0; l0 < El; l0 += 32) {
+            const int v = l0 + lane < El ? cnt[d * El + l0 + lane] : 0;
+            int upto = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int below = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += below;
+            }
+            if (l0 + lane < El) {
+                const int first = run + upto - v;
+                put[d * El + l0 + lane] += first;
+                if (tables && d == (int)me) {
+                    a.row_off[l0 + lane] = ok ? first : 0;
+                    a.recv_per_expert[l0 + lane] = ok ? v : 0;
+                    int off = first;
+                    for (uint32_t r = 0; r < W; r++) {
+                        a.src_off[(l0 + lane) * (int)W + (int)r] = ok ? off : 0;
+                        if (W > 1 && ok) off += __ldcg(tbl + r * E + me * El + l0 + lane);
+                    }
+                }
+            }
+            run += __shfl_sync(0xffffffffu, upto, 31);
+        }
+        if (tables && d == (int)me && lane == 0) a.row_off[El] = ok ? run : 0;
+    }
     __syncthreads();
-    MF_PROF_STOP(PF_WAIT_PEERS);
+    if (tables)
+        for (int e = threadIdx.x; e < E; e += blockDim.x) const_cast<int *>(a.d.put_off)[e] = ok ? put[e] : -1;
+    for (int x = threadIdx.x; x < own * 16; x += blockDim.x) {
+        const int j = x >> 4, k = x & 15;
+        if (k >= K) continue;
+        const int e = dst_rank[j][k];
+        if (e < 0) continue;
+        const int pos = put[e] + dst_pos[j][k];
+        dst_pos[j][k] = pos;
+        const bool fits = pos < a.d.sh.max_recv;
+        if (ok && !fits) atomicCAS(a.d.status, 0, 0x401);  // receive buffer too small: dropped, reported
+        dst_rank[j][k] = ok && fits ? e / El : -1;
+    }
+    __syncthreads();
+    MF_PROF_STOP(PF_LAYOUT);
+    MF_PROF_START(PF_DISPATCH);
+    for (int j = 0; j < own; j++) {
+        const int tok = (int)blockIdx.x + j * (int)gridDim.x;
+        uint4 nlo = make_uint4(0, 0, 0, 0), nhi = nlo;
+        if (j + 1 < own && vec < vecs) {
+            const uint4 *src = reinterpret_cast<const uint4 *>(a.d.x + (int64_t)(tok + (int)gridDim.x) * H + vec * 16);
+            nlo = __ldcg(src);
+            nhi = __ldcg(src + 1);
+        }
+        push_row(a.d, me, tok, vec, vecs, q, lo, hi, s_scale[j & 1], dst_rank[j], dst_pos[j], dst_w[j]);
+        if (j + 1 < own) {
+            lo = nlo;
+            hi = nhi;
+            q = quantise_16(a.d, lo, hi, smooth, smoothed, vec, vecs, s_scale[(j + 1) & 1]);
+            __syncthreads();
+        }
+    }
+    const bool last = finish_dispatch(a.d, me, a.epoch_dev);
+    MF_PROF_STOP(PF_DISPATCH);
+    if (last) ll_wait_rows(a, me);  // uniform over the CTA
 }
 
 struct LLCombineArgs {
@@ -877,7 +1061,7 @@ struct LLCombineArgs {
     uint32_t *done_count;       // counts this launch's CTAs, zero between launches (the dispatch's counter serves)
 };
 
-__global__ void __launch_bounds__(256) k_moe_ll_combine(LLCombineArgs a)
+__global__ void __launch_bounds__(512) k_moe_ll_combine(LLCombineArgs a)
 {
     const Team &t = a.p.team;
     const uint32_t me = team_rank(t);
@@ -887,21 +1071,16 @@ __global__ void __launch_bounds__(256) k_moe_ll_combine(LLCombineArgs a)
     MF_PROF_STOP(PF_PUSH);
     // The last CTA to finish pushing raises this rank's flag on every peer; every CTA waits for the peers' flags itself (its
     // own rank's among them, so nobody reduces before this rank's rows are stored): no grid-wide barrier on either side.
-    __shared__ int last_sh;
     __syncthreads();
     if (threadIdx.x == 0) {
-        fence_sys();
-        const uint32_t done = atomicAdd(a.done_count, 1u) + 1;
-        last_sh = done == gridDim.x ? 1 : 0;
-        if (done == gridDim.x) {
+        __threadfence();  // to the CTA that finishes last
+        if (atomicAdd(a.done_count, 1u) + 1 == gridDim.x) {
             *a.done_count = 0;
-            __threadfence();  // as in finish_dispatch
+            raise_flags(t, a.p.hp.flags + kMaxRanks * sizeof(uint32_t), me, a.epoch);
         }
     }
-    __syncthreads();
     if (blockIdx.x == 0) MF_PROF_START(PF_WAIT_PEERS);
     if (threadIdx.x < t.world) {
-        if (last_sh) st_release_sys(reinterpret_cast<uint32_t *>(peer_ptr(t, threadIdx.x, a.p.hp.flags)) + kMaxRanks + me, a.epoch);
         const uint32_t *f = reinterpret_cast<const uint32_t *>(peer_ptr(t, me, a.p.hp.flags)) + kMaxRanks + threadIdx.x;
         if (!wait_flag(f, a.epoch, t.spin_limit)) {
             report_timeout(t, me, 0x422, a.epoch);
@@ -1055,6 +1234,13 @@ int mf_moe_combine_push(const Team *team, const MoeHeap *hp, const void *y, int6
     return e == cudaSuccess ? 0 : (int)e;
 }
 
+// Whether a grid has a CTA per SM at most: the kernels of the low-latency pair that take most of an SM's registers are resident then.
+static bool one_per_sm(int ctas)
+{
+    int dev = 0, sms = 0;
+    return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && ctas <= sms;
+}
+
 // Cooperative: ctas must not exceed what the device can hold at once (one CTA per SM is always safe).
 int mf_moe_ll_dispatch(const DispatchArgs *d, int *tokens_per_expert, int *recv_per_expert, int *row_off, int *src_off, uint32_t *epoch_dev,
                        int ctas, void *stream)
@@ -1065,8 +1251,9 @@ int mf_moe_ll_dispatch(const DispatchArgs *d, int *tokens_per_expert, int *recv_
         return -1;
     LLDispatchArgs a{*d, tokens_per_expert, recv_per_expert, row_off, src_off, epoch_dev};
     void *params[] = {&a};
-    cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_moe_ll_dispatch), dim3(ctas), dim3(448), params, 0,
-                                                (cudaStream_t)stream);
+    const bool few = d->sh.T <= kLLTokens * ctas && d->sh.T * d->sh.K <= kLLEntries && one_per_sm(ctas);
+    cudaError_t e = cudaLaunchCooperativeKernel(few ? reinterpret_cast<const void *>(k_moe_ll_dispatch_few) : reinterpret_cast<const void *>(k_moe_ll_dispatch),
+                                                dim3(ctas), dim3(448), params, 0, (cudaStream_t)stream);
     return e == cudaSuccess ? 0 : (int)e;
 }
 
@@ -1078,7 +1265,7 @@ int mf_moe_ll_combine(const Team *team, const MoeHeap *hp, const MoeShape *sh, c
     LLCombineArgs a{{*team, *hp, static_cast<const __nv_bfloat16 *>(y), ldy, rows_dev, sh->H, sh->K, weighted}, *sh, topk_idx,
                     static_cast<__nv_bfloat16 *>(out), epoch, status, topk_w, epoch_dev, done_count};
     void *params[] = {&a};
-    cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_moe_ll_combine), dim3(ctas), dim3(256), params, 0,
+    cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_moe_ll_combine), dim3(ctas), dim3(one_per_sm(ctas) ? 512 : 256), params, 0,
                                                 (cudaStream_t)stream);
     return e == cudaSuccess ? 0 : (int)e;
 }

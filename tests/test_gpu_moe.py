@@ -590,6 +590,68 @@ def test_a_count_exchange_that_times_out_sends_and_receives_nothing(how, raw_bf1
     assert bool((data == 0x5A).all()), "a row was stored"
 
 
+def _ll_rank(rank, world, url, sync):
+    import torch
+    from memfabric_hybrid_b200.ops import moe as M
+    from memfabric_hybrid_b200.ops.gemm import check_status
+    from memfabric_hybrid_b200.ops.heap import SymmetricHeap
+    bad = []
+    heap = SymmetricHeap(url, 1, 0, 0, 256 << 20)
+    # (hidden, experts, copies, tokens): a token per CTA, up to four, and more (the kernel with a grid-wide barrier); entries that nobody selected
+    for H, E, K, sizes in ((512, 8, 2, (1, 3)), (7168, 32, 8, (1, 147, 149, 256)), (1152, 40, 5, (1, 7, 593, 600)), (640, 1024, 16, (2, 256, 257))):
+        mark = heap.mark()
+        comm = M.MoEComm(heap, max(sizes), H, E, K, max_recv=max(sizes) * K)
+        for T in sizes:
+            g = torch.Generator("cuda").manual_seed(T + H)
+            x = torch.randn(T, H, device="cuda", generator=g).to(torch.bfloat16)
+            idx = torch.stack([torch.randperm(E, device="cuda", generator=g)[:K] for _ in range(T)]).to(torch.int32)
+            if T > 2:
+                idx[1] = -1
+                idx[2, 0] = -1
+            w = torch.rand(T, K, device="cuda", generator=g)
+            for _ in range(2):   # the counter of calls moves on
+                d = comm.ll_dispatch(x, idx, w)
+                rows = int(d.row_off[-1])
+                q, s = comm.recv_x()[:rows].float(), comm.recv_scale()[:rows]
+                y = (q.view(rows, -1, 128) * s[:, :, None]).view(rows, H).to(torch.bfloat16)
+                info = comm.recv_info()[:rows].cpu()
+                out = comm.ll_combine(y, d)
+                torch.cuda.synchronize()
+                check_status()
+                flat = idx.cpu().view(-1)
+                counts = torch.bincount(flat[flat >= 0].long(), minlength=E)
+                off = torch.cat([torch.zeros(1, dtype=torch.long), counts.cumsum(0)])
+                ok = torch.equal(d.row_off.cpu().long(), off) and torch.equal(d.recv_per_expert.cpu().long(), counts) and torch.equal(d.tokens_per_expert.cpu().long(), counts)
+                ok = ok and torch.equal(d.put_off.cpu().long(), off[:-1]) and torch.equal(d.src_off.cpu().long(), off[:-1])
+                # every selected entry once, in its expert's group, where send_idx says
+                entry = info[:, 1].long() * K + info[:, 2].long()
+                ok = ok and torch.equal(entry.sort().values, (flat >= 0).nonzero().view(-1))
+                ok = ok and torch.equal(off[flat[entry].long()] + d.send_idx.cpu().long()[entry], torch.arange(rows))
+                ok = ok and torch.equal(info[:, 3].view(torch.float32), w.cpu().view(-1)[entry])
+                # a row is its token quantised; the sum of the weighted answers in bf16 steps
+                xq = y.cpu()
+                for a in {0, rows // 2, rows - 1} if rows else ():
+                    t = x[int(info[a, 1])].cpu().float()
+                    ok = ok and bool(((xq[a].float() - t).abs() <= t.abs() * 2.0 ** -4 + t.view(-1, 128).abs().amax(1).repeat_interleave(128) * 2.0 ** -9).all())
+                ref = torch.zeros(T, H)
+                ref.index_add_(0, info[:, 1].long(), (xq.float() * w.cpu().view(-1)[entry][:, None]).to(torch.bfloat16).float())
+                got = out.cpu().float()
+                ok = ok and bool(((got - ref).abs() <= ref.abs() * 2.0 ** -8 + 1e-5).all())
+                if not ok:
+                    bad.append((H, E, K, T))
+        heap.release_to(mark)
+    st = heap.status()[0]
+    heap.close()
+    SymmetricHeap.shutdown()
+    return bad, st
+
+
+def test_low_latency_pair_around_its_tokens_per_cta():
+    url = f"127.0.0.1:{free_port()}"
+    (bad, st), = run_ranks(_ll_rank, 1, (url,), timeout=300, with_barrier=True)
+    assert not bad and st == 0, (bad, st)
+
+
 def _refused_rank(rank, world, url, sync):
     import torch
     from memfabric_hybrid_b200.ops import moe as M
