@@ -219,6 +219,10 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_t
     const uint32_t tmem_base = *sm.tmem_slot();
     const int total = (g.max_rows / BM) * n_tiles;
     const uint32_t me = g.team.rank;
+    // MODE 2 by one rank: there are no partials to wait for, so a tile's epilogue writes its rows of y itself, under the next tile's MMAs. Adding up behind the
+    // last tile read 67 MB back and wrote as much with the tensor cores idle: 4096 x 8192 outputs, K 3584, 126 us, so (and without a second fence
+    // for the system per tile) 101; 1024 rows 43.2 / 36.0, 128 rows 23.3 / 20.0. With more ranks the loads of the other partials would hold the epilogue up.
+    const bool alone = g.team.world == 1;
 
     // linear tile -> (first row, column tile): blocks of rows owned by one rank, visited starting with this rank (MODE 1: the order in
     // which the shards arrive) or with the next rank (MODE 2: remote owners first, own rows last); inside a block the row tile varies fastest
@@ -502,16 +506,28 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_t
                         const unsigned long long d = __shfl_sync(0xffffffffu, dst, p * 8 + r);
                         const uint4 val = *reinterpret_cast<const uint4 *>(stg + r * kWideRowB + (lane & 15) * 16);
                         if (d != 0) *reinterpret_cast<uint4 *>(d + (unsigned long long)((lane & 15) * 16)) = val;
+                        if (MODE == 2 && alone) {
+                            // the only partial there is, rounded as it would be read back
+                            uint4 pk;
+                            const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&val);
+                            __nv_bfloat162 *o = reinterpret_cast<__nv_bfloat162 *>(&pk);
+#pragma unroll
+                            for (int e = 0; e < 4; e++) {
+                                const float2 f = __bfloat1622float2(h[e]);
+                                o[e] = __floats2bfloat162_rn(f.x * g.scale, f.y * g.scale);
+                            }
+                            *reinterpret_cast<uint4 *>(g.y_out + (int64_t)(row0 + quad * 32 + p * 8 + r) * g.ldy + nt * XBN + half * 128 + (lane & 15) * 8) = pk;
+                        }
                     }
                     __syncwarp();
                 }
                 if (MODE == 2) {
                     // all eight epilogue warps have stored their part of the tile: tell the owner
-                    named_bar_sync(9, 256);  // orders all eight warps' stores before the counting thread, whose fence + release publishes them
+                    named_bar_sync(9, 256);  // orders all eight warps' stores before the counting thread, whose release publishes them
                     if (warp == 4 && lane == 0) {
-                        __threadfence_system();
                         const int owner = row0 / g.rows_per_rank;
                         const int ltile = ((row0 - owner * g.rows_per_rank) / BM) * n_tiles + nt;
+                        if (alone) g.tile_uses[ltile]++;
                         uint32_t *cnt = reinterpret_cast<uint32_t *>(peer_ptr(g.team, (uint32_t)owner, g.rs_count_off)) + ltile;
                         asm volatile("red.release.sys.global.add.u32 [%0], 1;" ::"l"(cnt) : "memory");
                     }
@@ -529,14 +545,17 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_t
         const int per = (g.shard_rows + (int)gridDim.x - 1) / (int)gridDim.x;
         const int r0 = min(g.shard_rows, (int)blockIdx.x * per), r1 = min(g.shard_rows, r0 + per);
         auto raise = [&](uint32_t p) {
-            // the CTA that completes this rank's shard in the buffer of rank p raises the flag there
+            // The CTA that completes this rank's shard in the buffer of rank p raises the flag there: every CTA's fence and count hand its stores to that one,
+            // whose fence for the system covers all of them. A fence for the system takes about 3 us, and three of them in a row stood in front of the first
+            // tile of a call (N 7168, K 8192, SwiGLU, us, before / so: 128 rows 44.2 / 40.7, 1024 85.1 / 81.6, 4096 236 / 230).
             __syncwarp();
             if (lane == 0) {
-                __threadfence_system();  // covers the stores ordered before it by the barriers of the warp and of the quantising warps
+                __threadfence();  // covers the stores ordered before it by the barriers of the warp and of the quantising warps
                 const uint32_t done = atomicAdd(g.push_count + p, 1u) + 1;
                 if (done == gridDim.x * g.seq) {
-                    __threadfence_system();
-                    st_release_sys(reinterpret_cast<uint32_t *>(peer_ptr(g.team, p, g.ag_ready_off)) + me, g.epoch);
+                    fence_sys();
+                    asm volatile("st.relaxed.sys.global.u32 [%0], %1;" ::"l"(reinterpret_cast<uint32_t *>(peer_ptr(g.team, p, g.ag_ready_off)) + me), "r"(g.epoch)
+                                 : "memory");
                 }
             }
             __syncwarp();
@@ -564,14 +583,14 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_t
     }
     // MODE 2, thread 0: calls that had this CTA's first owned tile so far. Every tile counts its own: smaller calls leave some out.
     uint32_t uses = 0;
-    if (MODE == 2 && threadIdx.x == 0 && (int)blockIdx.x < (g.rows_per_rank / BM) * n_tiles) uses = g.tile_uses[blockIdx.x];
+    if (MODE == 2 && !alone && threadIdx.x == 0 && (int)blockIdx.x < (g.rows_per_rank / BM) * n_tiles) uses = g.tile_uses[blockIdx.x];
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem_base, kXTmemCols);
     }
-    if (MODE == 2) {
+    if (MODE == 2 && !alone) {
         // add up the W partial tiles of every tile whose rows this rank owns
         __shared__ int ok_sh;
         const int own_tiles = (g.rows_per_rank / BM) * n_tiles;
