@@ -1,6 +1,9 @@
 #include "mf_data_op.h"
 
 #include <sys/uio.h>
+#ifdef __SSE2__
+#include <emmintrin.h>
+#endif
 
 #include <algorithm>
 
@@ -176,7 +179,7 @@ int ComposeDataOp::RunKernel(const std::vector<const ResolvedCopy *> &items, voi
     // descriptor fetch. Multiples of 4 KiB keep the alignment of every chunk equal to that of its item.
     uint64_t sms = std::max(1, dev_->Caps().smCount);
     uint64_t chunk = AlignUp(std::max<uint64_t>(total / (sms * 8), 1), 4096);
-    chunk = std::min(std::max<uint64_t>(chunk, 16 * kKiB), chunk_);
+    chunk = std::min(std::max<uint64_t>(chunk, kMinCopyChunk), chunk_);
     MF_TRACE_BEGIN(TP_HYBM_BATCH_KERNEL);
     size_t i = 0;
     uint64_t off = 0;
@@ -319,7 +322,34 @@ int ComposeDataOp::Submit(std::vector<ResolvedCopy> &items, void *userStream, ui
 }
 
 // ------------------------------------------------------------------------------------------------
-KernelBatch::KernelBatch(ComposeDataOp &op, void *userStream, uint32_t flags, uint64_t totalBytes)
+// A piece that does not fit the share: the next one takes it where little room is left, else it is cut. What a share takes too much or too
+// little, the next one makes up for.
+uint64_t SpanCutter::Split(uint64_t len, uint32_t at, bool rest)
+{
+    const int64_t cost = rest ? 0 : kPieceCost;
+    if (room_ < cost + kMinCut && s_.start[cur_] != at && cur_ + 1 < s_.n) {  // a share has a piece at least
+        s_.start[++cur_] = at;
+        room_ += quota_;
+    }
+    int64_t n = (int64_t)len;
+    if (cost + n > room_ + kMinCut && cur_ + 1 < s_.n) {
+        const int64_t cut = (std::max(room_ - cost, kMinCut) + kCutAlign - 1) & -kCutAlign;
+        if (cut + kMinCut <= n) n = cut;
+    }
+    room_ -= n + cost;
+    return (uint64_t)n;
+}
+
+// Shares for a batch, 0: none. Up to a chunk of the smallest size per CTA, each chunk gets a CTA of its own (100 pieces of up to 16 KiB: one
+// latency for all of them); the chunks are at least as many as the runs and as the bytes would fill.
+static uint32_t SpansFor(const DeviceBackend *dev, const BatchShape &b)
+{
+    const uint32_t n = dev->CopySpanCount();
+    if ((b.alignMask & 15) == 0 || std::max(b.runs, b.bytes / kMinCopyChunk) <= n) return 0;
+    return b.bytes / n < (32u << 10) ? (n + 1) / 2 : n;  // 1500 pieces of up to 16 KiB: the host takes 0.7 us less, the kernel, which it hides, 1.6 more
+}
+
+KernelBatch::KernelBatch(ComposeDataOp &op, void *userStream, uint32_t flags, const BatchShape &shape)
     : op_(op), lock_(op.mu_), flags_(flags)
 {
     if (op_.dev_ == nullptr) {
@@ -331,17 +361,98 @@ KernelBatch::KernelBatch(ComposeDataOp &op, void *userStream, uint32_t flags, ui
     if (rc_ != OK) return;
     stream_ = op_.StreamFor(userStream, flags);
     uint64_t sms = std::max(1, op_.dev_->Caps().smCount);
-    uint64_t chunk = AlignUp(std::max<uint64_t>(totalBytes / (sms * 8), 1), 4096);
-    chunk_ = std::min(std::max<uint64_t>(chunk, 16 * kKiB), op_.chunk_);
+    uint64_t chunk = AlignUp(std::max<uint64_t>(shape.bytes / (sms * 8), 1), 4096);
+    chunk_ = std::min(std::max<uint64_t>(chunk, kMinCopyChunk), op_.chunk_);
+    bulk_ = (shape.alignMask & 15) == 0;
+    spans_ = SpansFor(op_.dev_, shape);
+    if (spans_ != 0) cut_.Begin(SpanCutter::Weight(shape), spans_);
+    most_ = shape.runs + (spans_ != 0 ? spans_ : shape.bytes / chunk_);
     first_ = op_.ringHead_;  // before a wrap: what earlier batches left in the ring has been launched by them
     if (op_.ringHead_ >= op_.ringCap_) Wrap();
+}
+
+// The ring is written once around before a line of it is written again, and read by the GPU: past the caches, no line is fetched to be overwritten. A call
+// with 1500 pieces 17.4 us without, 14.8 so.
+static inline void PutDescriptor(CopyItem *at, uint64_t src, uint64_t dst, uint64_t len)
+{
+#ifdef __SSE2__
+    _mm_stream_si64(reinterpret_cast<long long *>(&at->src), (long long)src);
+    _mm_stream_si64(reinterpret_cast<long long *>(&at->dst), (long long)dst);
+    _mm_stream_si64(reinterpret_cast<long long *>(&at->len), (long long)len);
+#else
+    *at = CopyItem{src, dst, len};
+#endif
+}
+static inline void DescriptorsDone()
+{
+#ifdef __SSE2__
+    _mm_sfence();
+#endif
+}
+
+// Everything that a descriptor needs in registers: through the members, which a descriptor's words may alias, a piece cost 3 ns more.
+template <bool SPANS> void KernelBatch::AddFast(const void *const *src, const void *const *dst, const uint64_t *len, uint32_t count)
+{
+    CopyItem *o = op_.ring_ + op_.ringHead_;
+    const CopyItem *const launch = op_.ring_ + first_;
+    const uint64_t chunk = chunk_;
+    int64_t room = cut_.room_;
+    uint64_t s = 0, d = 0, n = 0, merged = 0;
+    auto emit = [&]() {
+        uint64_t off = 0;
+        while (off < n) {
+            uint64_t k = n - off;
+            if (SPANS) {
+                const int64_t w = (int64_t)k + (off != 0 ? 0 : SpanCutter::kPieceCost);
+                if (w <= room) {
+                    room -= w;
+                } else {
+                    cut_.room_ = room;
+                    k = cut_.Split(k, (uint32_t)(o - launch), off != 0);
+                    room = cut_.room_;
+                }
+            } else if (k > chunk) {
+                k = chunk;
+            }
+            PutDescriptor(o++, s + off, d + off, k);
+            off += k;
+        }
+    };
+    for (uint32_t i = 0; i < count; i++) {
+        const uint64_t si = reinterpret_cast<uint64_t>(src[i]), di = reinterpret_cast<uint64_t>(dst[i]);
+        if (s + n == si && d + n == di && n != 0) {
+            n += len[i];
+            merged++;
+            continue;
+        }
+        emit();
+        s = si;
+        d = di;
+        n = len[i];
+    }
+    emit();
+    cut_.room_ = room;
+    op_.stats_.coalesced += merged;
+    op_.ringHead_ = (uint64_t)(o - op_.ring_);
+    DescriptorsDone();
+}
+
+void KernelBatch::AddAll(const void *const *src, const void *const *dst, const uint64_t *len, uint32_t count)
+{
+    if (op_.ringHead_ + most_ <= op_.ringCap_) {
+        if (spans_ != 0) AddFast<true>(src, dst, len, count);
+        else AddFast<false>(src, dst, len, count);
+        return;
+    }
+    for (uint32_t i = 0; i < count; i++) Add(reinterpret_cast<uint64_t>(src[i]), reinterpret_cast<uint64_t>(dst[i]), len[i]);
 }
 
 int KernelBatch::Launch()
 {
     uint64_t n = op_.ringHead_ - first_;
     if (n == 0) return OK;
-    int rc = op_.dev_->LaunchBatchCopy(op_.ring_ + first_, (uint32_t)n, stream_, (alignMask_ & 15) == 0);
+    int rc = spans_ != 0 ? op_.dev_->LaunchSpanCopy(op_.ring_ + first_, cut_.End((uint32_t)n), stream_)
+                         : op_.dev_->LaunchBatchCopy(op_.ring_ + first_, (uint32_t)n, stream_, bulk_);
     if (rc != OK) return rc;
     if (std::find(op_.ringUsers_.begin(), op_.ringUsers_.end(), stream_) == op_.ringUsers_.end()) op_.ringUsers_.push_back(stream_);
     op_.stats_.kernelLaunches++;
@@ -359,6 +470,7 @@ void KernelBatch::Wrap()
     op_.ringUsers_.clear();
     op_.ringHead_ = 0;
     first_ = 0;
+    if (spans_ != 0) cut_.Begin(cut_.Left(), spans_);  // the rest of the batch is shared among all CTAs again
 }
 
 int KernelBatch::Finish()
@@ -390,34 +502,45 @@ int ComposeDataOp::Prepare(const std::vector<ResolvedCopy> &items, PreparedBatch
     if (dev_ == nullptr) return ERR_NOT_INIT;
     // merge neighbours, then cut into equal work chunks exactly as RunKernel does
     std::vector<CopyItem> runs;
-    uint64_t total = 0, alignMask = 0;
+    BatchShape shape;
     for (const auto &c : items) {
         if (c.len == 0) continue;
         if (c.src.kind != EP_DEVICE || c.dst.kind != EP_DEVICE) return MF_FAIL(ERR_INVALID_PARAM, "a prepared batch holds device-to-device copies only");
-        total += c.len;
-        alignMask |= c.src.addr | c.dst.addr | c.len;
+        shape.bytes += c.len;
+        shape.alignMask |= c.src.addr | c.dst.addr | c.len;
         if (!runs.empty() && runs.back().src + runs.back().len == c.src.addr && runs.back().dst + runs.back().len == c.dst.addr) runs.back().len += c.len;
         else runs.push_back(CopyItem{c.src.addr, c.dst.addr, c.len});
     }
     if (runs.empty()) return MF_FAIL(ERR_INVALID_PARAM, "a prepared batch needs at least one non-empty copy");
     const uint64_t sms = std::max(1, dev_->Caps().smCount);
-    uint64_t chunk = AlignUp(std::max<uint64_t>(total / (sms * 8), 1), 4096);
-    chunk = std::min(std::max<uint64_t>(chunk, 16 * kKiB), chunk_);
-    uint64_t n = 0;
-    for (const auto &r : runs) n += (r.len + chunk - 1) / chunk;
+    uint64_t chunk = AlignUp(std::max<uint64_t>(shape.bytes / (sms * 8), 1), 4096);
+    chunk = std::min(std::max<uint64_t>(chunk, kMinCopyChunk), chunk_);
+    shape.runs = runs.size();
+    const uint32_t spans = SpansFor(dev_, shape);
+    SpanCutter cut;
+    auto each = [&](auto &&emit) {  // the descriptors, in order
+        uint64_t w = 0;
+        if (spans != 0) cut.Begin(SpanCutter::Weight(shape), spans);
+        for (const auto &r : runs)
+            for (uint64_t off = 0, len; off < r.len; off += len, w++) {
+                len = spans != 0 ? cut.Take(r.len - off, (uint32_t)w, off != 0) : std::min(chunk, r.len - off);
+                emit(w, CopyItem{r.src + off, r.dst + off, len});
+            }
+        return w;
+    };
+    const uint64_t n = each([](uint64_t, const CopyItem &) {});
     if (n > UINT32_MAX) return MF_FAIL(ERR_INVALID_PARAM, "batch too large");
     dev_->BindThread();
     void *mem = nullptr;
     int rc = dev_->HostAlloc(n * sizeof(CopyItem), &mem);
     if (rc != OK) return MF_FAIL(rc, "cannot allocate %lu pinned descriptors", (unsigned long)n);
     auto *d = static_cast<CopyItem *>(mem);
-    uint64_t w = 0;
-    for (const auto &r : runs)
-        for (uint64_t off = 0; off < r.len; off += chunk) d[w++] = CopyItem{r.src + off, r.dst + off, std::min(chunk, r.len - off)};
+    each([d](uint64_t w, const CopyItem &c) { d[w] = c; });
     out.desc = d;
     out.count = (uint32_t)n;
-    out.bytes = total;
-    out.bulkOk = (alignMask & 15) == 0;
+    if (spans != 0) out.spans = std::make_shared<const CopySpans>(cut.End((uint32_t)n));
+    out.bytes = shape.bytes;
+    out.bulkOk = (shape.alignMask & 15) == 0;
     return OK;
 }
 
@@ -425,7 +548,7 @@ int ComposeDataOp::LaunchPrepared(const PreparedBatch &b, void *stream)
 {
     if (dev_ == nullptr || b.desc == nullptr) return ERR_INVALID_PARAM;
     // no lock, no shared state: the descriptors belong to the batch; the launch is all there is (graph-capturable)
-    int rc = dev_->LaunchBatchCopy(b.desc, b.count, stream, b.bulkOk);
+    int rc = b.spans ? dev_->LaunchSpanCopy(b.desc, *b.spans, stream) : dev_->LaunchBatchCopy(b.desc, b.count, stream, b.bulkOk);
     if (rc == OK) {
         fastLaunches_.fetch_add(1, std::memory_order_relaxed);
         fastItems_.fetch_add(b.count, std::memory_order_relaxed);

@@ -156,6 +156,15 @@ public:
             memmove(reinterpret_cast<void *>(items[i].dst), reinterpret_cast<const void *>(items[i].src), items[i].len);
         return OK;
     }
+    uint32_t CopySpanCount() const override { return 12; }
+    int LaunchSpanCopy(const CopyItem *items, const CopySpans &spans, void *s) override
+    {
+        for (uint32_t i = 0; i < spans.n; i++) {
+            if (spans.start[i] > spans.start[i + 1]) return ERR_INVALID_PARAM;
+            if (spans.start[i] < spans.start[i + 1]) LaunchBatchCopy(items + spans.start[i], spans.start[i + 1] - spans.start[i], s, false);
+        }
+        return OK;
+    }
     // Reference arithmetic of the quantising copy, also used as the CPU oracle of the CUDA kernel.
     int LaunchQuantCopy(const QuantItem *items, uint32_t count, uint32_t unit, int inputFp16, int mode, void *) override
     {

@@ -33,6 +33,13 @@ struct QuantItem {
     uint64_t elems;  // number of input elements
 };
 
+// Shares of a launch's descriptors: CTA i copies items[start[i]] .. items[start[i + 1] - 1].
+constexpr uint32_t kMaxCopySpans = 600;
+struct CopySpans {
+    uint32_t n = 0;
+    uint32_t start[kMaxCopySpans + 1];
+};
+
 enum MemcpyKind : int { CPY_H2H = 0, CPY_H2D = 1, CPY_D2H = 2, CPY_D2D = 3, CPY_AUTO = 4 };
 
 struct DeviceCaps {
@@ -107,6 +114,9 @@ public:
     // bulkOk: every item has source, destination and length in multiples of 16 bytes and both ends in device
     // memory, so the backend may move it with the bulk-copy (TMA) variant of the kernel.
     virtual int LaunchBatchCopy(const CopyItem *items, uint32_t count, void *stream, bool bulkOk = false) = 0;
+    // CTAs that a large batch of pieces for the register-copy kernel is shared among (at most kMaxCopySpans), 0: this backend has no such launch.
+    virtual uint32_t CopySpanCount() const { return 0; }
+    virtual int LaunchSpanCopy(const CopyItem *items, const CopySpans &spans, void *stream) { return LaunchBatchCopy(items, spans.start[spans.n], stream, false); }
     // Code left by a copy kernel whose bounded wait ran out (0: none); `clear` resets it.
     virtual uint32_t CopyStatus(bool clear) { (void)clear; return 0; }
     // Debug aid (MF_XCOPY_DEBUG=1): the pool window the copy kernels check every descriptor against before their first

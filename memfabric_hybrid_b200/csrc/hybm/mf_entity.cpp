@@ -611,19 +611,23 @@ int Entity::BatchCopyData(const hybm_batch_copy_params &p, hybm_data_copy_direct
             }
             return len <= at.mapped && a - at.lo <= at.mapped - len;  // no sum that a huge len could wrap
         };
-        uint64_t total = 0;
+        BatchShape shape;
+        uint64_t endSrc = 0, endDst = 0;  // of the item in front: neighbours that continue one another are one run
         for (uint32_t i = 0; i < p.batchSize; i++) {
             uint64_t s = reinterpret_cast<uint64_t>(p.sources[i]), d = reinterpret_cast<uint64_t>(p.destinations[i]);
             uint64_t len = p.dataSizes[i];
             if (s == 0 || d == 0 || len == 0 || (srcPool && !poolOk(s, len, srcLast)) || (dstPool && !poolOk(d, len, dstLast)))
                 return MF_FAIL(ERR_INVALID_PARAM, "batch copy item %u (%p -> %p, %lu bytes): null, empty or outside the mapped pool",
                                i, p.sources[i], p.destinations[i], (unsigned long)len);
-            total += len;
+            shape.bytes += len;
+            shape.alignMask |= s | d | len;
+            shape.runs += endSrc != s || endDst != d;
+            endSrc = s + len;
+            endDst = d + len;
         }
-        KernelBatch kb(*ops_, stream, flags, total);
+        KernelBatch kb(*ops_, stream, flags, shape);
         if (kb.Ready()) {
-            for (uint32_t i = 0; i < p.batchSize; i++)
-                kb.Add(reinterpret_cast<uint64_t>(p.sources[i]), reinterpret_cast<uint64_t>(p.destinations[i]), p.dataSizes[i]);
+            kb.AddAll(p.sources, p.destinations, p.dataSizes, p.batchSize);
             return kb.Finish();
         }
     }

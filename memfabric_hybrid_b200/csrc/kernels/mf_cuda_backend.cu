@@ -150,6 +150,7 @@ public:
     int ConfigureBulkCopy(int pipes, int stages, int pieceKb) override
     {
         bulkPipes_ = 0;
+        spansOk_ = false;
         if (pipes <= 0) return OK;
         pipes = std::min(pipes, 4);
         stages = std::min(std::max(stages, 4), mfk::kBulkMaxStages);
@@ -174,6 +175,8 @@ public:
         const int perSm = std::max(1, std::min(8, (int)((227u * 1024u) / (smem + 1024u))));
         bulkGrid_ = perSm * caps_.smCount;
         bulkPipes_ = (uint32_t)pipes;
+        spansOk_ = cudaFuncSetAttribute(mfk::mf_xcopy_span_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mfk::kSpanSmem) == cudaSuccess;
+        if (!spansOk_) (void)cudaGetLastError();
         return OK;
     }
 
@@ -483,6 +486,17 @@ public:
         RT_CHECK(cudaGetLastError(), "xcopy batch launch");
         return OK;
     }
+    uint32_t CopySpanCount() const override { return spansOk_ ? std::min<uint32_t>((uint32_t)grid_, kMaxCopySpans) : 0; }
+    int LaunchSpanCopy(const CopyItem *items, const CopySpans &spans, void *s) override
+    {
+        static_assert(sizeof(CopySpans::start) == sizeof(mfk::SpanStarts), "shares of the register-copy kernel");
+        if (spans.n == 0 || spans.start[spans.n] == 0) return OK;
+        mfk::mf_xcopy_span_kernel<<<spans.n, mfk::kSpanThreads, mfk::kSpanSmem, (cudaStream_t)s>>>(reinterpret_cast<const mfk::CopyItem *>(items),
+                                                                                      *reinterpret_cast<const mfk::SpanStarts *>(spans.start),
+                                                                                      window_, copyStatus_);
+        RT_CHECK(cudaGetLastError(), "xcopy span launch");
+        return OK;
+    }
     bool SetCopyWindow(uint64_t base, uint64_t slot, uint32_t ranks, const uint64_t *mapped) override
     {
         if (copyStatus_ == nullptr || ranks > 64) return false;
@@ -601,6 +615,7 @@ private:
     };
     int dev_ = 0;
     int grid_ = 296;
+    bool spansOk_ = false;  // pieces at any alignment may go through the copy unit too
     uint32_t bulkPipes_ = 0, bulkStages_ = 4, bulkPiece_ = 16384;
     int bulkGrid_ = 148;
     uint32_t *copyStatus_ = nullptr;

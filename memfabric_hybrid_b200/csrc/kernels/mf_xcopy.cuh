@@ -2,6 +2,8 @@
 // device-visible addresses (local HBM, a peer's HBM mapped over NVLink, pinned pooled DRAM) goes
 // through these, issued from inside the kernel as 16-byte vector loads and stores.
 //   mf_xcopy_batch_kernel : list of (src, dst, len) work chunks in a pinned, device-visible ring
+//   mf_xcopy_bulk_kernel  : the same list where every address is a multiple of 16, through the copy unit
+//   mf_xcopy_span_kernel  : pieces at any alignment, a share of equal weight per CTA
 //   mf_xcopy_quant_kernel : bf16/fp16 -> int8 (per-unit scale) or fp8 e4m3 (1x128 scale) while pushing
 // Parity of role: src/hybm/csrc/copy_extend/hybm_copy_kernel.cpp:53-90 (contiguous), :114-136 (batch),
 // :163-235 (quantising batch).
@@ -97,8 +99,8 @@ __device__ __forceinline__ void cta_copy(const uint8_t *__restrict__ src, uint8_
 // A CTA fetches the descriptors of its next 32 chunks together (they lie in pinned host memory: a PCIe read of more than a microsecond),
 // and nothing but the list's end holds its warps back: a warp that has no vectors left in one chunk is already in the next. With a
 // descriptor and a barrier per chunk (one descriptor ahead), us before / now: 700 pieces of 256 B - 512 KiB at 2-byte offsets 26.2 / 24.5,
-// 1500 of up to 16 KiB at any offset 15.0 / 12.2, 200 of up to 512 KiB at 8-byte offsets 11.9 / 10.1. (Warps that take pieces of 2 to
-// 16 KiB by themselves: 9.7 for the 1500, but 26.6 for the 700.) Where no CTA has more than one chunk a list
+// 1500 of up to 16 KiB at any offset 15.0 / 12.2. (Large batches between device addresses go to mf_xcopy_span_kernel; batches with a leg in pinned host
+// memory, and all of them where the copy unit is switched off, come here.) Where no CTA has more than one chunk a list
 // and its barriers are in the way: replayed from a graph, one piece of up to 1 KiB takes 2.4 us with the single descriptor, 2.7 to 2.9 with a
 // list; 20 pieces of up to 16 KiB 3.8 and 4.2, 100 of them 4.1 and 4.4.
 __global__ void __launch_bounds__(kCopyThreads) mf_xcopy_batch_kernel(const CopyItem *__restrict__ items, uint32_t count,
@@ -249,6 +251,200 @@ __global__ void __launch_bounds__(128) mf_xcopy_bulk_kernel(const CopyItem *__re
         }
     }
     asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
+
+// ---- pieces at any alignment, cut into a share per CTA ---------------------------------------------
+// A large batch whose addresses are not all multiples of 16: the host has cut it into shares of equal weight (see SpanCutter), and CTA i copies
+// descriptors start[i] .. start[i + 1] - 1, which lie together in host memory; the shares travel with the launch. One thread walks the pieces and
+// has the copy unit load their whole granules into a ring of shared-memory stages, eight warps cut the destination's vectors out of
+// neighbouring granules and store them, one warp copies the few bytes in front of the first vector and behind the last. The loads of the next
+// pieces are on their way whatever the warps wait for, so that short pieces and the ends of long ones cost no latency of their own.
+// What bounds it: memory in large batches, latencies and the list's way from host memory in small ones. 700 pieces of 256 B - 512 KiB at 2-byte offsets (53
+// MB) took 28.9 us with register copies of chunks dealt out one by one, 28.2 with equal shares alone, 21.7 so (4.9 TB/s); 1500 of up to 512 KiB at 4-byte
+// offsets 51 / 41 (5.2 TB/s); 200 at 8-byte offsets 11.8 / 7.8; 1500 of up to 16 KiB at any offset 12.4 / 10.9 with half as many shares, 9.3 with all: a
+// share costs the host 5 ns, and such a batch waits for the host.
+struct SpanStarts {
+    uint32_t start[601];
+};
+constexpr int kSpanConsumers = 8, kSpanThreads = (kSpanConsumers + 2) * 32, kSpanStages = 6;
+constexpr uint32_t kSpanVecs = 1024, kSpanStageBytes = (kSpanVecs + 1) * 16, kSpanSmem = kSpanStages * kSpanStageBytes;
+
+// `head` bytes one by one, `vecs` destination vectors, the rest one by one; granules are loaded from src + head - shift on.
+__device__ __forceinline__ ShiftPlan span_plan(uint64_t src, uint64_t dst, uint64_t len)
+{
+    if (((src ^ dst) & 15) != 0) return shift_plan(src, dst, len);
+    ShiftPlan p;
+    p.head = (16 - (dst & 15)) & 15;
+    if (p.head > len) p.head = len;
+    p.vecs = (len - p.head) >> 4;
+    p.shift = 0;
+    return p;
+}
+
+__device__ __forceinline__ bool xc_wait(uint64_t *bar, uint32_t parity, volatile int *quit)
+{
+    uint64_t t0 = 0;
+    for (uint32_t spin = 0;; spin++) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred P;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+            "selp.b32 %0, 1, 0, P;\n\t}"
+            : "=r"(ok)
+            : "r"(xc_smem_u32(bar)), "r"(parity)
+            : "memory");
+        if (ok) return true;
+        if ((spin & 255u) == 255u) {  // time limit, not an iteration count: a try_wait may suspend for a while
+            if (quit != nullptr && *quit) return false;
+            uint64_t now;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+            if (t0 == 0) t0 = now;
+            else if (now - t0 > kBulkWaitNs) return false;
+        }
+    }
+}
+
+template <int Q> __device__ __forceinline__ void span_cut(const uint4 *g, uint4 *d, uint32_t vecs, uint32_t bits)
+{
+#pragma unroll
+    for (uint32_t u = 0; u < kSpanVecs / (kSpanConsumers * 32); u++) {
+        const uint32_t i = threadIdx.x + u * kSpanConsumers * 32;
+        if (i < vecs) __stcs(d + i, cut16<Q>(g[i], g[i + 1], bits));
+    }
+}
+
+__global__ void __launch_bounds__(kSpanThreads, 2) mf_xcopy_span_kernel(const CopyItem *__restrict__ items, const __grid_constant__ SpanStarts spans,
+                                                                        const CopyWindow *__restrict__ window, uint32_t *status)
+{
+    extern __shared__ __align__(128) uint8_t xc_smem[];
+    __shared__ __align__(8) uint64_t full[kSpanStages], empty[kSpanStages];
+    __shared__ uint64_t list[kCopyList * 3];
+    __shared__ int quit_sh;
+    volatile int *quit = &quit_sh;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t beg = spans.start[blockIdx.x], end = spans.start[blockIdx.x + 1];
+    const uint64_t *words = reinterpret_cast<const uint64_t *>(items);
+    auto fetch = [&](uint32_t first) -> uint64_t {
+        return threadIdx.x < kCopyList * 3 && first + threadIdx.x / 3 < end ? words[(uint64_t)first * 3 + threadIdx.x] : 0;
+    };
+    uint64_t next = fetch(beg);
+    if (threadIdx.x == 0) {
+        quit_sh = 0;
+        for (int s = 0; s < kSpanStages; s++) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(xc_smem_u32(&full[s])));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(xc_smem_u32(&empty[s])), "r"(kSpanConsumers));
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the initialised barriers as the copy unit sees them
+    }
+    uint32_t slot = 0, phase = 0;  // of the role's next stage
+    auto advance = [&]() {
+        if (++slot == kSpanStages) {
+            slot = 0;
+            phase ^= 1;
+        }
+    };
+    for (uint32_t first = beg; first < end; first += kCopyList) {
+        __syncthreads();  // the barriers are initialised; the previous list is no longer read
+        if (*quit) break;
+        if (threadIdx.x < kCopyList * 3) list[threadIdx.x] = next;
+        __syncthreads();
+        next = fetch(first + kCopyList);  // arrives while this list's pieces are copied
+        const uint32_t n = min(kCopyList, end - first);
+        if (window != nullptr) {
+            if (threadIdx.x < n && !xc_check(window, list[3 * threadIdx.x], list[3 * threadIdx.x + 1], list[3 * threadIdx.x + 2], status)) list[3 * threadIdx.x + 2] = 0;
+            __syncthreads();
+        }
+        if (warp == kSpanConsumers) {
+            if (lane != 0) continue;
+            for (uint32_t l = 0; l < n && !*quit; l++) {
+                const uint64_t src = list[3 * l];
+                const ShiftPlan p = span_plan(src, list[3 * l + 1], list[3 * l + 2]);
+                for (uint64_t v = 0; v < p.vecs; v += kSpanVecs) {
+                    const uint32_t bytes = ((uint32_t)min((uint64_t)kSpanVecs, p.vecs - v) + (p.shift != 0 ? 1 : 0)) * 16;
+                    if (!xc_wait(&empty[slot], phase ^ 1, quit)) {
+                        *quit = 1;
+                        break;
+                    }
+                    const uint32_t bar = xc_smem_u32(&full[slot]);
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                     xc_smem_u32(xc_smem + slot * kSpanStageBytes)),
+                                 "l"(src + p.head - p.shift + v * 16), "r"(bytes), "r"(bar)
+                                 : "memory");
+                    advance();
+                }
+            }
+        } else if (warp > kSpanConsumers) {
+            constexpr uint32_t kAtOnce = 4;
+            for (uint32_t l0 = 0; l0 < n; l0 += kAtOnce) {
+                uint8_t b[kAtOnce][2];
+                uint8_t *to[kAtOnce][2];
+#pragma unroll
+                for (uint32_t j = 0; j < kAtOnce; j++) {
+                    const uint32_t l = min(l0 + j, n - 1);
+                    const uint64_t src = list[3 * l], dst = list[3 * l + 1], len = list[3 * l + 2];
+                    const ShiftPlan p = span_plan(src, dst, len);
+                    const uint64_t edge = len - p.vecs * 16;  // at most 62: a head of up to 31 bytes and as many behind the vectors
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const uint32_t e = lane + 32 * h;
+                        const uint64_t at = e < p.head ? e : e + p.vecs * 16;
+                        to[j][h] = nullptr;
+                        if (e < edge && l0 + j < n) {
+                            b[j][h] = *reinterpret_cast<const uint8_t *>(src + at);
+                            to[j][h] = reinterpret_cast<uint8_t *>(dst + at);
+                        }
+                    }
+                }
+#pragma unroll
+                for (uint32_t j = 0; j < kAtOnce; j++)
+#pragma unroll
+                    for (int h = 0; h < 2; h++)
+                        if (to[j][h] != nullptr) *to[j][h] = b[j][h];
+            }
+        } else {
+            for (uint32_t l = 0; l < n && !*quit; l++) {
+                const uint64_t dst = list[3 * l + 1];
+                const ShiftPlan p = span_plan(list[3 * l], dst, list[3 * l + 2]);
+                uint4 *d = reinterpret_cast<uint4 *>(dst + p.head);
+                const uint32_t bits = (p.shift & 3) * 8;
+                for (uint64_t v = 0; v < p.vecs; v += kSpanVecs) {
+                    if (!xc_wait(&full[slot], phase, quit)) {
+                        if (!*quit) *reinterpret_cast<volatile uint32_t *>(status) = 0x702u;
+                        *quit = 1;
+                        break;
+                    }
+                    const uint4 *g = reinterpret_cast<const uint4 *>(xc_smem + slot * kSpanStageBytes);
+                    const uint32_t m = (uint32_t)min((uint64_t)kSpanVecs, p.vecs - v);
+                    if (p.shift == 0) {
+#pragma unroll
+                        for (uint32_t u = 0; u < kSpanVecs / (kSpanConsumers * 32); u++) {
+                            const uint32_t i = threadIdx.x + u * kSpanConsumers * 32;
+                            if (i < m) __stcs(d + v + i, g[i]);
+                        }
+                    } else {
+                        switch (p.shift >> 2) {  // uniform over the CTA
+                            case 0: span_cut<0>(g, d + v, m, bits); break;
+                            case 1: span_cut<1>(g, d + v, m, bits); break;
+                            case 2: span_cut<2>(g, d + v, m, bits); break;
+                            default: span_cut<3>(g, d + v, m, bits); break;
+                        }
+                    }
+                    __syncwarp();
+                    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(xc_smem_u32(&empty[slot])) : "memory");
+                    advance();
+                }
+            }
+        }
+    }
+    __syncthreads();
+    // a load that did not land in time: once more as long for what the copy unit still has in flight, then the CTA goes
+    if (*quit && warp == kSpanConsumers && lane == 0)
+        for (int s = 0; s < kSpanStages; s++) {
+            const uint32_t done = slot > (uint32_t)s ? phase : phase ^ 1;  // parity of the stage's last load
+            xc_wait(&full[s], done, nullptr);
+        }
 }
 
 // One WARP per (item, unit); a CTA of 8 warps walks the units of its item. The unit is read once when it fits in

@@ -419,6 +419,26 @@ uint64_t mf_t_ex_mapped_bytes(void *h, uint32_t rank)
     return seg ? seg->MappedBytes(rank) : 0;
 }
 
+// ---- shares of a copy batch ------------------------------------------------------------------------------
+// Cuts pieces of `len` bytes into `spans` shares as the copy operator does: first descriptor of every share and their number in start[0 .. spans],
+// bytes of every descriptor in out[0 .. cap). -> descriptors.
+uint32_t mf_t_copy_shares(const uint64_t *len, uint32_t n, uint32_t spans, uint32_t *start, uint64_t *out, uint32_t cap)
+{
+    mf::hybm::BatchShape shape;
+    shape.runs = n;
+    for (uint32_t i = 0; i < n; i++) shape.bytes += len[i];
+    mf::hybm::SpanCutter cut;
+    cut.Begin(mf::hybm::SpanCutter::Weight(shape), spans);
+    uint32_t w = 0;
+    for (uint32_t i = 0; i < n; i++)
+        for (uint64_t off = 0, k; off < len[i]; off += k, w++) {
+            k = cut.Take(len[i] - off, w, off != 0);
+            if (w < cap) out[w] = k;
+        }
+    memcpy(start, cut.End(w).start, (spans + 1) * sizeof(uint32_t));
+    return w;
+}
+
 // ---- fault points -------------------------------------------------------------------------------------
 // Runs the periodic TLS certificate check now; -> the smallest number of days left over the live contexts.
 int mf_t_tls_check_now(void) { return mf::net::TlsCheckAllNow(); }

@@ -292,3 +292,66 @@ def _ring_rank(rank, world, url):
 def test_a_batch_that_finds_the_descriptor_ring_full_launches_its_own_pieces_only():
     url = f"tcp://127.0.0.1:{free_port()}"
     assert run_ranks(_ring_rank, 1, (url,), timeout=120, env={"MF_DEVICE_BACKEND": "fake", "MF_XCOPY_RING_MB": "1"}) == [True]
+
+
+def test_shares_of_a_copy_batch():
+    """Every byte once and in order, a piece cut at multiples of 512 only, and no share much above the others."""
+    import hooks
+    r = np.random.default_rng(3)
+    for sizes in (np.exp(r.uniform(5, 13, 700)), r.integers(1, 16 << 10, 1500), [100] * 297, [16385] * 297, [1] * 5000 + [1 << 20] * 3,
+                  [50 << 20] + [100] * 3000, [1 << 40], [7]):
+        sizes = np.asarray(sizes, dtype=np.uint64)
+        for spans in (1, 12, 148, 600):
+            start, out = np.full(spans + 1, 99, dtype=np.uint32), np.zeros(len(sizes) + spans, dtype=np.uint64)
+            n = hooks.lib().mf_t_copy_shares(sizes.ctypes.data, len(sizes), spans, start.ctypes.data, out.ctypes.data, len(out))
+            assert n <= len(out) and start[0] == 0 and start[-1] == n and bool((np.diff(start.astype(np.int64)) >= 0).all())
+            out, left, cost = out[:n].astype(np.int64), 0, 4096
+            piece, weight = iter(sizes.astype(np.int64).tolist()), np.zeros(spans)
+            share = np.searchsorted(start[1:], np.arange(n), side="right")
+            for k, s in zip(out.tolist(), share.tolist()):
+                fresh = left == 0
+                left = next(piece) if fresh else left
+                assert 0 < k <= left and (k == left or k % 512 == 0)
+                left -= k
+                weight[s] += k + (cost if fresh else 0)
+            assert left == 0 and next(piece, None) is None
+            mean = (int(sizes.sum()) + cost * len(sizes)) / spans
+            assert weight.max() <= 2 * mean + 4 * cost, (spans, weight.max(), mean)
+
+
+def _shares_rank(rank, world, url):
+    import memfabric_hybrid as mf
+    from memfabric_hybrid import bm
+    assert mf.initialize() == 0
+    cfg = bm.BmConfig()
+    cfg.rank_id = 0
+    cfg.start_store = True
+    assert bm.initialize(url, 1, 0, cfg) == 0, mf.get_last_err_msg()
+    h = bm.create2(id=7, local_dram_size=0, max_dram_size=0, local_hbm_size=32 * MiB, max_hbm_size=32 * MiB)
+    assert h.join() == 0, mf.get_last_err_msg()
+    base = h.peer_rank_ptr(0, bm.BmMemType.DEVICE)
+    r, ok = np.random.default_rng(1), True
+    # few and many pieces, neighbours that merge, and (ring of 1 MiB) batches that reach the ring's end in the middle
+    for n, top, gap in ((40, 60000, 1), (3000, 300, 3), (3000, 5000, 0), (30000, 40, 1), (30000, 60, 2)):
+        size = r.integers(1, top, n).astype(np.uint64)
+        off = np.concatenate(([0], np.cumsum(size + np.uint64(gap) * r.integers(0, 2, n).astype(np.uint64))[:-1])).astype(np.uint64) + np.uint64(1)
+        total = int(off[-1] + size[-1])
+        src = r.integers(0, 256, total + 8, dtype=np.uint8)
+        z, got = np.full(total + 8, 9, dtype=np.uint8), np.zeros(total + 8, dtype=np.uint8)
+        assert h.copy_data(z.ctypes.data, base, z.nbytes, bm.BmCopyType.H2G, 0) == 0
+        assert h.copy_data_batch(off + np.uint64(src.ctypes.data), off + np.uint64(base), size, n, bm.BmCopyType.L2G, bm.ASYNC_COPY_FLAG) == 0
+        assert h.copy_data(base, got.ctypes.data, got.nbytes, bm.BmCopyType.G2H, 0) == 0
+        want = z.copy()
+        for o, s in zip(off.tolist(), size.tolist()):
+            want[o:o + s] = src[o:o + s]
+        ok = ok and bool(np.array_equal(got, want))
+    h.leave()
+    h.destroy()
+    bm.uninitialize(0)
+    mf.uninitialize()
+    return ok
+
+
+def test_batches_in_shares_against_the_pieces_one_by_one():
+    url = f"tcp://127.0.0.1:{free_port()}"
+    assert run_ranks(_shares_rank, 1, (url,), timeout=120, env={"MF_DEVICE_BACKEND": "fake", "MF_XCOPY_RING_MB": "1"}) == [True]

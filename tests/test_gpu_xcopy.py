@@ -256,6 +256,65 @@ def _shifted_rank(rank, world, url):
     return ok
 
 
+def _share_rank(rank, world, url):
+    import torch
+    import memfabric_hybrid as mf
+    from memfabric_hybrid import bm
+    torch.cuda.set_device(0)
+    assert mf.initialize() == 0
+    cfg = bm.BmConfig()
+    cfg.rank_id = 0
+    cfg.start_store = True
+    assert bm.initialize(url, 1, 0, cfg) == 0, mf.get_last_err_msg()
+    pool = 256 * MiB
+    h = bm.create2(id=5, local_dram_size=0, max_dram_size=0, local_hbm_size=pool, max_hbm_size=pool)
+    assert h.join() == 0, mf.get_last_err_msg()
+    base, bad = h.peer_rank_ptr(0, bm.BmMemType.DEVICE), []
+    stage = 16384   # bytes that a CTA moves at once
+    ends = [stage * k + e for k in (1, 2, 7) for e in (-17, -16, -1, 0, 1, 15, 16, 31, 33)]
+    # the ends of stages, at one offset and at two; more pieces than a CTA's list holds, of a few bytes and of a few vectors; one long piece cut into all shares
+    for name, lens, offs in (("stages", ends * 12, (0, 1, 4, 15)), ("tiny", [1, 5, 16, 17, 62, 63, 64] * 3000, (0, 3)), ("short", [300, 700, 1030] * 8000, (0, 8, 11)),
+                             ("long", [100_000_003], (5,)), ("same offset", [40_001] * 400, (7,))):
+        segs, so, do = [], 0, 0
+        for i, ln in enumerate(lens):
+            s, d = offs[i % len(offs)], offs[i // len(offs) % len(offs)]
+            segs.append((so + s, do + d, ln))
+            so += (s + ln + 31) // 16 * 16
+            do += (d + ln + 47) // 16 * 16
+        src = torch.randint(0, 256, (so + 64,), dtype=torch.uint8, device="cuda", generator=torch.Generator("cuda").manual_seed(len(lens)))
+        fill = torch.full((do + 64,), 77, dtype=torch.uint8, device="cuda")
+        want = fill.clone()
+        for s, d, n in segs:
+            want[d:d + n] = src[s:s + n]
+        lists = [src.data_ptr() + s for s, _, _ in segs], [base + d for _, d, _ in segs], [n for _, _, n in segs]
+        got = torch.empty_like(fill)
+        for prepared in (False, True):
+            torch.cuda.synchronize()
+            assert h.copy_data(fill.data_ptr(), base, fill.numel(), bm.BmCopyType.L2G, 0) == 0, mf.get_last_err_msg()
+            if prepared:
+                b = h.create_batch(*lists, bm.BmCopyType.L2G)
+                b.launch(torch.cuda.current_stream().cuda_stream)
+                torch.cuda.synchronize()
+                b.destroy()
+            else:
+                assert h.copy_data_batch(*lists, len(segs), bm.BmCopyType.L2G, 0) == 0, mf.get_last_err_msg()
+            assert h.copy_data(base, got.data_ptr(), got.numel(), bm.BmCopyType.G2L, 0) == 0, mf.get_last_err_msg()
+            torch.cuda.synchronize()
+            if not torch.equal(got, want):   # the bytes between the pieces included
+                bad.append((name, prepared))
+    h.leave()
+    h.destroy()
+    bm.uninitialize(0)
+    mf.uninitialize()
+    return bad
+
+
+@pytest.mark.parametrize("debug", ["0", "1"], ids=["plain", "descriptors_checked"])
+def test_unaligned_batches_in_shares(debug):
+    url = f"tcp://127.0.0.1:{free_port()}"
+    assert run_ranks(_share_rank, 1, (url,), timeout=240, env={"MF_XCOPY_DEBUG": debug}) == [[]]
+
+
 def test_pieces_at_every_pair_of_byte_offsets():
     url = f"tcp://127.0.0.1:{free_port()}"
     assert run_ranks(_shifted_rank, 1, (url,), timeout=180) == [True]
