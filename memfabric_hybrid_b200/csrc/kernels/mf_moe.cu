@@ -838,6 +838,8 @@ struct LLDispatchArgs {
     int *src_off;            // [El * W]
     uint32_t *epoch_dev;     // call counter in device memory: this call uses *epoch_dev + 1 and stores it back at the
                              // end, so a captured launch can be replayed (d.epoch is ignored, d.seq must be 0)
+    int *tokens_per_rank;       // [W], one rank's own dispatch only, as is_token_in_rank [T, W]
+    uint8_t *is_token_in_rank;
 };
 
 // The last CTA of a low-latency dispatch waits for every peer's rows.
@@ -900,10 +902,14 @@ __global__ void __launch_bounds__(448) k_moe_ll_dispatch(LLDispatchArgs a)
 // 256 24.1 / 18.3. A pass of the pair with a stand-in expert, 128 tokens: 81 before this kernel and the present combine, 66.
 constexpr int kLLTokens = 4;        // tokens of a CTA
 constexpr int kLLEntries = 4096;    // entries in all: a CTA looks at every entry once for each of its own
-__global__ void __launch_bounds__(448) k_moe_ll_dispatch_few(LLDispatchArgs a)
+// ALONE: the dispatch of the pair dispatch / combine by a group of one rank, which has no counts to exchange: layout, tables and push in one launch that
+// waits for nobody, in place of k_moe_prepare and k_moe_dispatch_warp (with more ranks the CTAs would hold their SMs while they wait for the
+// peers' counts, see finish_dispatch). MoE layer, 32 experts of 7168 x 2048, us, two launches / one: 1 token 106 / 91, 16 260 / 244, 128 270 / 253, 256 282 / 267, 512
+// 317 / 309.
+template <bool ALONE> __global__ void __launch_bounds__(448) k_moe_dispatch_few(LLDispatchArgs a)
 {
     const Team &t = a.d.team;
-    const uint32_t me = team_rank(t), W = t.world;
+    const uint32_t me = team_rank(t), W = ALONE ? 1 : t.world;
     const int T = a.d.sh.T, K = a.d.sh.K, E = a.d.sh.E, H = a.d.sh.H, n = T * K, El = E / (int)W;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (int)(blockDim.x >> 5);
     __shared__ uint16_t ids[kLLEntries];
@@ -912,9 +918,13 @@ __global__ void __launch_bounds__(448) k_moe_ll_dispatch_few(LLDispatchArgs a)
     __shared__ int dst_rank[kLLTokens][16], dst_pos[kLLTokens][16];
     __shared__ float dst_w[kLLTokens][16];
     __shared__ __align__(16) float s_scale[2][64];
-    __shared__ int ok_sh;
+    __shared__ int ok_sh, any_sh;
+    if (ALONE) {
+        after_predecessor();
+        start_successor();
+    }
     MF_PROF_START(PF_LAYOUT);
-    a.d.epoch = *reinterpret_cast<volatile uint32_t *>(a.epoch_dev) + 1;
+    if (!ALONE) a.d.epoch = *reinterpret_cast<volatile uint32_t *>(a.epoch_dev) + 1;
     const int vec = threadIdx.x, vecs = H / 16;
     uint4 lo, hi;
     dispatch_preload(a.d, lo, hi);
@@ -922,7 +932,10 @@ __global__ void __launch_bounds__(448) k_moe_ll_dispatch_few(LLDispatchArgs a)
         cnt[e] = 0;
         put[e] = 0;
     }
-    if (threadIdx.x == 0) ok_sh = 1;
+    if (threadIdx.x == 0) {
+        ok_sh = 1;
+        any_sh = 0;
+    }
     __syncthreads();
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         const int e = a.d.topk_idx[i];
@@ -962,6 +975,19 @@ __global__ void __launch_bounds__(448) k_moe_ll_dispatch_few(LLDispatchArgs a)
     const bool tables = blockIdx.x == gridDim.x - 1;  // this CTA leaves the tables for the caller
     if (tables)
         for (int e = threadIdx.x; e < E; e += blockDim.x) a.tokens_per_expert[e] = cnt[e];
+    if (ALONE && tables) {
+        int some = 0;
+        for (int tok = threadIdx.x; tok < T; tok += blockDim.x) {
+            bool in = false;
+            for (int k = 0; k < K; k++) in = in || ids[tok * K + k] != 0xffff;
+            a.is_token_in_rank[tok] = in ? 1 : 0;
+            some += in ? 1 : 0;
+        }
+        some = __reduce_add_sync(0xffffffffu, some);
+        if (lane == 0 && some != 0) atomicAdd(&any_sh, some);
+        __syncthreads();
+        if (threadIdx.x == 0) a.tokens_per_rank[0] = any_sh;
+    }
     if (W > 1) {
         if (threadIdx.x < W && !wait_flag(reinterpret_cast<const uint32_t *>(peer_ptr(t, me, bar)) + threadIdx.x, a.d.epoch, t.spin_limit)) {
             ok_sh = 0;
@@ -1044,9 +1070,9 @@ __global__ void __launch_bounds__(448) k_moe_ll_dispatch_few(LLDispatchArgs a)
             __syncthreads();
         }
     }
-    const bool last = finish_dispatch(a.d, me, a.epoch_dev);
+    const bool last = finish_dispatch(a.d, me, ALONE ? nullptr : a.epoch_dev);
     MF_PROF_STOP(PF_DISPATCH);
-    if (last) ll_wait_rows(a, me);  // uniform over the CTA
+    if (!ALONE && last) ll_wait_rows(a, me);  // uniform over the CTA
 }
 
 struct LLCombineArgs {
@@ -1203,6 +1229,18 @@ int mf_moe_dispatch(const DispatchArgs *a, int ctas, void *stream)
     return e == cudaSuccess ? 0 : (int)e;
 }
 
+// mf_moe_prepare and mf_moe_dispatch of one rank's few tokens in one launch; -3: more ranks or too many tokens, make the two calls. `ctas` as for
+// mf_moe_dispatch, whose completion counter it shares.
+int mf_moe_dispatch_alone(const DispatchArgs *d, int *tokens_per_expert, int *tokens_per_rank, uint8_t *is_token_in_rank, int *recv_per_expert,
+                          int *row_off, int *src_off, int ctas, void *stream)
+{
+    if (d == nullptr || d->team.emu || d->sh.T <= 0 || d->sh.K <= 0 || d->sh.K > 16 || d->sh.E <= 0 || d->sh.E > 1024 || d->sh.H % 128 != 0 || ctas <= 0) return -1;
+    if (d->team.world != 1 || d->sh.H / 16 > 448 || d->sh.T > kLLTokens * ctas || d->sh.T * d->sh.K > kLLEntries) return -3;
+    const LLDispatchArgs a{*d, tokens_per_expert, recv_per_expert, row_off, src_off, nullptr, tokens_per_rank, is_token_in_rank};
+    const cudaError_t e = launch_overlapped(k_moe_dispatch_few<true>, dim3((unsigned)ctas), dim3(448), 0, (cudaStream_t)stream, 1, a);
+    return e == cudaSuccess ? 0 : (int)e;
+}
+
 int mf_moe_wait_all(const Team *team, const MoeHeap *hp, int which, uint32_t epoch, int *status, void *stream)
 {
     const cudaError_t e = launch_overlapped(k_moe_wait_all, dim3(1), dim3(32), 0, (cudaStream_t)stream, 1, *team, *hp, which, epoch, status);
@@ -1249,10 +1287,10 @@ int mf_moe_ll_dispatch(const DispatchArgs *d, int *tokens_per_expert, int *recv_
     if (d == nullptr || d->team.emu || d->sh.H % 128 != 0 || d->sh.H / 16 > 448 || d->sh.K > 16 || d->sh.E > 1024 ||
         d->sh.E % (int)d->team.world != 0 || ctas <= 0)
         return -1;
-    LLDispatchArgs a{*d, tokens_per_expert, recv_per_expert, row_off, src_off, epoch_dev};
+    LLDispatchArgs a{*d, tokens_per_expert, recv_per_expert, row_off, src_off, epoch_dev, nullptr, nullptr};
     void *params[] = {&a};
     const bool few = d->sh.T <= kLLTokens * ctas && d->sh.T * d->sh.K <= kLLEntries && one_per_sm(ctas);
-    cudaError_t e = cudaLaunchCooperativeKernel(few ? reinterpret_cast<const void *>(k_moe_ll_dispatch_few) : reinterpret_cast<const void *>(k_moe_ll_dispatch),
+    cudaError_t e = cudaLaunchCooperativeKernel(few ? reinterpret_cast<const void *>(k_moe_dispatch_few<false>) : reinterpret_cast<const void *>(k_moe_ll_dispatch),
                                                 dim3(ctas), dim3(448), params, 0, (cudaStream_t)stream);
     return e == cudaSuccess ? 0 : (int)e;
 }

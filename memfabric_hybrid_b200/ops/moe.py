@@ -61,6 +61,8 @@ def _cu():
         l.mf_moe_prepare.argtypes = [P(TeamC), P(MoeHeapC), vp, ci, ci, ci, vp, vp, vp, vp, vp, vp, vp, vp, C.c_uint32, vp]
         l.mf_moe_dispatch.restype = ci
         l.mf_moe_dispatch.argtypes = [P(DispatchArgsC), ci, vp]
+        l.mf_moe_dispatch_alone.restype = ci
+        l.mf_moe_dispatch_alone.argtypes = [P(DispatchArgsC), vp, vp, vp, vp, vp, vp, ci, vp]
         l.mf_moe_wait_all.restype = ci
         l.mf_moe_wait_all.argtypes = [P(TeamC), P(MoeHeapC), ci, C.c_uint32, vp, vp]
         l.mf_moe_signal_all.restype = ci
@@ -297,23 +299,32 @@ class MoEComm:
             idx, tpe, tpr, sidx, inr = self.get_dispatch_layout(topk_idx)
         rpe, row_off, put_off, src_off = (torch.empty(n, **i32) for n in (self.El, self.El + 1, self.E, self.El * self.world))
         epoch = self._epoch + 1   # counts once the exchange is launched: a refused call must not put this rank out of step
-        if small:
-            # layout and count exchange in one launch
-            _ok(cu.mf_moe_prepare(C.byref(team), C.byref(self.hp), idx.data_ptr(), T, self.K, self.E, tpe.data_ptr(), tpr.data_ptr(),
-                                  sidx.data_ptr(), inr.data_ptr(), rpe.data_ptr(), row_off.data_ptr(), put_off.data_ptr(), src_off.data_ptr(),
-                                  epoch, _s()), "moe_prepare")
-        else:
-            _ok(cu.mf_moe_notify(C.byref(team), C.byref(self.hp), self.E, tpe.data_ptr(), rpe.data_ptr(), row_off.data_ptr(),
-                                 put_off.data_ptr(), src_off.data_ptr(), epoch, _s()), "moe_notify")
-        self._epoch = epoch
         w = topk_w.to(torch.float32).contiguous()
-        self._dispatches += 1
         a = DispatchArgsC(team, self.hp, self._shape(T), x.data_ptr(), idx.data_ptr(), w.data_ptr(), sidx.data_ptr(), put_off.data_ptr(),
-                          self._done.data_ptr(), self._epoch, self._dispatches, status_word(self.dev).data_ptr(), 1 if self.raw_bf16 else 0,
+                          self._done.data_ptr(), epoch, self._dispatches + 1, status_word(self.dev).data_ptr(), 1 if self.raw_bf16 else 0,
                           smooth.data_ptr() if smooth is not None else None)
+        rc = -3
+        if small and self.world == 1:
+            # nothing to exchange: layout, tables and push of a few tokens in one launch
+            rc = cu.mf_moe_dispatch_alone(C.byref(a), tpe.data_ptr(), tpr.data_ptr(), inr.data_ptr(), rpe.data_ptr(), row_off.data_ptr(), src_off.data_ptr(),
+                                          self._grid, _s())
+            if rc != -3:
+                _ok(rc, "moe_dispatch_alone")
+                self._epoch = epoch
+        if rc == -3:
+            if small:
+                # layout and count exchange in one launch
+                _ok(cu.mf_moe_prepare(C.byref(team), C.byref(self.hp), idx.data_ptr(), T, self.K, self.E, tpe.data_ptr(), tpr.data_ptr(),
+                                      sidx.data_ptr(), inr.data_ptr(), rpe.data_ptr(), row_off.data_ptr(), put_off.data_ptr(), src_off.data_ptr(),
+                                      epoch, _s()), "moe_prepare")
+            else:
+                _ok(cu.mf_moe_notify(C.byref(team), C.byref(self.hp), self.E, tpe.data_ptr(), rpe.data_ptr(), row_off.data_ptr(),
+                                     put_off.data_ptr(), src_off.data_ptr(), epoch, _s()), "moe_notify")
+            self._epoch = epoch
+            # one CTA per SM on every call: the completion counter of the kernel counts CTAs
+            _ok(_cu().mf_moe_dispatch(C.byref(a), self._grid, _s()), "moe_dispatch")
+        self._dispatches += 1
         self._keep = (w, idx, smooth)
-        # one CTA per SM on every call: the completion counter of the kernel counts CTAs
-        _ok(_cu().mf_moe_dispatch(C.byref(a), self._grid, _s()), "moe_dispatch")
         _ok(_cu().mf_moe_wait_all(C.byref(team), C.byref(self.hp), 0, self._epoch, status_word(self.dev).data_ptr(), _s()), "moe_wait")
         return DispatchState(T, idx, sidx, tpe, tpr, inr, rpe, row_off, put_off, src_off, self._epoch)
 
