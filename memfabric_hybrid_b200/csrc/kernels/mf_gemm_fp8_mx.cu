@@ -7,8 +7,9 @@
 // warp turns them into UE8M0 bytes (the fp32 exponent) in the tensor core's scale layout in shared
 // memory, four K blocks per 32-bit word; the MMA thread copies a group of them into TMEM (tcgen05.cp)
 // and picks the byte of the current K block through the instruction descriptor.
-// Tile 128 x 256 (48 KiB of operands per 128 of K: 3/4 of the L2 traffic per FLOP of a 128 x 128 tile),
-// four TMA stages, operands from THIS GPU's memory only, no multicast.
+// Tile 128 x 256 per CTA; the two CTAs of a pair (PAIR, tcgen05 cta_group::2) have neighbouring row tiles and share the weights' rows: each
+// fetches half of them, the leader issues the MMAs for both, everything behind the accumulator is a CTA's own. Operands from THIS GPU's memory
+// only, no multicast.
 // Warps: 0 TMA, 1 MMA (+ TMEM allocation), 2 scale producer, 4..11 epilogue (two per TMEM lane quadrant).
 // The epilogue warps first move their part of the accumulator into registers and hand TMEM back, so the
 // next tile's MMAs overlap the epilogue arithmetic and stores.
@@ -36,16 +37,16 @@
 namespace mfk {
 
 constexpr int XBN = 256;
-constexpr int XSTAGES = 4;
 constexpr int XSFBUFS = 4;
 constexpr int kXThreads = 384;
 constexpr int kXTmemCols = 512;
 constexpr uint32_t kXSfaCol = 256;  // TMEM columns [256, 260): scales of A; [260, 268): scales of B
 constexpr uint32_t kXSfbCol = 260;
 
-struct XSmem {
+template <bool PAIR> struct XSmem {
+    static constexpr int XSTAGES = PAIR ? 6 : 4;
     static constexpr int kABytes = BM * 128;
-    static constexpr int kBBytes = XBN * 128;
+    static constexpr int kBBytes = (PAIR ? XBN / 2 : XBN) * 128;  // a CTA of a pair fetches half of the weights' rows
     static constexpr int kStageBytes = kABytes + kBBytes;
     static constexpr int kSfOff = XSTAGES * kStageBytes;
     static constexpr int kSfBufBytes = 512 + 1024;  // A chunk, two B chunks
@@ -73,7 +74,7 @@ struct XSmem {
     __device__ float *amax(int parity) const { return reinterpret_cast<float *>(base + kAmaxOff) + parity * 256; }
     __device__ uint8_t *out_stage(int epi_warp) const { return base + kOutOff + epi_warp * 32 * kOutRowB; }
 };
-static_assert(XSmem::kDynBytes <= 227 * 1024, "shared memory of the block-scaled fp8 GEMM");
+static_assert(XSmem<false>::kDynBytes <= 227 * 1024 && XSmem<true>::kDynBytes <= 227 * 1024, "shared memory of the block-scaled fp8 GEMM");
 
 struct XArgs {
     TmaPair tm;            // A: [rows, K] fp8; B: [N, K] fp8
@@ -182,10 +183,15 @@ __device__ __noinline__ void ag_quant_rows(const XArgs &g, uint32_t me, int wq, 
     }
 }
 
-template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_tp_fp8_mx(const __grid_constant__ XArgs g)
+template <int MODE, int EPI, bool PAIR> __global__ void __launch_bounds__(kXThreads, 1) k_tp_fp8_mx(const __grid_constant__ XArgs g)
 {
+    using Smem = XSmem<PAIR>;
+    constexpr int XSTAGES = Smem::XSTAGES;
     extern __shared__ uint8_t smem_raw[];
-    XSmem sm(smem_raw);
+    Smem sm(smem_raw);
+    const uint32_t crank = PAIR ? cluster_ctarank() : 0;
+    const int walker = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, walkers = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
+    constexpr int kTileRows = PAIR ? 2 * BM : BM;  // of a pair or a single CTA
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int n_tiles = g.N / XBN;
@@ -200,24 +206,30 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_t
             mbar_init(sm.empty(s), 1);
         }
         for (int i = 0; i < XSFBUFS; i++) {
-            mbar_init(sm.sf_full(i), 32);
+            mbar_init(sm.sf_full(i), PAIR ? 2 : 1);  // the scale producers (of a pair: counted in the leader)
             mbar_init(sm.sf_empty(i), 1);
         }
         mbar_init(sm.tfull(), 1);
-        mbar_init(sm.tempty(), 8);
+        mbar_init(sm.tempty(), PAIR ? 16 : 8);  // the epilogue warps (of a pair: counted in the leader)
         mbar_fence_init();
         tma_prefetch_desc(&g.tm.a);
         tma_prefetch_desc(&g.tm.b);
     }
     if (warp == 1) {
-        tmem_alloc(sm.tmem_slot(), kXTmemCols);
-        tmem_relinquish();
+        if (PAIR) {
+            tmem_alloc_pair(sm.tmem_slot(), kXTmemCols);
+            tmem_relinquish_pair();
+        } else {
+            tmem_alloc(sm.tmem_slot(), kXTmemCols);
+            tmem_relinquish();
+        }
     }
     tc_fence_before();
     __syncthreads();
+    if (PAIR) cluster_sync_all();  // both CTAs' barriers are initialised and both halves of the tensor memory are allocated
     tc_fence_after();
     const uint32_t tmem_base = *sm.tmem_slot();
-    const int total = (g.max_rows / BM) * n_tiles;
+    const int total = (g.max_rows / kTileRows) * n_tiles;
     const uint32_t me = g.team.rank;
     // MODE 2 by one rank: there are no partials to wait for, so a tile's epilogue writes its rows of y itself, under the next tile's MMAs. Adding up behind the
     // last tile read 67 MB back and wrote as much with the tensor cores idle: 4096 x 8192 outputs, K 3584, 126 us, so (and without a second fence
@@ -228,13 +240,13 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_t
     // which the shards arrive) or with the next rank (MODE 2: remote owners first, own rows last); inside a block the row tile varies fastest
     auto locate = [&](int t, int &row0, int &nt) {
         const int rows = MODE == 1 ? g.shard_rows : g.rows_per_rank;
-        const int mt_per = rows / BM;
+        const int mt_per = rows / kTileRows;
         const int per_block = mt_per * n_tiles;
         const int i = t / per_block;
         const int owner = (int)((me + (MODE == 2 ? 1 : 0) + i) % g.team.world);
         const int r = t - i * per_block;
         nt = r / mt_per;
-        row0 = (owner * mt_per + r % mt_per) * BM;
+        row0 = (owner * mt_per + r % mt_per) * kTileRows + (int)crank * BM;  // of this CTA
     };
 
     if (MODE == 1 && warp >= 3) {
@@ -246,7 +258,7 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_t
         if (elect_one()) {
             PipeState ps;
             bool fine = true;
-            for (int t = blockIdx.x; t < total && fine; t += gridDim.x) {
+            for (int t = walker; t < total && fine; t += walkers) {
                 int row0, nt;
                 locate(t, row0, nt);
                 if (MODE == 1) {
@@ -262,50 +274,76 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_t
                 for (int kb = 0; kb < k_blocks; kb++) {
                     fine = mbar_wait(sm.empty(ps.stage), ps.phase ^ 1, ac, 0x602);
                     if (!fine) break;
-                    mbar_expect_tx(sm.full(ps.stage), XSmem::kStageBytes);
-                    tma_load_2d(sm.a(ps.stage), &g.tm.a, kb * 128, row0, sm.full(ps.stage));
-                    tma_load_2d(sm.b(ps.stage), &g.tm.b, kb * 128, nt * XBN, sm.full(ps.stage));
+                    if (PAIR) {
+                        // both CTAs' bytes are counted on the leader's barrier
+                        if (crank == 0) mbar_expect_tx(sm.full(ps.stage), 2 * Smem::kStageBytes);
+                        const uint32_t lead = mapa_u32(smem_u32(sm.full(ps.stage)), 0);
+                        tma_load_2d_pair(sm.a(ps.stage), &g.tm.a, kb * 128, row0, lead);
+                        tma_load_2d_pair(sm.b(ps.stage), &g.tm.b, kb * 128, nt * XBN + (int)crank * (XBN / 2), lead);
+                    } else {
+                        mbar_expect_tx(sm.full(ps.stage), Smem::kStageBytes);
+                        tma_load_2d(sm.a(ps.stage), &g.tm.a, kb * 128, row0, sm.full(ps.stage));
+                        tma_load_2d(sm.b(ps.stage), &g.tm.b, kb * 128, nt * XBN, sm.full(ps.stage));
+                    }
                     ps.advance<XSTAGES>();
                 }
             }
         }
     } else if (warp == 1) {
-        if (elect_one()) {
+        if (crank == 0 && elect_one()) {
+            // of a pair the leader issues for both: a commit that the other CTA waits for as well goes to both CTAs' barriers
+            auto commit = [&](uint64_t *bar) {
+                if (PAIR) {
+                    umma_commit_pair(smem_u32(bar));
+                    umma_commit_pair(mapa_u32(smem_u32(bar), 1));
+                } else {
+                    umma_commit(bar);
+                }
+            };
             PipeState ps, sf;
             uint32_t tphase = 0;
             bool fine = true;
             const uint32_t sfa = tmem_base + kXSfaCol, sfb = tmem_base + kXSfbCol;
-            for (int t = blockIdx.x; t < total && fine; t += gridDim.x) {
-                fine = mbar_wait(sm.tempty(), tphase ^ 1, ac, 0x603);  // the epilogue has taken the previous tile out of TMEM
+            for (int t = walker; t < total && fine; t += walkers) {
+                fine = mbar_wait<PAIR>(sm.tempty(), tphase ^ 1, ac, 0x603);  // the epilogue has taken the previous tile out of TMEM
                 if (!fine) break;
+                tc_fence_after();
                 tphase ^= 1;
                 for (int kb = 0; kb < k_blocks; kb++) {
                     if ((kb & 3) == 0) {
-                        fine = mbar_wait(sm.sf_full(sf.stage), sf.phase, ac, 0x606);
+                        fine = mbar_wait<PAIR>(sm.sf_full(sf.stage), sf.phase, ac, 0x606);
                         if (!fine) break;
                         tc_fence_after();
                         const uint8_t *chunk = sm.sf(sf.stage);
-                        tmem_cp_sf(sfa, umma_desc_sf(chunk));
-                        tmem_cp_sf(sfb, umma_desc_sf(chunk + 512));
-                        tmem_cp_sf(sfb + 4, umma_desc_sf(chunk + 1024));
+                        if (PAIR) {
+                            tmem_cp_sf_pair(sfa, umma_desc_sf(chunk));
+                            tmem_cp_sf_pair(sfb, umma_desc_sf(chunk + 512));
+                            tmem_cp_sf_pair(sfb + 4, umma_desc_sf(chunk + 1024));
+                        } else {
+                            tmem_cp_sf(sfa, umma_desc_sf(chunk));
+                            tmem_cp_sf(sfb, umma_desc_sf(chunk + 512));
+                            tmem_cp_sf(sfb + 4, umma_desc_sf(chunk + 1024));
+                        }
                     }
                     fine = mbar_wait(sm.full(ps.stage), ps.phase, ac, 0x604);
                     if (!fine) break;
                     tc_fence_after();
                     const uint64_t da = umma_desc_sw128(sm.a(ps.stage));
                     const uint64_t db = umma_desc_sw128(sm.b(ps.stage));
-                    const uint32_t idesc = umma_idesc_bs(BM, XBN, (uint32_t)(kb & 3), (uint32_t)(kb & 3));
+                    const uint32_t idesc = umma_idesc_bs(kTileRows, XBN, (uint32_t)(kb & 3), (uint32_t)(kb & 3));
 #pragma unroll
-                    for (int k = 0; k < 4; k++)  // 32 bytes = 32 fp8 = one UMMA K step
-                        umma_fp8_bs(tmem_base, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb | k) != 0, sfa, sfb);
-                    umma_commit(sm.empty(ps.stage));
+                    for (int k = 0; k < 4; k++) {  // 32 bytes = 32 fp8 = one UMMA K step
+                        if (PAIR) umma_fp8_bs_pair(tmem_base, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb | k) != 0, sfa, sfb);
+                        else umma_fp8_bs(tmem_base, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb | k) != 0, sfa, sfb);
+                    }
+                    commit(sm.empty(ps.stage));
                     ps.advance<XSTAGES>();
                     if ((kb & 3) == 3 || kb == k_blocks - 1) {
-                        umma_commit(sm.sf_empty(sf.stage));  // the scale chunk has been copied and its MMAs are done
+                        commit(sm.sf_empty(sf.stage));  // the scale chunk has been copied and its MMAs are done
                         sf.advance<XSFBUFS>();
                     }
                 }
-                if (fine) umma_commit(sm.tfull());
+                if (fine) commit(sm.tfull());
             }
         }
     } else if (warp == 2) {
@@ -314,7 +352,7 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_t
         PipeState sf;
         const int nblocks = g.N / 128;
         bool fine = true;
-        for (int t = blockIdx.x; t < total && fine; t += gridDim.x) {
+        for (int t = walker; t < total && fine; t += walkers) {
             int row0, nt;
             locate(t, row0, nt);
             int nb0, nb1;
@@ -378,7 +416,12 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_t
                 *reinterpret_cast<uint4 *>(chunk + 512 + lane * 16) = make_uint4(wb0, wb0, wb0, wb0);
                 *reinterpret_cast<uint4 *>(chunk + 1024 + lane * 16) = make_uint4(wb1, wb1, wb1, wb1);
                 fence_proxy_async_smem();  // the tensor core's copy unit reads these bytes through the async proxy
-                mbar_arrive(sm.sf_full(sf.stage));
+                __syncwarp();
+                if (lane == 0) {
+                    // each CTA's tensor core copies its own chunks, but the leader has both do it: the other CTA's bytes are released to the cluster
+                    if (crank == 0) mbar_arrive(sm.sf_full(sf.stage));
+                    else mbar_arrive_cluster_smem(mapa_u32(smem_u32(sm.sf_full(sf.stage)), 0));
+                }
                 sf.advance<XSFBUFS>();
             }
         }
@@ -389,8 +432,8 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_t
         const int half = (warp - 4) >> 2;
         uint32_t tphase = 0;
         uint8_t *stg = sm.out_stage(warp - 4);
-        constexpr int kRowB = XSmem::kOutRowB;
-        for (int t = blockIdx.x; t < total; t += gridDim.x) {
+        constexpr int kRowB = Smem::kOutRowB;
+        for (int t = walker; t < total; t += walkers) {
             int row0, nt;
             locate(t, row0, nt);
             const int row = row0 + quad * 32 + lane;
@@ -412,7 +455,10 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_t
             tmem_ld_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(sm.tempty());  // the accumulator is in registers: the next tile may start
+            if (lane == 0) {  // the accumulator is in registers: the next tile may start
+                if (crank == 0) mbar_arrive(sm.tempty());
+                else mbar_arrive_cluster_smem(mapa_u32(smem_u32(sm.tempty()), 0));
+            }
             if (EPI == 1 || EPI == 3) {
                 float o[64];
 #pragma unroll
@@ -586,9 +632,11 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_t
     if (MODE == 2 && !alone && threadIdx.x == 0 && (int)blockIdx.x < (g.rows_per_rank / BM) * n_tiles) uses = g.tile_uses[blockIdx.x];
     tc_fence_before();
     __syncthreads();
+    if (PAIR) cluster_sync_all();  // nobody signals a barrier of a CTA that has left, and both halves of the tensor memory are freed together
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, kXTmemCols);
+        if (PAIR) tmem_dealloc_pair(tmem_base, kXTmemCols);
+        else tmem_dealloc(tmem_base, kXTmemCols);
     }
     if (MODE == 2 && !alone) {
         // add up the W partial tiles of every tile whose rows this rank owns
@@ -622,21 +670,44 @@ template <int MODE, int EPI> __global__ void __launch_bounds__(kXThreads, 1) k_t
 using namespace mfk;
 
 namespace {
-template <int MODE, int EPI> int launch_mx(const XArgs &g, int grid, cudaStream_t s)
+template <int MODE, int EPI, bool PAIR> int launch_mx_as(const XArgs &g, int grid, cudaStream_t s)
 {
-    auto kern = k_tp_fp8_mx<MODE, EPI>;
+    auto kern = k_tp_fp8_mx<MODE, EPI, PAIR>;
     static bool attr_set = false;
     if (!attr_set) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, XSmem::kDynBytes) != cudaSuccess) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, XSmem<PAIR>::kDynBytes) != cudaSuccess) {
             (void)cudaGetLastError();
             return -2;
         }
         attr_set = true;
     }
     // a grid whose CTAs wait for the peers' starts when the kernel in front of it has left the SMs
-    kern<<<grid, kXThreads, XSmem::kDynBytes, s>>>(g);
-    cudaError_t e = cudaGetLastError();
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(kXThreads);
+    cfg.dynamicSmemBytes = XSmem<PAIR>::kDynBytes;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = PAIR ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, g);
+    if (e != cudaSuccess) (void)cudaGetLastError();
     return e == cudaSuccess ? 0 : (int)e;
+}
+
+// `rows`: of a rank's block. Whole 256-row tiles go to CTA pairs: a CTA fetches 32 KiB per 128 of K for what takes 48 KiB alone, which an SM's path from the
+// L2 does not deliver under the MMAs (512 clocks). One rank, N 7168 / K 8192 (SwiGLU, fp8 out) and N 8192 / K 3584, us, single CTAs / pairs: 256 rows 46 / 40
+// and 25 / 20, 512 50 / 46 and 26 / 21, 1024 81.6 / 76 and 36 / 33.5, 2048 138 / 137 and 62 / 55, 4096 230 / 229 and 101 / 89.5.
+template <int MODE, int EPI> int launch_mx(XArgs &g, const void *b, int rows, int sms, cudaStream_t s)
+{
+    const bool pair = rows % (2 * BM) == 0 && (sms & 1) == 0 && sms >= 2;  // the same grid either way: the flags' counters count its CTAs
+    const int rc = make_tmap_2d(&g.tm.b, b, 1, (uint64_t)g.N, (uint64_t)g.K, (uint64_t)g.K, pair ? XBN / 2 : XBN, true);
+    if (rc != 0) return rc;
+    return pair ? launch_mx_as<MODE, EPI, true>(g, sms, s) : launch_mx_as<MODE, EPI, false>(g, sms, s);
 }
 }  // namespace
 
@@ -661,7 +732,6 @@ int mf_ag_gemm_fp8(const Team *team, const void *x_local, int64_t ldx, int shard
     const int M = shard_rows * (int)team->world;
     const uint64_t slot = team->heap_base + (uint64_t)team->rank * team->stride;
     int rc = make_tmap_2d(&g.tm.a, reinterpret_cast<const void *>(slot + ag_buf_off), 1, (uint64_t)M, (uint64_t)K, (uint64_t)K, BM, true);
-    if (rc == 0) rc = make_tmap_2d(&g.tm.b, B, 1, (uint64_t)N, (uint64_t)K, (uint64_t)K, XBN, true);
     if (rc != 0) return rc;
     g.a_scale = reinterpret_cast<const float *>(slot + ag_scale_off);
     g.b_scale = b_scale;
@@ -685,9 +755,9 @@ int mf_ag_gemm_fp8(const Team *team, const void *x_local, int64_t ldx, int shard
     cudaStream_t s = (cudaStream_t)stream;
     // every CTA carries a copy warp whose work peers wait for: the grid must be fully resident (one CTA per SM)
     switch (epi) {
-        case 0: return launch_mx<1, 0>(g, sms, s);
-        case 1: return launch_mx<1, 1>(g, sms, s);
-        case 3: return launch_mx<1, 3>(g, sms, s);
+        case 0: return launch_mx<1, 0>(g, B, shard_rows, sms, s);
+        case 1: return launch_mx<1, 1>(g, B, shard_rows, sms, s);
+        case 3: return launch_mx<1, 3>(g, B, shard_rows, sms, s);
         default: return -1;
     }
 }
@@ -704,7 +774,6 @@ int mf_gemm_rs_fp8(const Team *team, const void *A, const float *a_scale, const 
     XArgs g{};
     const int M = rows_per_rank * (int)team->world;
     int rc = make_tmap_2d(&g.tm.a, A, 1, (uint64_t)M, (uint64_t)K, (uint64_t)K, BM, true);
-    if (rc == 0) rc = make_tmap_2d(&g.tm.b, B, 1, (uint64_t)N, (uint64_t)K, (uint64_t)K, XBN, true);
     if (rc != 0) return rc;
     g.a_scale = a_scale;
     g.b_scale = b_scale;
@@ -721,7 +790,7 @@ int mf_gemm_rs_fp8(const Team *team, const void *A, const float *a_scale, const 
     g.y_out = static_cast<__nv_bfloat16 *>(y_out);
     g.ldy = ldy;
     g.scale = scale;
-    return launch_mx<2, 0>(g, sms, (cudaStream_t)stream);
+    return launch_mx<2, 0>(g, B, rows_per_rank, sms, (cudaStream_t)stream);
 }
 
 }  // extern "C"
