@@ -258,6 +258,22 @@ template <int MODE, int EPI, bool PAIR> __global__ void __launch_bounds__(kXThre
         if (elect_one()) {
             PipeState ps;
             bool fine = true;
+            auto load_b = [&](int stage, int kb, int nt) {
+                if (PAIR) tma_load_2d_pair(sm.b(stage), &g.tm.b, kb * 128, nt * XBN + (int)crank * (XBN / 2), mapa_u32(smem_u32(sm.full(stage)), 0));
+                else tma_load_2d(sm.b(stage), &g.tm.b, kb * 128, nt * XBN, sm.full(stage));
+            };
+            auto expect = [&](int stage) {  // of a pair both CTAs' bytes are counted on the leader's barrier
+                if (!PAIR) mbar_expect_tx(sm.full(stage), Smem::kStageBytes);
+                else if (crank == 0) mbar_expect_tx(sm.full(stage), 2 * Smem::kStageBytes);
+            };
+            // the weights of the first stages do not wait for any shard
+            const int ahead = MODE == 1 && walker < total ? min(XSTAGES, k_blocks) : 0;
+            for (int kb = 0; kb < ahead; kb++) {
+                int row0, nt;
+                locate(walker, row0, nt);
+                expect(kb);
+                load_b(kb, kb, nt);
+            }
             for (int t = walker; t < total && fine; t += walkers) {
                 int row0, nt;
                 locate(t, row0, nt);
@@ -272,19 +288,14 @@ template <int MODE, int EPI, bool PAIR> __global__ void __launch_bounds__(kXThre
                     asm volatile("fence.proxy.async.global;" ::: "memory");  // peers' generic-proxy stores before our TMA reads
                 }
                 for (int kb = 0; kb < k_blocks; kb++) {
-                    fine = mbar_wait(sm.empty(ps.stage), ps.phase ^ 1, ac, 0x602);
-                    if (!fine) break;
-                    if (PAIR) {
-                        // both CTAs' bytes are counted on the leader's barrier
-                        if (crank == 0) mbar_expect_tx(sm.full(ps.stage), 2 * Smem::kStageBytes);
-                        const uint32_t lead = mapa_u32(smem_u32(sm.full(ps.stage)), 0);
-                        tma_load_2d_pair(sm.a(ps.stage), &g.tm.a, kb * 128, row0, lead);
-                        tma_load_2d_pair(sm.b(ps.stage), &g.tm.b, kb * 128, nt * XBN + (int)crank * (XBN / 2), lead);
-                    } else {
-                        mbar_expect_tx(sm.full(ps.stage), Smem::kStageBytes);
-                        tma_load_2d(sm.a(ps.stage), &g.tm.a, kb * 128, row0, sm.full(ps.stage));
-                        tma_load_2d(sm.b(ps.stage), &g.tm.b, kb * 128, nt * XBN, sm.full(ps.stage));
+                    if (t != walker || kb >= ahead) {
+                        fine = mbar_wait(sm.empty(ps.stage), ps.phase ^ 1, ac, 0x602);
+                        if (!fine) break;
+                        expect(ps.stage);
+                        load_b(ps.stage, kb, nt);
                     }
+                    if (PAIR) tma_load_2d_pair(sm.a(ps.stage), &g.tm.a, kb * 128, row0, mapa_u32(smem_u32(sm.full(ps.stage)), 0));
+                    else tma_load_2d(sm.a(ps.stage), &g.tm.a, kb * 128, row0, sm.full(ps.stage));
                     ps.advance<XSTAGES>();
                 }
             }
@@ -599,7 +610,8 @@ template <int MODE, int EPI, bool PAIR> __global__ void __launch_bounds__(kXThre
                 __threadfence();  // covers the stores ordered before it by the barriers of the warp and of the quantising warps
                 const uint32_t done = atomicAdd(g.push_count + p, 1u) + 1;
                 if (done == gridDim.x * g.seq) {
-                    fence_sys();
+                    if (p == me) __threadfence();  // read by this GPU only
+                    else fence_sys();
                     asm volatile("st.relaxed.sys.global.u32 [%0], %1;" ::"l"(reinterpret_cast<uint32_t *>(peer_ptr(g.team, p, g.ag_ready_off)) + me), "r"(g.epoch)
                                  : "memory");
                 }
