@@ -32,6 +32,7 @@
 
 #include "mf_fp8.cuh"
 #include "mf_gemm.cuh"
+#include "mf_launch.cuh"
 #include "mf_team.cuh"
 
 namespace mfk {
@@ -71,6 +72,7 @@ template <bool PAIR> struct XSmem {
     __device__ uint64_t *tempty() const { return bar(2 * XSTAGES + 2 * XSFBUFS + 1); }
     __device__ uint32_t *tmem_slot() const { return reinterpret_cast<uint32_t *>(base + kBarOff + 256); }
     __device__ volatile int *abort_flag() const { return reinterpret_cast<volatile int *>(base + kBarOff + 264); }
+    __device__ uint32_t *stored(int parity) const { return reinterpret_cast<uint32_t *>(base + kBarOff + 272) + parity; }  // MODE 2: warps that have stored a tile
     __device__ float *amax(int parity) const { return reinterpret_cast<float *>(base + kAmaxOff) + parity * 256; }
     __device__ uint8_t *out_stage(int epi_warp) const { return base + kOutOff + epi_warp * 32 * kOutRowB; }
 };
@@ -201,6 +203,7 @@ template <int MODE, int EPI, bool PAIR> __global__ void __launch_bounds__(kXThre
 
     if (threadIdx.x == 0) {
         *sm.abort_flag() = 0;
+        *sm.stored(0) = *sm.stored(1) = 0;
         for (int s = 0; s < XSTAGES; s++) {
             mbar_init(sm.full(s), 1);
             mbar_init(sm.empty(s), 1);
@@ -235,6 +238,9 @@ template <int MODE, int EPI, bool PAIR> __global__ void __launch_bounds__(kXThre
     // last tile read 67 MB back and wrote as much with the tensor cores idle: 4096 x 8192 outputs, K 3584, 126 us, so (and without a second fence
     // for the system per tile) 101; 1024 rows 43.2 / 36.0, 128 rows 23.3 / 20.0. With more ranks the loads of the other partials would hold the epilogue up.
     const bool alone = g.team.world == 1;
+
+    after_predecessor();  // one rank's launch may start under the kernel in front of it; else this returns at once
+    if (alone) start_successor();
 
     // linear tile -> (first row, column tile): blocks of rows owned by one rank, visited starting with this rank (MODE 1: the order in
     // which the shards arrive) or with the next rank (MODE 2: remote owners first, own rows last); inside a block the row tile varies fastest
@@ -579,18 +585,41 @@ template <int MODE, int EPI, bool PAIR> __global__ void __launch_bounds__(kXThre
                     __syncwarp();
                 }
                 if (MODE == 2) {
-                    // all eight epilogue warps have stored their part of the tile: tell the owner
-                    named_bar_sync(9, 256);  // orders all eight warps' stores before the counting thread, whose release publishes them
-                    if (warp == 4 && lane == 0) {
-                        const int owner = row0 / g.rows_per_rank;
-                        const int ltile = ((row0 - owner * g.rows_per_rank) / BM) * n_tiles + nt;
-                        if (alone) g.tile_uses[ltile]++;
-                        uint32_t *cnt = reinterpret_cast<uint32_t *>(peer_ptr(g.team, (uint32_t)owner, g.rs_count_off)) + ltile;
-                        asm volatile("red.release.sys.global.add.u32 [%0], 1;" ::"l"(cnt) : "memory");
-                    }
+                    __syncwarp();
+                    if (lane == 0)
+                        asm volatile("red.release.cta.shared::cta.add.u32 [%0], 1;" ::"r"(smem_u32(sm.stored((int)tphase))) : "memory");
                 }
             }
             tphase ^= 1;
+        }
+    } else if (MODE == 2 && warp == 3) {
+        // Counts every tile at its owner once all eight epilogue warps have stored their part. The release waits until a tile's stores have been
+        // performed at the owner (4 to 5 us after the burst of a round's tiles): in the epilogue it held the next tile up, and K = 3584 was
+        // bound by it (10.4 us a tile for 8.7 of MMAs; 4096 x 8192 outputs 89.5 us, so 78). One counter per parity: no warp is two tiles ahead of another, because a tile's MMAs start
+        // when all of them have taken the previous accumulator out.
+        if (lane == 0) {
+            int it = 0;
+            for (int t = walker; t < total; t += walkers, it++) {
+                int row0, nt;
+                locate(t, row0, nt);
+                const uint32_t want = 8u * (uint32_t)(it / 2 + 1), at = smem_u32(sm.stored(it & 1));
+                uint32_t have = 0;
+                for (uint32_t i = 0; i < kMbarSpinLimit && !*ac.abort_smem; i++) {
+                    asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(have) : "r"(at) : "memory");
+                    if (have >= want) break;
+                    __nanosleep(64);
+                }
+                if (have < want) break;
+                const int owner = row0 / g.rows_per_rank;
+                const int ltile = ((row0 - owner * g.rows_per_rank) / BM) * n_tiles + nt;
+                uint32_t *cnt = reinterpret_cast<uint32_t *>(peer_ptr(g.team, (uint32_t)owner, g.rs_count_off)) + ltile;
+                if (alone) {
+                    g.tile_uses[ltile]++;
+                    asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(cnt) : "memory");  // nobody waits for it
+                } else {
+                    asm volatile("red.release.sys.global.add.u32 [%0], 1;" ::"l"(cnt) : "memory");
+                }
+            }
         }
     } else if (MODE == 1 && warp == 3) {
         // all-gather side, after every warp's part of the quantisation: this CTA's rows and scales to every peer, nearest
@@ -693,7 +722,11 @@ template <int MODE, int EPI, bool PAIR> int launch_mx_as(const XArgs &g, int gri
         }
         attr_set = true;
     }
-    // a grid whose CTAs wait for the peers' starts when the kernel in front of it has left the SMs
+    // a grid whose CTAs wait for the peers' starts when the kernel in front of it has left the SMs; one rank waits for nobody (4 us of every call)
+    if (g.team.world == 1) {
+        const cudaError_t e = launch_overlapped(kern, dim3((unsigned)grid), dim3(kXThreads), XSmem<PAIR>::kDynBytes, s, PAIR ? 2 : 1, g);
+        return e == cudaSuccess ? 0 : (int)e;
+    }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(kXThreads);
