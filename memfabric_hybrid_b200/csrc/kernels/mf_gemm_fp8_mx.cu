@@ -114,74 +114,79 @@ __device__ __forceinline__ void named_bar_sync(int id, int threads) { asm volati
 // All-gather side, first pass: this CTA's rows of the rank's bf16 shard -> e4m3 + one power-of-two scale per 128 elements,
 // into the rank's OWN gather buffer. Nine warps share it (the epilogue warps have nothing else to do until the first tile is
 // finished, and no tile can start before the shard is complete): a unit is 2048 elements of a row (lane = 16 elements, 8
-// lanes = one 128-group, four steps of 512), two units in flight per warp. 4096 rows of 8192 by one warp per SM held the first
-// tile back by more than 100 us; the whole all-gather GEMM (N = 7168, SwiGLU) went from 350 to 234 us.
+// lanes = one 128-group, four steps of 512). The next unit's loads are on their way while a unit's four steps, side by side, are
+// worked on: with nine warps nothing else hides the latencies of either. 4096 rows of 8192: one warp per SM held the first tile back by more
+// than 100 us, nine warps with two units at a time, loads and arithmetic in turns, by 45, so by 35 (copying the rows alone takes 25: nine warps).
+// One 16-byte load per lane and run of 256, whole lines but more shuffles: 38; a third unit on its way: no difference.
+constexpr int kQuantUnit = 2048;
+struct QuantUnit {
+    uint4 raw[4][2];
+    int row, col;  // first row of the shard and column; row < 0: nothing to do
+};
+__device__ __forceinline__ void quant_load(const XArgs &g, QuantUnit &u, int row, int col, int r1, int lane)
+{
+    u.row = row < r1 ? row : -1;
+    u.col = col;
+    if (row >= r1) return;  // uniform over the warp
+    const __nv_bfloat16 *src = g.x_local + (int64_t)row * g.ldx;
+#pragma unroll
+    for (int v = 0; v < 4; v++) {
+        const int c = min(col + v * 512, g.K - 512) + lane * 16;  // K is a multiple of 512: a step is there or not, for the whole warp
+        u.raw[v][0] = __ldcg(reinterpret_cast<const uint4 *>(src + c));
+        u.raw[v][1] = __ldcg(reinterpret_cast<const uint4 *>(src + c) + 1);
+    }
+}
+__device__ __forceinline__ void quant_store(const QuantUnit &u, int K, uint8_t *own_q, float *own_s, int lane)
+{
+    if (u.row < 0) return;
+    __nv_bfloat162 m[4];
+    float scale[4];
+#pragma unroll
+    for (int v = 0; v < 4; v++) m[v] = __hmax2(amax_bf16(u.raw[v][0]), amax_bf16(u.raw[v][1]));
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1)
+#pragma unroll
+        for (int v = 0; v < 4; v++) m[v] = __hmax2(m[v], shfl_xor_bf162(m[v], o));
+#pragma unroll
+    for (int v = 0; v < 4; v++) scale[v] = pow2_scale_e4m3(amax_of(m[v]));
+    uint8_t *q = own_q + (int64_t)u.row * K + u.col + lane * 16;
+    float *s = own_s + (int64_t)u.row * (K / 128) + u.col / 128 + lane / 8;
+#pragma unroll
+    for (int v = 0; v < 4; v++) {
+        const __nv_bfloat162 mul = inverse_bf162(scale[v]);
+        const uint2 lo = pack8_e4m3(u.raw[v][0], mul), hi = pack8_e4m3(u.raw[v][1], mul);
+        if (u.col + v * 512 < K) {
+            *reinterpret_cast<uint4 *>(q + v * 512) = make_uint4(lo.x, lo.y, hi.x, hi.y);
+            if ((lane & 7) == 0) s[v * 4] = scale[v];
+        }
+    }
+}
 __device__ __noinline__ void ag_quant_rows(const XArgs &g, uint32_t me, int wq, int lane)
 {
-    constexpr int kWarps = 9, kUnit = 2048, kU = 2;
+    constexpr int kWarps = 9;
     const int per = (g.shard_rows + (int)gridDim.x - 1) / (int)gridDim.x;
     const int r0 = min(g.shard_rows, (int)blockIdx.x * per), r1 = min(g.shard_rows, r0 + per);
-    const int K = g.K, kg = K / 128, per_row = (K + kUnit - 1) / kUnit;
+    const int K = g.K, per_row = (K + kQuantUnit - 1) / kQuantUnit;
     uint8_t *own_q = peer_ptr(g.team, me, g.ag_buf_off) + (int64_t)me * g.shard_rows * K;
-    float *own_s = reinterpret_cast<float *>(peer_ptr(g.team, me, g.ag_scale_off)) + (int64_t)me * g.shard_rows * kg;
-    const int units = (r1 - r0) * per_row;
-    for (int u0 = wq; u0 < units; u0 += kWarps * kU) {
-        uint4 raw[kU][4][2];
-        int row[kU], col[kU];
-#pragma unroll
-        for (int j = 0; j < kU; j++) {
-            const int u = u0 + j * kWarps;
-            const bool on = u < units;
-            row[j] = r0 + (on ? u / per_row : 0);
-            col[j] = on ? (u % per_row) * kUnit : K;  // K: nothing to do
-            const __nv_bfloat16 *src = g.x_local + (int64_t)row[j] * g.ldx;
-#pragma unroll
-            for (int v = 0; v < 4; v++) {
-                const int c = col[j] + v * 512 + lane * 16;
-                if (c < K) {
-                    raw[j][v][0] = __ldcg(reinterpret_cast<const uint4 *>(src + c));
-                    raw[j][v][1] = __ldcg(reinterpret_cast<const uint4 *>(src + c) + 1);
-                } else {
-                    raw[j][v][0] = raw[j][v][1] = make_uint4(0, 0, 0, 0);
-                }
-            }
+    float *own_s = reinterpret_cast<float *>(peer_ptr(g.team, me, g.ag_scale_off)) + (int64_t)me * g.shard_rows * (K / 128);
+    const int rows_on = kWarps / per_row, parts_on = kWarps - rows_on * per_row;  // from a warp's unit to its next
+    int row = r0 + wq / per_row, part = wq % per_row;
+    auto next = [&](QuantUnit &u) {
+        quant_load(g, u, row, part * kQuantUnit, r1, lane);
+        row += rows_on;
+        part += parts_on;
+        if (part >= per_row) {
+            part -= per_row;
+            row++;
         }
-#pragma unroll
-        for (int j = 0; j < kU; j++) {
-#pragma unroll
-            for (int v = 0; v < 4; v++) {
-                const int c = col[j] + v * 512 + lane * 16;
-                float f[16];
-                const __nv_bfloat162 *h0 = reinterpret_cast<const __nv_bfloat162 *>(&raw[j][v][0]);
-                const __nv_bfloat162 *h1 = reinterpret_cast<const __nv_bfloat162 *>(&raw[j][v][1]);
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    float2 pr = __bfloat1622float2(h0[i]);
-                    f[2 * i] = pr.x;
-                    f[2 * i + 1] = pr.y;
-                    pr = __bfloat1622float2(h1[i]);
-                    f[8 + 2 * i] = pr.x;
-                    f[8 + 2 * i + 1] = pr.y;
-                }
-                float amax = 0.f;
-#pragma unroll
-                for (int i = 0; i < 16; i++) amax = fmaxf(amax, fabsf(f[i]));
-                amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-                amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-                amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-                const float scale = pow2_scale_e4m3(amax);
-                const float mul = 1.f / scale;
-                if (c < K) {
-                    uint4 q;
-                    q.x = pack4_e4m3(f[0], f[1], f[2], f[3], mul);
-                    q.y = pack4_e4m3(f[4], f[5], f[6], f[7], mul);
-                    q.z = pack4_e4m3(f[8], f[9], f[10], f[11], mul);
-                    q.w = pack4_e4m3(f[12], f[13], f[14], f[15], mul);
-                    *reinterpret_cast<uint4 *>(own_q + (int64_t)row[j] * K + c) = q;
-                    if ((lane & 7) == 0) own_s[(int64_t)row[j] * kg + c / 128] = scale;
-                }
-            }
-        }
+    };
+    QuantUnit a, b;
+    next(a);
+    while (a.row >= 0) {
+        next(b);
+        quant_store(a, K, own_q, own_s, lane);
+        next(a);
+        quant_store(b, K, own_q, own_s, lane);
     }
 }
 
