@@ -2,6 +2,7 @@
 // (plain loads/stores on mapped peer memory) and fuses the x scale and the output cast into the same
 // pass. One launch per collective; CTA b of every rank works on the same element ranges as CTA b of
 // every other rank and synchronises only with those (lane flags), so no grid-wide barrier is needed.
+//   allreduce  small    : packets of data and flags straight into the peers' signal areas, no staging, no handshake
 //   allreduce  one-shot : stage -> sync -> every rank reads all W copies, reduces, writes its output
 //   allreduce  two-shot : stage -> sync -> reduce own 1/W into own staging -> sync -> pull every rank's part
 //   reduce_scatter      : stage -> sync -> reduce own 1/W straight into the output
@@ -13,6 +14,8 @@
 // Parity of role: app/zbal/src/csrc/operators/npu/aicore/ops/classic/zbal_kernel_{allreduce,
 // reducescatter,allgather,alltoallv,broadcast,send,recv,barrier}.* of the reference.
 #include <cooperative_groups.h>
+
+#include <algorithm>
 
 #include "mf_coll.cuh"
 #include "mf_shift.cuh"
@@ -35,7 +38,7 @@ struct CollArgs {
     uint32_t epoch;
     uint32_t zero_copy;        // 1: input already sits at stage_a of every slot; 2: direct mode (buffers inside the slices);
                                // 3: direct mode through the multicast alias (team.mc_base)
-    uint32_t root;
+    uint32_t root;             // allreduce: how many CTAs a call in packets may have (0: as many as the launch asks for)
     uint32_t algo;             // allreduce: 0 one-shot, 1 two-shot; rooted copy: 0 broadcast, 1 scatter
     uint64_t part_stride;      // elements between consecutive members' parts in the user buffer (0: packed):
                                // reduce_scatter input rows, allgather output rows, scatter source parts
@@ -394,6 +397,145 @@ template <typename T, typename TO, bool INT, int W> __global__ void __launch_bou
     MF_PROF_START(PF_COPY_OUT);
     fetch_parts<TO>(t, me, a.stage_b, a.n, C, sub, out);
     MF_PROF_STOP(PF_COPY_OUT);
+}
+
+// ------------------------------------------------------------------------------------------------
+// Small all-reduce. Data travels in packets whose every four bytes carry the call's epoch beside them: a store of eight bytes arrives whole, so a receiver
+// that reads this call's epoch has the data, and nobody fences, raises a flag or waits for one. (The handshake of the staged
+// kernel is a release for the system, 3 us here, and a second trip.) A packet carries eight bytes of the input in 16.
+//   algo 2: every rank sends everything to every rank, which sums it up: one trip, W times the data;
+//   algo 3: a rank sums up its part of the elements and sends the results: two trips, twice the data both ways.
+// A half of the packet area is written again two calls later, when every rank has left this one (as with the staging sets): a call ends when the rank
+// has received something that all ranks have contributed to. The whole input is read in front of the CTA's barrier, the
+// output is written behind it.
+// What bounds it: the launch, then latencies. 8 emulated ranks, kernel, us, staged / so: 64 bf16 values 5.5 / 2.5, 3 584 6.3 / 4.1, 32 768 7.9 / 4.4, 8 192 fp32 6.1 / 4.1;
+// a call of 28 672 bf16 values that is waited for 22 / 18.
+template <typename T> struct Packet {
+    static constexpr int N = 8 / sizeof(T);  // elements
+    union {
+        uint2 u;
+        T v[N];
+    };
+    __device__ __forceinline__ void load(const T *p, uint64_t have)  // `have` elements are there
+    {
+        if (have >= N && (reinterpret_cast<uint64_t>(p) & 7) == 0) {
+            u = __ldcg(reinterpret_cast<const uint2 *>(p));
+            return;
+        }
+        u = make_uint2(0, 0);
+#pragma unroll
+        for (int i = 0; i < N; i++)
+            if ((uint64_t)i < have) v[i] = p[i];
+    }
+    __device__ __forceinline__ void store(T *p, uint64_t room) const
+    {
+        if (room >= N && (reinterpret_cast<uint64_t>(p) & 7) == 0) {
+            *reinterpret_cast<uint2 *>(p) = u;
+            return;
+        }
+#pragma unroll
+        for (int i = 0; i < N; i++)
+            if ((uint64_t)i < room) p[i] = v[i];
+    }
+};
+__device__ __forceinline__ void send_packet(uint8_t *to, uint2 data, uint32_t epoch)
+{
+    asm volatile("st.relaxed.sys.global.v2.u64 [%0], {%1, %2};" ::"l"(to), "l"((uint64_t)data.x | (uint64_t)epoch << 32), "l"((uint64_t)data.y | (uint64_t)epoch << 32)
+                 : "memory");
+}
+__device__ __forceinline__ bool try_packet(const uint8_t *from, uint32_t epoch, uint2 &data)
+{
+    uint64_t a, b;
+    asm volatile("ld.relaxed.sys.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(from) : "memory");
+    data = make_uint2((uint32_t)a, (uint32_t)b);
+    return (uint32_t)(a >> 32) == epoch && (uint32_t)(b >> 32) == epoch;
+}
+// Packets from[0], from[stride], .. of this call, all on their way at once; false: the wait ran out.
+template <int M> __device__ __forceinline__ bool wait_packets(const Team &t, const uint8_t *from, uint64_t stride, int count, uint32_t epoch, uint2 (&data)[M])
+{
+    for (uint32_t i = 0; i < t.spin_limit; i++) {
+        bool all = true;
+#pragma unroll
+        for (int r = 0; r < M; r++)
+            if (r < count) all = try_packet(from + r * stride, epoch, data[r]) && all;
+        if (all) return true;
+        if (i > 64) __nanosleep(i > 4096 ? 256 : 32);
+    }
+    return false;
+}
+
+template <typename T, typename TO, bool INT, int W> __global__ void __launch_bounds__(512) k_allreduce_packets(CollArgs a)
+{
+    const Team &t = a.team;
+    const uint32_t me = team_rank(t);
+    const uint32_t world = W > 0 ? (uint32_t)W : t.world;
+    const T *in = reinterpret_cast<const T *>(a.in + (uint64_t)me * a.in_rank_stride);
+    TO *out = reinterpret_cast<TO *>(a.out + (uint64_t)me * a.out_rank_stride);
+    constexpr uint32_t P = Packet<T>::N;
+    const uint32_t n = (uint32_t)a.n;
+    const bool parts = a.algo == 3;
+    const uint32_t C = parts ? (uint32_t)part_of_two_shot(a.n, world) : (n + P - 1) / P * P;  // elements of a row of packets
+    const uint32_t np = C / P, per = (np + gridDim.x - 1) / gridDim.x;
+    const uint32_t beg = min(np, blockIdx.x * per), cnt = min(np, beg + per) - beg;           // this CTA's packets of every row
+    const uint64_t area = kPacketOff + (a.epoch & 1) * kPacketBytes;
+    const uint64_t second = area + (uint64_t)world * np * 16;
+    auto slot = [&](uint32_t rank, uint64_t base, uint32_t row, uint32_t p) { return peer_ptr(t, rank, base) + ((uint64_t)row * np + p) * 16; };
+    // row k of the input: the part of rank me + k, or all of it for that rank
+    for (uint32_t i = threadIdx.x; i < world * cnt; i += blockDim.x) {
+        const uint32_t k = i / cnt, p = beg + i - k * cnt, c = (me + k) % world;
+        const uint32_t e = (parts ? c * C : 0) + p * P;
+        if (e >= n) continue;
+        Packet<T> x;
+        x.load(in + e, n - e);
+        send_packet(slot(c, area, me, p), x.u, a.epoch);
+    }
+    __syncthreads();
+    bool ok = true;
+    for (uint32_t i = threadIdx.x; i < cnt && ok; i += blockDim.x) {
+        const uint32_t p = beg + i, e = (parts ? me * C : 0) + p * P;
+        if (e >= n) continue;
+        float acc[P];
+        constexpr int M = W > 0 ? W : 4;
+        for (uint32_t r0 = 0; r0 < world && ok; r0 += M) {
+            uint2 d[M];
+            const int have = (int)min((uint32_t)M, world - r0);
+            ok = wait_packets<M>(t, slot(me, area, r0, p), (uint64_t)np * 16, have, a.epoch, d);
+#pragma unroll
+            for (int r = 0; r < M; r++) {
+                if (r >= have) continue;
+                Packet<T> x;
+                x.u = d[r];
+#pragma unroll
+                for (uint32_t k = 0; k < P; k++) acc[k] = r0 + r == 0 ? Vec<T>::to_f(x.v[k]) : red_apply<INT>(acc[k], Vec<T>::to_f(x.v[k]), a.op);
+            }
+        }
+        if (!ok) break;
+        Packet<TO> y;
+        y.u = make_uint2(0, 0);
+        static_assert(Packet<TO>::N >= (int)P, "the results of a packet fit one");
+#pragma unroll
+        for (uint32_t k = 0; k < P; k++) y.v[k] = Vec<TO>::from_f(!INT && a.scale != 1.f ? acc[k] * a.scale : acc[k]);
+        if (parts) {
+            for (uint32_t k = 0; k < world; k++) send_packet(slot((me + k) % world, second, me, p), y.u, a.epoch);
+        } else if (Packet<TO>::N == (int)P) {
+            y.store(out + e, n - e);
+        } else {
+            for (uint32_t k = 0; k < P && e + k < n; k++) out[e + k] = y.v[k];
+        }
+    }
+    for (uint32_t i = threadIdx.x; parts && i < world * cnt && ok; i += blockDim.x) {
+        const uint32_t k = i / cnt, p = beg + i - k * cnt, c = (me + k) % world, e = c * C + p * P;
+        if (e >= n) continue;
+        uint2 d[1];
+        ok = wait_packets<1>(t, slot(me, second, c, p), 0, 1, a.epoch, d);
+        if (!ok) break;
+        Packet<TO> y;
+        y.u = d[0];
+        if (Packet<TO>::N == (int)P) y.store(out + e, n - e);
+        else
+            for (uint32_t q = 0; q < P && e + q < n; q++) out[e + q] = y.v[q];
+    }
+    if (!ok) report_timeout(t, me, 0x102, a.epoch);
 }
 
 // reduce_scatter: input n = W * m elements, output m elements (rank r gets the reduction of chunk r)
@@ -1387,8 +1529,41 @@ bool pipe_pays(const CollArgs &a, uint64_t part_stride, uint64_t es, int threads
     return !a.zero_copy && threads == kPipeThreads && a.team.world > 1 && a.team.world * a.n * es >= kPipeMinBytes && part_stride * es % 16 == 0;
 }
 
+constexpr uint64_t kOneTripBytes = 16 << 10;  // received by a rank; above it two trips of less data are as fast on one GPU
+constexpr uint64_t kPacketCtaBytes = 4 << 10;  // a CTA: 8 ranks, 38 000 bf16 values back to back, us: with 1, 4, 8, 14, 18 CTAs a rank 20.5, 9.9, 8.3, 6.5, 6.2
+bool own_buffers(const CollArgs &a, uint64_t es, uint64_t oes)  // input and output (of all emulated ranks) are one buffer or share nothing
+{
+    const uint64_t more = a.team.emu ? a.team.world - 1 : 0;
+    const uint64_t in_end = a.in + more * a.in_rank_stride + a.n * es, out_end = a.out + more * a.out_rank_stride + a.n * oes;
+    return (a.in == a.out && es == oes && (!a.team.emu || a.in_rank_stride == a.out_rank_stride)) || in_end <= a.out || out_end <= a.in;
+}
+// Packets for a small all-reduce: 2 (one trip), 3 (two trips), 0: staged. The same on every rank: what a rank's own buffers look like plays no part; emulated
+// ranks' buffers are all known, and where one rank's output lies in another's input the staged kernel's exchange keeps them apart.
+uint32_t packets_for(const CollArgs &a, uint64_t es, bool own)
+{
+    const uint64_t world = a.team.world, bytes = a.n * es;
+    if (a.zero_copy || a.algo != 0 || world < 2 || a.n == 0 || bytes > kPacketBytes || (a.team.emu && !own)) return 0;
+    const uint64_t packet = 8 / es;  // elements
+    if (world * bytes <= kOneTripBytes && world * ((a.n + packet - 1) / packet) * 16 <= kPacketBytes) return 2;
+    return 2 * world * (part_of_two_shot(a.n, (uint32_t)world) / packet) * 16 <= kPacketBytes ? 3 : 0;
+}
+
 template <typename T, typename TO, bool INT> int launch_allreduce(const CollArgs &a, int ctas, int threads, cudaStream_t s)
 {
+    const bool own = own_buffers(a, sizeof(T), sizeof(TO));
+    if (const uint32_t algo = packets_for(a, sizeof(T), own)) {
+        CollArgs b = a;
+        b.algo = algo;
+        // a CTA waits for nothing but its own packets, so that ranks may differ in the number of CTAs; a single one keeps an overlap of the buffers in order
+        const uint64_t bytes = a.n * sizeof(T) * (algo == 2 ? a.team.world : 1);
+        ctas = !own ? 1 : a.root ? (int)std::min<uint64_t>((bytes + kPacketCtaBytes - 1) / kPacketCtaBytes, a.root) : ctas;
+        switch (a.team.world) {
+            case 2: return launch(k_allreduce_packets<T, TO, INT, 2>, b, ctas, threads, s, false);
+            case 4: return launch(k_allreduce_packets<T, TO, INT, 4>, b, ctas, threads, s, false);
+            case 8: return launch(k_allreduce_packets<T, TO, INT, 8>, b, ctas, threads, s, false);
+            default: return launch(k_allreduce_packets<T, TO, INT, 0>, b, ctas, threads, s, false);
+        }
+    }
     const uint64_t C = part_of_two_shot(a.n, a.team.world);
     // a row per rank has to fit the staging area, which ends in front of the results'
     if (a.algo == 1 && pipe_pays(a, C, sizeof(T), threads) && a.stage_b >= a.stage_a + a.team.world * C * sizeof(T)) {
@@ -1647,7 +1822,7 @@ const char *mf_noalloc_strerror(int code)
         case MF_NOALLOC_E_TOO_LARGE: return "vector larger than MF_NOALLOC_MAX_BYTES (1 MiB): the built-in scratch cannot stage it";
         case MF_NOALLOC_E_SETUP: return "could not obtain the device address of the built-in scratch array";
         case MF_NOALLOC_E_LAUNCH: return "kernel launch refused";
-        case MF_NOALLOC_E_TIMEOUT: return "a bounded wait inside an earlier call ran out: that call did not write its output";
+        case MF_NOALLOC_E_TIMEOUT: return "a bounded wait inside an earlier call ran out: that call did not complete its output";
         default: return "unknown code";
     }
 }

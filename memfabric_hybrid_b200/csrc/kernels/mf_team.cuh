@@ -37,6 +37,10 @@ constexpr int kPhases = 4;
 constexpr uint32_t kXchgOff = 256 * 1024;
 //   [384 KiB, 384 KiB + 32 KiB)  chunk progress  [cta 0..255][rank 0..15] x u64 {epoch, chunks delivered}
 constexpr uint32_t kChunkOff = 384 * 1024;
+//   [416 KiB, 1 MiB)             packets {4 bytes of data, epoch} x 2, 16 bytes each: two halves by the parity of the epoch. Every word behind
+//                                four bytes of data is an epoch, whatever the size of the call, so nothing else is ever stored here
+constexpr uint32_t kPacketOff = 416 * 1024;
+constexpr uint32_t kPacketBytes = (kSignalBytes - kPacketOff) / 2;
 
 enum MfStatus : uint32_t { ST_OK = 0, ST_TIMEOUT = 1, ST_BAD_ARG = 2 };
 

@@ -169,7 +169,7 @@ int AllReduce(Comm &c, const void *in, void *out, uint64_t n, int kdt, int odt, 
     uint64_t done = 0;
     while (done < n) {
         const uint64_t cnt = std::min(piece, n - done);
-        MfCollArgs a = BaseArgs(c, static_cast<const char *>(in) + done * es, static_cast<char *>(out) + done * oes, cnt, scale, op, 0,
+        MfCollArgs a = BaseArgs(c, static_cast<const char *>(in) + done * es, static_cast<char *>(out) + done * oes, cnt, scale, op, c.maxCtas,
                                 cnt * es <= kOneShotMax ? 0 : 1);
         int rc = Launched(L->coll(0, kdt, odt, &a, c.Ctas(cnt * es), 512, stream), "all_reduce");
         if (rc != Z_OK) return rc;

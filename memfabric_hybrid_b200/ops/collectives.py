@@ -221,7 +221,7 @@ class Communicator:
         while done < n:
             cnt = min(piece, n - done)
             use = a if a is not None else (0 if cnt * es <= ONE_SHOT_MAX else 1)
-            self._launch(0, x, out, cnt, cnt * es, "all_reduce", scale, op, 0, use, 0, xl, ol, (done * es, done * oes))
+            self._launch(0, x, out, cnt, cnt * es, "all_reduce", scale, op, self.max_ctas, use, 0, xl, ol, (done * es, done * oes))
             done += cnt
         return out
 

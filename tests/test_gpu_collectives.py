@@ -65,6 +65,47 @@ def test_all_reduce_fused_cast_and_ops(comms, world):
     assert torch.equal(c.all_reduce(xi, op="max", algo="twoshot")[world - 1], xi.max(0).values)
 
 
+@pytest.mark.parametrize("world", [2, 3, 8])
+def test_small_all_reduce_in_packets(world):
+    """Sizes that change from call to call (what an earlier call left in the packet area must not count), odd ones, inputs off eight bytes, in place, an output in
+    the input's memory, every type: the fp32 sum in rank order, rounded once. 76 KiB is about where the staged kernel takes over."""
+    from memfabric_hybrid_b200.ops.heap import EmulatedHeap
+    from memfabric_hybrid_b200.ops.collectives import Communicator
+    heap = EmulatedHeap(world, (1 << 20) + 4 * (1 << 20) + 4096)
+    c = Communicator(heap, stage_bytes=1 << 20)
+    for k, n in enumerate([1, 7, 40_000, 513, 8, 38_912, 1021, 4096, 38_913, 19_456, 19_459, 3, 2048 // world, 2048 // world + 1]):
+        g = torch.Generator("cuda").manual_seed(n)
+        for dtype, out_dtype in ((torch.bfloat16, None), (torch.float32, None), (torch.float32, torch.bfloat16), (torch.float16, None), (torch.int32, None)):
+            if dtype == torch.int32:
+                x = torch.randint(-1000, 1000, (world, n), device="cuda", generator=g, dtype=dtype)
+                want = x.sum(0).to(dtype)
+            else:
+                x = torch.randn(world, n, device="cuda", generator=g).to(dtype)
+                acc = x[0].float()
+                for r in range(1, world):
+                    acc = acc + x[r].float()
+                want = (acc * 0.5).to(out_dtype or dtype)
+            scale = 1.0 if dtype == torch.int32 else 0.5
+            want = want.expand(world, n)
+            room = torch.full((world * n + 16,), 7, device="cuda", dtype=out_dtype or dtype)
+            off = k % 8
+            got = c.all_reduce(x, out=room[off:off + world * n].view(world, n), scale=scale, out_dtype=out_dtype)
+            assert torch.equal(got, want) and bool((room[:off] == 7).all()) and bool((room[off + world * n:] == 7).all()), (n, dtype, out_dtype)
+            assert torch.equal(c.all_reduce(x, scale=scale, out_dtype=out_dtype), want), (n, dtype, out_dtype)
+            if out_dtype is None:
+                wide = torch.empty(world * n + 5, dtype=dtype, device="cuda")
+                y = wide[1:1 + world * n].view(world, n)
+                y.copy_(x)
+                assert torch.equal(c.all_reduce(y, out=y, scale=scale), want), (n, dtype)
+                if n * x.element_size() <= 16 << 10:   # one CTA per rank: any overlap is fine
+                    y.copy_(x)
+                    assert torch.equal(c.all_reduce(y, out=wide[4:4 + world * n].view(world, n), scale=scale), want), (n, dtype)
+        if n > 1 and world == 8:
+            assert torch.equal(c.all_reduce(x, op="max")[0], x.max(0).values)
+    torch.cuda.synchronize()
+    assert heap.status()[0] == 0
+
+
 @pytest.mark.parametrize("world", [2, 4, 8])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("m", [8, 1024, 50_000, 400_000])
