@@ -2,8 +2,8 @@
 //
 // What bounds it: reading B once from memory. The persistent kernel of mf_gemm.cu gives one SM a whole 128 x 256 tile over all
 // of K, so a layer with N = 7168 keeps 28 SMs busy and the other 120 idle. Measured with B from memory, launches from a CUDA graph (us,
-// the persistent kernel's better tiling / this kernel): 32 x 7168 x 8192 42.6 / 23.4, 32 x 8192 x 3584 22.9 / 14.4, 16 x 1024 x 8192
-// 42.1 / 9.2. (Alone, with cold caches under ncu, the first two take 51.5 / 27.2 and 24.7 / 16.5.) Here a tile is 128 x 128 and the S
+// the persistent kernel's better tiling / this kernel): 32 x 7168 x 8192 43.1 / 22.6, 32 x 8192 x 3584 23.2 / 13.8, 1 x 1024 x 4096
+// 23.8 / 5.6. Of the 22.6, 18.5 are the loads (6.3 TB/s; the first ones arrive after 2.3), 2.5 the exchange. Here a tile is 128 x 128 and the S
 // CTAs of a cluster each take 1/S of K into their own tensor memory; the partial sums meet through distributed shared memory (every CTA adds up
 // and stores 1/S of the tile, in CTA order: the result does not depend on timing). No workspace, no second launch.
 // Two CTAs share an SM (about 100 KB of stages each), so one CTA's prologue and reduction run under the other's loads.
@@ -25,6 +25,8 @@ namespace mfk {
 constexpr int kSkBN = 128;
 constexpr int kSkThreads = 192;              // warp 0 TMA, warp 1 MMA, warps 2..5 read the accumulator, all six reduce
 constexpr int kSkMaxSplit = 8;               // portable cluster size
+constexpr int kSkAtOnce = 8;                 // partial sums on their way to a thread at once
+static_assert(kSkMaxSplit <= kSkAtOnce, "one item's parts");
 constexpr int kSkStageArea = 100 * 1024;     // two CTAs per SM
 constexpr int kSkRowFloats = kSkBN + 4;      // 528-byte rows: eight lanes' 16-byte writes to eight rows hit all banks once
 constexpr int kSkMaxStages = kSkStageArea / (8 * KSPAN + kSkBN * KSPAN);  // A's box is at least 8 rows
@@ -45,6 +47,98 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr)
     float4 v;
     asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
     return v;
+}
+
+__device__ __forceinline__ float4 ld_shared_f4(uint32_t addr)
+{
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+// Every thread on its own (threads of a warp come to it at different places).
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
+// This CTA's share of the tile: the S partial sums of four columns (with SwiGLU: four gate columns and their up projections) per item, added in CTA order.
+// What bounds it: the way from the neighbours' shared memory. Lanes read 16 bytes side by side, a CTA's own part does not leave the SM, and the reads
+// of several items are on their way at once. Before, a thread read 32 bytes with gaps, the own part the same way, one part after another: with a tile's
+// 32 rows in 4 CTAs 2.9 us from the last partial tile to the end, 1.7 so; 128 rows in 2 CTAs 5.6, 4.2; gate/up and down product (N, K = 7168, 8192 and
+// 8192, 3584) in a row, us before / so: 1 row 35.1 / 34.3, 32 rows 41.6 / 37.4, 64 46.0 / 41.5, 128 55.8 / 48.2, 256 61.0 / 58.0.
+template <int EPI, int S> __device__ __forceinline__ void add_up(const SplitArgs &g, uint32_t part0, __nv_bfloat16 *C, int rows, int nt, uint32_t rank, uint32_t split)
+{
+    constexpr int kOutCols = EPI == 1 ? kSkBN / 2 : kSkBN;   // output columns of the tile
+    constexpr int kVecs = kOutCols / 4;
+    constexpr int H = EPI == 1 ? 2 : 1;
+    constexpr int P = S ? S : kSkAtOnce, U = kSkAtOnce / P;  // parts, items at once
+    const int n_out = EPI == 1 ? g.N / 2 : g.N;
+    const bool vec_ok = (g.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(C) & 7) == 0;
+    const int total = rows * kVecs, step = (int)(S ? S : split) * kSkThreads;
+    int it = (int)(rank * kSkThreads + threadIdx.x);
+    if (it >= total) cluster_arrive();
+    for (; it < total; it += U * step) {
+        float4 v[U][P][H];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int i = it + u * step;
+            if (i >= total) continue;
+            const uint32_t at = part0 + (uint32_t)((i / kVecs) * kSkRowFloats + (i % kVecs) * 4) * 4;
+#pragma unroll
+            for (uint32_t p = 0; p < (uint32_t)P; p++) {
+                if (S == 0 && p >= split) continue;
+                const uint32_t from = mapa_u32(at, p);
+#pragma unroll
+                for (int h = 0; h < H; h++) v[u][p][h] = p == rank ? ld_shared_f4(at + (uint32_t)(h * (kSkBN / 2) * 4)) : ld_cluster_f4(from + (uint32_t)(h * (kSkBN / 2) * 4));
+            }
+        }
+        float acc[U][H * 4];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+#pragma unroll
+            for (int e = 0; e < H * 4; e++) acc[u][e] = 0.f;
+            if (it + u * step >= total) continue;
+#pragma unroll
+            for (uint32_t p = 0; p < (uint32_t)P; p++) {
+                if (S == 0 && p >= split) continue;
+#pragma unroll
+                for (int h = 0; h < H; h++) {
+                    acc[u][h * 4] += v[u][p][h].x;
+                    acc[u][h * 4 + 1] += v[u][p][h].y;
+                    acc[u][h * 4 + 2] += v[u][p][h].z;
+                    acc[u][h * 4 + 3] += v[u][p][h].w;
+                }
+            }
+        }
+        // the last reads of the neighbours' tiles: they may go once all have arrived, while the stores below are on their way
+        if (it + U * step >= total) cluster_arrive();
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int i = it + u * step;
+            if (i >= total) continue;
+            float o[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                if (EPI == 1) {
+                    const float gt = acc[u][e], up = acc[u][H * 4 - 4 + e];
+                    o[e] = gt / (1.f + __expf(-gt)) * up;
+                } else {
+                    o[e] = acc[u][e];
+                }
+            }
+            const int col = nt * kOutCols + (i % kVecs) * 4;
+            __nv_bfloat16 *dst = C + (int64_t)(i / kVecs) * g.ldc + col;
+            if (vec_ok && col + 4 <= n_out) {
+                uint2 pk;
+                __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(&pk);
+                h[0] = __floats2bfloat162_rn(o[0], o[1]);
+                h[1] = __floats2bfloat162_rn(o[2], o[3]);
+                *reinterpret_cast<uint2 *>(dst) = pk;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; e++)
+                    if (col + e < n_out) dst[e] = __float2bfloat16_rn(o[e]);
+            }
+        }
+    }
 }
 
 template <int EPI> __global__ void __launch_bounds__(kSkThreads, 2) k_gemm_bf16_splitk(const __grid_constant__ SplitArgs g)
@@ -145,75 +239,38 @@ template <int EPI> __global__ void __launch_bounds__(kSkThreads, 2) k_gemm_bf16_
             if (quad * 32 < g.M - mt * BM) {  // uniform over the warp: the reads below are collective
                 float *mine = reinterpret_cast<float *>(base) + row * kSkRowFloats;
 #pragma unroll
-                for (int c = 0; c < kSkBN / 32; c++) {
-                    uint32_t v[32];
-                    tmem_ld32(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(c * 32), v);
+                for (int c = 0; c < kSkBN / 64; c++) {
+                    uint32_t v[2][32];
+                    tmem_ld32(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(c * 64), v[0]);
+                    tmem_ld32(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(c * 64 + 32), v[1]);
                     tmem_ld_wait();
 #pragma unroll
-                    for (int q = 0; q < 8; q++)
-                        *reinterpret_cast<uint4 *>(mine + c * 32 + q * 4) = make_uint4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);
+                    for (int q = 0; q < 16; q++) {
+                        const uint32_t *w = v[q / 8] + q % 8 * 4;
+                        *reinterpret_cast<uint4 *>(mine + c * 64 + q * 4) = make_uint4(w[0], w[1], w[2], w[3]);
+                    }
                 }
             }
             tc_fence_before();
         }
     }
-    __syncthreads();
+    __syncwarp();
+    cluster_sync_all();  // every CTA's partial tile is in its shared memory (every CTA arrives: the waits above are bounded)
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem, kSkBN);
     }
-    cluster_sync_all();  // every CTA's partial tile is in its shared memory (every CTA arrives: the waits above are bounded)
 
     const int rows = min(BM, g.M - mt * BM);
-    constexpr int kOutCols = EPI == 1 ? kSkBN / 2 : kSkBN;   // output columns of the tile
-    constexpr int kVecs = kOutCols / 8;
-    const int n_out = EPI == 1 ? g.N / 2 : g.N;
-    const bool vec_ok = (g.ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(g.C) & 15) == 0;
     const uint32_t part0 = smem_u32(base);
-    for (int it = (int)(rank * kSkThreads + threadIdx.x); it < rows * kVecs; it += (int)split * kSkThreads) {
-        const int r = it / kVecs, c = (it % kVecs) * 8;
-        const uint32_t at = part0 + (uint32_t)(r * kSkRowFloats + c) * 4;
-        float acc[EPI == 1 ? 16 : 8];
-#pragma unroll
-        for (int e = 0; e < (EPI == 1 ? 16 : 8); e++) acc[e] = 0.f;
-        for (uint32_t p = 0; p < split; p++) {
-            const uint32_t from = mapa_u32(at, p);
-#pragma unroll
-            for (int h = 0; h < (EPI == 1 ? 4 : 2); h++) {
-                // SwiGLU: columns c.. are gate, c + 64.. the matching up projections
-                const float4 v = ld_cluster_f4(from + (uint32_t)((h & 1) * 16 + (h >> 1) * (kSkBN / 2) * 4));
-                acc[h * 4] += v.x;
-                acc[h * 4 + 1] += v.y;
-                acc[h * 4 + 2] += v.z;
-                acc[h * 4 + 3] += v.w;
-            }
-        }
-        float o[8];
-#pragma unroll
-        for (int e = 0; e < 8; e++) {
-            if (EPI == 1) {
-                const float gt = acc[e], up = acc[8 + e];
-                o[e] = gt / (1.f + __expf(-gt)) * up;
-            } else {
-                o[e] = acc[e];
-            }
-        }
-        const int col = nt * kOutCols + c;
-        __nv_bfloat16 *dst = g.C + (int64_t)(mt * BM + r) * g.ldc + col;
-        if (vec_ok && col + 8 <= n_out) {
-            uint4 pk;
-            __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(&pk);
-#pragma unroll
-            for (int e = 0; e < 4; e++) h[e] = __floats2bfloat162_rn(o[2 * e], o[2 * e + 1]);
-            *reinterpret_cast<uint4 *>(dst) = pk;
-        } else {
-#pragma unroll
-            for (int e = 0; e < 8; e++)
-                if (col + e < n_out) dst[e] = __float2bfloat16_rn(o[e]);
-        }
+    __nv_bfloat16 *C = g.C + (int64_t)mt * BM * g.ldc;
+    switch (split) {
+        case 1: add_up<EPI, 1>(g, part0, C, rows, nt, rank, split); break;
+        case 2: add_up<EPI, 2>(g, part0, C, rows, nt, rank, split); break;
+        case 4: add_up<EPI, 4>(g, part0, C, rows, nt, rank, split); break;
+        default: add_up<EPI, 0>(g, part0, C, rows, nt, rank, split); break;
     }
-    __syncwarp();
-    cluster_sync_all();  // nobody leaves while a peer still reads its partial tile
+    cluster_wait();  // nobody leaves while a peer still reads its partial tile
 }
 
 }  // namespace mfk

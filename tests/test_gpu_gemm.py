@@ -79,6 +79,33 @@ def test_gemm_bf16_swiglu_few_rows(M, F, K):
     assert ((c.float() - one.float()).norm() / one.float().norm()).item() <= 2.0 ** -8
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 256, 512), (31, 512, 576), (129, 256, 2048)])
+@pytest.mark.parametrize("split", [1, 2, 3, 4, 8])
+@pytest.mark.parametrize("swiglu", [0, 1])
+def test_partial_tiles_added_by_any_number_of_ctas(M, N, K, split, swiglu):
+    """Items of four columns, several of them at once for 1, 2 and 4 CTAs, rows of C at 2, 4, 8 and 16 bytes. One bf16 rounding (2^-8 of the value) plus fp32 accumulation
+    (K 2^-24 of the terms), which SwiGLU scales by |up| times the slope of silu (at most 1.1) and by |silu|; its exponential and quotient stay below 2^-16."""
+    from memfabric_hybrid_b200.ops import gemm
+    torch.manual_seed(M + N + K)
+    a = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    b = (torch.randn(N, K, device="cuda") * 0.05).to(torch.bfloat16)
+    n_out = N // 2 if swiglu else N
+    ref, err = a.double() @ b.double().t(), (a.double().abs() @ b.double().abs().t()) * K * 2.0 ** -24
+    if swiglu:
+        (g, u), (eg, eu) = (t.view(M, N // 256, 2, 128).permute(2, 0, 1, 3).reshape(2, M, n_out) for t in (ref, err))
+        ref = torch.nn.functional.silu(g) * u
+        err = 1.1 * eg * u.abs() + torch.nn.functional.silu(g).abs() * eu + ref.abs() * 2.0 ** -16
+    for ld, off in ((n_out + 8, 0), (n_out + 4, 4), (n_out + 2, 2), (n_out + 1, 1)):
+        buf = torch.full((off + M * ld,), 7.0, device="cuda", dtype=torch.bfloat16)
+        c = buf[off:].view(M, ld)
+        assert gemm._cu().mf_gemm_bf16_splitk(a.data_ptr(), b.data_ptr(), c.data_ptr(), M, N, K, K, K, ld, gemm.status_word().data_ptr(), gemm.sm_count(), swiglu,
+                                              split, torch.cuda.current_stream().cuda_stream) == 0
+        torch.cuda.synchronize()
+        gemm.check_status()
+        assert ((c[:, :n_out].double() - ref).abs() <= ref.abs() * 2.0 ** -8 + err).all(), ld
+        assert bool((c[:, n_out:] == 7.0).all()) and bool((buf[:off] == 7.0).all()), "columns past N were written"
+
+
 @pytest.mark.parametrize("M", [32, 4096])
 def test_gemm_bf16_in_a_cuda_graph(M):
     """Two products in a row, captured: the second may start under the end of the first (few rows) and must still see all of it."""
