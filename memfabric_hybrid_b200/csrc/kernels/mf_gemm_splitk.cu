@@ -63,7 +63,7 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 // What bounds it: the way from the neighbours' shared memory. Lanes read 16 bytes side by side, a CTA's own part does not leave the SM, and the reads
 // of several items are on their way at once. Before, a thread read 32 bytes with gaps, the own part the same way, one part after another: with a tile's
 // 32 rows in 4 CTAs 2.9 us from the last partial tile to the end, 1.7 so; 128 rows in 2 CTAs 5.6, 4.2; gate/up and down product (N, K = 7168, 8192 and
-// 8192, 3584) in a row, us before / so: 1 row 35.1 / 34.3, 32 rows 41.6 / 37.4, 64 46.0 / 41.5, 128 55.8 / 48.2, 256 61.0 / 58.0.
+// 8192, 3584) in a row, us before / so: 1 row 35.1 / 34.3, 32 rows 41.6 / 37.4, 64 46.1 / 41.5, 128 55.6 / 48.2, 256 60.8 / 57.9.
 template <int EPI, int S> __device__ __forceinline__ void add_up(const SplitArgs &g, uint32_t part0, __nv_bfloat16 *C, int rows, int nt, uint32_t rank, uint32_t split)
 {
     constexpr int kOutCols = EPI == 1 ? kSkBN / 2 : kSkBN;   // output columns of the tile
@@ -301,12 +301,13 @@ extern "C" {
 // CTAs that share a tile: 1, 2, 4 or 8 (clusters of 3, 5, 6 leave more of a GPC unused and were slower throughout).
 // Cost in steps of K (64 elements of a 128 x 128 tile), for rounds of resident clusters: two CTAs per SM; clusters of two fit
 // everywhere, of the larger ones a tenth does not fit the rest of a GPC. A round takes K / s steps, or what memory takes for all
-// tiles' steps (1.35 steps per SM at a time); sharing a tile costs 2.5 steps, and every CTA of it adds its exchange, which
-// grows with the rows and with how many CTAs exchange at once. The constants fit 975 products of 1 - 1024 rows, 1 - 74 tiles of 128 x
-// 256 and K 512 - 16384 (launches from a graph, weights from memory): the choice is 1.2 % from the best of the four on average.
-// Measured (us, persistent kernels' better tiling | s = 1, 2, 4, 8): 32 x 7168 x 8192 42.6 | 33.7, 24.2, 23.4, 31.6; 1 x 1024 x 4096 24.2 |
-// 16.7, 10.5, 7.2, 5.8; 128 x 1024 x 8192 42.4 | 46.9, 27.1, 17.6, 15.0; 256 x 4096 x 8192 42.8 | 47.1, 28.8, 26.1, 47.7; 256 x 9216 x 8192 44.0 | 50.8,
-// 42.5, 67.0, 107; 1024 x 2304 x 16384 78.5 | 90.9, 68.1, 114, 153; 1024 x 1280 x 1024 10.6 | 7.9, 11.2, 21.5, 45.3.
+// tiles' steps (1.35 steps per SM at a time), and its exchange: a barrier, what grows with the rows and with how many CTAs exchange at once, and
+// most of all whether clusters share their SMs (a cluster's slowest CTA counts: 17 tiles in clusters of eight, 6 x 2624 x 1856, 6.5, in clusters of
+// four 5.6; 16 tiles, 3 x 2016 x 2432, 5.9, 5.9). The constants fit 181 products of 1 - 1024 rows, 1 - 74 tiles of 128 x
+// 256 and K 512 - 8192 (launches from a graph, weights from memory): the choice is 0.3 % from the best of the four on average (0.5 % for 107 others; 4.4 and 4.8 with the constants of the slower exchange).
+// Measured (us, persistent kernels' better tiling | s = 1, 2, 4, 8): 32 x 7168 x 8192 43.1 | 34.3, 24.3, 22.6, 27.9; 1 x 1024 x 4096 23.8 |
+// 16.9, 10.1, 6.8, 5.6; 128 x 1024 x 8192 41.9 | 47.5, 26.4, 16.1, 11.8; 256 x 4096 x 8192 43.2 | 48.2, 28.7, 22.7, 33.6; 256 x 9216 x 8192 44.8 | 52.0,
+// 41.0, 58.9, 74.4; 1024 x 2304 x 16384 79.2 | 93.2, 66.4, 90.6, 101; 1024 x 1280 x 1024 10.0 | 9.5, 9.8, 15.0, 25.9.
 int mf_gemm_bf16_split(int M, int N, int K, int sms)
 {
     const int tiles = split_tiles(M, N), k_iters = split_k_iters(K), n = sms > 0 ? sms : 148;
@@ -317,7 +318,8 @@ int mf_gemm_bf16_split(int M, int N, int K, int sms)
         const double resident = (s <= 2 ? 2.0 : 1.8) * n / s;
         const double rounds = std::ceil(tiles / std::max(1.0, std::floor(resident)));
         const double busy = std::min(1.0, (double)tiles * s / (2.0 * n));
-        const double cost = std::max(rounds * ((k_iters + s - 1) / s), memory) + (s > 1 ? 2.5 : 0.0) + s * (1 + 8.0 * split_box_rows(M) / BM * busy);
+        const double exchange = s > 1 ? 1.7 + 1.8 * s * split_box_rows(M) / BM * busy + (tiles > std::floor(resident / 2) ? 5.25 : 0.0) : 0.0;
+        const double cost = std::max(rounds * ((k_iters + s - 1) / s), memory) + rounds * (0.3 * s + exchange);
         if (split == 0 || cost < best) {
             best = cost;
             split = s;

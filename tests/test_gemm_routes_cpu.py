@@ -21,6 +21,12 @@ def test_split_is_the_measured_best(split, M, N, K, best):
     assert split(M, N, K, 148) == best
 
 
+@pytest.mark.parametrize("M,N,K,best", [(1, 2048, 2432, 8), (6, 2624, 1856, 4), (31, 4096, 704, 4), (31, 4680, 704, 2)])
+def test_split_leaves_clusters_their_sms(split, M, N, K, best):
+    """16 and 17 tiles in clusters of eight, 32 and 37 in clusters of four: behind the edge clusters would share SMs."""
+    assert split(M, N, K, 148) == best
+
+
 @pytest.mark.parametrize("sms", [0, 1, 16, 132, 148, 160])
 def test_split_never_exceeds_the_steps_of_k(split, sms):
     for M in (1, 8, 100, 128, 129, 2000):
