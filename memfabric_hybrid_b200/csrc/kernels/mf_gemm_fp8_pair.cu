@@ -682,7 +682,7 @@ template <int EPI> __global__ void __launch_bounds__(kPThreads, 1) k_grouped_fp8
             __threadfence();
             if (atomicAdd(g.done_count, 1u) + 1 == gridDim.x) {
                 *g.done_count = 0;
-                fence_sys();
+                fence_group(g.team);
                 for (uint32_t r = 0; r < g.team.world; r++)
                     asm volatile("st.relaxed.sys.global.u32 [%0], %1;" ::"l"(reinterpret_cast<uint32_t *>(peer_ptr(g.team, r, g.flag_off)) + g.team.rank), "r"(g.epoch)
                                  : "memory");

@@ -322,10 +322,11 @@ __device__ __forceinline__ void dispatch_preload(const DispatchArgs &a, uint4 &l
 // By the thread that has counted the last CTA of a grid: this rank's flag of the row at `flags` on every rank. A CTA's barrier orders its stores before its
 // counting thread, whose fence for this GPU hands them to the last one, whose fence hands all of them to the system (release is cumulative, whatever
 // the scope of the steps in front); the stores behind that fence need no order of their own. A fence for the system waits about 3 us here:
-// with one in every CTA and a release store per flag the low-latency pair of 128 tokens took 14.2 + 15.6 us, so 10.3 + 12.4.
+// with one in every CTA and a release store per flag the low-latency pair of 128 tokens took 14.2 + 15.6 us, so 10.3 + 12.4. One
+// rank's fence is for its GPU: a pass of the pair 66.9 -> 64.2.
 __device__ __forceinline__ void raise_flags(const Team &t, uint64_t flags, uint32_t me, uint32_t epoch)
 {
-    fence_sys();
+    fence_group(t);
     for (uint32_t r = 0; r < t.world; r++)
         asm volatile("st.relaxed.sys.global.u32 [%0], %1;" ::"l"(reinterpret_cast<uint32_t *>(peer_ptr(t, r, flags)) + me), "r"(epoch) : "memory");
 }
@@ -899,13 +900,13 @@ __global__ void __launch_bounds__(448) k_moe_ll_dispatch(LLDispatchArgs a)
 // nothing in front of its stores. What bounds it are the latencies that are left: routing and rows from memory, the stores' way to
 // memory, the counter of finished CTAs, the flag. The ranks need not take the same kernel: the exchange is the other one's.
 // Tokens of 7168, 8 of 32 experts, one rank, us, the other kernel / this one (the fences of finish_dispatch not counted): 1 token 16.3 / 11.0, 128 19.5 / 14.2,
-// 256 24.1 / 18.3. A pass of the pair with a stand-in expert, 128 tokens: 81 before this kernel and the present combine, 66.
+// 256 24.1 / 18.3. A pass of the pair with a stand-in expert, 128 tokens: 81 before this kernel and the present combine, 66 (64 with the fence of one rank).
 constexpr int kLLTokens = 4;        // tokens of a CTA
 constexpr int kLLEntries = 4096;    // entries in all: a CTA looks at every entry once for each of its own
 // ALONE: the dispatch of the pair dispatch / combine by a group of one rank, which has no counts to exchange: layout, tables and push in one launch that
 // waits for nobody, in place of k_moe_prepare and k_moe_dispatch_warp (with more ranks the CTAs would hold their SMs while they wait for the
-// peers' counts, see finish_dispatch). MoE layer, 32 experts of 7168 x 2048, us, two launches / one: 1 token 106 / 91, 16 260 / 244, 128 270 / 253, 256 282 / 267, 512
-// 317 / 309.
+// peers' counts, see finish_dispatch). Its end is all that the next kernel on the stream waits for: no flag, no count of CTAs, no k_moe_wait_all. MoE layer, 32 experts of 7168 x 2048, us, three launches / one: 1 token 106 / 84, 16 260 / 237, 128 270 / 245, 256 282 / 257, 512
+// 317 / 297.
 template <bool ALONE> __global__ void __launch_bounds__(448) k_moe_dispatch_few(LLDispatchArgs a)
 {
     const Team &t = a.d.team;
@@ -1070,9 +1071,8 @@ template <bool ALONE> __global__ void __launch_bounds__(448) k_moe_dispatch_few(
             __syncthreads();
         }
     }
-    const bool last = finish_dispatch(a.d, me, ALONE ? nullptr : a.epoch_dev);
+    if (!ALONE && finish_dispatch(a.d, me, a.epoch_dev)) ll_wait_rows(a, me);  // uniform over the CTA
     MF_PROF_STOP(PF_DISPATCH);
-    if (!ALONE && last) ll_wait_rows(a, me);  // uniform over the CTA
 }
 
 struct LLCombineArgs {
@@ -1229,8 +1229,8 @@ int mf_moe_dispatch(const DispatchArgs *a, int ctas, void *stream)
     return e == cudaSuccess ? 0 : (int)e;
 }
 
-// mf_moe_prepare and mf_moe_dispatch of one rank's few tokens in one launch; -3: more ranks or too many tokens, make the two calls. `ctas` as for
-// mf_moe_dispatch, whose completion counter it shares.
+// mf_moe_prepare, mf_moe_dispatch and mf_moe_wait_all of one rank's few tokens in one launch; -3: more ranks or too many tokens, make the three calls. `ctas` as
+// for mf_moe_dispatch, whose completion counter it leaves alone.
 int mf_moe_dispatch_alone(const DispatchArgs *d, int *tokens_per_expert, int *tokens_per_rank, uint8_t *is_token_in_rank, int *recv_per_expert,
                           int *row_off, int *src_off, int ctas, void *stream)
 {

@@ -81,6 +81,12 @@ __device__ __forceinline__ uint32_t ld_relaxed_sys(const uint32_t *p)
 // Orders this thread's (and, behind a CTA barrier, its CTA's) accesses for observers on every GPU: release and acquire, which is
 // all that a counter or a flag behind it needs. (__threadfence_system() is the sequentially consistent fence.)
 __device__ __forceinline__ void fence_sys() { asm volatile("fence.acq_rel.sys;" ::: "memory"); }
+// In front of flags that every rank's GPU reads. A group of one rank has them read by this GPU alone: its fence takes 0.7-1 us for 3.
+__device__ __forceinline__ void fence_group(const Team &t)
+{
+    if (t.world > 1) fence_sys();
+    else __threadfence();
+}
 
 __device__ __forceinline__ void report_timeout(const Team &t, uint32_t me, uint32_t where, uint32_t epoch)
 {

@@ -235,6 +235,7 @@ class MoEComm:
         self._done = torch.zeros(1, dtype=torch.int32, device=self.dev)
         self._push_done = torch.zeros(1, dtype=torch.int32, device=self.dev)  # finished CTAs of the down projection, zero between launches
         self._dispatches = 0
+        self._counted = 0   # of these, the calls whose kernel counts its CTAs in _done
         self._ll_done = torch.zeros(1, dtype=torch.int32, device=self.dev)
         self._ll_grid = None
         self._grid = sm_count(self.dev)
@@ -301,7 +302,7 @@ class MoEComm:
         epoch = self._epoch + 1   # counts once the exchange is launched: a refused call must not put this rank out of step
         w = topk_w.to(torch.float32).contiguous()
         a = DispatchArgsC(team, self.hp, self._shape(T), x.data_ptr(), idx.data_ptr(), w.data_ptr(), sidx.data_ptr(), put_off.data_ptr(),
-                          self._done.data_ptr(), epoch, self._dispatches + 1, status_word(self.dev).data_ptr(), 1 if self.raw_bf16 else 0,
+                          self._done.data_ptr(), epoch, self._counted + 1, status_word(self.dev).data_ptr(), 1 if self.raw_bf16 else 0,
                           smooth.data_ptr() if smooth is not None else None)
         rc = -3
         if small and self.world == 1:
@@ -311,6 +312,7 @@ class MoEComm:
             if rc != -3:
                 _ok(rc, "moe_dispatch_alone")
                 self._epoch = epoch
+                self._keep = (w, idx, smooth)
         if rc == -3:
             if small:
                 # layout and count exchange in one launch
@@ -323,9 +325,10 @@ class MoEComm:
             self._epoch = epoch
             # one CTA per SM on every call: the completion counter of the kernel counts CTAs
             _ok(_cu().mf_moe_dispatch(C.byref(a), self._grid, _s()), "moe_dispatch")
+            self._counted += 1
+            self._keep = (w, idx, smooth)
+            _ok(_cu().mf_moe_wait_all(C.byref(team), C.byref(self.hp), 0, self._epoch, status_word(self.dev).data_ptr(), _s()), "moe_wait")
         self._dispatches += 1
-        self._keep = (w, idx, smooth)
-        _ok(_cu().mf_moe_wait_all(C.byref(team), C.byref(self.hp), 0, self._epoch, status_word(self.dev).data_ptr(), _s()), "moe_wait")
         return DispatchState(T, idx, sidx, tpe, tpr, inr, rpe, row_off, put_off, src_off, self._epoch)
 
     def dispatch_cached(self, x: torch.Tensor, st: DispatchState, topk_w: torch.Tensor) -> DispatchState:
@@ -336,10 +339,11 @@ class MoEComm:
         import dataclasses
         self._epoch += 1
         self._dispatches += 1
+        self._counted += 1
         team = self.heap.team()
         w = topk_w.to(torch.float32).contiguous()   # the weights travel with the rows again
         a = DispatchArgsC(team, self.hp, self._shape(st.T), x.data_ptr(), st.topk_idx.data_ptr(), w.data_ptr(), st.send_idx.data_ptr(),
-                          st.put_off.data_ptr(), self._done.data_ptr(), self._epoch, self._dispatches, status_word(self.dev).data_ptr(),
+                          st.put_off.data_ptr(), self._done.data_ptr(), self._epoch, self._counted, status_word(self.dev).data_ptr(),
                           1 if self.raw_bf16 else 0, None)
         self._keep = (w, st.topk_idx, None)
         _ok(_cu().mf_moe_dispatch(C.byref(a), self._grid, _s()), "moe_dispatch")

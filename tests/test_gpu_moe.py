@@ -652,6 +652,39 @@ def test_low_latency_pair_around_its_tokens_per_cta():
     assert not bad and st == 0, (bad, st)
 
 
+def _mixed_rank(rank, world, url, sync):
+    import torch
+    from memfabric_hybrid_b200.ops import moe as M
+    from memfabric_hybrid_b200.ops.gemm import status_word
+    from memfabric_hybrid_b200.ops.heap import SymmetricHeap
+    H, E, K = 512, 8, 8
+    heap = SymmetricHeap(url, 1, 0, 0, 64 << 20)
+    comm = M.MoEComm(heap, 700, H, E, K, max_recv=700 * K)
+    g = torch.Generator("cuda").manual_seed(3)
+    fine = []
+    for step, T in enumerate((4, 4, 700, 64, 700, 1, 1)):
+        x = torch.randn(T, H, device="cuda", generator=g).to(torch.bfloat16)
+        w = torch.rand(T, K, device="cuda", generator=g)
+        if step in (1, 6):
+            st = comm.dispatch_cached(x, st, w)
+        else:
+            st = comm.dispatch(x, torch.rand(T, E, device="cuda", generator=g).argsort(1).to(torch.int32), w)
+        comm.combine_push(torch.ones(T * K, H, dtype=torch.bfloat16, device="cuda"), st)
+        want = w.to(torch.bfloat16).float().sum(1, keepdim=True).expand(T, H)   # of rows that were rounded to bf16 when they were pushed
+        fine.append(bool(((comm.combine(st).float() - want).abs() <= want * 2.0 ** -8).all()) and int(st.row_off[-1]) == T * K)
+    fine.append(int(status_word("cuda").item()) == 0 and heap.status()[0] == 0)
+    heap.close()
+    SymmetricHeap.shutdown()
+    return fine
+
+
+def test_dispatch_kernels_that_count_and_do_not_count_their_ctas_take_turns():
+    """One rank's few tokens leave the counter of finished CTAs and the flag alone; calls of the kernels that use both follow in any order."""
+    url = f"127.0.0.1:{free_port()}"
+    (fine,) = run_ranks(_mixed_rank, 1, (url,), timeout=300, with_barrier=True)
+    assert all(fine), fine
+
+
 def _refused_rank(rank, world, url, sync):
     import torch
     from memfabric_hybrid_b200.ops import moe as M
