@@ -652,6 +652,30 @@ def test_low_latency_pair_around_its_tokens_per_cta():
     assert not bad and st == 0, (bad, st)
 
 
+@pytest.mark.parametrize("T,K", [(1, 1), (127, 16), (341, 3), (1025, 1), (4099, 8)])
+@pytest.mark.parametrize("world,E", [(1, 32), (3, 96), (8, 1024), (16, 64)])
+def test_layout_of_tokens_cut_over_ctas(T, K, world, E):
+    """Positions in token order, counts per expert and per rank, and each token's ranks, whatever the outputs held before; ids outside of [0, E) count nowhere."""
+    from memfabric_hybrid_b200.ops import moe as M
+    g = torch.Generator().manual_seed(T + K)
+    idx = torch.randint(-3, E + 3, (T, K), generator=g, dtype=torch.int32)
+    tpe, tpr, sidx = (torch.full((n,), -7, dtype=torch.int32, device="cuda") for n in (E, world, T * K))
+    inr = torch.full((T, world), 9, dtype=torch.uint8, device="cuda")
+    d = idx.cuda()
+    for _ in range(2):
+        assert M._cu().mf_moe_layout(d.data_ptr(), T, K, E, world, tpe.data_ptr(), tpr.data_ptr(), sidx.data_ptr(), inr.data_ptr(),
+                                     torch.cuda.current_stream().cuda_stream) == 0
+    flat = idx.view(-1).long()
+    on = (flat >= 0) & (flat < E)
+    hot = torch.nn.functional.one_hot(torch.where(on, flat, E), E + 1)[:, :E]
+    before = (hot.cumsum(0) - hot)
+    assert torch.equal(tpe.cpu().long(), hot.sum(0))
+    assert torch.equal(sidx.cpu().long(), torch.where(on, before.gather(1, flat.clamp(0, E - 1)[:, None])[:, 0], 0))
+    ranks = hot.view(T, K, world, E // world).sum((1, 3)) > 0
+    assert torch.equal(inr.cpu().bool(), ranks) and int(inr.max()) <= 1
+    assert torch.equal(tpr.cpu().long(), ranks.sum(0))
+
+
 def _mixed_rank(rank, world, url, sync):
     import torch
     from memfabric_hybrid_b200.ops import moe as M
