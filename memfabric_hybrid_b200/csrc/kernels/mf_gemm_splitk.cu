@@ -25,8 +25,7 @@ namespace mfk {
 constexpr int kSkBN = 128;
 constexpr int kSkThreads = 192;              // warp 0 TMA, warp 1 MMA, warps 2..5 read the accumulator, all six reduce
 constexpr int kSkMaxSplit = 8;               // portable cluster size
-constexpr int kSkAtOnce = 8;                 // partial sums on their way to a thread at once
-static_assert(kSkMaxSplit <= kSkAtOnce, "one item's parts");
+constexpr int kSkAtOnce = 4;                 // partial sums on their way to a thread at once, from which on items follow one another
 constexpr int kSkStageArea = 100 * 1024;     // two CTAs per SM
 constexpr int kSkRowFloats = kSkBN + 4;      // 528-byte rows: eight lanes' 16-byte writes to eight rows hit all banks once
 constexpr int kSkMaxStages = kSkStageArea / (8 * KSPAN + kSkBN * KSPAN);  // A's box is at least 8 rows
@@ -63,13 +62,14 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 // What bounds it: the way from the neighbours' shared memory. Lanes read 16 bytes side by side, a CTA's own part does not leave the SM, and the reads
 // of several items are on their way at once. Before, a thread read 32 bytes with gaps, the own part the same way, one part after another: with a tile's
 // 32 rows in 4 CTAs 2.9 us from the last partial tile to the end, 1.7 so; 128 rows in 2 CTAs 5.6, 4.2; gate/up and down product (N, K = 7168, 8192 and
-// 8192, 3584) in a row, us before / so: 1 row 35.1 / 34.3, 32 rows 41.6 / 37.4, 64 46.1 / 41.5, 128 55.6 / 48.2, 256 60.8 / 57.9.
+// 8192, 3584) in a row, us before / so: 1 row 35.1 / 34.1, 32 rows 41.6 / 37.1, 64 46.1 / 39.7, 128 55.6 / 47.9, 256 60.8 / 57.4. With eight reads at once
+// 1 % slower (the code of a short kernel is fetched cold), with sixteen 6 %; with two as fast, but 64 x 8192 x 1024 6.6 for 6.2.
 template <int EPI, int S> __device__ __forceinline__ void add_up(const SplitArgs &g, uint32_t part0, __nv_bfloat16 *C, int rows, int nt, uint32_t rank, uint32_t split)
 {
     constexpr int kOutCols = EPI == 1 ? kSkBN / 2 : kSkBN;   // output columns of the tile
     constexpr int kVecs = kOutCols / 4;
     constexpr int H = EPI == 1 ? 2 : 1;
-    constexpr int P = S ? S : kSkAtOnce, U = kSkAtOnce / P;  // parts, items at once
+    constexpr int P = S ? S : kSkMaxSplit, U = kSkAtOnce / P > 0 ? kSkAtOnce / P : 1;  // parts, items at once
     const int n_out = EPI == 1 ? g.N / 2 : g.N;
     const bool vec_ok = (g.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(C) & 7) == 0;
     const int total = rows * kVecs, step = (int)(S ? S : split) * kSkThreads;
