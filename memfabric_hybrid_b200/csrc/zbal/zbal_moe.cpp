@@ -313,7 +313,7 @@ int32_t zbal_combine_normal(zbal_moe_t moe, const void *srcTokens, int64_t ld, c
     if (rc != Z_OK) return rc;
     MoeShape sh = c->sh;
     sh.T = (int)tokens;
-    return Launched(L->combineReduce(&c->comm->team, &c->hp, &sh, topkIndex, destTokens, (int)std::min<int64_t>(tokens, c->grid * 4), stream), "combine reduce");
+    return Launched(L->combineReduce(&c->comm->team, &c->hp, &sh, topkIndex, destTokens, c->grid * 4, stream), "combine reduce");
 }
 
 int32_t zbal_dispatch_low_latency(zbal_moe_t moe, const void *x, int64_t tokens, const int32_t *topkIndex, const float *topkWeights,
@@ -430,7 +430,7 @@ int32_t zbal_fused_deep_moe(zbal_moe_t moe, const void *x, int64_t tokens, const
     if (rc != Z_OK) return rc;
     MoeShape sh = c->sh;
     sh.T = (int)tokens;
-    return Launched(L->combineReduce(&c->comm->team, &c->hp, &sh, topkIndex, xOut, (int)std::min<int64_t>(tokens, c->grid * 4), stream), "combine reduce");
+    return Launched(L->combineReduce(&c->comm->team, &c->hp, &sh, topkIndex, xOut, c->grid * 4, stream), "combine reduce");
 }
 
 }  // extern "C"

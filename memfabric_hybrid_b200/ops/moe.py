@@ -397,7 +397,7 @@ class MoEComm:
         _ok(_cu().mf_moe_wait_all(C.byref(team), C.byref(self.hp), 1, st.epoch, status_word(self.dev).data_ptr(), _s()), "moe_wait")
         sh = self._shape(st.T)
         _ok(_cu().mf_moe_combine_reduce(C.byref(team), C.byref(self.hp), C.byref(sh), st.topk_idx.data_ptr(), out.data_ptr(),
-                                        min(st.T, self._grid * 4), _s()), "moe_combine_reduce")
+                                        self._grid * 4, _s()), "moe_combine_reduce")
         if self._canary:
             torch.cuda.synchronize()
             self.check_canaries()
