@@ -123,7 +123,9 @@ MfCollArgs BaseArgs(Comm &c, const void *in, void *out, uint64_t n, float scale,
     return a;
 }
 
-constexpr uint64_t kOneShotMax = 256u << 10;
+// One shot has a handshake less than two and moves more bytes: the line and its reasons are those of ops/collectives.py.
+constexpr uint64_t kOneShotMax = 256u << 10, kOneShotReads = 32u << 20;
+bool OneShot(const Comm &c, uint64_t bytes) { return bytes <= kOneShotMax || (uint64_t)c.size * c.size * bytes <= kOneShotReads; }
 
 // Direct mode: a buffer that lies inside this rank's slice of the symmetric heap (a tensor from the
 // symmetric allocator) is reachable by the peers, so the kernels skip the staging copies. Small payloads
@@ -170,7 +172,7 @@ int AllReduce(Comm &c, const void *in, void *out, uint64_t n, int kdt, int odt, 
     while (done < n) {
         const uint64_t cnt = std::min(piece, n - done);
         MfCollArgs a = BaseArgs(c, static_cast<const char *>(in) + done * es, static_cast<char *>(out) + done * oes, cnt, scale, op, c.maxCtas,
-                                cnt * es <= kOneShotMax ? 0 : 1);
+                                OneShot(c, cnt * es) ? 0 : 1);
         int rc = Launched(L->coll(0, kdt, odt, &a, c.Ctas(cnt * es), 512, stream), "all_reduce");
         if (rc != Z_OK) return rc;
         done += cnt;

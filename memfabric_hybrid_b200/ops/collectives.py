@@ -23,7 +23,12 @@ from .heap import TeamC, _HeapBase, current_stream_ptr as _stream
 
 DT = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2, torch.int32: 3}
 OPS = {"sum": 0, "max": 1, "min": 2, "prod": 3}
-ONE_SHOT_MAX = 256 << 10
+# One shot (every rank reads all of every rank's staged copy) has a handshake less than two shots (4-5 us) and moves (W - 1) n bytes per rank for 2 (W - 1) / W n.
+# Emulated ranks on one GPU, all-reduce, us, one shot / two: 2 ranks 400 KiB 8.0 / 12.5, 8 MiB 17.2 / 20.4; 4 ranks 512 KiB 9.0 / 14.3, 2 MiB 14.1 / 16.6, 4 MiB 21.2 / 20.7;
+# 8 ranks 400 KiB 12.4 / 16.6, 700 KiB 15.1 / 17.2, 1 MiB 19.2 / 18.0 (fp32 a little later): even at W * W * n of 56 MiB. Over NVLink the further bytes take as long as the
+# handshake (by their count, 770 GB/s) at 2 MiB with 4 ranks and 0.6 MiB with 8: the line is drawn in front of both.
+ONE_SHOT_MAX = 256 << 10      # always
+ONE_SHOT_READS = 32 << 20     # above it: up to so many bytes read by all ranks
 DIRECT_MIN = 256 << 10  # above this, buffers that live in the heap are used in place (no staging copies)
 
 
@@ -220,7 +225,7 @@ class Communicator:
         done = 0
         while done < n:
             cnt = min(piece, n - done)
-            use = a if a is not None else (0 if cnt * es <= ONE_SHOT_MAX else 1)
+            use = a if a is not None else (0 if cnt * es <= ONE_SHOT_MAX or self.world * self.world * cnt * es <= ONE_SHOT_READS else 1)
             self._launch(0, x, out, cnt, cnt * es, "all_reduce", scale, op, self.max_ctas, use, 0, xl, ol, (done * es, done * oes))
             done += cnt
         return out

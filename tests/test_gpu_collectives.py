@@ -65,6 +65,24 @@ def test_all_reduce_fused_cast_and_ops(comms, world):
     assert torch.equal(c.all_reduce(xi, op="max", algo="twoshot")[world - 1], xi.max(0).values)
 
 
+@pytest.mark.parametrize("world,m", [(2, 8 << 20), (4, 2 << 20), (8, 512 << 10)])
+def test_all_reduce_on_both_sides_of_one_shot(world, m):
+    """The largest calls of one shot and the smallest of two, in one buffer and in pieces of the staging area: the same sum in rank order, rounded once."""
+    from memfabric_hybrid_b200.ops.heap import EmulatedHeap
+    from memfabric_hybrid_b200.ops.collectives import Communicator
+    for stage in (m + 4096, (m // 3 + 4095) // 4096 * 4096):
+        heap = EmulatedHeap(world, (1 << 20) + 4 * stage + 4096)
+        c = Communicator(heap, stage_bytes=stage)
+        for n in (m // 2 - 1, m // 2, m // 2 + 1):
+            x = torch.randn(world, n, device="cuda", generator=torch.Generator("cuda").manual_seed(n)).to(torch.bfloat16)
+            acc = x[0].float()
+            for r in range(1, world):
+                acc = acc + x[r].float()
+            assert torch.equal(c.all_reduce(x), acc.to(torch.bfloat16).expand(world, n)), (stage, n)
+        torch.cuda.synchronize()
+        assert heap.status()[0] == 0
+
+
 @pytest.mark.parametrize("world", [2, 3, 8])
 def test_small_all_reduce_in_packets(world):
     """Sizes that change from call to call (what an earlier call left in the packet area must not count), odd ones, inputs off eight bytes, in place, an output in
