@@ -340,12 +340,12 @@ uint64_t SpanCutter::Split(uint64_t len, uint32_t at, bool rest)
     return (uint64_t)n;
 }
 
-// Shares for a batch, 0: none. Up to a chunk of the smallest size per CTA, each chunk gets a CTA of its own (100 pieces of up to 16 KiB: one
+// Shares for a batch, 0: none (the pieces are dealt out one by one; on a device without the copy unit always). Up to a chunk of the smallest size per CTA, each chunk gets a CTA of its own (100 pieces of up to 16 KiB: one
 // latency for all of them); the chunks are at least as many as the runs and as the bytes would fill.
 static uint32_t SpansFor(const DeviceBackend *dev, const BatchShape &b)
 {
     const uint32_t n = dev->CopySpanCount();
-    if ((b.alignMask & 15) == 0 || std::max(b.runs, b.bytes / kMinCopyChunk) <= n) return 0;
+    if (n == 0 || (b.alignMask & 15) == 0 || std::max(b.runs, b.bytes / kMinCopyChunk) <= n) return 0;
     return b.bytes / n < (32u << 10) ? (n + 1) / 2 : n;  // 1500 pieces of up to 16 KiB: the host takes 0.7 us less, the kernel, which it hides, 1.6 more
 }
 

@@ -156,7 +156,12 @@ public:
             memmove(reinterpret_cast<void *>(items[i].dst), reinterpret_cast<const void *>(items[i].src), items[i].len);
         return OK;
     }
-    uint32_t CopySpanCount() const override { return 12; }
+    int ConfigureBulkCopy(int pipes, int, int) override  // as on a GPU: without the copy unit there is no launch by shares
+    {
+        spans_ = pipes > 0 ? 12 : 0;
+        return OK;
+    }
+    uint32_t CopySpanCount() const override { return spans_; }
     int LaunchSpanCopy(const CopyItem *items, const CopySpans &spans, void *s) override
     {
         for (uint32_t i = 0; i < spans.n; i++) {
@@ -206,6 +211,7 @@ private:
         return sign ? -v : v;
     }
     int dev_ = 0;
+    uint32_t spans_ = 12;
     DeviceCaps caps_;
     std::mutex mu_;
     std::map<uint64_t, uint64_t> allocs_;

@@ -439,6 +439,26 @@ uint32_t mf_t_copy_shares(const uint64_t *len, uint32_t n, uint32_t spans, uint3
     return w;
 }
 
+// A prepared batch on the fake device, which launches by shares or not: laid out, launched and released. -> code of the first step that failed.
+int mf_t_prepared_copy(const uint64_t *src, const uint64_t *dst, const uint64_t *len, uint32_t n, int shares)
+{
+    using namespace mf::hybm;
+    std::unique_ptr<DeviceBackend> dev(CreateFakeBackend());
+    dev->ConfigureBulkCopy(shares, 0, 0);
+    ComposeDataOp op(dev.get(), 0);
+    std::vector<ResolvedCopy> items(n);
+    for (uint32_t i = 0; i < n; i++) {
+        items[i].src = {src[i], EP_DEVICE, 0};
+        items[i].dst = {dst[i], EP_DEVICE, 0};
+        items[i].len = len[i];
+    }
+    PreparedBatch b;
+    int rc = op.Prepare(items, b);
+    if (rc == mf::OK) rc = op.LaunchPrepared(b, nullptr);
+    op.ReleasePrepared(b);
+    return rc;
+}
+
 // ---- fault points -------------------------------------------------------------------------------------
 // Runs the periodic TLS certificate check now; -> the smallest number of days left over the live contexts.
 int mf_t_tls_check_now(void) { return mf::net::TlsCheckAllNow(); }

@@ -73,6 +73,7 @@ def lib():
     s(l, "mf_t_ex_import", i32, vp, cp, u32, i32)
     s(l, "mf_t_ex_mapped_bytes", u64, vp, u32)
     s(l, "mf_t_copy_shares", u32, vp, u32, u32, vp, vp, u32)
+    s(l, "mf_t_prepared_copy", i32, vp, vp, vp, u32, i32)
     s(l, "mf_t_backend_set_reachable", None, cp, i32)
     s(l, "mf_t_backend_reset", None, cp)
     s(l, "mf_t_group_new", vp, vp, u32, u32, u64, i32, CHANGE_CB)

@@ -1,6 +1,7 @@
 """The HBM-pool code path (VMM segment, fd channel, batch descriptors, partial results) on a machine
 without a GPU, against the fake device backend whose "device memory" is memfd-backed host memory."""
 import numpy as np
+import pytest
 
 from conftest import free_port
 from mp_util import run_ranks
@@ -319,7 +320,7 @@ def test_shares_of_a_copy_batch():
             assert weight.max() <= 2 * mean + 4 * cost, (spans, weight.max(), mean)
 
 
-def _shares_rank(rank, world, url):
+def _shares_rank(rank, world, url, copy_unit=True):
     import memfabric_hybrid as mf
     from memfabric_hybrid import bm
     assert mf.initialize() == 0
@@ -329,6 +330,9 @@ def _shares_rank(rank, world, url):
     assert bm.initialize(url, 1, 0, cfg) == 0, mf.get_last_err_msg()
     h = bm.create2(id=7, local_dram_size=0, max_dram_size=0, local_hbm_size=32 * MiB, max_hbm_size=32 * MiB)
     assert h.join() == 0, mf.get_last_err_msg()
+    if not copy_unit:
+        from memfabric_hybrid_b200 import _native as N
+        assert N.lib().mf_xcopy_bulk_config(0, 0, 0) == 0
     base = h.peer_rank_ptr(0, bm.BmMemType.DEVICE)
     r, ok = np.random.default_rng(1), True
     # few and many pieces, neighbours that merge, and (ring of 1 MiB) batches that reach the ring's end in the middle
@@ -355,3 +359,33 @@ def _shares_rank(rank, world, url):
 def test_batches_in_shares_against_the_pieces_one_by_one():
     url = f"tcp://127.0.0.1:{free_port()}"
     assert run_ranks(_shares_rank, 1, (url,), timeout=120, env={"MF_DEVICE_BACKEND": "fake", "MF_XCOPY_RING_MB": "1"}) == [True]
+
+
+def test_unaligned_batches_of_a_device_without_a_launch_by_shares():
+    """The copy unit switched off: the pieces are dealt out one by one."""
+    url = f"tcp://127.0.0.1:{free_port()}"
+    assert run_ranks(_shares_rank, 1, (url, False), timeout=60, env={"MF_DEVICE_BACKEND": "fake", "MF_XCOPY_RING_MB": "1"}) == [True]
+
+
+def _prepared_rank(rank, world, shares):
+    import hooks
+    r = np.random.default_rng(2)
+    for n, top in ((1, 100), (1, 3 << 20), (40, 60000), (3000, 300)):
+        size = r.integers(1, top, n).astype(np.uint64)
+        off = np.concatenate(([0], np.cumsum(size + r.integers(0, 2, n).astype(np.uint64))[:-1])).astype(np.uint64) + np.uint64(1)
+        src = r.integers(0, 256, int(off[-1] + size[-1]) + 8, dtype=np.uint8)
+        got = np.full_like(src, 9)
+        want = got.copy()
+        s, d = off + np.uint64(src.ctypes.data), off + np.uint64(got.ctypes.data)
+        if hooks.lib().mf_t_prepared_copy(s.ctypes.data, d.ctypes.data, size.ctypes.data, n, shares) != 0:
+            return False
+        for o, k in zip(off.tolist(), size.tolist()):
+            want[o:o + k] = src[o:o + k]
+        if not np.array_equal(got, want):
+            return False
+    return True
+
+
+@pytest.mark.parametrize("shares", [0, 1])
+def test_prepared_unaligned_batches_with_and_without_shares(shares):
+    assert run_ranks(_prepared_rank, 1, (shares,), timeout=60) == [True]

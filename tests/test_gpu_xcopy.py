@@ -315,6 +315,12 @@ def test_unaligned_batches_in_shares(debug):
     assert run_ranks(_share_rank, 1, (url,), timeout=240, env={"MF_XCOPY_DEBUG": debug}) == [[]]
 
 
+def test_unaligned_batches_without_the_copy_unit():
+    """MF_XCOPY_BULK=0: the same batches, direct and prepared, through the register copy kernel."""
+    url = f"tcp://127.0.0.1:{free_port()}"
+    assert run_ranks(_share_rank, 1, (url,), timeout=240, env={"MF_XCOPY_BULK": "0"}) == [[]]
+
+
 def test_pieces_at_every_pair_of_byte_offsets():
     url = f"tcp://127.0.0.1:{free_port()}"
     assert run_ranks(_shifted_rank, 1, (url,), timeout=180) == [True]
