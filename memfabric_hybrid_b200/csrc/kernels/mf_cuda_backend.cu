@@ -685,3 +685,21 @@ extern "C" int mf_xcopy_debug_probe(const uint64_t *triples, uint32_t n, uint64_
     cudaFreeHost(mem);
     return rc;
 }
+
+// Test aid: lets a wait of mf_xcopy_span_kernel's loader or of its storers run out (limits in microseconds, at most a second) on the default stream. Returns the
+// status that is reported, or a negative number when the launch could not be made or a role has not left.
+extern "C" int mf_xcopy_wait_probe(uint32_t loader_us, uint32_t storer_us)
+{
+    if (loader_us > 1000000 || storer_us > 1000000) return -1;
+    uint32_t *status = nullptr;
+    if (cudaHostAlloc(reinterpret_cast<void **>(&status), 64, cudaHostAllocMapped) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return -2;
+    }
+    memset(status, 0, 64);
+    mfk::mf_xcopy_wait_probe_kernel<<<1, 64>>>(status, loader_us * 1000ull, storer_us * 1000ull);
+    int rc = cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess ? -4 : 0;
+    if (rc == 0) rc = status[1] == 2 ? (int)status[0] : -5;
+    cudaFreeHost(status);
+    return rc;
+}

@@ -281,7 +281,8 @@ __device__ __forceinline__ ShiftPlan span_plan(uint64_t src, uint64_t dst, uint6
     return p;
 }
 
-__device__ __forceinline__ bool xc_wait(uint64_t *bar, uint32_t parity, volatile int *quit)
+enum XcWait : int { kXcArrived, kXcToldToQuit, kXcRanOut };
+__device__ __forceinline__ XcWait xc_wait(uint64_t *bar, uint32_t parity, volatile int *quit, uint64_t limit_ns)
 {
     uint64_t t0 = 0;
     for (uint32_t spin = 0;; spin++) {
@@ -293,15 +294,27 @@ __device__ __forceinline__ bool xc_wait(uint64_t *bar, uint32_t parity, volatile
             : "=r"(ok)
             : "r"(xc_smem_u32(bar)), "r"(parity)
             : "memory");
-        if (ok) return true;
+        if (ok) return kXcArrived;
         if ((spin & 255u) == 255u) {  // time limit, not an iteration count: a try_wait may suspend for a while
-            if (quit != nullptr && *quit) return false;
+            if (quit != nullptr && *quit) return kXcToldToQuit;
             uint64_t now;
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
             if (t0 == 0) t0 = now;
-            else if (now - t0 > kBulkWaitNs) return false;
+            else if (now - t0 > limit_ns) return kXcRanOut;
         }
     }
+}
+// The wait of a role whose CTA goes as soon as one of its waits runs out. Loader and storers wait for the same stage with the same limit, so either may be
+// the first: whoever runs out reports it, before the others learn of it.
+constexpr uint32_t kSpanLoadMissing = 0x702, kSpanStageMissing = 0x703;
+__device__ __forceinline__ bool span_wait(uint64_t *bar, uint32_t parity, volatile int *quit, uint32_t *status, uint32_t code, uint64_t limit_ns = kBulkWaitNs)
+{
+    const XcWait w = xc_wait(bar, parity, quit, limit_ns);
+    if (w == kXcRanOut) {
+        *reinterpret_cast<volatile uint32_t *>(status) = code;
+        *quit = 1;
+    }
+    return w == kXcArrived;
 }
 
 template <int Q> __device__ __forceinline__ void span_cut(const uint4 *g, uint4 *d, uint32_t vecs, uint32_t bits)
@@ -362,10 +375,7 @@ __global__ void __launch_bounds__(kSpanThreads, 2) mf_xcopy_span_kernel(const Co
                 const ShiftPlan p = span_plan(src, list[3 * l + 1], list[3 * l + 2]);
                 for (uint64_t v = 0; v < p.vecs; v += kSpanVecs) {
                     const uint32_t bytes = ((uint32_t)min((uint64_t)kSpanVecs, p.vecs - v) + (p.shift != 0 ? 1 : 0)) * 16;
-                    if (!xc_wait(&empty[slot], phase ^ 1, quit)) {
-                        *quit = 1;
-                        break;
-                    }
+                    if (!span_wait(&empty[slot], phase ^ 1, quit, status, kSpanStageMissing)) break;
                     const uint32_t bar = xc_smem_u32(&full[slot]);
                     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
                     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
@@ -410,11 +420,7 @@ __global__ void __launch_bounds__(kSpanThreads, 2) mf_xcopy_span_kernel(const Co
                 uint4 *d = reinterpret_cast<uint4 *>(dst + p.head);
                 const uint32_t bits = (p.shift & 3) * 8;
                 for (uint64_t v = 0; v < p.vecs; v += kSpanVecs) {
-                    if (!xc_wait(&full[slot], phase, quit)) {
-                        if (!*quit) *reinterpret_cast<volatile uint32_t *>(status) = 0x702u;
-                        *quit = 1;
-                        break;
-                    }
+                    if (!span_wait(&full[slot], phase, quit, status, kSpanLoadMissing)) break;
                     const uint4 *g = reinterpret_cast<const uint4 *>(xc_smem + slot * kSpanStageBytes);
                     const uint32_t m = (uint32_t)min((uint64_t)kSpanVecs, p.vecs - v);
                     if (p.shift == 0) {
@@ -443,8 +449,27 @@ __global__ void __launch_bounds__(kSpanThreads, 2) mf_xcopy_span_kernel(const Co
     if (*quit && warp == kSpanConsumers && lane == 0)
         for (int s = 0; s < kSpanStages; s++) {
             const uint32_t done = slot > (uint32_t)s ? phase : phase ^ 1;  // parity of the stage's last load
-            xc_wait(&full[s], done, nullptr);
+            xc_wait(&full[s], done, nullptr, kBulkWaitNs);
         }
+}
+
+// The two roles on stages of their own that nothing ever fills or frees, each with a limit of its own: word 0 of `status` is what is reported, word 1 counts
+// the roles that have left.
+__global__ void __launch_bounds__(64) mf_xcopy_wait_probe_kernel(uint32_t *status, uint64_t loader_ns, uint64_t storer_ns)
+{
+    __shared__ __align__(8) uint64_t full, empty;
+    __shared__ int quit_sh;
+    if (threadIdx.x == 0) {
+        quit_sh = 0;
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(xc_smem_u32(&full)));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(xc_smem_u32(&empty)));
+    }
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) {
+        const bool loader = threadIdx.x == 0;
+        if (!span_wait(loader ? &empty : &full, 0, &quit_sh, status, loader ? kSpanStageMissing : kSpanLoadMissing, loader ? loader_ns : storer_ns))
+            atomicAdd_system(status + 1, 1u);
+    }
 }
 
 // One WARP per (item, unit); a CTA of 8 warps walks the units of its item. The unit is read once when it fits in

@@ -321,6 +321,17 @@ def test_unaligned_batches_without_the_copy_unit():
     assert run_ranks(_share_rank, 1, (url,), timeout=240, env={"MF_XCOPY_BULK": "0"}) == [[]]
 
 
+@pytest.mark.parametrize("loader_us,storer_us,code", [(500, 500_000, 0x703), (500_000, 500, 0x702)], ids=["loader_first", "storers_first"])
+def test_a_wait_of_the_span_kernel_that_runs_out_is_reported(loader_us, storer_us, code):
+    """Whichever role gives up first: the status is set before the other one, which then leaves without a word, is told."""
+    import ctypes as C
+    from memfabric_hybrid_b200 import _native as N
+    cu = N.cuda()
+    cu.mf_xcopy_wait_probe.restype = C.c_int
+    cu.mf_xcopy_wait_probe.argtypes = [C.c_uint32, C.c_uint32]
+    assert cu.mf_xcopy_wait_probe(loader_us, storer_us) == code
+
+
 def test_pieces_at_every_pair_of_byte_offsets():
     url = f"tcp://127.0.0.1:{free_port()}"
     assert run_ranks(_shifted_rank, 1, (url,), timeout=180) == [True]
