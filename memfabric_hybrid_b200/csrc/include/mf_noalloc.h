@@ -23,8 +23,8 @@
  *     numbered, so they never need clearing); two calls that overlap on the GPU, from different streams
  *     or threads, race on it: serialise them;
  *   - it calls no cudaMalloc, cudaFree or allocating library routine;
- *   - every wait inside the kernel is bounded. A wait that runs out makes the kernel return without
- *     writing `out`; the launching call has long returned MF_NOALLOC_OK by then, so after synchronising
+ *   - every wait inside the kernel is bounded. A wait that runs out makes the kernel return with `out`
+ *     not or only partly written; the launching call has long returned MF_NOALLOC_OK by then, so after synchronising
  *     the stream a careful caller asks mf_noalloc_status() whether that happened.
  */
 #ifndef MF_B200_NOALLOC_H

@@ -106,3 +106,23 @@ def test_no_alloc_rejects_oversize_and_bad_arguments():
     assert fn(None, x.data_ptr(), 2, 16, 2, 0, 1.0, None) == -1
     assert lib.mf_noalloc_status(None, 0) == -1
     assert b"bounded wait" in lib.mf_noalloc_strerror(-5)
+
+
+@pytest.mark.parametrize("world,n", [(8, 2049), (8, 16_384), (8, 38_912), (8, 38_913), (3, 1021), (2, 4096), (1, 5000)])
+def test_no_alloc_calls_in_packets_of_several_ctas(world, n):
+    """Up to about 76 KiB the call goes in packets, a CTA of a rank per 4 KiB: the fp32 sum in rank order, rounded once, also in place."""
+    lib, fn = _sym()
+    stream = torch.cuda.current_stream().cuda_stream
+    x = torch.randn(world, n, device="cuda", generator=torch.Generator("cuda").manual_seed(n)).to(torch.bfloat16)
+    acc = x[0].float()
+    for r in range(1, world):
+        acc = acc + x[r].float()
+    want = acc.to(torch.bfloat16).expand(world, n)
+    got = torch.empty_like(x)
+    for _ in range(3):
+        assert fn(x.data_ptr(), got.data_ptr(), world, n, 0, 0, 1.0, stream) == 0
+        assert torch.equal(got, want)
+        got.zero_()
+    assert fn(x.data_ptr(), x.data_ptr(), world, n, 0, 0, 1.0, stream) == 0
+    assert torch.equal(x, want)
+    assert _status(lib) == (0, [0, 0, 0, 0])
