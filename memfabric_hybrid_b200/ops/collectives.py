@@ -166,9 +166,9 @@ class Communicator:
         return t.data_ptr(), 0, t.numel()
 
     def _launch(self, kind: int, x, out, n: int, nbytes: int, what: str, scale=1.0, op="sum", root=0, algo=0, zero_copy=0, x_local=None, o_local=None,
-                skip=(0, 0), dtypes=None) -> None:
+                skip=(0, 0), dtypes=(0, 0)) -> None:
         """One launch of the collective ``kind`` (see ``mf_coll_launch``) with the next epoch and staging buffers. ``skip``: bytes of the input and of
-        the output that earlier launches of the call have done."""
+        the output that earlier launches of the call have done. ``dtypes``: codes of the input's and the output's values."""
         xin, xs, _ = x_local or self._local(x)
         xo, os_, _ = o_local or self._local(out)
         self._epoch += 1
@@ -180,8 +180,7 @@ class Communicator:
             block = buf, C.byref(CollArgsC.from_buffer(buf))
         _COLL_ARGS.pack_into(block[0], 0, h.base, h.stride, h.mc_base, h.rank, h.world, 1 if h.emu else 0, h.spin_limit, xin + skip[0], xo + skip[1], xs, os_, n, a, b,
                              scale, OPS[op], self._epoch & 0xFFFFFFFF, zero_copy, root, algo, 0)
-        dt = dtypes or (DT[x.dtype], DT[out.dtype])
-        rc = _cu().mf_coll_launch(kind, dt[0], dt[1], block[1], self._ctas(nbytes), 512, _stream())
+        rc = _cu().mf_coll_launch(kind, dtypes[0], dtypes[1], block[1], self._ctas(nbytes), 512, _stream())
         self._block = block
         if rc != 0:
             _check(rc, what)
@@ -210,14 +209,16 @@ class Communicator:
         n = xl[2]
         if out is None:
             out = torch.empty_like(x) if od is x.dtype and x.dim() == (2 if self.heap.emu else 1) else self._empty_like(x, n, od)
-        es = x.element_size()
+        es, oes = x.element_size(), out.element_size()
+        if oes < od.itemsize:
+            od = out.dtype   # values of `od` would not fit
+        dt = DT[x.dtype], DT[od]   # `out` may be of another type of the same size: it receives the bits
         if algo in (None, "direct") and n * es > DIRECT_MIN and self._in_heap(x) and self._in_heap(out):
             # with a multicast alias of the heap the switch does the adding (sum of one floating type, no cast)
             mc = op == "sum" and od == x.dtype and x.dtype != torch.int32 and self._multicast("all_reduce", n * es)
-            self._launch(0, x, out, n, n * es, "all_reduce (direct)", scale, op, 0, 1, 3 if mc else 2, xl)
+            self._launch(0, x, out, n, n * es, "all_reduce (direct)", scale, op, 0, 1, 3 if mc else 2, xl, dtypes=dt)
             return out
         assert algo != "direct", "direct mode needs input and output inside the symmetric heap"
-        oes = out.element_size()
         ol = self._local(out)
         piece = self.stage_bytes // max(es, oes)
         piece -= piece % (8 * self.world)
@@ -226,7 +227,7 @@ class Communicator:
         while done < n:
             cnt = min(piece, n - done)
             use = a if a is not None else (0 if cnt * es <= ONE_SHOT_MAX or self.world * self.world * cnt * es <= ONE_SHOT_READS else 1)
-            self._launch(0, x, out, cnt, cnt * es, "all_reduce", scale, op, self.max_ctas, use, 0, xl, ol, (done * es, done * oes))
+            self._launch(0, x, out, cnt, cnt * es, "all_reduce", scale, op, self.max_ctas, use, 0, xl, ol, (done * es, done * oes), dt)
             done += cnt
         return out
 

@@ -65,6 +65,28 @@ def test_all_reduce_fused_cast_and_ops(comms, world):
     assert torch.equal(c.all_reduce(xi, op="max", algo="twoshot")[world - 1], xi.max(0).values)
 
 
+@pytest.mark.parametrize("n", [100, 200_000])
+def test_all_reduce_into_a_given_output(comms, n):
+    """What is stored are values of out_dtype, or of the input's type: an output of another type of that size receives their bits. Where they would not fit the output's
+    elements, values of its own type."""
+    c, world = comms[4], 4
+    x = torch.randn(world, n, device="cuda", generator=torch.Generator("cuda").manual_seed(n)).to(torch.bfloat16)
+    bits = torch.zeros(world, n, dtype=torch.int16, device="cuda")
+    assert c.all_reduce(x, out=bits) is bits
+    want = c.all_reduce(x)
+    assert torch.equal(bits.view(torch.bfloat16), want)
+    y = x.float()
+    words = torch.zeros(world, n, dtype=torch.int32, device="cuda")
+    assert torch.equal(c.all_reduce(y, out=words).view(torch.float32), c.all_reduce(y))
+    assert torch.equal(c.all_reduce(y, out=torch.empty_like(x)), want)   # the same sums, rounded once
+    wide = torch.zeros(world, n, dtype=torch.float32, device="cuda")
+    c.all_reduce(y, out=wide, out_dtype=torch.bfloat16)
+    got = wide.view(torch.bfloat16)   # rows of the output are 2 n values apart
+    assert torch.equal(got[:, :n], want) and not bool(got[:, n:].any())
+    torch.cuda.synchronize()
+    assert c.heap.status()[0] == 0
+
+
 @pytest.mark.parametrize("world,m", [(2, 8 << 20), (4, 2 << 20), (8, 512 << 10)])
 def test_all_reduce_on_both_sides_of_one_shot(world, m):
     """The largest calls of one shot and the smallest of two, in one buffer and in pieces of the staging area: the same sum in rank order, rounded once."""
