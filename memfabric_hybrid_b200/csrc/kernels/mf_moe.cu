@@ -750,6 +750,7 @@ struct CombinePushArgs {
     const __nv_bfloat16 *y;
     int64_t ldy;
     const int *rows_dev;
+    int max_rows;  // rows of the receive buffers: a dispatch that drops rows for want of room still counts them
     int H, K, weighted;
 };
 
@@ -757,7 +758,7 @@ __device__ __forceinline__ void combine_push_body(const CombinePushArgs &a)
 {
     const Team &t = a.team;
     const uint32_t me = team_rank(t);
-    const int rows = *a.rows_dev;
+    const int rows = min(*a.rows_dev, a.max_rows);
     const int vecs = a.H / 8;
     const int4 *info = reinterpret_cast<const int4 *>(peer_ptr(t, me, a.hp.recv_info));
     // A warp takes a piece of a row, at most eight 16-byte loads per lane, all in flight before the first store: at decode sizes the push is bound by
@@ -1295,11 +1296,11 @@ int mf_moe_combine_reduce(const Team *team, const MoeHeap *hp, const MoeShape *s
     return e == cudaSuccess ? 0 : (int)e;
 }
 
-int mf_moe_combine_push(const Team *team, const MoeHeap *hp, const void *y, int64_t ldy, const int *rows_dev, int H, int K, int weighted,
+int mf_moe_combine_push(const Team *team, const MoeHeap *hp, const void *y, int64_t ldy, const int *rows_dev, int max_rows, int H, int K, int weighted,
                         int ctas, void *stream)
 {
     if (team == nullptr || hp == nullptr || team->emu || H % 8 != 0 || ctas <= 0) return -1;
-    CombinePushArgs a{*team, *hp, static_cast<const __nv_bfloat16 *>(y), ldy, rows_dev, H, K, weighted};
+    CombinePushArgs a{*team, *hp, static_cast<const __nv_bfloat16 *>(y), ldy, rows_dev, max_rows, H, K, weighted};
     k_moe_combine_push<<<ctas, 256, 0, (cudaStream_t)stream>>>(a);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : (int)e;
@@ -1333,7 +1334,7 @@ int mf_moe_ll_combine(const Team *team, const MoeHeap *hp, const MoeShape *sh, c
                       int *status, int ctas, void *stream)
 {
     if (team == nullptr || hp == nullptr || sh == nullptr || team->emu || sh->H % 8 != 0 || ctas <= 0 || done_count == nullptr) return -1;
-    LLCombineArgs a{{*team, *hp, static_cast<const __nv_bfloat16 *>(y), ldy, rows_dev, sh->H, sh->K, weighted}, *sh, topk_idx,
+    LLCombineArgs a{{*team, *hp, static_cast<const __nv_bfloat16 *>(y), ldy, rows_dev, sh->max_recv, sh->H, sh->K, weighted}, *sh, topk_idx,
                     static_cast<__nv_bfloat16 *>(out), epoch, status, topk_w, epoch_dev, done_count};
     void *params[] = {&a};
     cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k_moe_ll_combine), dim3(ctas), dim3(one_per_sm(ctas) ? 512 : 256), params, 0,

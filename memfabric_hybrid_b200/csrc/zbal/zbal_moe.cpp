@@ -49,7 +49,7 @@ struct MoeLaunchers {
     int (*waitAll)(const MfTeam *, const MoeHeap *, int, uint32_t, int *, void *) = nullptr;
     int (*signalAll)(const MfTeam *, const MoeHeap *, int, uint32_t, void *) = nullptr;
     int (*combineReduce)(const MfTeam *, const MoeHeap *, const MoeShape *, const int *, void *, int, void *) = nullptr;
-    int (*combinePush)(const MfTeam *, const MoeHeap *, const void *, int64_t, const int *, int, int, int, int, void *) = nullptr;
+    int (*combinePush)(const MfTeam *, const MoeHeap *, const void *, int64_t, const int *, int, int, int, int, int, void *) = nullptr;
     int (*llDispatch)(const DispatchArgs *, int *, int *, int *, int *, uint32_t *, int, void *) = nullptr;
     int (*llCombine)(const MfTeam *, const MoeHeap *, const MoeShape *, const void *, int64_t, const int *, int, const int *, const float *,
                      void *, uint32_t, const uint32_t *, uint32_t *, int *, int, void *) = nullptr;
@@ -307,7 +307,7 @@ int32_t zbal_combine_normal(zbal_moe_t moe, const void *srcTokens, int64_t ld, c
     if (!srcTokens || !rowsDev || !topkIndex || !destTokens || tokens <= 0 || tokens > c->sh.T) return MF_FAIL(Z_INVALID_PARAM, "combine: NULL tensor or bad token count");
     std::lock_guard<std::mutex> g(c->mu);
     const MoeLaunchers *L = Moe();
-    int rc = Launched(L->combinePush(&c->comm->team, &c->hp, srcTokens, ld, rowsDev, c->sh.H, c->sh.K, weighted, c->grid * 2, stream), "combine push");
+    int rc = Launched(L->combinePush(&c->comm->team, &c->hp, srcTokens, ld, rowsDev, c->sh.max_recv, c->sh.H, c->sh.K, weighted, c->grid * 2, stream), "combine push");
     if (rc == Z_OK) rc = Launched(L->signalAll(&c->comm->team, &c->hp, 1, c->epoch, stream), "combine signal");
     if (rc == Z_OK) rc = Launched(L->waitAll(&c->comm->team, &c->hp, 1, c->epoch, c->status, stream), "combine wait");
     if (rc != Z_OK) return rc;

@@ -70,7 +70,7 @@ def _cu():
         l.mf_moe_combine_reduce.restype = ci
         l.mf_moe_combine_reduce.argtypes = [P(TeamC), P(MoeHeapC), P(MoeShapeC), vp, vp, ci, vp]
         l.mf_moe_combine_push.restype = ci
-        l.mf_moe_combine_push.argtypes = [P(TeamC), P(MoeHeapC), vp, C.c_int64, vp, ci, ci, ci, ci, vp]
+        l.mf_moe_combine_push.argtypes = [P(TeamC), P(MoeHeapC), vp, C.c_int64, vp, ci, ci, ci, ci, ci, vp]
         l.mf_moe_ll_dispatch.restype = ci
         l.mf_moe_ll_dispatch.argtypes = [P(DispatchArgsC), vp, vp, vp, vp, vp, ci, vp]
         l.mf_moe_ll_combine.restype = ci
@@ -409,7 +409,7 @@ class MoEComm:
         the combine slot of its token on the token's home rank and raises the combine flag."""
         assert y.dtype == torch.bfloat16 and y.shape[1] == self.H and y.stride(1) == 1
         team = self.heap.team()
-        _ok(_cu().mf_moe_combine_push(C.byref(team), C.byref(self.hp), y.data_ptr(), y.stride(0), st.row_off[self.El:].data_ptr(), self.H,
+        _ok(_cu().mf_moe_combine_push(C.byref(team), C.byref(self.hp), y.data_ptr(), y.stride(0), st.row_off[self.El:].data_ptr(), self.max_recv, self.H,
                                       self.K, 1 if weighted else 0, self._grid * 2, _s()), "moe_combine_push")
         _ok(_cu().mf_moe_signal_all(C.byref(team), C.byref(self.hp), 1, st.epoch, _s()), "moe_signal")
 

@@ -709,6 +709,48 @@ def test_dispatch_kernels_that_count_and_do_not_count_their_ctas_take_turns():
     assert all(fine), fine
 
 
+def _overfull_rank(rank, world, url, sync):
+    import torch
+    from memfabric_hybrid_b200.ops import moe as M
+    from memfabric_hybrid_b200.ops.gemm import status_word
+    from memfabric_hybrid_b200.ops.heap import SymmetricHeap
+    H, E, K, T, room = 512, 8, 2, 32, 40
+    heap = SymmetricHeap(url, 1, 0, 0, 16 << 20)
+    comm = M.MoEComm(heap, T, H, E, K, max_recv=room)
+    idx = torch.stack([torch.randperm(E - 1, generator=torch.Generator().manual_seed(t))[:K] for t in range(T)]).to(torch.int32)
+    idx[0, 0] = E - 1   # the last row of all: dropped
+    order = idx.view(-1).argsort(stable=True)
+    kept = torch.zeros(T * K)
+    kept[order[:room]] = 1
+    want = kept.view(T, K).sum(1, keepdim=True).expand(T, H)
+    x, w, d = torch.ones(T, H, dtype=torch.bfloat16, device="cuda"), torch.ones(T, K, device="cuda"), idx.cuda()
+    y = torch.full((T * K, H), float("nan"), dtype=torch.bfloat16, device="cuda")   # what lies behind the caller's `room` rows
+    y[:room] = 1
+    right = []
+    for pair in ("normal", "low latency"):
+        heap.view(comm.hp.recv_info, (comm.hp.comb - comm.hp.recv_info + T * K * H * 2,), torch.uint8).zero_()
+        if pair == "normal":
+            st = comm.dispatch(x, d, w)
+            comm.combine_push(y[:room], st)
+            out = comm.combine(st)
+        else:
+            st = comm.ll_dispatch(x, d, w)
+            out = comm.ll_combine(y[:room], st)
+        right.append(torch.equal(out.float().cpu(), want) and int(st.row_off[-1]) == T * K and int(status_word(comm.dev).item()) == 0x401)
+        status_word(comm.dev).zero_()
+    torch.cuda.synchronize()
+    right.append(heap.status()[0] == 0)
+    heap.close()
+    SymmetricHeap.shutdown()
+    return right
+
+
+def test_combine_of_a_receive_buffer_that_was_too_small():
+    """Rows without room are dropped and reported; the rows of the answers end where the receive buffer ends, and nothing behind them is read or sent."""
+    url = f"127.0.0.1:{free_port()}"
+    assert run_ranks(_overfull_rank, 1, (url,), timeout=300, with_barrier=True) == [[True, True, True]]
+
+
 def _refused_rank(rank, world, url, sync):
     import torch
     from memfabric_hybrid_b200.ops import moe as M
