@@ -36,7 +36,9 @@ def _cu():
 
 
 def status_word(device=None) -> torch.Tensor:
-    dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
+    dev = torch.device("cuda" if device is None else device)
+    if dev.index is None and dev.type == "cuda":   # the current device's word, not one of its own
+        dev = torch.device("cuda", torch.cuda.current_device())
     t = _status.get(dev)
     if t is None:
         t = torch.zeros(1, dtype=torch.int32, device=dev)

@@ -131,3 +131,13 @@ def test_gemm_bf16_in_a_cuda_graph(M):
         ref = h.float() @ w2.float().t()
         assert ((h.float() - a.float() @ w1.float().t()).norm() / h.float().norm()).item() <= 2.0 ** -8
         assert ((y.float() - ref).norm() / ref.norm()).item() <= 2.0 ** -8
+
+
+def test_status_word_of_a_device_without_an_index_is_the_current_one():
+    from memfabric_hybrid_b200.ops import gemm
+    here = torch.device("cuda", torch.cuda.current_device())
+    assert gemm.status_word("cuda") is gemm.status_word(here) and gemm.status_word() is gemm.status_word(here)
+    gemm.status_word().fill_(0x401)
+    with pytest.raises(RuntimeError, match="0x401"):
+        gemm.check_status("cuda")
+    gemm.check_status()
