@@ -234,8 +234,7 @@ class MoEComm:
         self._epoch = 0
         self._done = torch.zeros(1, dtype=torch.int32, device=self.dev)
         self._push_done = torch.zeros(1, dtype=torch.int32, device=self.dev)  # finished CTAs of the down projection, zero between launches
-        self._dispatches = 0
-        self._counted = 0   # of these, the calls whose kernel counts its CTAs in _done
+        self._counted = 0   # dispatches whose kernel counts its CTAs in _done
         self._ll_done = torch.zeros(1, dtype=torch.int32, device=self.dev)
         self._ll_grid = None
         self._grid = sm_count(self.dev)
@@ -328,7 +327,6 @@ class MoEComm:
             self._counted += 1
             self._keep = (w, idx, smooth)
             _ok(_cu().mf_moe_wait_all(C.byref(team), C.byref(self.hp), 0, self._epoch, status_word(self.dev).data_ptr(), _s()), "moe_wait")
-        self._dispatches += 1
         return DispatchState(T, idx, sidx, tpe, tpr, inr, rpe, row_off, put_off, src_off, self._epoch)
 
     def dispatch_cached(self, x: torch.Tensor, st: DispatchState, topk_w: torch.Tensor) -> DispatchState:
@@ -338,7 +336,6 @@ class MoEComm:
         assert x.dtype == torch.bfloat16 and x.is_contiguous() and x.shape == (st.T, self.H)
         import dataclasses
         self._epoch += 1
-        self._dispatches += 1
         self._counted += 1
         team = self.heap.team()
         w = topk_w.to(torch.float32).contiguous()   # the weights travel with the rows again

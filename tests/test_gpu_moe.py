@@ -755,20 +755,34 @@ def _refused_rank(rank, world, url, sync):
     import torch
     from memfabric_hybrid_b200.ops import moe as M
     from memfabric_hybrid_b200.ops.heap import SymmetricHeap
-    H, E, K = 512, 8, 2
-    heap = SymmetricHeap(url, 1, 0, 0, 16 << 20)
-    comm = M.MoEComm(heap, 4096, H, E, K, max_recv=64)
-    x, idx, w = torch.randn(4, H, device="cuda").to(torch.bfloat16), torch.zeros(4, K, dtype=torch.int32, device="cuda"), torch.ones(4, K, device="cuda")
+    H, E, K, many = 512, 8, 2, 2100   # more than 4096 entries: layout and count exchange have launches of their own
+    heap = SymmetricHeap(url, 1, 0, 0, 32 << 20)
+    comm = M.MoEComm(heap, 4096, H, E, K, max_recv=many * K)
+    x, idx, w = torch.randn(many, H, device="cuda").to(torch.bfloat16), torch.zeros(many, K, dtype=torch.int32, device="cuda"), torch.ones(many, K, device="cuda")
     idx[:, 1] = 5
+    lib = M._cu()
+
+    class Refusing:
+        """The library, with some calls answered on the host."""
+        answers = {}
+
+        def __getattr__(self, name):
+            return (lambda *a: self.answers[name]) if name in self.answers else getattr(lib, name)
+
+    fake = Refusing()
+    M._cu = lambda: fake
     numbers = []
-    for t in (4, 0, 4):
+    for t, answers in ((4, {}), (0, {}), (4, {}), (many, {}), (many, {"mf_moe_layout": -1}), (many, {"mf_moe_notify": -1}), (many, {}),
+                       (4, {"mf_moe_dispatch_alone": -3, "mf_moe_prepare": -1}), (4, {"mf_moe_dispatch_alone": -3}), (many, {"mf_moe_dispatch": -1}), (many, {}),
+                       (4, {"mf_moe_dispatch_alone": -1}), (4, {})):
+        fake.answers = answers
         try:
             st = comm.dispatch(x[:t], idx[:t], w[:t])
-            comm.combine_push(torch.ones(8, H, dtype=torch.bfloat16, device="cuda"), st)
+            comm.combine_push(torch.ones(t * K, H, dtype=torch.bfloat16, device="cuda"), st)
             y = comm.combine(st)
-            numbers.append((comm._epoch, comm._dispatches, bool((y == 2).all())))
+            numbers.append((comm._epoch, comm._counted, bool((y == 2).all())))
         except RuntimeError:
-            numbers.append((comm._epoch, comm._dispatches, None))
+            numbers.append((comm._epoch, comm._counted, None))
     torch.cuda.synchronize()
     st = heap.status()[0]
     heap.close()
@@ -777,7 +791,10 @@ def _refused_rank(rank, world, url, sync):
 
 
 def test_a_refused_dispatch_leaves_the_ranks_in_step():
-    """No tokens: refused before anything is launched. The call numbers that the ranks' flags carry must not advance on the rank
-    that was refused, or its next call waits for a number that no peer sends."""
+    """Refused by the library (no tokens), or any of the calls of a dispatch by a stand-in for it. The call numbers that the ranks' flags carry must not advance on
+    the rank that was refused, or its next call waits for a number that no peer sends; nor may the number that the counter of finished CTAs is
+    compared with. An exchange that was launched counts, even if the push behind it was refused."""
     url = f"127.0.0.1:{free_port()}"
-    assert run_ranks(_refused_rank, 1, (url,), timeout=300, with_barrier=True) == [([(1, 1, True), (1, 1, None), (2, 2, True)], 0)]
+    assert run_ranks(_refused_rank, 1, (url,), timeout=300, with_barrier=True) == [
+        ([(1, 0, True), (1, 0, None), (2, 0, True), (3, 1, True), (3, 1, None), (3, 1, None), (4, 2, True), (4, 2, None), (5, 3, True), (6, 3, None), (7, 4, True),
+          (7, 4, None), (8, 4, True)], 0)]
