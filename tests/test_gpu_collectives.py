@@ -270,6 +270,39 @@ def test_large_reductions_whose_parts_are_pushed_in_chunks(world, stage_mb):
     assert heap.status()[0] == 0
 
 
+@pytest.mark.parametrize("world", [2, 3])
+def test_collectives_whose_peers_never_come(world):
+    """One rank alone with the slots of a group: what it sends lands in slots that nobody reads, and every wait of the calls ends at its limit, is reported with where it
+    gave up and with the call's number, and leaves the GPU to the next call."""
+    from memfabric_hybrid_b200.ops.heap import EmulatedHeap
+    from memfabric_hybrid_b200.ops.collectives import Communicator
+    stage = 32 << 20
+    heap = EmulatedHeap(world, (1 << 20) + 4 * stage + 4096)
+    heap.emu, heap.spin_limit = False, 2000   # under a millisecond
+    c = Communicator(heap, stage_bytes=stage)
+    big = (60 << 20) // world // 4 + 24       # fp32 values from which on the parts are pushed in chunks
+    big -= big % (8 * world)
+    big += 8 * world
+    calls = [(0x102, lambda: c.all_reduce(torch.ones(64, device="cuda", dtype=torch.bfloat16))),            # packets, one trip
+             (0x102, lambda: c.all_reduce(torch.ones(20_000, device="cuda", dtype=torch.bfloat16))),        # two trips
+             (0x100, lambda: c.all_reduce(torch.ones(100_000, device="cuda", dtype=torch.bfloat16))),       # staged, one shot
+             (0x110, lambda: c.all_reduce(torch.ones(100_000, device="cuda", dtype=torch.bfloat16), algo="twoshot")),
+             (0x118, lambda: c.all_reduce(torch.ones(big, device="cuda"), algo="twoshot")),
+             (0x128, lambda: c.reduce_scatter(torch.ones(big, device="cuda"))),
+             (0x120, lambda: c.reduce_scatter(torch.ones(8 * world, device="cuda"))),
+             (0x130, lambda: c.all_gather(torch.ones(1000, device="cuda")))]
+    for where, call in calls:
+        call()
+        torch.cuda.synchronize()
+        code, at, epoch, count = heap.status()
+        assert (code, at, epoch) == (1, where, c._epoch) and count > 0, (hex(at), hex(where))
+        heap.clear_status()
+    whole = EmulatedHeap(world, (1 << 20) + 4 * (1 << 20) + 4096)
+    assert bool((Communicator(whole, stage_bytes=1 << 20).all_reduce(torch.ones(world, 64, device="cuda")) == world).all())
+    torch.cuda.synchronize()
+    assert whole.status()[0] == 0
+
+
 @pytest.mark.parametrize("world", [2, 8])
 def test_broadcast_scatter_alltoallv(comms, world):
     c = comms[world]
