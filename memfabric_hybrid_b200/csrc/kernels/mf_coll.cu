@@ -215,7 +215,8 @@ template <typename T> __device__ __forceinline__ void cta_fanout_copy(const T *s
 // Several sources, one destination each (all-gather, second half of the two-shot all-reduce): part k is cnt[k] elements from srcs[k] to dsts[k]. The
 // vectors of all parts are numbered through, so that eight loads are in flight per thread however short a part is: part by part,
 // every part of a small message cost a memory latency of its own (over NVLink a round trip to the peer). The stores are streaming ones: outputs
-// as large as the L2 otherwise push the staged parts out (8 ranks, all-gather of 983 040 bf16 values each 46 us, 40 so).
+// as large as the L2 otherwise push the staged parts out (8 ranks, all-gather of 983 040 bf16 values each 46 us, 40 so). All figures are of ranks that
+// share one GPU's memory and L2; not measured on two GPUs, where a fetch is a round trip behind the flag and a push is not.
 template <typename T> __device__ __forceinline__ void cta_gather_copy(const T *const *srcs, T *const *dsts, const uint32_t *cnt, uint32_t parts)
 {
     constexpr uint32_t VN = 16 / sizeof(T);
@@ -329,7 +330,7 @@ template <typename TO, bool INT> __device__ __forceinline__ void emit(TO *dst, u
 
 // Second half of the two-shot all-reduce: every rank fetches the finished parts from their owners. As many bytes cross NVLink as when the owners
 // push them, but a part is written to memory once instead of once per rank and copied out of nobody's staging area. 8 emulated ranks, us, pushed /
-// so: 983 040 bf16 27.5 / 24, fp32 40 / 34.5.
+// so: 983 040 bf16 27.5 / 24, fp32 40 / 34.5. Not measured on two GPUs (see cta_gather_copy).
 template <typename TO> __device__ __forceinline__ void fetch_parts(const Team &t, uint32_t me, uint64_t stage_b, uint64_t n, uint64_t C, const Range &sub, TO *out)
 {
     __shared__ const TO *srcs[kMaxRanks];

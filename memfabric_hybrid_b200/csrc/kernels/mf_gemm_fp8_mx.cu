@@ -242,6 +242,7 @@ template <int MODE, int EPI, bool PAIR> __global__ void __launch_bounds__(kXThre
     // MODE 2 by one rank: there are no partials to wait for, so a tile's epilogue writes its rows of y itself, under the next tile's MMAs. Adding up behind the
     // last tile read 67 MB back and wrote as much with the tensor cores idle: 4096 x 8192 outputs, K 3584, 126 us, so (and without a second fence
     // for the system per tile) 101; 1024 rows 43.2 / 36.0, 128 rows 23.3 / 20.0. With more ranks the loads of the other partials would hold the epilogue up.
+    // The tiles are stored in the landing zone and counted all the same, as by every number of ranks, though only y is read behind the call.
     const bool alone = g.team.world == 1;
 
     after_predecessor();  // one rank's launch may start under the kernel in front of it; else this returns at once

@@ -7,9 +7,10 @@
 
 Every rank must issue the same sequence of calls (the flag epochs advance in lockstep). With an
 ``EmulatedHeap`` the tensors carry a leading ``world`` dimension and one launch runs all ranks.
-Algorithm choice follows the message size: one-shot all-reduce up to 256 KiB, two-shot above; the
-number of CTAs grows with the size (the analogue of the reference's per-size block-count table,
-zbal_kernel_utils.h:117-152).
+Algorithm choice follows the message size. Staged all-reduce: packets that carry the call's number beside the data up
+to about 76 KiB, one shot up to 256 KiB and for as long as all ranks together read 32 MiB at most, two shots above. Buffers
+inside the symmetric heap of more than 256 KiB are used in place. The number of CTAs grows with the size (the analogue of
+the reference's per-size block-count table, zbal_kernel_utils.h:117-152).
 """
 from __future__ import annotations
 
@@ -25,8 +26,9 @@ DT = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2, torch.int32: 3}
 OPS = {"sum": 0, "max": 1, "min": 2, "prod": 3}
 # One shot (every rank reads all of every rank's staged copy) has a handshake less than two shots (4-5 us) and moves (W - 1) n bytes per rank for 2 (W - 1) / W n.
 # Emulated ranks on one GPU, all-reduce, us, one shot / two: 2 ranks 400 KiB 8.0 / 12.5, 8 MiB 17.2 / 20.4; 4 ranks 512 KiB 9.0 / 14.3, 2 MiB 14.1 / 16.6, 4 MiB 21.2 / 20.7;
-# 8 ranks 400 KiB 12.4 / 16.6, 700 KiB 15.1 / 17.2, 1 MiB 19.2 / 18.0 (fp32 a little later): even at W * W * n of 56 MiB. Over NVLink the further bytes take as long as the
-# handshake (by their count, 770 GB/s) at 2 MiB with 4 ranks and 0.6 MiB with 8: the line is drawn in front of both.
+# 8 ranks 400 KiB 12.4 / 16.6, 700 KiB 15.1 / 17.2, 1 MiB 19.2 / 18.0 (fp32 a little later): even at W * W * n of 56 MiB. Not measured with ranks on GPUs of
+# their own: counted at 770 GB/s over NVLink, the further bytes take as long as the handshake at 2 MiB with 4 ranks, which is where the line lies, and at 0.6 MiB with 8, behind it (0.5); with
+# 2 ranks (line at 8 MiB) both ways move the same bytes.
 ONE_SHOT_MAX = 256 << 10      # always
 ONE_SHOT_READS = 32 << 20     # above it: up to so many bytes read by all ranks
 DIRECT_MIN = 256 << 10  # above this, buffers that live in the heap are used in place (no staging copies)
