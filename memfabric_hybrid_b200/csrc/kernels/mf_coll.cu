@@ -667,7 +667,7 @@ __device__ __forceinline__ bool pipe_reduce(const Team &t, uint32_t me, const Pi
     constexpr uint32_t VN = Vec<T>::N, kPiece = kPieceBytes / sizeof(T);
     __shared__ uint64_t done[kMaxChunks];
     __shared__ int ok_sh;
-    const uint32_t world = W > 0 ? (uint32_t)W : t.world;
+    constexpr uint32_t world = W;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t parts = p.own ? world - 1 : world;
     const uint64_t span = sub.end > sub.beg ? sub.end - sub.beg : 0;
@@ -735,38 +735,27 @@ __device__ __forceinline__ bool pipe_reduce(const Team &t, uint32_t me, const Pi
             const uint64_t b = sub.beg + q * chunk, e = min(end, b + chunk);
             if (b >= e) continue;
             const uint64_t vend = b + (e - b) / VN * VN;
-            constexpr int U = W == 0 ? 1 : 2;
+            constexpr int U = 2;
             for (uint64_t i = b + (uint64_t)tid * VN; i < vend; i += (uint64_t)U * kReduceWarps * 32 * VN) {
-                if (W > 0) {
-                    uint4 raw[U][W > 0 ? W : 1];
+                uint4 raw[U][W];
 #pragma unroll
-                    for (int u = 0; u < U; u++)
+                for (int u = 0; u < U; u++)
 #pragma unroll
-                        for (int r = 0; r < W; r++)
-                            if (u == 0 || i + u * kReduceWarps * 32 * VN < vend)
-                                raw[u][r] = __ldcs(reinterpret_cast<const uint4 *>(row(r) + i + u * kReduceWarps * 32 * VN));
+                    for (int r = 0; r < W; r++)
+                        if (u == 0 || i + u * kReduceWarps * 32 * VN < vend)
+                            raw[u][r] = __ldcs(reinterpret_cast<const uint4 *>(row(r) + i + u * kReduceWarps * 32 * VN));
 #pragma unroll
-                    for (int u = 0; u < U; u++) {
-                        if (u != 0 && i + u * kReduceWarps * 32 * VN >= vend) continue;
-                        float acc[VN];
-#pragma unroll
-                        for (int r = 0; r < W; r++) {
-                            float f[VN];
-                            Vec<T>::unpack(raw[u][r], f);
-#pragma unroll
-                            for (uint32_t k = 0; k < VN; k++) acc[k] = r == 0 ? f[k] : red_apply<INT>(acc[k], f[k], op);
-                        }
-                        sink(i + u * kReduceWarps * 32 * VN, acc, VN);
-                    }
-                } else {
+                for (int u = 0; u < U; u++) {
+                    if (u != 0 && i + u * kReduceWarps * 32 * VN >= vend) continue;
                     float acc[VN];
-                    for (uint32_t r = 0; r < world; r++) {
+#pragma unroll
+                    for (int r = 0; r < W; r++) {
                         float f[VN];
-                        Vec<T>::load(row(r) + i, f);
+                        Vec<T>::unpack(raw[u][r], f);
 #pragma unroll
                         for (uint32_t k = 0; k < VN; k++) acc[k] = r == 0 ? f[k] : red_apply<INT>(acc[k], f[k], op);
                     }
-                    sink(i, acc, VN);
+                    sink(i + u * kReduceWarps * 32 * VN, acc, VN);
                 }
             }
             for (uint64_t i = vend + tid; i < e; i += kReduceWarps * 32) {
@@ -1523,11 +1512,14 @@ template <typename K, typename A> int launch(K kernel, const A &args, int ctas, 
 // the two passes of the others. Emulated ranks, fp32, us, two passes / pipelined by the bytes of all ranks: reduce-scatter of 32 MB 18.2 / 21.0 (4
 // ranks), 63 MB 36.4 / 32.6, 64 MB 36.2 / 35.3 (8 ranks), 128 MB 66 / 60, 252 MB 125 / 107; two-shot all-reduce of 33 MB 36.8 / 38.9 (2 ranks), 67 MB 62.6 /
 // 60.4, 8 ranks of 32 MB 207 / 185. Real ranks, not measured here, follow the same line (8 ranks: 7.5 MB each): there the copy into the own staging area
-// in front of the exchange goes away as well. Parts off 16 bytes have to be shifted, which the two passes do with more warps (139 / 143).
+// in front of the exchange goes away as well. Parts off 16 bytes have to be shifted, which the two passes do with more warps (139 / 143). Other numbers of
+// ranks than 2, 4 and 8: the loads of all ranks' parts are not unrolled, and eight warps of the pipelined kernel then have too few on their way where the two
+// passes have sixteen: reduce-scatter of 63 MB by 3 ranks 53 / 69, of 96 MB by 16 93 / 103, of 256 MB by 16 221 / 317.
 constexpr uint64_t kPipeMinBytes = 60ull << 20;
 bool pipe_pays(const CollArgs &a, uint64_t part_stride, uint64_t es, int threads)
 {
-    return !a.zero_copy && threads == kPipeThreads && a.team.world > 1 && a.team.world * a.n * es >= kPipeMinBytes && part_stride * es % 16 == 0;
+    const uint32_t world = a.team.world;
+    return !a.zero_copy && threads == kPipeThreads && (world == 2 || world == 4 || world == 8) && world * a.n * es >= kPipeMinBytes && part_stride * es % 16 == 0;
 }
 
 constexpr uint64_t kOneTripBytes = 16 << 10;  // received by a rank; above it two trips of less data are as fast on one GPU
@@ -1571,8 +1563,7 @@ template <typename T, typename TO, bool INT> int launch_allreduce(const CollArgs
         switch (a.team.world) {
             case 2: return launch(k_allreduce_pipe<T, TO, INT, 2>, a, ctas, threads, s, false);
             case 4: return launch(k_allreduce_pipe<T, TO, INT, 4>, a, ctas, threads, s, false);
-            case 8: return launch(k_allreduce_pipe<T, TO, INT, 8>, a, ctas, threads, s, false);
-            default: return launch(k_allreduce_pipe<T, TO, INT, 0>, a, ctas, threads, s, false);
+            default: return launch(k_allreduce_pipe<T, TO, INT, 8>, a, ctas, threads, s, false);
         }
     }
     switch (a.team.world) {
@@ -1624,8 +1615,7 @@ template <typename T, typename TO, bool INT> int launch_rs(const CollArgs &a, in
         switch (a.team.world) {
             case 2: return launch(k_reduce_scatter_pipe<T, TO, INT, 2>, a, ctas, threads, s, false);
             case 4: return launch(k_reduce_scatter_pipe<T, TO, INT, 4>, a, ctas, threads, s, false);
-            case 8: return launch(k_reduce_scatter_pipe<T, TO, INT, 8>, a, ctas, threads, s, false);
-            default: return launch(k_reduce_scatter_pipe<T, TO, INT, 0>, a, ctas, threads, s, false);
+            default: return launch(k_reduce_scatter_pipe<T, TO, INT, 8>, a, ctas, threads, s, false);
         }
     }
     switch (a.team.world) {

@@ -233,10 +233,10 @@ def test_reduce_scatter_and_all_gather_whose_output_lies_in_the_input(comms, wor
         assert torch.equal(out, shard.reshape(1, -1).expand(world, -1)), off
 
 
-@pytest.mark.parametrize("world,stage_mb", [(2, 32), (3, 21), (4, 16), (8, 8)])
+@pytest.mark.parametrize("world,stage_mb", [(2, 32), (3, 21), (4, 16), (5, 14), (8, 8), (16, 6)])
 def test_large_reductions_whose_parts_are_pushed_in_chunks(world, stage_mb):
     """From 60 MiB over all ranks on, the parts travel in chunks while they are reduced: ends of chunks and of CTA ranges, inputs on and off 16 bytes, an
-    output in the input's memory, every rank's sum in rank order bit for bit; just below, the two passes."""
+    output in the input's memory, every rank's sum in rank order bit for bit; just below, and by other numbers of ranks than 2, 4 and 8, the two passes."""
     from memfabric_hybrid_b200.ops.heap import EmulatedHeap
     from memfabric_hybrid_b200.ops.collectives import Communicator
     heap = EmulatedHeap(world, (1 << 20) + 4 * (stage_mb << 20) + (1 << 20))
@@ -280,15 +280,15 @@ def test_collectives_whose_peers_never_come(world):
     heap = EmulatedHeap(world, (1 << 20) + 4 * stage + 4096)
     heap.emu, heap.spin_limit = False, 2000   # under a millisecond
     c = Communicator(heap, stage_bytes=stage)
-    big = (60 << 20) // world // 4 + 24       # fp32 values from which on the parts are pushed in chunks
+    big = (60 << 20) // world // 4 + 24       # fp32 values from which on two ranks push their parts in chunks
     big -= big % (8 * world)
     big += 8 * world
     calls = [(0x102, lambda: c.all_reduce(torch.ones(64, device="cuda", dtype=torch.bfloat16))),            # packets, one trip
              (0x102, lambda: c.all_reduce(torch.ones(20_000, device="cuda", dtype=torch.bfloat16))),        # two trips
              (0x100, lambda: c.all_reduce(torch.ones(100_000, device="cuda", dtype=torch.bfloat16))),       # staged, one shot
              (0x110, lambda: c.all_reduce(torch.ones(100_000, device="cuda", dtype=torch.bfloat16), algo="twoshot")),
-             (0x118, lambda: c.all_reduce(torch.ones(big, device="cuda"), algo="twoshot")),
-             (0x128, lambda: c.reduce_scatter(torch.ones(big, device="cuda"))),
+             (0x118 if world == 2 else 0x110, lambda: c.all_reduce(torch.ones(big, device="cuda"), algo="twoshot")),
+             (0x128 if world == 2 else 0x120, lambda: c.reduce_scatter(torch.ones(big, device="cuda"))),
              (0x120, lambda: c.reduce_scatter(torch.ones(8 * world, device="cuda"))),
              (0x130, lambda: c.all_gather(torch.ones(1000, device="cuda")))]
     for where, call in calls:
