@@ -105,6 +105,30 @@ def test_all_reduce_on_both_sides_of_one_shot(world, m):
         assert heap.status()[0] == 0
 
 
+@pytest.mark.parametrize("world,n", [(2, 262_145), (2, 262_143), (2, 1_000_003), (3, 262_149), (4, 700_001), (8, 147_465)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_one_shot_into_outputs_off_16_bytes(world, n, dtype):
+    """Around two vectors per thread, where the sums start to go through the staging area: every offset of the output, also in place; the fp32 sum in rank order."""
+    from memfabric_hybrid_b200.ops.heap import EmulatedHeap
+    from memfabric_hybrid_b200.ops.collectives import Communicator
+    heap = EmulatedHeap(world, (1 << 20) + 4 * (3 << 20) + 4096)
+    c = Communicator(heap, stage_bytes=3 << 20)
+    x = torch.randn(world, n, device="cuda", generator=torch.Generator("cuda").manual_seed(n)).to(dtype)
+    acc = x[0].float()
+    for r in range(1, world):
+        acc = acc + x[r].float()
+    want = (acc * 0.5).to(dtype).expand(world, n)
+    for off in range(8):
+        room = torch.full((world * n + 16,), 7, device="cuda", dtype=dtype)
+        got = room[off:off + world * n].view(world, n)
+        c.all_reduce(x, out=got, scale=0.5, algo="oneshot")
+        assert torch.equal(got, want) and bool((room[:off] == 7).all()) and bool((room[off + world * n:] == 7).all()), off
+        got.copy_(x)
+        assert torch.equal(c.all_reduce(got, out=got, scale=0.5, algo="oneshot"), want), off
+    torch.cuda.synchronize()
+    assert heap.status()[0] == 0
+
+
 @pytest.mark.parametrize("world", [2, 3, 8])
 def test_small_all_reduce_in_packets(world):
     """Sizes that change from call to call (what an earlier call left in the packet area must not count), odd ones, inputs off eight bytes, in place, an output in
