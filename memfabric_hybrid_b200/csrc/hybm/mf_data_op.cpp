@@ -340,13 +340,17 @@ uint64_t SpanCutter::Split(uint64_t len, uint32_t at, bool rest)
     return (uint64_t)n;
 }
 
-// Shares for a batch, 0: none (the pieces are dealt out one by one; on a device without the copy unit always). Up to a chunk of the smallest size per CTA, each chunk gets a CTA of its own (100 pieces of up to 16 KiB: one
-// latency for all of them); the chunks are at least as many as the runs and as the bytes would fill.
-static uint32_t SpansFor(const DeviceBackend *dev, const BatchShape &b)
+// Shares for a batch, 0: none (the pieces are dealt out one by one; on a device without the copy unit always). Up to a chunk of the smallest size per CTA,
+// each chunk gets a CTA of its own (100 pieces of up to 16 KiB: one latency for all of them); the chunks are at least as many as the runs and as the bytes would fill.
+// `laidOutOnce`: the host does not cut the batch on every call. Else half as many shares do for few bytes per share, since a share costs the host 5 ns
+// (1500 pieces of up to 16 KiB: 0.7 us less, the kernel, which the host hides, 1.6 more), but not for many tiny pieces: the latencies of a share's pieces
+// follow one another (3000 pieces of up to 1 KiB, kernel: dealt out one by one 13.0, half of the shares 16.5, all 12.4; the call the same 20).
+static uint32_t SpansFor(const DeviceBackend *dev, const BatchShape &b, bool laidOutOnce)
 {
     const uint32_t n = dev->CopySpanCount();
     if (n == 0 || (b.alignMask & 15) == 0 || std::max(b.runs, b.bytes / kMinCopyChunk) <= n) return 0;
-    return b.bytes / n < (32u << 10) ? (n + 1) / 2 : n;  // 1500 pieces of up to 16 KiB: the host takes 0.7 us less, the kernel, which it hides, 1.6 more
+    const bool manyTiny = b.bytes / b.runs < (2u << 10) && b.runs > 4ull * n;
+    return !laidOutOnce && !manyTiny && b.bytes / n < (32u << 10) ? (n + 1) / 2 : n;
 }
 
 KernelBatch::KernelBatch(ComposeDataOp &op, void *userStream, uint32_t flags, const BatchShape &shape)
@@ -364,7 +368,7 @@ KernelBatch::KernelBatch(ComposeDataOp &op, void *userStream, uint32_t flags, co
     uint64_t chunk = AlignUp(std::max<uint64_t>(shape.bytes / (sms * 8), 1), 4096);
     chunk_ = std::min(std::max<uint64_t>(chunk, kMinCopyChunk), op_.chunk_);
     bulk_ = (shape.alignMask & 15) == 0;
-    spans_ = SpansFor(op_.dev_, shape);
+    spans_ = SpansFor(op_.dev_, shape, false);
     if (spans_ != 0) cut_.Begin(SpanCutter::Weight(shape), spans_);
     most_ = shape.runs + (spans_ != 0 ? spans_ : shape.bytes / chunk_);
     first_ = op_.ringHead_;  // before a wrap: what earlier batches left in the ring has been launched by them
@@ -516,7 +520,7 @@ int ComposeDataOp::Prepare(const std::vector<ResolvedCopy> &items, PreparedBatch
     uint64_t chunk = AlignUp(std::max<uint64_t>(shape.bytes / (sms * 8), 1), 4096);
     chunk = std::min(std::max<uint64_t>(chunk, kMinCopyChunk), chunk_);
     shape.runs = runs.size();
-    const uint32_t spans = SpansFor(dev_, shape);
+    const uint32_t spans = SpansFor(dev_, shape, true);
     SpanCutter cut;
     auto each = [&](auto &&emit) {  // the descriptors, in order
         uint64_t w = 0;
