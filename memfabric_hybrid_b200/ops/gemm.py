@@ -36,6 +36,9 @@ def _cu():
 
 
 def status_word(device=None) -> torch.Tensor:
+    t = _status.get(device)   # keys name their index
+    if t is not None:
+        return t
     dev = torch.device("cuda" if device is None else device)
     if dev.index is None and dev.type == "cuda":   # the current device's word, not one of its own
         dev = torch.device("cuda", torch.cuda.current_device())
