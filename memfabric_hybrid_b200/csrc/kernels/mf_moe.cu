@@ -450,9 +450,11 @@ __device__ __forceinline__ void push_row(const DispatchArgs &a, uint32_t me, int
         const int64_t pos = d_pos[k];
         if (vec < vecs) {
             if (a.raw_bf16) {
-                uint4 *row = reinterpret_cast<uint4 *>(peer_ptr(t, d, a.hp.recv_x) + pos * H * 2 + vec * 32);
-                row[0] = raw_lo;
-                row[1] = raw_hi;
+                // A whole 32-byte sector per store (rows start on 256 bytes): as two halves, the sooner the stores of a row leave the more of its sectors reach memory
+                // in parts. Along known routing, with its wait, 7168 columns, 8 copies, us, two stores / one: 592 tokens 24.8 / 17.7, 1 024 40.8 / 33.3.
+                asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(peer_ptr(t, d, a.hp.recv_x) + pos * H * 2 + vec * 32), "r"(raw_lo.x), "r"(raw_lo.y),
+                             "r"(raw_lo.z), "r"(raw_lo.w), "r"(raw_hi.x), "r"(raw_hi.y), "r"(raw_hi.z), "r"(raw_hi.w)
+                             : "memory");
             } else {
                 *reinterpret_cast<uint4 *>(peer_ptr(t, d, a.hp.recv_x) + pos * H + vec * 16) = q;
             }

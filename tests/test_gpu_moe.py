@@ -709,6 +709,46 @@ def test_dispatch_kernels_that_count_and_do_not_count_their_ctas_take_turns():
     assert all(fine), fine
 
 
+def _raw_rank(rank, world, url, sync):
+    import torch
+    from memfabric_hybrid_b200.ops import moe as M
+    from memfabric_hybrid_b200.ops.gemm import check_status
+    from memfabric_hybrid_b200.ops.heap import SymmetricHeap
+    heap, E, K, bad = SymmetricHeap(url, 1, 0, 0, 256 << 20), 16, 4, []
+    for H in (128, 1152, 7168):
+        mark = heap.mark()
+        comm = M.MoEComm(heap, 1100, H, E, K, max_recv=1100 * K, raw_bf16=True)
+        for T in (1, 3, 149, 593, 1100):    # one launch of few tokens, the small exchange, launches of their own
+            x = torch.randn(T, H, device="cuda", generator=torch.Generator("cuda").manual_seed(T)).to(torch.bfloat16)
+            idx = torch.rand(T, E, device="cuda").topk(K, 1).indices.to(torch.int32)
+            idx[T // 2, 1] = -1
+            for how in ("dispatch", "cached", "low latency"):
+                comm.recv_x().fill_(7.0)
+                if how == "cached":
+                    st = comm.dispatch_cached(x, st, torch.rand(T, K, device="cuda"))
+                else:
+                    st = (comm.dispatch if how == "dispatch" else comm.ll_dispatch)(x, idx, torch.rand(T, K, device="cuda"))
+                rows = int(st.row_off[-1])
+                got, tok = comm.recv_x(), comm.recv_info()[:rows, 1].long()
+                if rows != T * K - 1 or not torch.equal(got[:rows], x[tok]) or not bool((got[rows:] == 7.0).all()):
+                    bad.append((H, T, how))
+                if how == "low latency":
+                    comm.ll_combine(got[:rows].clone(), st)   # the pair: the next call counts on it
+        heap.release_to(mark)
+    torch.cuda.synchronize()
+    check_status()
+    ok = heap.status()[0] == 0
+    heap.close()
+    SymmetricHeap.shutdown()
+    return bad, ok
+
+
+def test_rows_that_travel_as_bf16():
+    """Every row whole, where the tables say, and nothing behind the last one."""
+    url = f"127.0.0.1:{free_port()}"
+    assert run_ranks(_raw_rank, 1, (url,), timeout=300, with_barrier=True) == [([], True)]
+
+
 def _overfull_rank(rank, world, url, sync):
     import torch
     from memfabric_hybrid_b200.ops import moe as M
