@@ -1262,13 +1262,15 @@ int mf_moe_dispatch(const DispatchArgs *a, int ctas, void *stream)
     return e == cudaSuccess ? 0 : (int)e;
 }
 
+// The most tokens that mf_moe_dispatch_alone takes with `ctas`, 0: none (a caller that asks spares itself the refused call, 2 us from Python).
+int mf_moe_dispatch_alone_max(int world, int H, int K, int ctas) { return world != 1 || H / 16 > 448 || K <= 0 ? 0 : std::min(kLLTokens * ctas, kLLEntries / K); }
 // mf_moe_prepare, mf_moe_dispatch and mf_moe_wait_all of one rank's few tokens in one launch; -3: more ranks or too many tokens, make the three calls. `ctas` as
 // for mf_moe_dispatch, whose completion counter it leaves alone.
 int mf_moe_dispatch_alone(const DispatchArgs *d, int *tokens_per_expert, int *tokens_per_rank, uint8_t *is_token_in_rank, int *recv_per_expert,
                           int *row_off, int *src_off, int ctas, void *stream)
 {
     if (d == nullptr || d->team.emu || d->sh.T <= 0 || d->sh.K <= 0 || d->sh.K > 16 || d->sh.E <= 0 || d->sh.E > 1024 || d->sh.H % 128 != 0 || ctas <= 0) return -1;
-    if (d->team.world != 1 || d->sh.H / 16 > 448 || d->sh.T > kLLTokens * ctas || d->sh.T * d->sh.K > kLLEntries) return -3;
+    if (d->sh.T > mf_moe_dispatch_alone_max((int)d->team.world, d->sh.H, d->sh.K, ctas)) return -3;
     const LLDispatchArgs a{*d, tokens_per_expert, recv_per_expert, row_off, src_off, nullptr, tokens_per_rank, is_token_in_rank};
     const cudaError_t e = launch_overlapped(k_moe_dispatch_few<true>, dim3((unsigned)ctas), dim3(448), 0, (cudaStream_t)stream, 1, a);
     return e == cudaSuccess ? 0 : (int)e;

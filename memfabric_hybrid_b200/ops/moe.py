@@ -61,6 +61,8 @@ def _cu():
         l.mf_moe_prepare.argtypes = [P(TeamC), P(MoeHeapC), vp, ci, ci, ci, vp, vp, vp, vp, vp, vp, vp, vp, C.c_uint32, vp]
         l.mf_moe_dispatch.restype = ci
         l.mf_moe_dispatch.argtypes = [P(DispatchArgsC), ci, vp]
+        l.mf_moe_dispatch_alone_max.restype = ci
+        l.mf_moe_dispatch_alone_max.argtypes = [ci, ci, ci, ci]
         l.mf_moe_dispatch_alone.restype = ci
         l.mf_moe_dispatch_alone.argtypes = [P(DispatchArgsC), vp, vp, vp, vp, vp, vp, ci, vp]
         l.mf_moe_wait_all.restype = ci
@@ -238,6 +240,7 @@ class MoEComm:
         self._ll_done = torch.zeros(1, dtype=torch.int32, device=self.dev)
         self._ll_grid = None
         self._grid = sm_count(self.dev)
+        self._alone = _cu().mf_moe_dispatch_alone_max(self.world, hidden, topk, self._grid)   # tokens of a dispatch in one launch, 0: never
         self._inter = intermediate
         self._h = self._hq = self._hs = None
         torch.cuda.synchronize()
@@ -304,7 +307,7 @@ class MoEComm:
                           self._done.data_ptr(), epoch, self._counted + 1, status_word(self.dev).data_ptr(), 1 if self.raw_bf16 else 0,
                           smooth.data_ptr() if smooth is not None else None)
         rc = -3
-        if small and self.world == 1:
+        if small and T <= self._alone:
             # nothing to exchange: layout, tables and push of a few tokens in one launch
             rc = cu.mf_moe_dispatch_alone(C.byref(a), tpe.data_ptr(), tpr.data_ptr(), inr.data_ptr(), rpe.data_ptr(), row_off.data_ptr(), src_off.data_ptr(),
                                           self._grid, _s())
