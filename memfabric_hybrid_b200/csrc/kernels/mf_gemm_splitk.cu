@@ -303,8 +303,9 @@ extern "C" {
 // everywhere, of the larger ones a tenth does not fit the rest of a GPC. A round takes K / s steps, or what memory takes for all
 // tiles' steps (1.35 steps per SM at a time), and its exchange: a barrier, what grows with the rows and with how many CTAs exchange at once, and
 // most of all whether clusters share their SMs (a cluster's slowest CTA counts: 17 tiles in clusters of eight, 6 x 2624 x 1856, 6.5, in clusters of
-// four 5.6; 16 tiles, 3 x 2016 x 2432, 5.9, 5.9). The constants fit 181 products of 1 - 1024 rows, 1 - 74 tiles of 128 x
-// 256 and K 512 - 8192 (launches from a graph, weights from memory): the choice is 0.3 % from the best of the four on average (0.5 % for 107 others; 4.4 and 4.8 with the constants of the slower exchange).
+// four 5.6; 16 tiles, 3 x 2016 x 2432, 5.9, 5.9; of 128 rows and K 4096, clusters of four / eight: 15 tiles 10.5 / 9.3, 16 10.6 / 11.4, 17 10.7 / 12.1, 24 11.6 / 13.1). The constants fit
+// 181 products of 1 - 1024 rows, 1 - 74 tiles of 128 x 256 and K 512 - 8192 (launches from a graph, weights from memory), and what clusters of eight share 350 more of 8 to
+// 40 tiles and 8 to 1024 rows: the choice is 0.3 % from the best of the four on average, 10 % at most (with one penalty for any number of rows 1 % and 26 %: 947 x 304 x 7040 in clusters of eight 14.1, of four 11.2).
 // Measured (us, persistent kernels' better tiling | s = 1, 2, 4, 8): 32 x 7168 x 8192 43.1 | 34.3, 24.3, 22.6, 27.9; 1 x 1024 x 4096 23.8 |
 // 16.9, 10.1, 6.8, 5.6; 128 x 1024 x 8192 41.9 | 47.5, 26.4, 16.1, 11.8; 256 x 4096 x 8192 43.2 | 48.2, 28.7, 22.7, 33.6; 256 x 9216 x 8192 44.8 | 52.0,
 // 41.0, 58.9, 74.4; 1024 x 2304 x 16384 79.2 | 93.2, 66.4, 90.6, 101; 1024 x 1280 x 1024 10.0 | 9.5, 9.8, 15.0, 25.9.
@@ -318,7 +319,10 @@ int mf_gemm_bf16_split(int M, int N, int K, int sms)
         const double resident = (s <= 2 ? 2.0 : 1.8) * n / s;
         const double rounds = std::ceil(tiles / std::max(1.0, std::floor(resident)));
         const double busy = std::min(1.0, (double)tiles * s / (2.0 * n));
-        const double exchange = s > 1 ? 1.7 + 1.8 * s * split_box_rows(M) / BM * busy + (tiles > std::floor(resident / 2) ? 5.25 : 0.0) : 0.0;
+        const double rows = (double)split_box_rows(M) / BM, edge = std::floor(resident / 2);
+        // clusters of eight share SMs from one tile earlier on, half of them at first, and share more between them the more rows they exchange
+        const double shared = s < 8 ? (tiles > edge ? 5.25 : 0.0) : (tiles > edge ? 1.0 : tiles == edge ? 0.5 : 0.0) * (6 + 8 * rows);
+        const double exchange = s > 1 ? 1.7 + 1.8 * s * rows * busy + shared : 0.0;
         const double cost = std::max(rounds * ((k_iters + s - 1) / s), memory) + rounds * (0.3 * s + exchange);
         if (split == 0 || cost < best) {
             best = cost;

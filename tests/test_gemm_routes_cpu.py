@@ -27,6 +27,12 @@ def test_split_leaves_clusters_their_sms(split, M, N, K, best):
     assert split(M, N, K, 148) == best
 
 
+@pytest.mark.parametrize("M,N,K,best", [(947, 304, 7040, 4), (700, 304, 7040, 4), (962, 224, 4928, 4), (128, 1920, 4096, 8), (800, 200, 8192, 8)])
+def test_split_of_whole_tiles_around_the_last_clusters_of_eight_with_sms_of_their_own(split, M, N, K, best):
+    """24, 18 and 16 tiles of 128 rows: what clusters of eight share costs them 14 to 27 %; with 15 and 14 tiles they are the fastest by as much."""
+    assert split(M, N, K, 148) == best
+
+
 @pytest.mark.parametrize("sms", [0, 1, 16, 132, 148, 160])
 def test_split_never_exceeds_the_steps_of_k(split, sms):
     for M in (1, 8, 100, 128, 129, 2000):
