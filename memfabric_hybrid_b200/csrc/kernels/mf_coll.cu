@@ -582,7 +582,7 @@ template <typename T, typename TO, bool INT, int W> __global__ void __launch_bou
 }
 
 // ------------------------------------------------------------------------------------------------
-// Pipelined reduce (reduce-scatter and first half of the two-shot all-reduce, large parts). A CTA's range of every part is cut into chunks; seven warps
+// Pipelined reduce (reduce-scatter and first half of the two-shot all-reduce, large parts, 2, 4 or 8 ranks). A CTA's range of every part is cut into chunks; seven warps
 // push chunk after chunk of the input into the staging areas of the ranks that reduce them, one warp tells these
 // ranks how many chunks have arrived, eight warps reduce the chunks that the peers have pushed here. A chunk is read a few microseconds after it
 // was written, out of the L2, and no rank waits for the whole of another's input.
