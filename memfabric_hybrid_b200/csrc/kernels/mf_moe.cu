@@ -14,6 +14,7 @@
 // zbal_kernel_{dispatch_layout,notify_dispatch,dispatch_normal,combine_normal}.h of the reference.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
+#include <limits.h>
 #include <stdlib.h>
 
 #include <algorithm>
@@ -715,10 +716,10 @@ __global__ void __launch_bounds__(256, 4) k_moe_combine_reduce(Team t, MoeHeap h
 
 // Rows of bf16 -> fp8 e4m3 with one power-of-two scale per 128 elements (the activation format of the expert GEMMs).
 // rows_dev: device int with the number of valid rows (the receive count), read here so the host never waits.
-__global__ void __launch_bounds__(256) k_quant_rows_fp8(const __nv_bfloat16 *__restrict__ x, int64_t ldx, const int *rows_dev, int cols,
+__global__ void __launch_bounds__(256) k_quant_rows_fp8(const __nv_bfloat16 *__restrict__ x, int64_t ldx, const int *rows_dev, int max_rows, int cols,
                                                         uint8_t *__restrict__ q, float *__restrict__ scales)
 {
-    const int rows = *rows_dev;
+    const int rows = min(*rows_dev, max_rows);
     const int groups = cols / kQuantGroup;
     const int lane = threadIdx.x & 31;
     const int warps_total = gridDim.x * (blockDim.x >> 5);
@@ -1346,13 +1347,18 @@ int mf_moe_ll_combine(const Team *team, const MoeHeap *hp, const MoeShape *sh, c
     return e == cudaSuccess ? 0 : (int)e;
 }
 
-int mf_quant_rows_fp8(const void *x, int64_t ldx, const int *rows_dev, int cols, void *q, float *scales, int ctas, void *stream)
+// max_rows: of the buffers; a dispatch that drops rows for want of room still counts them in *rows_dev.
+int mf_quant_rows_fp8_max(const void *x, int64_t ldx, const int *rows_dev, int max_rows, int cols, void *q, float *scales, int ctas, void *stream)
 {
     if (cols % 128 != 0) return -1;
-    k_quant_rows_fp8<<<ctas, 256, 0, (cudaStream_t)stream>>>(static_cast<const __nv_bfloat16 *>(x), ldx, rows_dev, cols,
+    k_quant_rows_fp8<<<ctas, 256, 0, (cudaStream_t)stream>>>(static_cast<const __nv_bfloat16 *>(x), ldx, rows_dev, max_rows, cols,
                                                              static_cast<uint8_t *>(q), scales);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : (int)e;
+}
+int mf_quant_rows_fp8(const void *x, int64_t ldx, const int *rows_dev, int cols, void *q, float *scales, int ctas, void *stream)
+{
+    return mf_quant_rows_fp8_max(x, ldx, rows_dev, INT_MAX, cols, q, scales, ctas, stream);
 }
 
 }  // extern "C"

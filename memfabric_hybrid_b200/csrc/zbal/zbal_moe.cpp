@@ -53,7 +53,7 @@ struct MoeLaunchers {
     int (*llDispatch)(const DispatchArgs *, int *, int *, int *, int *, uint32_t *, int, void *) = nullptr;
     int (*llCombine)(const MfTeam *, const MoeHeap *, const MoeShape *, const void *, int64_t, const int *, int, const int *, const float *,
                      void *, uint32_t, const uint32_t *, uint32_t *, int *, int, void *) = nullptr;
-    int (*quantRows)(const void *, int64_t, const int *, int, void *, float *, int, void *) = nullptr;
+    int (*quantRows)(const void *, int64_t, const int *, int, int, void *, float *, int, void *) = nullptr;
     int (*groupedGemm)(const void *, const float *, int, const void *, const float *, const int *, int, int, int, void *, int64_t, int,
                        const MfTeam *, const void *, uint64_t, int, int *, int, void *) = nullptr;
     int (*groupedGemmMx)(const void *, const float *, int, const void *, const float *, const int *, int, int, int, void *, int64_t, float *, int,
@@ -79,7 +79,7 @@ const MoeLaunchers *Moe()
         SYM(combinePush, "mf_moe_combine_push");
         SYM(llDispatch, "mf_moe_ll_dispatch");
         SYM(llCombine, "mf_moe_ll_combine");
-        SYM(quantRows, "mf_quant_rows_fp8");
+        SYM(quantRows, "mf_quant_rows_fp8_max");
         SYM(groupedGemm, "mf_grouped_gemm_fp8");
         SYM(groupedGemmMx, "mf_grouped_gemm_fp8_mx");
         SYM(mxSupported, "mf_grouped_gemm_fp8_mx_supported");
@@ -420,7 +420,7 @@ int32_t zbal_fused_deep_moe(zbal_moe_t moe, const void *x, int64_t tokens, const
     } else {
         rc = Launched(L->groupedGemm(recvX, recvS, (int)R, gmm1Weight, gmm1Scale, rowOff, (int)El, (int)(2 * inter), c->sh.H, h, inter, 1, nullptr, nullptr, 0,
                                      c->sh.K, c->status, c->grid, stream), "grouped GEMM (gate/up)");
-        if (rc == Z_OK) rc = Launched(L->quantRows(h, inter, rowOff + El, (int)inter, hq, hs, c->grid * 4, stream), "requantisation");
+        if (rc == Z_OK) rc = Launched(L->quantRows(h, inter, rowOff + El, (int)R, (int)inter, hq, hs, c->grid * 4, stream), "requantisation");
         if (rc == Z_OK)
             rc = Launched(L->groupedGemm(hq, hs, (int)R, gmm2Weight, gmm2Scale, rowOff, (int)El, c->sh.H, (int)inter, nullptr, 0, 2, &c->comm->team, recvInfo,
                                          c->hp.comb, c->sh.K, c->status, c->grid, stream), "grouped GEMM (down + combine)");

@@ -77,6 +77,8 @@ def _cu():
         l.mf_moe_ll_dispatch.argtypes = [P(DispatchArgsC), vp, vp, vp, vp, vp, ci, vp]
         l.mf_moe_ll_combine.restype = ci
         l.mf_moe_ll_combine.argtypes = [P(TeamC), P(MoeHeapC), P(MoeShapeC), vp, C.c_int64, vp, ci, vp, vp, vp, C.c_uint32, vp, vp, vp, ci, vp]
+        l.mf_quant_rows_fp8_max.restype = ci
+        l.mf_quant_rows_fp8_max.argtypes = [vp, C.c_int64, vp, ci, ci, vp, vp, ci, vp]
         l.mf_quant_rows_fp8.restype = ci
         l.mf_quant_rows_fp8.argtypes = [vp, C.c_int64, vp, ci, vp, vp, ci, vp]
         l.mf_grouped_gemm_fp8.restype = ci
@@ -383,8 +385,8 @@ class MoEComm:
         _ok(cu.mf_grouped_gemm_fp8(self.heap.ptr(self.rank, self.hp.recv_x), self.heap.ptr(self.rank, self.hp.recv_scale), self.max_recv,
                                    w1q.data_ptr(), w1s.data_ptr(), st.row_off.data_ptr(), El, two_i, H, self._h.data_ptr(), I, 1, None, None,
                                    0, self.K, stw, self._grid, _s()), "grouped_gemm_fp8 (gate/up)")
-        _ok(cu.mf_quant_rows_fp8(self._h.data_ptr(), I, st.row_off[El:].data_ptr(), I, self._hq.data_ptr(), self._hs.data_ptr(),
-                                 self._grid * 4, _s()), "quant_rows_fp8")
+        _ok(cu.mf_quant_rows_fp8_max(self._h.data_ptr(), I, st.row_off[El:].data_ptr(), self.max_recv, I, self._hq.data_ptr(), self._hs.data_ptr(),
+                                     self._grid * 4, _s()), "quant_rows_fp8")
         _ok(cu.mf_grouped_gemm_fp8(self._hq.data_ptr(), self._hs.data_ptr(), self.max_recv, w2q.data_ptr(), w2s.data_ptr(),
                                    st.row_off.data_ptr(), El, H, I, None, 0, 2, C.byref(team), self.heap.ptr(self.rank, self.hp.recv_info),
                                    self.hp.comb, self.K, stw, self._grid, _s()), "grouped_gemm_fp8 (down+combine)")

@@ -791,6 +791,38 @@ def test_combine_of_a_receive_buffer_that_was_too_small():
     assert run_ranks(_overfull_rank, 1, (url,), timeout=300, with_barrier=True) == [[True, True, True]]
 
 
+def _overfull_ffn_rank(rank, world, url, sync):
+    import torch
+    from memfabric_hybrid_b200.ops import moe as M
+    from memfabric_hybrid_b200.ops.gemm import status_word
+    from memfabric_hybrid_b200.ops.heap import SymmetricHeap
+    H, I, E, K, T, room = 640, 256, 8, 2, 32, 40   # 640 columns: the kernels with a re-quantisation pass of its own
+    heap = SymmetricHeap(url, 1, 0, 0, 16 << 20)
+    comm = M.MoEComm(heap, T, H, E, K, max_recv=room)
+    q, s = torch.full((T * K, I), 0x5A, dtype=torch.uint8, device="cuda"), torch.full((T * K, I // 128), 7.0, device="cuda")
+    comm._hq, comm._hs = q[:room], s[:room]
+    w1, w2 = torch.zeros(E, 2 * I, H, dtype=torch.uint8, device="cuda"), torch.zeros(E, H, I, dtype=torch.uint8, device="cuda")
+    idx = torch.stack([torch.randperm(E, generator=torch.Generator().manual_seed(t))[:K] for t in range(T)]).to(torch.int32).cuda()
+    heap.view(comm.hp.comb, (T * K * H * 2,), torch.uint8).zero_()
+    st = comm.dispatch(torch.ones(T, H, dtype=torch.bfloat16, device="cuda"), idx, torch.ones(T, K, device="cuda"))
+    comm.expert_ffn(st, w1, torch.ones(E, 2 * I // 128, H // 128, device="cuda"), w2, torch.ones(E, H // 128, I // 128, device="cuda"))
+    y = comm.combine(st)
+    torch.cuda.synchronize()
+    ok = int(status_word(comm.dev).item()) == 0x401 and int(st.row_off[-1]) == T * K
+    ok = ok and bool((q[room:] == 0x5A).all()) and bool((s[room:] == 7.0).all()) and not bool(q[:room].any()) and not bool(y.any())
+    status_word(comm.dev).zero_()
+    ok = ok and heap.status()[0] == 0
+    heap.close()
+    SymmetricHeap.shutdown()
+    return ok
+
+
+def test_expert_ffn_of_a_receive_buffer_that_was_too_small():
+    """The activations are quantised up to the last row of the buffers, whatever the dispatch has counted."""
+    url = f"127.0.0.1:{free_port()}"
+    assert run_ranks(_overfull_ffn_rank, 1, (url,), timeout=300, with_barrier=True) == [True]
+
+
 def _refused_rank(rank, world, url, sync):
     import torch
     from memfabric_hybrid_b200.ops import moe as M
